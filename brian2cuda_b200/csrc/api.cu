@@ -425,6 +425,56 @@ struct MemberTmp {
   }
 };
 
+std::vector<std::pair<void*, size_t>> state_arrays(b2b_net* net);
+
+// Puts the STDP weights of a projection in post-grouped order (on_post walks contiguous
+// weights, on_pre reaches them through rec_of) or back in synapse order.  The live weights
+// and every stored copy of them (snapshots) are permuted together, so a later restore
+// finds them in the order in use.
+b2b_status set_record_order(b2b_net* net, Proj& pr, bool post_grouped) {
+  if ((pr.dev.rec_of != nullptr) == post_grouped) return B2B_OK;
+  cudaStream_t s = net->stream;
+  if (post_grouped && !pr.rec_buf) {
+    CU(dalloc(pr, &pr.rec_buf, (size_t)pr.n_syn));
+    CU(build_rec_of(pr.dev.post_syn, pr.n_syn, pr.rec_buf, s));
+  }
+  const size_t bytes = real_size(pr.dtype) * (size_t)pr.n_syn;
+  std::vector<void*> copies = {pr.dev.stdp_w};
+  const auto state = state_arrays(net);
+  for (size_t k = 0; k < state.size(); ++k) {
+    if (state[k].first != pr.dev.stdp_w) continue;
+    for (const Snapshot& sn : net->snapshots)
+      if (sn.valid && k < sn.buffers.size()) copies.push_back(sn.buffers[k]);
+  }
+  void* tmp = nullptr;
+  CU(cudaMalloc(&tmp, bytes ? bytes : 1));
+  cudaError_t e = cudaSuccess;
+  for (void* a : copies) {
+    if (e == cudaSuccess)
+      e = permute_stdp_weights(a, tmp, pr.dev.post_syn, pr.n_syn, pr.dtype, post_grouped, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(a, tmp, bytes, cudaMemcpyDeviceToDevice, s);
+  }
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  cudaFree(tmp);
+  if (e != cudaSuccess) return fail(net, B2B_ERR_CUDA, "record order: %s", cudaGetErrorString(e));
+  pr.dev.rec_of = post_grouped ? pr.rec_buf : nullptr;
+  if (net->graph) {   // the graph holds the projection's parameters
+    cudaGraphExecDestroy(net->graph);
+    net->graph = nullptr;
+  }
+  return B2B_OK;
+}
+
+// The built-in order of an STDP projection's weights.  A strided visit moves a 32-byte sector
+// per weight, which counts once the weights are more than a few MB; below that a step is
+// latency, and synapse order saves on_pre the load of the weight's place.  Measured (us per
+// step in synapse / post-grouped order, Poisson inputs at 15 Hz, targets at 1-5 kHz): float32
+// 1000 x 100 (0.4 MB) 7.6 / 8.0, 2000 x 500 (4 MB) 10.1 / 10.5, 4000 x 500 (8 MB) 12.2 / 11.4,
+// 10000 x 1000 (40 MB) 65.1 / 19.6; float64 3001 x 257 (6.2 MB) 12.9 / 12.5.
+bool stdp_post_grouped(const Proj& pr) {
+  return (int64_t)real_size(pr.dtype) * pr.n_syn >= 6000000;
+}
+
 b2b_status build_proj(b2b_net* net, int pj) {
   Proj& pr = net->projs[pj];
   const Pop& src = net->pops[pr.src_pop];
@@ -567,14 +617,15 @@ b2b_status build_proj(b2b_net* net, int pj) {
   if (pr.effect == B2B_EFFECT_STDP) {
     const b2b_stdp_params& sp = net->syns[pr.members[0]].stdp;
     CHECK(pr.n_syn < (1ll << 31), B2B_ERR_UNSUPPORTED, "STDP projection above 2^31 synapses");
-    // one interleaved record per synapse; the scattered initial weights move into it
-    CU(dalloc(pr, (uint8_t**)&D.syn4, 4 * rs * (size_t)pr.n_syn));
-    CU(pack_stdp(pr.w, D.syn4, pr.dtype, pr.n_syn, s));
-    CU(cudaStreamSynchronize(s));
-    pr.allocs.erase(std::remove(pr.allocs.begin(), pr.allocs.end(), pr.w), pr.allocs.end());
-    cudaFree(pr.w);
+    CHECK(nkeys < (1ll << 31), B2B_ERR_UNSUPPORTED, "STDP source size x delay range above 2^31");
+    // the scattered initial weights are the synapses' weights; the traces start at 0
+    D.stdp_w = pr.w;
     pr.w = nullptr;
     D.w = nullptr;
+    CU(dalloc(pr, (uint8_t**)&D.tr_pre, 2 * rs * (size_t)nkeys));
+    CU(dalloc(pr, (uint8_t**)&D.tr_post, 2 * rs * (size_t)dst.n));
+    CU(cudaMemsetAsync(D.tr_pre, 0, 2 * rs * (size_t)nkeys, s));
+    CU(cudaMemsetAsync(D.tr_post, 0, 2 * rs * (size_t)dst.n, s));
     D.taupre = sp.taupre; D.taupost = sp.taupost; D.dApre = sp.dApre; D.dApost = sp.dApost;
     D.wmin = sp.wmin; D.wmax = sp.wmax; D.pre_adds_weight = sp.pre_adds_weight;
     int64_t* poff = nullptr;
@@ -591,6 +642,11 @@ b2b_status build_proj(b2b_net* net, int pj) {
     D.post_chunks = (int32_t)std::max<int64_t>(1, (maxp + kChunk - 1) / kChunk);
     D.post_off = poff;
     D.post_syn = psyn;
+    int32_t* key_of = nullptr;
+    CU(dalloc(pr, &key_of, (size_t)pr.n_syn));
+    CU(build_key_of(psyn, pr.off, nkeys, pr.n_syn, key_of, s));
+    D.key_of = key_of;
+    if (b2b_status st = set_record_order(net, pr, stdp_post_grouped(pr))) return st;
   }
   return B2B_OK;
 }
@@ -1063,7 +1119,11 @@ std::vector<std::pair<void*, size_t>> state_arrays(b2b_net* net) {
   }
   for (Proj& pr : net->projs) {
     if (pr.effect != B2B_EFFECT_STDP) continue;
-    out.emplace_back(pr.dev.syn4, 4 * real_size(pr.dtype) * pr.n_syn);
+    const size_t rs = real_size(pr.dtype);
+    out.emplace_back(pr.dev.stdp_w, rs * pr.n_syn);
+    out.emplace_back(pr.dev.tr_pre,
+                     2 * rs * (size_t)(net->pops[pr.src_pop].n * (int64_t)pr.dev.nd));
+    out.emplace_back(pr.dev.tr_post, 2 * rs * (size_t)pr.dst_n);
   }
   return out;
 }
@@ -1996,44 +2056,6 @@ b2b_status b2b_profile_graph(b2b_net* net, int64_t n_steps, double* mean_ms,
 // ---- autotuner ------------------------------------------------------------------------------
 namespace {
 
-// Puts the STDP records of a projection in post-grouped order (on_post walks contiguous
-// records, on_pre reaches them through rec_of) or back in synapse order.  The live records
-// and every stored copy of them (snapshots) are permuted together, so a later restore
-// finds them in the order in use.
-b2b_status set_record_order(b2b_net* net, Proj& pr, bool post_grouped) {
-  if ((pr.dev.rec_of != nullptr) == post_grouped) return B2B_OK;
-  cudaStream_t s = net->stream;
-  if (post_grouped && !pr.rec_buf) {
-    CU(dalloc(pr, &pr.rec_buf, (size_t)pr.n_syn));
-    CU(build_rec_of(pr.dev.post_syn, pr.n_syn, pr.rec_buf, s));
-  }
-  const size_t bytes = 4 * real_size(pr.dtype) * (size_t)pr.n_syn;
-  std::vector<void*> copies = {pr.dev.syn4};
-  const auto state = state_arrays(net);
-  for (size_t k = 0; k < state.size(); ++k) {
-    if (state[k].first != pr.dev.syn4) continue;
-    for (const Snapshot& sn : net->snapshots)
-      if (sn.valid && k < sn.buffers.size()) copies.push_back(sn.buffers[k]);
-  }
-  void* tmp = nullptr;
-  CU(cudaMalloc(&tmp, bytes ? bytes : 1));
-  cudaError_t e = cudaSuccess;
-  for (void* a : copies) {
-    if (e == cudaSuccess)
-      e = permute_stdp_records(a, tmp, pr.dev.post_syn, pr.n_syn, pr.dtype, post_grouped, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(a, tmp, bytes, cudaMemcpyDeviceToDevice, s);
-  }
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  cudaFree(tmp);
-  if (e != cudaSuccess) return fail(net, B2B_ERR_CUDA, "record order: %s", cudaGetErrorString(e));
-  pr.dev.rec_of = post_grouped ? pr.rec_buf : nullptr;
-  if (net->graph) {   // the graph holds the projection's parameters
-    cudaGraphExecDestroy(net->graph);
-    net->graph = nullptr;
-  }
-  return B2B_OK;
-}
-
 constexpr double kTuneMargin = 0.98;
 
 // Launch shape of the delivery launch of a net run with two launches per step (pending.cu):
@@ -2538,18 +2560,21 @@ b2b_status b2b_autotune(b2b_net* net, int32_t trial_steps, b2b_tune_result* out,
       res.push_back(b2b_tune_result{11, 0, form, form >= 2 ? one_grid : 0, form_ms[form],
                                     form_ms[builtin]});
     }
-    // STDP projections: order of the synapse records (0 synapse order, 1 post-grouped)
+    // STDP projections: order of the weights (0 synapse order, 1 post-grouped), the built-in
+    // one first
     for (size_t p = 0; p < net->projs.size() && st == B2B_OK; ++p) {
       Proj& pr = net->projs[p];
       if (pr.effect != B2B_EFFECT_STDP) continue;
       b2b_tune_result r{8, (int32_t)p, 0, 0, 0.0, 0.0};
       double best = 1e30;
-      for (int c = 0; c < 2 && st == B2B_OK; ++c) {
+      const int builtin = stdp_post_grouped(pr) ? 1 : 0;
+      for (int c : {builtin, 1 - builtin}) {
+        if (st != B2B_OK) break;
         st = set_record_order(net, pr, c == 1);
         double ms = 0;
         if (st == B2B_OK) st = trial(&ms);
-        if (c == 0) r.default_ms = ms;
-        if (st == B2B_OK && (c == 0 || ms < kTuneMargin * best)) {
+        if (c == builtin) r.default_ms = ms;
+        if (st == B2B_OK && (c == builtin || ms < kTuneMargin * best)) {
           best = ms;
           r.choice_a = c;
         }
@@ -3147,23 +3172,19 @@ b2b_status b2b_syn_get(b2b_net* net, int32_t sid, int32_t var, void* host, int64
   const Group& gpre = net->groups[sy.pre_gid];
   const Group& gpost = net->groups[sy.post_gid];
   const int32_t nd = pr.dmax - pr.dmin + 1;
-  const void* arr = nullptr;
-  int64_t stride = 1;
-  if (pr.effect == B2B_EFFECT_STDP && var >= B2B_SYN_W) {
-    // component (var - W) of the interleaved {w, Apre, Apost, lastupdate} records
-    arr = static_cast<const uint8_t*>(pr.dev.syn4) + real_size(pr.dtype) * (var - B2B_SYN_W);
-    stride = 4;
-  } else if (var == B2B_SYN_W) {
-    arr = pr.w;
-  }
+  const bool stdp = pr.effect == B2B_EFFECT_STDP;
+  const void* arr = var == B2B_SYN_W ? (stdp ? pr.dev.stdp_w : pr.w) : nullptr;
   const int64_t* inv = sy.inv;  // NULL for generated synapses: positions are the numbering
   const size_t es = (var <= B2B_SYN_DELAY) ? 4 : real_size(pr.dtype);
   void* d_out = nullptr;
   CU(cudaMalloc(&d_out, es * n));
-  cudaError_t e = gather_syn_var(pr, var, inv, sy.base, n,
-                                 (gpre.offset + sy.pre_lo) * (int64_t)nd,
-                                 (gpre.offset + sy.pre_hi) * (int64_t)nd, gpre.offset,
-                                 gpost.offset, arr, stride, sy.w_scalar, d_out, net->stream);
+  const int64_t key_lo = (gpre.offset + sy.pre_lo) * (int64_t)nd;
+  const int64_t key_hi = (gpre.offset + sy.pre_hi) * (int64_t)nd;
+  cudaError_t e =
+      var > B2B_SYN_W
+          ? gather_syn_trace(pr, var, inv, sy.base, n, key_lo, key_hi, d_out, net->stream)
+          : gather_syn_var(pr, var, inv, sy.base, n, key_lo, key_hi, gpre.offset, gpost.offset,
+                           arr, sy.w_scalar, d_out, net->stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(host, d_out, es * n, cudaMemcpyDeviceToHost, net->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(net->stream);
   cudaFree(d_out);

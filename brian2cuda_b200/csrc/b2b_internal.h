@@ -143,9 +143,13 @@ struct ProjDev {
   const int8_t* mem_var;
   const double* mem_w;            // per-member scalar weight (members differ), or NULL
   void* targets[3];               // per variable v, ge, gi
-  // STDP
-  void* syn4;                     // per synapse {w, Apre, Apost, lastupdate}, interleaved so
-                                  // that a strided (on_post) visit touches one sector
+  // STDP: one weight per synapse, and the event-driven traces once per neuron that drives
+  // them (propagate.cu): {value at the last event, time of the last event} per bundle
+  // (pre, delay) for Apre and per postsynaptic neuron for Apost
+  void* stdp_w;                   // [n_syn], in the order rec_of gives
+  void* tr_pre;                   // [n_src*nd] by bundle key
+  void* tr_post;                  // [n_post]
+  const int32_t* key_of;          // [n_syn] bundle key of each synapse, post-grouped order
   double taupre, taupost, dApre, dApost, wmin, wmax;
   int32_t pre_adds_weight;
   int32_t aggregate;              // warp-aggregate atomics (few targets)
@@ -157,9 +161,9 @@ struct ProjDev {
   int32_t post_chunks;
   const int64_t* post_off;        // [n_post + 1]
   const int32_t* post_syn;        // synapse positions grouped by post
-  // Order of the STDP records: NULL, record s belongs to synapse position s; otherwise the
-  // records follow the post-grouped index (record r is synapse post_syn[r], so on_post walks
-  // contiguous records) and rec_of[s] is the record of synapse position s.
+  // Order of the STDP weights: NULL, weight s belongs to synapse position s; otherwise the
+  // weights follow the post-grouped index (weight r is synapse post_syn[r]'s, so on_post walks
+  // contiguous weights) and rec_of[s] is the place of synapse position s's weight.
   const int32_t* rec_of;
 };
 
@@ -327,7 +331,7 @@ struct Proj {
   int32_t* post = nullptr;
   void* w = nullptr;
   std::vector<void*> allocs;
-  int32_t* rec_buf = nullptr;                // STDP: record of each synapse, post-grouped order
+  int32_t* rec_buf = nullptr;                // STDP: place of each synapse in post-grouped order
   // A projection retired by b2b_syn_set_delays: it only delivers the spikes sent before the
   // change (dev.src_hi) and is dropped once the last of them has arrived (after this step).
   // Retired projections follow the live ones in b2b_net::projs and belong to no Synapses.

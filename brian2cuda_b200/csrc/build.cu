@@ -152,7 +152,7 @@ __global__ void gather_kernel(int var, int64_t n, int64_t pos_base, const int64_
                               const int64_t* __restrict__ off, int64_t key_lo, int64_t key_hi,
                               int32_t nd, int32_t dmin, int64_t src_offset,
                               const int32_t* __restrict__ post, int64_t dst_offset,
-                              const R* __restrict__ arr, int64_t stride,
+                              const R* __restrict__ arr,
                               const int32_t* __restrict__ rec, double w_scalar, void* out) {
   for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < n;
        q += (int64_t)gridDim.x * blockDim.x) {
@@ -170,7 +170,7 @@ __global__ void gather_kernel(int var, int64_t n, int64_t pos_base, const int64_
                                            : (int32_t)(lo % nd + dmin);
       static_cast<int32_t*>(out)[q] = val;
     } else {
-      static_cast<R*>(out)[q] = arr ? arr[(rec ? (int64_t)rec[pos] : pos) * stride] : (R)w_scalar;
+      static_cast<R*>(out)[q] = arr ? arr[rec ? (int64_t)rec[pos] : pos] : (R)w_scalar;
     }
   }
 }
@@ -243,18 +243,61 @@ cudaError_t member_sort_scatter(uint32_t* d_keys, uint32_t* d_vals, int64_t n,
 }
 
 namespace {
-// STDP records between synapse order and post-grouped order (record r of the post-grouped
-// order is synapse post_syn[r]).
+// STDP weights between synapse order and post-grouped order (weight r of the post-grouped
+// order is synapse post_syn[r]'s).
 template <typename R>
-__global__ void permute_records_kernel(const R* __restrict__ in, R* __restrict__ out,
+__global__ void permute_weights_kernel(const R* __restrict__ in, R* __restrict__ out,
                                        const int32_t* __restrict__ post_syn, int64_t n,
                                        bool to_post) {
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n;
        r += (int64_t)gridDim.x * blockDim.x) {
     const int64_t s = post_syn[r];
-    const R* src = in + 4 * (to_post ? s : r);
-    R* dst = out + 4 * (to_post ? r : s);
-    for (int c = 0; c < 4; ++c) dst[c] = src[c];
+    out[to_post ? r : s] = in[to_post ? s : r];
+  }
+}
+
+// Bundle key of the synapse at position pos: the largest key of [lo, hi) with off[key] <= pos.
+__device__ __forceinline__ int64_t key_at(const int64_t* __restrict__ off, int64_t lo, int64_t hi,
+                                          int64_t pos) {
+  --hi;
+  while (lo < hi) {
+    const int64_t mid = (lo + hi + 1) >> 1;
+    if (off[mid] <= pos) lo = mid; else hi = mid - 1;
+  }
+  return lo;
+}
+
+__global__ void key_of_kernel(const int32_t* __restrict__ post_syn,
+                              const int64_t* __restrict__ off, int64_t nkeys, int64_t n,
+                              int32_t* __restrict__ key_of) {
+  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n;
+       r += (int64_t)gridDim.x * blockDim.x)
+    key_of[r] = (int32_t)key_at(off, 0, nkeys, post_syn[r]);
+}
+
+// Apre, Apost or lastupdate of STDP synapses in input order, from the bundles' and targets'
+// traces ({value, time} pairs): lastupdate is the later of the two events, and both traces
+// are decayed to it.
+template <typename R>
+__global__ void gather_trace_kernel(int var, int64_t n, int64_t pos_base,
+                                    const int64_t* __restrict__ inv,
+                                    const int64_t* __restrict__ off, int64_t key_lo,
+                                    int64_t key_hi, const int32_t* __restrict__ post,
+                                    const R* __restrict__ tr_pre, const R* __restrict__ tr_post,
+                                    double taupre, double taupost, R* __restrict__ out) {
+  for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < n;
+       q += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t pos = inv ? inv[q] : pos_base + q;
+    const R* a = tr_pre + 2 * key_at(off, key_lo, key_hi, pos);
+    const R* b = tr_post + 2 * (int64_t)post[pos];
+    const R lu = a[1] > b[1] ? a[1] : b[1];
+    if (var == B2B_SYN_LASTUPDATE) {
+      out[q] = lu;
+    } else {
+      const R* x = var == B2B_SYN_APRE ? a : b;
+      const double tau = var == B2B_SYN_APRE ? taupre : taupost;
+      out[q] = x[0] * dexp((R)(((double)x[1] - (double)lu) / tau));
+    }
   }
 }
 
@@ -266,14 +309,14 @@ __global__ void rec_of_kernel(const int32_t* __restrict__ post_syn, int64_t n,
 }
 }  // namespace
 
-cudaError_t permute_stdp_records(const void* d_in, void* d_out, const int32_t* d_post_syn,
+cudaError_t permute_stdp_weights(const void* d_in, void* d_out, const int32_t* d_post_syn,
                                  int64_t n, int dtype, bool to_post, cudaStream_t s) {
   if (n == 0) return cudaSuccess;
   if (dtype == B2B_F32)
-    permute_records_kernel<float><<<grid_for(n), 256, 0, s>>>(
+    permute_weights_kernel<float><<<grid_for(n), 256, 0, s>>>(
         static_cast<const float*>(d_in), static_cast<float*>(d_out), d_post_syn, n, to_post);
   else
-    permute_records_kernel<double><<<grid_for(n), 256, 0, s>>>(
+    permute_weights_kernel<double><<<grid_for(n), 256, 0, s>>>(
         static_cast<const double*>(d_in), static_cast<double*>(d_out), d_post_syn, n, to_post);
   return cudaGetLastError();
 }
@@ -282,6 +325,31 @@ cudaError_t build_rec_of(const int32_t* d_post_syn, int64_t n, int32_t* d_rec_of
                          cudaStream_t s) {
   if (n == 0) return cudaSuccess;
   rec_of_kernel<<<grid_for(n), 256, 0, s>>>(d_post_syn, n, d_rec_of);
+  return cudaGetLastError();
+}
+
+cudaError_t build_key_of(const int32_t* d_post_syn, const int64_t* d_off, int64_t nkeys,
+                         int64_t n, int32_t* d_key_of, cudaStream_t s) {
+  if (n == 0) return cudaSuccess;
+  key_of_kernel<<<grid_for(n), 256, 0, s>>>(d_post_syn, d_off, nkeys, n, d_key_of);
+  return cudaGetLastError();
+}
+
+cudaError_t gather_syn_trace(const Proj& pr, int var, const int64_t* d_inv, int64_t pos_base,
+                             int64_t n, int64_t key_lo, int64_t key_hi, void* d_out,
+                             cudaStream_t s) {
+  if (n == 0) return cudaSuccess;
+  const ProjDev& D = pr.dev;
+  if (pr.dtype == B2B_F32)
+    gather_trace_kernel<float><<<grid_for(n), 256, 0, s>>>(
+        var, n, pos_base, d_inv, pr.off, key_lo, key_hi, pr.post,
+        static_cast<const float*>(D.tr_pre), static_cast<const float*>(D.tr_post), D.taupre,
+        D.taupost, static_cast<float*>(d_out));
+  else
+    gather_trace_kernel<double><<<grid_for(n), 256, 0, s>>>(
+        var, n, pos_base, d_inv, pr.off, key_lo, key_hi, pr.post,
+        static_cast<const double*>(D.tr_pre), static_cast<const double*>(D.tr_post), D.taupre,
+        D.taupost, static_cast<double*>(d_out));
   return cudaGetLastError();
 }
 
@@ -364,23 +432,22 @@ cudaError_t build_post_index(const int32_t* d_post, int64_t n_syn, int64_t dst_l
 
 cudaError_t gather_syn_var(const Proj& pr, int var, const int64_t* d_inv, int64_t pos_base,
                            int64_t n, int64_t key_lo, int64_t key_hi, int64_t src_offset,
-                           int64_t dst_offset, const void* d_arr, int64_t stride,
-                           double w_scalar, void* d_out, cudaStream_t s) {
+                           int64_t dst_offset, const void* d_arr, double w_scalar,
+                           void* d_out, cudaStream_t s) {
   if (n == 0) return cudaSuccess;
-  // STDP record components are read through the record order
-  const int32_t* rec = stride == 4 ? pr.dev.rec_of : nullptr;
+  const int32_t* rec = pr.dev.rec_of;   // STDP weights are read through their order
   if (pr.dtype == B2B_F32)
     gather_kernel<float><<<grid_for(n), 256, 0, s>>>(var, n, pos_base, d_inv, pr.off, key_lo,
                                                      key_hi, pr.dmax - pr.dmin + 1, pr.dmin,
                                                      src_offset, pr.post, dst_offset,
                                                      static_cast<const float*>(d_arr),
-                                                     stride, rec, w_scalar, d_out);
+                                                     rec, w_scalar, d_out);
   else
     gather_kernel<double><<<grid_for(n), 256, 0, s>>>(var, n, pos_base, d_inv, pr.off, key_lo,
                                                       key_hi, pr.dmax - pr.dmin + 1, pr.dmin,
                                                       src_offset, pr.post, dst_offset,
                                                       static_cast<const double*>(d_arr),
-                                                      stride, rec, w_scalar, d_out);
+                                                      rec, w_scalar, d_out);
   return cudaGetLastError();
 }
 
@@ -400,32 +467,6 @@ cudaError_t add_out_degree(const int64_t* d_off, int32_t nd, int64_t first, int6
                            int32_t* d_out, cudaStream_t s) {
   const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 4096));
   out_degree_kernel<<<(unsigned)blocks, 256, 0, s>>>(d_off, nd, first, n, d_out);
-  return cudaGetLastError();
-}
-
-// STDP synapse records {w, 0, 0, 0} from the per-synapse initial weights.
-namespace {
-template <typename R>
-__global__ void pack_stdp_kernel(const R* __restrict__ w, R* __restrict__ syn4, int64_t n) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    syn4[4 * i] = w[i];
-    syn4[4 * i + 1] = (R)0;
-    syn4[4 * i + 2] = (R)0;
-    syn4[4 * i + 3] = (R)0;
-  }
-}
-}  // namespace
-
-cudaError_t pack_stdp(const void* d_w, void* d_syn4, int dtype, int64_t n, cudaStream_t s) {
-  if (n == 0) return cudaSuccess;
-  const unsigned g = (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 8192));
-  if (dtype == B2B_F32)
-    pack_stdp_kernel<float><<<g, 256, 0, s>>>(static_cast<const float*>(d_w),
-                                              static_cast<float*>(d_syn4), n);
-  else
-    pack_stdp_kernel<double><<<g, 256, 0, s>>>(static_cast<const double*>(d_w),
-                                               static_cast<double*>(d_syn4), n);
   return cudaGetLastError();
 }
 

@@ -131,9 +131,10 @@ __device__ __forceinline__ int find_delay_block(const int* s_pref, int nd, int s
   return lo;
 }
 
-// Calls item(b0, b1, len, pre) for every work item of projection J due at step ts: the
-// synapse positions [b0, b1) of one chunk of the bundle of presynaptic neuron pre (b1 == b0
-// for a lane group without an item).  Work items go to warps warp0, warp0 + nwarps, ...;
+// Calls item(b0, b1, len, pre, head_key) for every work item of projection J due at step ts:
+// the synapse positions [b0, b1) of one chunk of the bundle of presynaptic neuron pre (b1 == b0
+// for a lane group without an item); head_key is the bundle's key in its first chunk's item,
+// -1 in the others.  Work items go to warps warp0, warp0 + nwarps, ...;
 // inside a warp, groups of GROUP lanes take one item each, so 32/GROUP items' dependent loads
 // (spike index, bundle offsets, synapse data) are in flight together.  All 32 lanes of a warp
 // call item together; len, the longest b1 - b0 of the warp's groups, is the same in every
@@ -177,7 +178,7 @@ __device__ __forceinline__ void for_each_due_item(const ProjDev& J, int64_t ts, 
     } else {
       di = find_delay_block(s_pref, J.nd, sp, &kk);
     }
-    int64_t b0 = 0, b1 = 0;
+    int64_t b0 = 0, b1 = 0, head_key = -1;
     int32_t pre = 0;
     if (have) {
       const int slot = ring_back(base, J.dmin + di, J.src_ring_len);
@@ -186,12 +187,13 @@ __device__ __forceinline__ void for_each_due_item(const ProjDev& J, int64_t ts, 
       b0 = J.off[key] + (int64_t)ch * kChunk;
       b1 = J.off[key + 1];
       if (b1 > b0 + kChunk) b1 = b0 + kChunk;
+      if (ch == 0) head_key = key;
     }
     // rounds until the longest bundle of this warp's groups is done (warp-uniform)
     int64_t len = b1 - b0;
 #pragma unroll
     for (int o = 16; o >= GROUP; o >>= 1) len = max(len, __shfl_xor_sync(kFull, len, o));
-    item(b0, b1, len, pre);
+    item(b0, b1, len, pre, head_key);
   }
 }
 
@@ -203,7 +205,8 @@ __device__ __forceinline__ void for_each_due(const ProjDev& J, int64_t ts, int64
                                              int64_t nwarps, int* s_pref, Body body) {
   const int glane = (threadIdx.x & 31) % GROUP;
   for_each_due_item<WARP_PREFIX, GROUP>(J, ts, warp0, nwarps, s_pref,
-                                        [&](int64_t b0, int64_t b1, int64_t len, int32_t pre) {
+                                        [&](int64_t b0, int64_t b1, int64_t len, int32_t pre,
+                                            int64_t) {
     for (int64_t off = 0; off < len; off += GROUP) {
       const int64_t s = b0 + off + glane;
       body(s, s < b1, pre);

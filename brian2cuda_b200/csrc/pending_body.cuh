@@ -26,7 +26,8 @@ __device__ __forceinline__ void deliver_pending_body(const PendingDev& F,
     const R* W = static_cast<const R*>(J.w);
     MemberCache<R> mc;
     for_each_due_item<WARP_PREFIX, GROUP>(J, ts, warp0, nwarps, s_pref,
-                                          [&](int64_t b0, int64_t b1, int64_t len, int32_t pre) {
+                                          [&](int64_t b0, int64_t b1, int64_t len, int32_t pre,
+                                              int64_t) {
       member_lookup<R>(J, pre, mc);
       // the loads of kPendingUnroll rounds first, then their atomics
       for (int64_t off = 0; off < len; off += kPendingUnroll * GROUP) {

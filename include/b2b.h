@@ -405,9 +405,9 @@ b2b_status b2b_profile_graph(b2b_net* net, int64_t n_steps, double* mean_ms, int
  * steps run as b2b_run runs them (graph replays), so a shape is judged by the step time it
  * gives.  Populations: neurons per thread (1, 2 or 4) x threads per CTA (128 or 256), or, with a
  * gating surrogate, CTAs per SM (2..6); additive delivery launches: lanes per work item
- * (2, 4, 8, 16, 32) x CTAs (1/2, 1, 2, 4, 8 per SM); STDP projections: the order of the synapse
- * records (0 synapse order, 1 grouped by postsynaptic neuron, where on_post reads contiguous
- * records; the live records and every snapshot are permuted together, and b2b_syn_get reads
+ * (2, 4, 8, 16, 32) x CTAs (1/2, 1, 2, 4, 8 per SM); STDP projections: the order of the synapses'
+ * weights (0 synapse order, 1 grouped by postsynaptic neuron, where on_post reads contiguous
+ * weights; the live weights and every snapshot are permuted together, and b2b_syn_get reads
  * through the order); a net that can run every step as two concurrent launches: the pending
  * delivery's lanes per item x CTAs (kind 5), then the form itself (kind 11: choice_a 2 one
  * launch per step holding both halves, with choice_b delivering CTAs (of 256 threads; 0: the
@@ -418,7 +418,7 @@ b2b_status b2b_profile_graph(b2b_net* net, int64_t n_steps, double* mean_ms, int
  * rule) to be chosen.  A choice of 0 means the built-in rule won.  The trials should cover a
  * representative stretch of the run (bursts included). */
 typedef struct {
-  int32_t site_kind;     /* 1 population, 6 additive delivery launch, 8 STDP records,
+  int32_t site_kind;     /* 1 population, 6 additive delivery launch, 8 STDP weights,
                             5 pending delivery of the two-launch step, 11 step form
                             (0 per-step kernels, 1 two launches, 2 one launch,
                             3 one launch chained),
@@ -431,7 +431,7 @@ typedef struct {
                             effects at the targets                                        */
   int32_t site_index;    /* population / delivery launch / projection index              */
   int32_t choice_a;      /* neurons per thread (surrogate: CTAs per SM) / lanes per item /
-                            record order / step form                                      */
+                            weight order / step form                                      */
   int32_t choice_b;      /* threads per CTA / CTAs                                       */
   double best_ms;        /* mean device time of one whole step with the chosen shape     */
   double default_ms;     /* the same with the built-in rule                              */
