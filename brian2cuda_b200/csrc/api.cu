@@ -548,6 +548,10 @@ b2b_status build_proj(b2b_net* net, int pj) {
   int64_t maxb = 0;
   CU(counts_to_offsets(pr.off, nkeys, &maxb, s));
   pr.max_bundle = maxb;
+  double bundles = 0;
+  for (int sid : pr.members)
+    bundles += (double)(net->syns[sid].pre_hi - net->syns[sid].pre_lo) * nd;
+  pr.mean_bundle = bundles > 0 ? (double)pr.n_syn / bundles : 0;
   CU(dalloc(pr, &pr.post, (size_t)pr.n_syn));
   if (need_w) CU(dalloc(pr, (uint8_t**)&pr.w, rs * (size_t)pr.n_syn));
   // 3) sort + scatter
@@ -862,6 +866,14 @@ b2b_status setup_small(b2b_net* net) {
   return B2B_OK;
 }
 
+// Lanes per work item of the pending delivery, by the largest projection's bundles.
+int builtin_pending_lanes(const b2b_net* net) {
+  const Proj* big = nullptr;
+  for (const Proj& pr : net->projs)
+    if (!big || pr.n_syn > big->n_syn) big = &pr;
+  return pending_lanes(big ? big->mean_bundle : 0, net->pops[0].n);
+}
+
 // Populations up to this size run the two concurrent launches unless tuned otherwise
 // (measured: 1e5 HH neurons 38.6 vs 50.9 ms per simulated second).  Above it the pending
 // input's read and clear (16 B per neuron and step for ge and gi in float32) costs more HBM
@@ -913,7 +925,7 @@ b2b_status setup_two_launch(b2b_net* net) {
   }
   int sms = kNumSMs;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, net->cfg.device);
-  F.group = 8;
+  F.group = builtin_pending_lanes(net);
   net->pending_grid = 2 * sms;
   // the update launch is the per-step neuron kernel, adding in the input that the previous
   // step's delivery left in acc
@@ -971,7 +983,7 @@ b2b_status enqueue_steps(b2b_net* net, int kk) {
       CU(prof_mark(net, k, 0, 1, s));
       ++net->launches;
     }
-    CU(launch_fold_pending(net->pdev, pop.dtype, net->d_clock, kk - 1, s));
+    CU(launch_fold_pending(net->pdev, pop.dtype, kk - 1, s));
     CU(launch_tick(net->d_clock, kk, s));
     net->launches += 2;
     return B2B_OK;
@@ -1000,7 +1012,7 @@ b2b_status enqueue_steps(b2b_net* net, int kk) {
       net->launches += 2;
     }
     CU(cudaStreamWaitEvent(s, net->ev_d[(kk - 1) & 1], 0));
-    CU(launch_fold_pending(net->pdev, pop.dtype, net->d_clock, kk - 1, s));
+    CU(launch_fold_pending(net->pdev, pop.dtype, kk - 1, s));
     CU(launch_tick(net->d_clock, kk, s));
     net->launches += 2;
     return B2B_OK;
@@ -1927,7 +1939,11 @@ b2b_status b2b_profile(b2b_net* net, int64_t n_steps, double* mean_ms, int32_t* 
       ++net->launches;
     }
     if (result != B2B_OK) break;
-    cudaError_t e = launch_tick(net->d_clock, 1, net->stream);
+    // every profiled step is a chunk of its own (step 0 of it): its pending input is folded in
+    cudaError_t e = net->two_launch
+                        ? launch_fold_pending(net->pdev, net->pops[0].dtype, 0, net->stream)
+                        : cudaSuccess;
+    if (e == cudaSuccess) e = launch_tick(net->d_clock, 1, net->stream);
     ++net->launches;
     if (e == cudaSuccess) e = cudaStreamSynchronize(net->stream);
     if (e != cudaSuccess) { result = fail(net, B2B_ERR_CUDA, "profile: %s", cudaGetErrorString(e)); break; }
@@ -1940,11 +1956,6 @@ b2b_status b2b_profile(b2b_net* net, int64_t n_steps, double* mean_ms, int32_t* 
     net->last_chunk_steps = 1;
   }
   for (auto& e : ev) cudaEventDestroy(e);
-  if (result == B2B_OK && net->two_launch) {
-    cudaError_t e = launch_fold_pending(net->pdev, net->pops[0].dtype, net->d_clock, -1, net->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(net->stream);
-    if (e != cudaSuccess) result = fail(net, B2B_ERR_CUDA, "profile fold: %s", cudaGetErrorString(e));
-  }
   if (result != B2B_OK) return result;
   *n_sites = (int32_t)ns;
   for (size_t k = 0; k < ns && (int32_t)k < cap; ++k) {
@@ -2058,8 +2069,6 @@ namespace {
 
 constexpr double kTuneMargin = 0.98;
 
-// Launch shape of the delivery launch of a net run with two launches per step (pending.cu):
-// lanes per work item (0: 8) and CTAs (0: two per SM).
 // The pull form's connectivity split by the slices of sdev (cluster and slice set): for each
 // rank, offsets by presynaptic neuron and slice-local targets, uploaded to the device; false
 // when a slice's targets do not fit a CTA's shared memory.
@@ -2182,11 +2191,13 @@ void set_one_launch_grid(b2b_net* net, int grid) {
   }
 }
 
+// Launch shape of the delivery launch of a net run with two launches per step (pending.cu):
+// lanes per work item (0: built in) and CTAs (0: two per SM).
 void set_pending_shape(b2b_net* net, int group, int grid) {
   int sms = kNumSMs;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, net->cfg.device);
   net->pending_grid = grid > 0 ? grid : 2 * sms;
-  net->pdev.group = group > 0 ? group : 8;
+  net->pdev.group = group > 0 ? group : builtin_pending_lanes(net);
   if (net->graph) {
     cudaGraphExecDestroy(net->graph);
     net->graph = nullptr;
@@ -2493,10 +2504,7 @@ b2b_status b2b_autotune(b2b_net* net, int32_t trial_steps, b2b_tune_result* out,
         // threads): they share the grid with the delivery's, and fewer, larger CTAs shorten
         // the launch
         const std::pair<int, int> one_shapes[] = {{1, 128}, {1, 256}, {2, 128}, {2, 256}};
-        auto eff = [](int e, int b) {
-          return std::make_pair(e == 2 || e == 4 ? 2 : 1, b > 0 ? b : kBlock);
-        };
-        const auto cur = eff(pop0.tune_e, pop0.tune_block);
+        const std::pair<int, int> cur = {pop0.tune_e, pop0.tune_block};   // (0, 0): built in
         for (const auto& sh : one_shapes) {
           if (sh == cur || st != B2B_OK) continue;
           const int pe = pop0.tune_e, pb = pop0.tune_block;

@@ -201,7 +201,7 @@ struct PendingDev {
   ProjDev proj[kMaxProjBatch];
   int32_t n_proj, nd_max;
   void* acc[3];                   // per target variable (v, ge, gi): [2][pop.n] or NULL
-  int32_t group;                  // delivery: lanes per work item (4, 8 or 16)
+  int32_t group;                  // delivery: lanes per work item (2, 4, 8 or 16)
   int32_t pad_group;
 };
 
@@ -326,6 +326,7 @@ struct Proj {
   int32_t dmin = 0, dmax = 0;
   int64_t n_syn = 0;
   int64_t max_bundle = 0, max_post_bundle = 0;
+  double mean_bundle = 0;                    // synapses per (pre, delay) bundle of the members
   ProjDev dev{};
   int64_t* off = nullptr;
   int32_t* post = nullptr;
@@ -437,6 +438,10 @@ cudaError_t launch_proj_post(const Proj& pr, const int64_t* clock, int k, double
 // One launch for n (<= kMaxProjBatch) additive projections of equal dtype / weight mode.
 cudaError_t launch_proj_add_batch(const Proj* const* prs, int n, const int64_t* clock, int k,
                                   cudaStream_t s, const AddTune* tune = nullptr);
+// Lanes per work item of an additive delivery without tuning: for the per-step launch of
+// bundles of mean_bundle synapses, and for the delivery into the pending input (n neurons).
+int delivery_lanes(double mean_bundle);
+int pending_lanes(double mean_bundle, int64_t n);
 // Whether such a launch can accumulate in thread-block clusters (AddTune::cluster).
 bool add_batch_cluster_capable(const Proj* const* prs, int n);
 cudaError_t launch_tick(int64_t* clock, int steps, cudaStream_t s);
@@ -474,6 +479,5 @@ bool one_launch_supported(const Pop& pop, const PendingDev& F);
 cudaError_t launch_one_launch_step(const Pop& pop, const PopDev& U, const PendingDev& F,
                                    int deliver_ctas, bool chained, const int64_t* clock, int k,
                                    double dt, int32_t* status, cudaStream_t s);
-cudaError_t launch_fold_pending(const PendingDev& F, int dtype, const int64_t* clock, int k_last,
-                                cudaStream_t s);
+cudaError_t launch_fold_pending(const PendingDev& F, int dtype, int k_last, cudaStream_t s);
 }  // namespace b2b

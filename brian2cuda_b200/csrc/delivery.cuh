@@ -163,7 +163,11 @@ __device__ __forceinline__ void for_each_due_item(const ProjDev& J, int64_t ts, 
   for (int64_t r0 = warp0 * G; r0 < items; r0 += nwarps * G) {
     const int64_t it = r0 + grp;
     const bool have = it < items;
-    const int sp = have ? (int)(it / J.chunks) : 0;
+    // (one chunk per bundle is the ordinary case; a 64-bit quotient is slow)
+    const int sp = !have ? 0
+                   : J.chunks == 1 ? (int)it
+                   : items <= INT32_MAX ? (int)((uint32_t)it / (uint32_t)J.chunks)
+                                        : (int)(it / J.chunks);
     const int ch = have ? (int)(it - (int64_t)sp * J.chunks) : 0;
     int kk = 0, di = 0;
     if constexpr (WARP_PREFIX && G >= 4) {

@@ -65,8 +65,11 @@ __device__ __forceinline__ int block_exclusive_scan(int c, int* s_warp, int* tot
   return s_warp[warp] + x - c;
 }
 
-// Floor modulo of a (possibly negative) step by the ring length.
+// Floor modulo of a (possibly negative) step by the ring length.  Every kernel of a step
+// starts with it, so steps below 2^31 (all but days of simulated time) take the 32-bit
+// remainder: a 64-bit one is a long serial sequence in software.
 __device__ __forceinline__ int ring_slot(int64_t step, int ring_len) {
+  if ((uint64_t)step <= (uint64_t)INT32_MAX) return (int)((uint32_t)step % (uint32_t)ring_len);
   int64_t r = step % ring_len;
   return (int)(r < 0 ? r + ring_len : r);
 }

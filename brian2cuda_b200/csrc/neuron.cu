@@ -24,14 +24,16 @@
 namespace b2b {
 
 namespace {
-// Adds the input delivered during the previous step (fold buffer of variable v, parity
-// (ts-1) & 1) into pack X and returns the pack's address in the buffer, to be cleared after
-// the update's stores; no-op when the population has no fold buffer for v.
+// Adds the input delivered during the previous step (fold buffer of variable v, the row that
+// step k-1 of the chunk filled) into pack X and returns the pack's address in the buffer, to be
+// cleared after the update's stores; no-op when the population has no fold buffer for v.  The
+// row goes by the step's place in its chunk (both rows are empty between chunks), a launch
+// argument, so its load does not wait for the clock's.
 template <typename R, int E>
-__device__ __forceinline__ R* fold_in(const PopDev& P, int v, int64_t ts, int64_t q,
+__device__ __forceinline__ R* fold_in(const PopDev& P, int v, int k, int64_t q,
                                       Pack<R, E>& X) {
   if (!P.fold[v]) return nullptr;
-  R* a = static_cast<R*>(P.fold[v]) + (int64_t)((ts & 1) ^ 1) * P.n;
+  R* a = static_cast<R*>(P.fold[v]) + (int64_t)((k & 1) ^ 1) * P.n;
   const Pack<R, E> A = load_pack<R, E>(a, q);
 #pragma unroll
   for (int e = 0; e < E; ++e) X.x[e] += A.x[e];
@@ -73,8 +75,8 @@ __device__ __forceinline__ void lif_step_body(const PopDev& P, const int64_t* __
     Pack<R, E> GI = load_pack<R, E>(P.var[B2B_VAR_GI], q);
     Pack<R, E> LS;
     if (refr) LS = load_pack<R, E>(P.var[B2B_VAR_LASTSPIKE], q);
-    R* fge = fold_in<R, E>(P, B2B_VAR_GE, ts, q, GE);
-    R* fgi = fold_in<R, E>(P, B2B_VAR_GI, ts, q, GI);
+    R* fge = fold_in<R, E>(P, B2B_VAR_GE, k, q, GE);
+    R* fgi = fold_in<R, E>(P, B2B_VAR_GI, k, q, GI);
     uint32_t NRout = 0;
 #pragma unroll
     for (int e = 0; e < E; ++e) {
@@ -150,8 +152,8 @@ __device__ __forceinline__ void hh_step_body(const PopDev& P, const int64_t* __r
     Pack<R, E> GI = load_pack<R, E>(P.var[B2B_VAR_GI], q);
     Pack<R, E> LS;
     if (refr) LS = load_pack<R, E>(P.var[B2B_VAR_LASTSPIKE], q);
-    R* fge = fold_in<R, E>(P, B2B_VAR_GE, ts, q, GE);
-    R* fgi = fold_in<R, E>(P, B2B_VAR_GI, ts, q, GI);
+    R* fge = fold_in<R, E>(P, B2B_VAR_GE, k, q, GE);
+    R* fgi = fold_in<R, E>(P, B2B_VAR_GI, k, q, GI);
     uint32_t NRout = 0;
 #pragma unroll
     for (int e = 0; e < E; ++e) {
@@ -199,7 +201,7 @@ hh_step_kernel(PopDev P, const int64_t* __restrict__ clock, int k, double dt,
 // The update of step t and the delivery of step t into the pending input are independent
 // (pending.cu); here they are one grid: CTAs [0, n_upd) do the per-step update (one neuron
 // per thread, folding in the input pending from step t-1), the CTAs after them deliver the
-// bundles due at step t into acc[t & 1].  Consecutive steps are consecutive launches on one
+// bundles due at step t into acc[t & 1] (t counted from the chunk's start).  Consecutive steps are consecutive launches on one
 // stream, so one launch boundary orders step t+1 after both halves of step t, where the two
 // concurrent launches need a boundary each and dependencies across two streams.
 template <typename R, int KIND, int E, int GROUP>
@@ -312,8 +314,8 @@ hh_stream_kernel(PopDev P, const int64_t* __restrict__ clock, int k, double dt,
       const HhRun<R> g = hh_run(prm[cur.grp], R());
       const GroupInputs* gin = INPUTS ? P.inputs + cur.grp : nullptr;
       const bool refr = g.ref_steps >= 0;
-      R* fge = fold_in<R, 4>(P, B2B_VAR_GE, ts, q, cur.GE);
-      R* fgi = fold_in<R, 4>(P, B2B_VAR_GI, ts, q, cur.GI);
+      R* fge = fold_in<R, 4>(P, B2B_VAR_GE, k, q, cur.GE);
+      R* fgi = fold_in<R, 4>(P, B2B_VAR_GI, k, q, cur.GI);
       uint32_t NRout = 0;
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
@@ -386,11 +388,19 @@ poisson_step_kernel(PopDev P, const int64_t* __restrict__ clock, int k, double d
 }
 
 // ---- SpikeGeneratorGroup: entries sorted by step, one CTA ---------------------------------
-__device__ __forceinline__ int64_t lower_bound_i64(const int64_t* a, int64_t n, int64_t key) {
-  int64_t lo = 0, hi = n;
-  while (lo < hi) {
-    int64_t mid = (lo + hi) >> 1;
-    if (a[mid] < key) lo = mid + 1; else hi = mid;
+// Entries of the sorted a[0, n) below key, by a whole warp: 32 probes per round, so that 1e6
+// entries take 4 dependent loads instead of a binary search's 20.
+__device__ __forceinline__ int64_t warp_lower_bound(const int64_t* __restrict__ a, int64_t n,
+                                                    int64_t key) {
+  const int lane = threadIdx.x & 31;
+  int64_t lo = 0, hi = n;                       // the answer lies in [lo, hi]
+  while (lo < hi) {                             // warp-uniform
+    const int64_t step = (hi - lo + 31) / 32;
+    const int64_t at = lo + lane * step;
+    const int below = __popc(__ballot_sync(kFull, at < hi && a[at] < key));
+    if (below == 0) return lo;
+    hi = min(hi, lo + below * step);
+    lo += (below - 1) * step + 1;
   }
   return lo;
 }
@@ -399,21 +409,23 @@ __global__ void spikegen_step_kernel(PopDev P, const int64_t* __restrict__ clock
                                      int32_t* status) {
   const int64_t ts = clock[0] + k;
   const int slot = ring_slot(ts, P.ring_len);
-  __shared__ int64_t s_lo, s_hi;
+  __shared__ int64_t s_bound[2];
   __shared__ unsigned long long s_mbase;
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < 64) {
     // with a period, step ts emits the entries of bin ts mod period
-    // (brian2cuda/templates/spikegenerator.cu:42-49)
+    // (brian2cuda/templates/spikegenerator.cu:42-49); one warp per bound
     const int64_t bin = P.sg_period > 0 ? ts % P.sg_period : ts;
-    s_lo = lower_bound_i64(P.sg_step, P.sg_n, bin);
-    s_hi = lower_bound_i64(P.sg_step, P.sg_n, bin + 1);
-    const int cnt = (int)(s_hi - s_lo);
-    P.ring_cnt[slot] = cnt;
+    const int64_t b = warp_lower_bound(P.sg_step, P.sg_n, bin + (threadIdx.x >> 5));
+    if ((threadIdx.x & 31) == 0) s_bound[threadIdx.x >> 5] = b;
+  }
+  __syncthreads();
+  const int64_t s_lo = s_bound[0], cnt = s_bound[1] - s_bound[0];
+  if (threadIdx.x == 0) {
+    P.ring_cnt[slot] = (int)cnt;
     P.ring_cnt[ring_slot(ts + 1, P.ring_len)] = 0;
     if (P.mon_cnt) s_mbase = atomicAdd(P.mon_cnt, (unsigned long long)cnt);
   }
   __syncthreads();
-  const int64_t cnt = s_hi - s_lo;
   int32_t* out = P.ring_idx + (int64_t)slot * P.n;
   for (int64_t r = threadIdx.x; r < cnt; r += blockDim.x) {
     const int32_t idx = P.sg_idx[s_lo + r];
@@ -446,13 +458,34 @@ __global__ void lif_late_reset_kernel(PopDev P, const int64_t* __restrict__ cloc
   }
 }
 
-// Four neurons per thread once that still gives every SM several CTAs' worth of warps.
-bool wide(int64_t n) { return n / 4 >= (int64_t)kNumSMs * 4 * kBlock; }
+// Neurons per thread and threads per CTA of a population's update: the autotuner's choice, else
+// by kind, type and size.  Small populations are bound by one neuron's chain of loads and
+// arithmetic, so every neuron gets a thread, in CTAs of 128 that spread over more SMs; once a
+// thread per neuron is more than a wave of CTAs, the per-thread work (the clock, the group's
+// constants, the addresses) counts and two, then four neurons share it.  Measured, us per step
+// at 1 / 2 / 4 neurons per thread of 128 (256: 1-8 % slower): HH f32 20,000 2.48 / 2.75 / 3.27,
+// 100,000 3.16 / 3.18 / 3.70 (two are 5 % faster beside a delivery), 220,000 4.59 / 3.94 /
+// 4.18, 300,000 5.41 / 5.09 / 4.67, 600,000 8.61 / 7.50 / 7.12; LIF f32 100,000 2.96 / 2.93 /
+// 3.12, 300,000 4.71 / 3.45 / 3.44, 600,000 7.06 / 5.47 / 4.29; LIF f64 100,000 2.94 / 3.15 /
+// 3.65, 150,000 3.40 / 3.28 / 3.72, 600,000 7.92 / 6.96 / 8.24; HH f64 (two or more
+// serialise its exponentials) 8000-450,000: one; Poisson 100,000 2.69 / 2.65 / 2.65, 300,000
+// 3.42 / 3.10 / 3.03.
+struct UpdateShape {
+  int e, block;
+};
+UpdateShape update_shape(const Pop& pop, int64_t n) {
+  const bool f32 = pop.dtype == B2B_F32;
+  int e = 1;
+  if (pop.kind == KIND_POISSON) e = n >= 200000 ? 4 : 2;
+  else if (f32) e = n >= 280000 ? 4 : (n >= 90000 ? 2 : 1);
+  else if (pop.kind == KIND_LIF) e = n >= 130000 ? 2 : 1;
+  return {pop.tune_e > 0 ? pop.tune_e : e, pop.tune_block > 0 ? pop.tune_block : 128};
+}
 
 template <int E, bool IN>
 cudaError_t launch_e(const Pop& pop, const PopDev& P, const int64_t* clock, int k, double dt,
                      int32_t* status, cudaStream_t s) {
-  const int block = pop.tune_block > 0 ? pop.tune_block : kBlock;   // <= kBlock
+  const int block = update_shape(pop, P.n).block;   // <= kBlock
   const unsigned grid = (unsigned)((P.n / E + block - 1) / block);
   const bool f32 = pop.dtype == B2B_F32;
   switch (pop.kind) {
@@ -498,8 +531,7 @@ cudaError_t launch_pop_step_dev(const Pop& pop, const PopDev& dev, const int64_t
     spikegen_step_kernel<<<1, kBlock, 0, s>>>(pop.dev, clock, k, status);
     return cudaGetLastError();
   }
-  // neurons per thread: the autotuner's choice (1, 2 or 4), else 4 for wide populations
-  const int e = pop.tune_e > 0 ? pop.tune_e : (wide(pop.dev.n) ? 4 : 1);
+  const int e = update_shape(pop, pop.dev.n).e;
   if (pop.inputs) {
     if (e == 4) return launch_e<4, true>(pop, dev, clock, k, dt, status, s);
     if (e == 2) return launch_e<2, true>(pop, dev, clock, k, dt, status, s);
@@ -519,11 +551,11 @@ cudaError_t launch_one_launch_step(const Pop& pop, const PopDev& U, const Pendin
                                    int deliver_ctas, bool chained, const int64_t* clock, int k,
                                    double dt, int32_t* status, cudaStream_t s) {
   if (!one_launch_supported(pop, F) || deliver_ctas < 1) return cudaErrorInvalidValue;
-  // the update half takes the population's tuned shape (neurons per thread 1 or 2, 128 or
-  // 256 threads per CTA); the delivery half the same threads per CTA, deliver_ctas counted
-  // in CTAs of kBlock threads
-  const int e = pop.tune_e == 2 || pop.tune_e == 4 ? 2 : 1;
-  const int block = pop.tune_block > 0 ? pop.tune_block : kBlock;
+  // the update half takes the population's shape (neurons per thread 1 or 2, 128 or 256
+  // threads per CTA); the delivery half the same threads per CTA, deliver_ctas counted in
+  // CTAs of kBlock threads
+  const UpdateShape shape = update_shape(pop, U.n);
+  const int e = shape.e >= 2 ? 2 : 1, block = shape.block;
   const int n_upd = (int)((U.n / e + block - 1) / block);
   const unsigned grid = (unsigned)(n_upd + (int64_t)deliver_ctas * kBlock / block);
   const bool f32 = pop.dtype == B2B_F32;

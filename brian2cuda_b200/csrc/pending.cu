@@ -9,7 +9,8 @@
 //
 //   delivery of step t:  the bundles due at step t are added into acc[t & 1] (this file);
 //   update of step t:    the per-step neuron kernel (neuron.cu), which adds in the input
-//                        that arrived during step t-1, acc[(t-1) & 1], and clears it.
+//                        that arrived during step t-1, acc[(t-1) & 1], and clears it
+// (t counted from the start of the chunk of steps, when both rows are empty).
 //
 // The library launches the two side by side, the delivery on a second stream: the delivery
 // of step t waits for the update of step t-1, the update of step t for the update and the
@@ -23,7 +24,7 @@ namespace b2b {
 
 namespace {
 
-// Bundles due at step clock+k (spikes of steps ts - d, d >= 1) added into acc[ts & 1].
+// Bundles due at step clock+k (spikes of steps ts - d, d >= 1) added into acc[k & 1].
 template <typename R, bool WARP_PREFIX, int GROUP>
 __global__ void __launch_bounds__(kPendingBlock)
 deliver_pending_kernel(const __grid_constant__ PendingDev F, const int64_t* __restrict__ clock,
@@ -34,9 +35,8 @@ deliver_pending_kernel(const __grid_constant__ PendingDev F, const int64_t* __re
 
 // Adds the input delivered in step clock+k_last into the target variables and zeroes it.
 template <typename R>
-__global__ void fold_pending_kernel(const __grid_constant__ PendingDev F,
-                                    const int64_t* __restrict__ clock, int k_last) {
-  const int last = (int)((clock[0] + k_last) & 1);
+__global__ void fold_pending_kernel(const __grid_constant__ PendingDev F, int k_last) {
+  const int last = k_last & 1;
   const int64_t n = F.pop.n;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int v = B2B_VAR_GE; v <= B2B_VAR_GI; ++v) {
@@ -78,14 +78,13 @@ cudaError_t launch_pending_delivery(const PendingDev& F, int dtype, int grid,
             : launch_pending_r<double, false>(F, g, smem, clock, k, s);
 }
 
-cudaError_t launch_fold_pending(const PendingDev& F, int dtype, const int64_t* clock, int k_last,
-                                cudaStream_t s) {
+cudaError_t launch_fold_pending(const PendingDev& F, int dtype, int k_last, cudaStream_t s) {
   const int64_t n = F.pop.n;
   int64_t blocks = (n + kPendingBlock - 1) / kPendingBlock;
   if (blocks > 4 * kNumSMs) blocks = 4 * kNumSMs;
   const dim3 g((unsigned)blocks);
-  if (dtype == B2B_F32) fold_pending_kernel<float><<<g, kPendingBlock, 0, s>>>(F, clock, k_last);
-  else fold_pending_kernel<double><<<g, kPendingBlock, 0, s>>>(F, clock, k_last);
+  if (dtype == B2B_F32) fold_pending_kernel<float><<<g, kPendingBlock, 0, s>>>(F, k_last);
+  else fold_pending_kernel<double><<<g, kPendingBlock, 0, s>>>(F, k_last);
   return cudaGetLastError();
 }
 

@@ -1,7 +1,7 @@
 // The delivery half of the step forms whose every synaptic delay is at least one step
 // (pending.cu: its own launch beside the update; neuron.cu: the CTAs after the update's in
 // the one-launch step): the bundles due at step clock+k are added into the pending input
-// acc[ts & 1] instead of the target variables.
+// acc[k & 1] instead of the target variables.
 #pragma once
 #include "delivery.cuh"
 
@@ -19,7 +19,7 @@ __device__ __forceinline__ void deliver_pending_body(const PendingDev& F,
   const int64_t ts = clock[0] + k;
   const int64_t warp0 = (blk * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = (nblk * blockDim.x) >> 5;
-  const int64_t row = (int64_t)(ts & 1) * F.pop.n;
+  const int64_t row = (int64_t)(k & 1) * F.pop.n;
   const int glane = (threadIdx.x & 31) % GROUP;
   for (int p = 0; p < F.n_proj; ++p) {
     const ProjDev& J = F.proj[p];

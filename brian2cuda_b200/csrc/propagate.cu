@@ -466,6 +466,27 @@ void launch_stdp_pre(const ProjDev& P, unsigned grid, bool ag, bool wp, size_t s
 
 }  // namespace
 
+// A work item is a bundle (up to kChunk synapses): as many lanes as keep most of them busy, so
+// that short bundles leave lanes to other items and long ones need few dependent rounds.
+// Measured, us per step at 2 / 4 / 8 / 16 / 32 lanes: 80 synapses per bundle (CUBA 4000) 8.81 /
+// 7.28 / 6.46 / 6.00 / 5.53; 40 (1e5 -> 1e5 at 300 Hz, 4 CTAs per SM) 54.0 / 51.8 / 52.2 / 49.8 /
+// 55.7; 12 (2e4 -> 3e4) 7.83 / 7.25 / 6.74 / 7.48 / 8.15; 6 (40 merged COBAHH networks, 4 CTAs
+// per SM) 17.1 / 16.8 / 17.4 / 20.2 / 24.0.
+int delivery_lanes(double mean_bundle) {
+  return mean_bundle >= 64 ? 32 : mean_bundle >= 24 ? 16 : mean_bundle >= 8 ? 8 : 4;
+}
+
+// The pending delivery runs beside the update and is mostly latency: in a small network few
+// items are due, and wide items spread them over more warps (two launches, us per step at 4 / 8
+// / 16 lanes: COBAHH 4000 3.82 / 3.79 / 3.78, CUBA with delays 20,000 3.80 / 3.78 / 3.74; COBAHH
+// 30,000 3.05 / 2.99 / 2.97).  Larger ones go by the bundle: 40 synapses (COBAHH 1e5) 3.83 / 3.74
+// / 3.69, 4-5 (8 merged networks) 5.38 / 5.47 / 6.18, (CUBA with delays 150,000) 4.66 / 4.62 /
+// 4.53.
+int pending_lanes(double mean_bundle, int64_t n) {
+  if (n <= 40000 || mean_bundle >= 24) return 16;
+  return 8;
+}
+
 cudaError_t launch_proj_add_batch(const Proj* const* prs, int n, const int64_t* clock, int k,
                                   cudaStream_t s, const AddTune* tune) {
   if (n <= 0 || n > kMaxProjBatch) return cudaErrorInvalidValue;
@@ -480,7 +501,14 @@ cudaError_t launch_proj_add_batch(const Proj* const* prs, int n, const int64_t* 
   }
   const bool wp = nd <= kWarpPrefixMaxDelays;
   const size_t smem = sizeof(int) * (size_t)(nd + 1);
-  const int group = tune && tune->group > 0 ? tune->group : 8;
+  double mean = 0;
+  int64_t most = -1;
+  for (int i = 0; i < n; ++i)
+    if (prs[i]->n_syn > most) {
+      most = prs[i]->n_syn;
+      mean = prs[i]->mean_bundle;
+    }
+  const int group = tune && tune->group > 0 ? tune->group : delivery_lanes(mean);
   ClusterAcc A;
   if (tune && tune->cluster && cluster_layout(prs, n, &A)) {
     const int pref_ints = ((nd + 1 + 3) / 4) * 4;

@@ -56,12 +56,13 @@ __host__ __device__ inline SmallLayout small_layout(int kind) {
   return L;
 }
 
-// Delivery of the bundles of projection J due at step ts by every warp of the CTA: a work
+// Delivery of the bundles of projection J due at step ts (ring slot base) by every warp of the CTA: a work
 // item is 32 synapses of one due bundle (one synapse per lane), items go to the warps in
 // turn, so the few bundles of a small network's step are spread over the whole CTA rather
 // than walked by one warp while the others wait at the next barrier.
 template <typename R, bool WP>
-__device__ __forceinline__ void small_deliver(const ProjDev& J, int64_t ts, int* s_pref) {
+__device__ __forceinline__ void small_deliver(const ProjDev& J, int64_t ts, int base,
+                                              int* s_pref) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   DuePrefix wp{};
   int nspk;
@@ -75,7 +76,6 @@ __device__ __forceinline__ void small_deliver(const ProjDev& J, int64_t ts, int*
   }
   const int sub = J.chunks * (kChunk / 32);
   const int64_t items = (int64_t)nspk * sub;
-  const int base = ring_slot(ts, J.src_ring_len);
   const R* W = static_cast<const R*>(J.w);
   MemberCache<R> mc;
   for (int64_t it = warp; it < items; it += nwarps) {   // warp-uniform
@@ -154,10 +154,12 @@ small_net_kernel(const __grid_constant__ SmallDev D, const int64_t* __restrict__
   __syncthreads();
 
   const double inv_dt = 1.0 / dt;
-  for (int k = 0; k < steps; ++k) {
+  // the ring slots of step ts and of the next one, counted along
+  int slot = ring_slot(ts0, P.ring_len), next;
+  for (int k = 0; k < steps; ++k, slot = next) {
+    next = slot + 1 == P.ring_len ? 0 : slot + 1;
     const int64_t ts = ts0 + k;
     const double t = (double)ts * dt;
-    const int slot = ring_slot(ts, P.ring_len);
     // ---- groups and thresholds: neurons 4*tid .. 4*tid + 3
     unsigned fl = 0;
     const int64_t q4 = (int64_t)tid;
@@ -220,7 +222,6 @@ small_net_kernel(const __grid_constant__ SmallDev D, const int64_t* __restrict__
     const int c = __popc(fl);
     const int excl = block_exclusive_scan(c, s_warp, &total);
     if (tid == 0) {
-      const int next = ring_slot(ts + 1, P.ring_len);
       P.ring_cnt[slot] = total;
       P.ring_cnt[next] = 0;
       s_ring_cnt[slot] = total;
@@ -257,8 +258,8 @@ small_net_kernel(const __grid_constant__ SmallDev D, const int64_t* __restrict__
     }
     // ---- synapses: bundles due at step ts, effects into the shared-memory targets
     for (int p = 0; p < D.n_proj; ++p) {
-      if (D.warp_prefix) small_deliver<R, true>(J[p], ts, s_pref);
-      else small_deliver<R, false>(J[p], ts, s_pref);
+      if (D.warp_prefix) small_deliver<R, true>(J[p], ts, slot, s_pref);
+      else small_deliver<R, false>(J[p], ts, slot, s_pref);
       __syncthreads();
     }
     // ---- resets deferred after the synapses (a synapse writes the reset variable)
@@ -405,14 +406,13 @@ namespace cg = cooperative_groups;
 
 template <typename R>
 __device__ __forceinline__ void cluster_deliver(const cg::cluster_group& cl, const ProjDev& J,
-                                                int64_t ts, int64_t S, int64_t wid,
+                                                int64_t ts, int base, int64_t S, int64_t wid,
                                                 int64_t nw) {
   const int lane = threadIdx.x & 31;
   const DuePrefix wp = due_prefix_warp(J.src_ring_cnt, J.src_ring_len, ts, J.dmin, J.nd,
                                        J.src_lo, J.src_hi);
   const int sub = J.chunks * (kChunk / 32);
   const int64_t items = (int64_t)wp.total * sub;
-  const int base = ring_slot(ts, J.src_ring_len);
   const R* W = static_cast<const R*>(J.w);
   MemberCache<R> mc;
   for (int64_t it = wid; it < items; it += nw) {   // warp-uniform
@@ -487,10 +487,12 @@ small_cluster_kernel(const __grid_constant__ SmallDev D, const int64_t* __restri
   const int64_t nw = (int64_t)C * nwarps;
 
   const double inv_dt = 1.0 / dt;
-  for (int k = 0; k < steps; ++k) {
+  // the ring slots of step ts and of the next one, counted along
+  int slot = ring_slot(ts0, P.ring_len), next;
+  for (int k = 0; k < steps; ++k, slot = next) {
+    next = slot + 1 == P.ring_len ? 0 : slot + 1;
     const int64_t ts = ts0 + k;
     const double t = (double)ts * dt;
-    const int slot = ring_slot(ts, P.ring_len);
     // ---- groups and thresholds: local neuron tid
     const int64_t j0 = tid;
     const unsigned fl =
@@ -511,7 +513,6 @@ small_cluster_kernel(const __grid_constant__ SmallDev D, const int64_t* __restri
       }
       s_off = off;
       s_tot = tot;
-      const int next = ring_slot(ts + 1, P.ring_len);
       s_ring_cnt[slot] = tot;
       s_ring_cnt[next] = 0;
       if (rank == 0) {
@@ -543,7 +544,7 @@ small_cluster_kernel(const __grid_constant__ SmallDev D, const int64_t* __restri
     cl.sync();   // the ring slot is complete, and every CTA has read the counts
     if (tid == 0) s_mon += (unsigned long long)s_tot;
     // ---- synapses: every warp of the cluster, effects into the owners' shared memory
-    for (int p = 0; p < D.n_proj; ++p) cluster_deliver<R>(cl, J[p], ts, S, wid, nw);
+    for (int p = 0; p < D.n_proj; ++p) cluster_deliver<R>(cl, J[p], ts, slot, S, wid, nw);
     cl.sync();   // every effect has landed
     // ---- resets deferred after the synapses, each CTA for its own neurons
     if constexpr (KIND == KIND_LIF) {
@@ -667,10 +668,12 @@ small_pull_kernel(const __grid_constant__ SmallDev D, const int64_t* __restrict_
   __syncthreads();
 
   const double inv_dt = 1.0 / dt;
-  for (int k = 0; k < steps; ++k) {
+  // the ring slots of step ts and of the next one, counted along
+  int slot = ring_slot(ts0, P.ring_len), next;
+  for (int k = 0; k < steps; ++k, slot = next) {
+    next = slot + 1 == P.ring_len ? 0 : slot + 1;
     const int64_t ts = ts0 + k;
     const double t = (double)ts * dt;
-    const int slot = ring_slot(ts, P.ring_len);
     const int par = k & 1;
     int32_t* mylist = lists + par * S;
     // ---- groups and thresholds: local neuron tid
@@ -724,7 +727,7 @@ small_pull_kernel(const __grid_constant__ SmallDev D, const int64_t* __restrict_
       }
       if (tid == 0 && rank == 0) {
         P.ring_cnt[slot] = tot;
-        P.ring_cnt[ring_slot(ts + 1, P.ring_len)] = 0;
+        P.ring_cnt[next] = 0;
       }
     }
     __syncthreads();
