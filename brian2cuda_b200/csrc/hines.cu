@@ -16,13 +16,21 @@
 // Kirchhoff's current law at the nodes (node 0: the sealed start of the root section, node
 // s+1: the end of section s) gives a tree-shaped system in the node voltages.
 //
-// Here one CTA owns one neuron and keeps its whole morphology (matrix rows, state,
-// per-section and per-node arrays) in shared memory across a chunk of steps; the only
+// Here one CTA owns one neuron and keeps it on chip across a chunk of steps (the state of its
+// compartments in registers, everything the phases exchange in shared memory); the only
 // global traffic inside the chunk is the soma spike count.  Per step: compartment-parallel
 // channels, section-parallel tridiagonal solves, node-parallel assembly of the node
 // equations, then elimination (each node pulls in its children) and substitution level by
 // level over the section tree (nodes of equal depth are independent), and a
 // compartment-parallel combination.
+//
+// A step is a chain of latencies (an SM holds 2-5 neurons), so each phase is written for its
+// chain: operands that do not depend on the previous link are loaded ahead of it, a node's
+// children are read without branches (a dummy child adds 0), and a node's four numbers are
+// two 16-byte pairs.  Cycles per step of a 375-compartment, 15-level neuron alone on its SM,
+// before / after (clock64 in a copy of the kernel, float64 channels): channels 6450 / 3170,
+// sections 3310 / 2340, node equations 1000 / 880, elimination 14190 / 2370, substitution 6300 /
+// 1350, combination 810 / 220.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -36,8 +44,9 @@ namespace {
 
 constexpr int kHinesBlock = 256;
 constexpr int kHinesMaxStepsPerLaunch = 1000;
-constexpr int kHinesLargeCtas = 3;   // CTAs per SM of the large class (shared-memory bound)
-constexpr int kHinesSmallCtas = 5;   // and of the small class
+constexpr int kHinesWide = 512;      // threads per CTA when every neuron has an SM to itself
+constexpr int kHinesMaxInRegs = 1024;  // largest neuron whose state the registers hold
+constexpr int kHinesSmallCtas = 5;   // CTAs per SM that the small class's images fit
 
 struct HinesDev {
   int32_t n_neurons;
@@ -55,10 +64,14 @@ struct HinesDev {
   const double *g0, *gn, *rhs_first, *rhs_last;
   const int32_t* child_off;   // per node (global node index = sec_off[b] + b + i), global edges
   const int32_t* child_sec;   // neuron-local section index per edge
-  // per node slot, nodes sorted by depth: {node, parent node (-1 for node 0), first child
-  // edge, end of its child edges} (neuron-local), 4 ints
-  const int32_t* level_rec;
-  const int32_t* level_off;   // per neuron at lvl_base[b]: nlev+1 offsets into level_rec
+  // per node slot, nodes sorted by depth: neuron-local indices times 16 (byte offsets of 16-byte
+  // entries) of {node, end nodes of its first and second child section (node ns + 1, a dummy,
+  // where there is none), parent node}; and the edges of its further children, first | end << 16
+  const int4* level_rec;
+  const int32_t* more_rec;
+  // per neuron at lvl_base[b]: offsets into level_rec of its groups of at most 32 nodes of one
+  // depth, and their end
+  const int32_t* level_off;
   double* v;
   void *m, *h, *n;
   double* Ic;
@@ -79,16 +92,30 @@ __device__ __forceinline__ RC hh_expeuler(RC x, RC a, RC b, RC dt) {
   return -BA + (BA + x) * dexp(A * dt);
 }
 
+// x / c for a literal c, correctly rounded: the product with the rounded reciprocal, corrected
+// by its residual (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000
+// processor", 1990: with 1/c correctly rounded one fused residual step rounds the quotient
+// correctly).  Three operations without a branch, where the general quotient's range checks
+// keep the exponentials around it from overlapping.  An infinite quotient is kept as it is; x in
+// the subnormal range, whose residual is inexact, only feeds exponentials that round to 1.
+template <typename RC>
+__device__ __forceinline__ RC div_lit(RC x, double c) {
+  const RC b = (RC)c, y = (RC)(1.0 / (double)b);
+  const RC q = x * y;
+  const RC r = dfma(-q, b, x);
+  return fabs(q) <= (RC)3e38 ? dfma(r, y, q) : q;
+}
+
 // Hodgkin-Huxley 1952 rates (examples/compartmental/hh_with_spikes_cuda.py:41-46), v in
 // volts measured from rest, rates in 1/s; x/(exp(x/a) - 1) forms through z_over_expm1.
 template <typename RC>
 __device__ __forceinline__ void hh_gates(RC v, RC dt, RC& m, RC& h, RC& n) {
-  const RC am = (RC)1000 * z_over_expm1(((RC)25e-3 - v) / (RC)10e-3);
-  const RC bm = (RC)4000 * dexp(-v / (RC)18e-3);
-  const RC ah = (RC)70 * dexp(-v / (RC)20e-3);
-  const RC bh = (RC)1000 / (dexp(((RC)30e-3 - v) / (RC)10e-3) + (RC)1);
-  const RC an = (RC)100 * z_over_expm1(((RC)10e-3 - v) / (RC)10e-3);
-  const RC bn = (RC)125 * dexp(-v / (RC)80e-3);
+  const RC am = (RC)1000 * z_over_expm1(div_lit<RC>((RC)25e-3 - v, 10e-3));
+  const RC bm = (RC)4000 * dexp(div_lit<RC>(-v, 18e-3));
+  const RC ah = (RC)70 * dexp(div_lit<RC>(-v, 20e-3));
+  const RC bh = (RC)1000 / (dexp(div_lit<RC>((RC)30e-3 - v, 10e-3)) + (RC)1);
+  const RC an = (RC)100 * z_over_expm1(div_lit<RC>((RC)10e-3 - v, 10e-3));
+  const RC bn = (RC)125 * dexp(div_lit<RC>(-v, 80e-3));
   m = hh_expeuler(m, am, bm, dt);
   h = hh_expeuler(h, ah, bh, dt);
   n = hh_expeuler(n, an, bn, dt);
@@ -108,64 +135,68 @@ __device__ __forceinline__ double recip(double x) {
   return fma(y, e, y);
 }
 
-// MINB: CTAs per SM the register budget is sized for.  The large class runs 3 per SM (its
-// shared memory allows no more), so its kernel may keep its values in 80 registers instead of
-// spilling; the small class runs 5 per SM.
-template <typename RC, int MINB>
-__global__ void __launch_bounds__(kHinesBlock, MINB)
+// KC: compartments per thread whose state (v, the gates, the constant matrix diagonal) lives in
+// registers, the matrix couplings then in shared memory; 0: neurons of any size, the state in
+// shared memory and the matrix read through the read-only cache.  BS threads per CTA; MINB: CTAs
+// per SM the register budget is sized for (hines_variant).
+template <typename RC, int KC, int BS, int MINB>
+__global__ void __launch_bounds__(BS, MINB)
 hines_kernel(HinesDev H, int n_steps, int write_currents) {
   extern __shared__ __align__(16) uint8_t sm[];
   const int b = H.order[blockIdx.x];
-  const int tid = threadIdx.x, bs = blockDim.x;
+  const int tid = threadIdx.x;
   const int64_t c0 = H.comp_off[b];
   const int nc = (int)(H.comp_off[b + 1] - c0);
   const int s0 = H.sec_off[b];
   const int ns = H.sec_off[b + 1] - s0;
-  const int nB = ns + 1;
+  const int nB = ns + 1;                     // nodes; node nB is the dummy child
   const int nb0 = s0 + b;
   const int l0 = H.lvl_base[b];
   const int nlev = H.lvl_base[b + 1] - l0 - 1;
-  const int NC = H.nc_max, NS = H.ns_max, NB = H.ns_max + 1;
+  const int NC = H.nc_max, NS = H.ns_max, ND = H.ns_max + 2;
 
-  int4* REC = reinterpret_cast<int4*>(sm);   // level records, first (16-byte aligned)
-  // The constant matrix rows (low, diag, up) and the compartment-to-section map are read
-  // through the read-only cache rather than kept here, so that three CTAs fit an SM and one
-  // neuron's serial phases overlap other neurons' parallel ones.
-  double* V = reinterpret_cast<double*>(REC + NB);
-  double* X = V + NC;          // x*, first the right-hand side of the membrane solve
-  double* UE = X + NC;         // u_end
-  double* US = UE + NC;        // u_start
-  double* DG = US + NC;        // diagonal with the membrane conductance of the step, then
-                               // the eliminated super-diagonal
-  double* DN = DG + NC;        // node equations: diagonal,
-  double* TOWARD = DN + NB;    // coefficient of the parent node (node >= 1),
-  double* RHSN = TOWARD + NB;  // right-hand side,
-  double* INTO = RHSN + NB;    // per node >= 1: its coefficient in its parent's equation
-  double* INV = INTO + NB;     // 1 / final diagonal, per node
-  double* G0 = INV + NB;
+  int4* REC = reinterpret_cast<int4*>(sm);                    // level records
+  // a node's equation {diagonal, right-hand side}, after its elimination {1 / diagonal,
+  // right-hand side}, at last the right-hand side the node's voltage; and its coefficient in
+  // its parent's equation and the parent's in its own
+  double2* EQ = reinterpret_cast<double2*>(REC + ND);
+  double2* IT = EQ + ND;
+  // per compartment: the membrane solve's {diagonal, right-hand side}, after the forward pass
+  // {eliminated super-diagonal, right-hand side}, at last {u_end, x*}; and u_start
+  double2* DX = IT + ND;
+  double2* LU = DX + NC;                                      // KC > 0: {low, up} couplings
+  double* US = reinterpret_cast<double*>(LU + (KC > 0 ? NC : 0));
+  double* G0 = US + NC;
   double* GN = G0 + NS;
   double* RF = GN + NS;
   double* RL = RF + NS;
-  RC* M = reinterpret_cast<RC*>(RL + NS);
-  RC* Hh = M + NC;
-  RC* N = Hh + NC;
-  int32_t* SST = reinterpret_cast<int32_t*>(N + NC);
+  double* Vs = RL + NS;                                       // KC == 0: the state
+  RC* Ms = reinterpret_cast<RC*>(Vs + (KC > 0 ? 0 : NC));
+  RC* Hs = Ms + (KC > 0 ? 0 : NC);
+  RC* Ns = Hs + (KC > 0 ? 0 : NC);
+  int32_t* SST = reinterpret_cast<int32_t*>(Ns + (KC > 0 ? 0 : NC));
   int32_t* SEN = SST + NS;
   int32_t* SPN = SEN + NS;
-  int32_t* COFF = SPN + NS;
-  int32_t* CSEC = COFF + NB + 1;
-  int32_t* LOFF = CSEC + NS;
+  int32_t* CSEC = SPN + NS;
+  int32_t* MORE = CSEC + NS;   // edges of a node's children past the second, first | end << 16
+  int32_t* LOFF = MORE + ND;
 
-  const RC* gm = static_cast<const RC*>(H.m);
-  const RC* gh = static_cast<const RC*>(H.h);
-  const RC* gn = static_cast<const RC*>(H.n);
-  for (int j = tid; j < nc; j += bs) {
-    V[j] = H.v[c0 + j];
-    M[j] = gm[c0 + j];
-    Hh[j] = gh[c0 + j];
-    N[j] = gn[c0 + j];
-  }
-  for (int s = tid; s < ns; s += bs) {
+  constexpr int K1 = KC > 0 ? KC : 1;
+  double vr[K1], dr[K1];
+  RC mr[K1], hr[K1], nr[K1];
+  int32_t nodes[K1];           // start node | section << 16 of each compartment
+  // every compartment of this thread: f(j, its register slot)
+  auto for_comps = [&](auto f) {
+    if constexpr (KC > 0) {
+#pragma unroll
+      for (int c = 0; c < KC; ++c)
+        if (tid + c * BS < nc) f(tid + c * BS, c);
+    } else {
+      for (int j = tid; j < nc; j += BS) f(j, 0);
+    }
+  };
+
+  for (int s = tid; s < ns; s += BS) {
     SST[s] = H.sec_start[s0 + s];
     SEN[s] = H.sec_end[s0 + s];
     SPN[s] = H.sec_pnode[s0 + s];
@@ -175,13 +206,42 @@ hines_kernel(HinesDev H, int n_steps, int write_currents) {
     RL[s] = H.rhs_last[s0 + s];
   }
   const int e0 = H.child_off[nb0];
-  for (int i = tid; i <= nB; i += bs) COFF[i] = H.child_off[nb0 + i] - e0;
-  for (int e = tid; e < ns; e += bs) CSEC[e] = H.child_sec[e0 + e];
-  for (int k = tid; k < nB; k += bs)
-    REC[k] = make_int4(H.level_rec[4 * (nb0 + k)], H.level_rec[4 * (nb0 + k) + 1],
-                       H.level_rec[4 * (nb0 + k) + 2], H.level_rec[4 * (nb0 + k) + 3]);
-  for (int L = tid; L <= nlev; L += bs) LOFF[L] = H.level_off[l0 + L];
-  __syncthreads();
+  for (int e = tid; e < ns; e += BS) CSEC[e] = H.child_sec[e0 + e];
+  bool more = false;           // some node has more than two children
+  for (int k = tid; k < nB; k += BS) {
+    REC[k] = H.level_rec[nb0 + k];
+    MORE[k] = H.more_rec[nb0 + k];
+    more |= (MORE[k] & 0xffff) != (int)((unsigned)MORE[k] >> 16);
+  }
+  if (tid == 0) {
+    EQ[nB] = make_double2(1.0, 0.0);
+    IT[nB] = make_double2(0.0, 0.0);
+    IT[0] = make_double2(0.0, 0.0);
+  }
+  for (int L = tid; L <= nlev; L += BS) LOFF[L] = H.level_off[l0 + L];
+  const bool any_more = __syncthreads_or(more);
+  {
+    const RC* gm = static_cast<const RC*>(H.m);
+    const RC* gh = static_cast<const RC*>(H.h);
+    const RC* gn = static_cast<const RC*>(H.n);
+    for_comps([&](int j, int c) {
+      if constexpr (KC > 0) {
+        vr[c] = H.v[c0 + j];
+        mr[c] = gm[c0 + j];
+        hr[c] = gh[c0 + j];
+        nr[c] = gn[c0 + j];
+        dr[c] = H.diag[c0 + j];
+        LU[j] = make_double2(H.low[c0 + j], H.up[c0 + j]);
+        const int s = H.sec_of_comp[c0 + j];
+        nodes[c] = SPN[s] | s << 16;
+      } else {
+        Vs[j] = H.v[c0 + j];
+        Ms[j] = gm[c0 + j];
+        Hs[j] = gh[c0 + j];
+        Ns[j] = gn[c0 + j];
+      }
+    });
+  }
 
   const double cdt = H.Cm / H.dt;
   const double Isoma = H.soma_I[b];
@@ -191,131 +251,203 @@ hines_kernel(HinesDev H, int n_steps, int write_currents) {
 
   for (int step = 0; step < n_steps; ++step) {
     // (1) channels: conductance and current at the start of the step, then the gates
-    for (int j = tid; j < nc; j += bs) {
-      const double v = V[j];
-      RC m = M[j], h = Hh[j], n = N[j];
+    for_comps([&](int j, int c) {
+      const double v = KC > 0 ? vr[c] : Vs[j];
+      RC m = KC > 0 ? mr[c] : Ms[j], h = KC > 0 ? hr[c] : Hs[j], n = KC > 0 ? nr[c] : Ns[j];
       const double md = (double)m, hd = (double)h, nd = (double)n;
       const double gna = H.gNa * (md * md * md * hd);
       const double gk = H.gK * (nd * nd * nd * nd);
       const double gtot = H.gl + gna + gk;
       double I0 = H.gl * H.El + gna * H.ENa + gk * H.EK;
       if (j == 0) I0 += Isoma;
-      DG[j] = __ldg(H.diag + c0 + j) - gtot;
-      X[j] = -cdt * v - I0;
+      DX[j] = make_double2((KC > 0 ? dr[c] : __ldg(H.diag + c0 + j)) - gtot, -cdt * v - I0);
       hh_gates<RC>((RC)v, dtR, m, h, n);
-      M[j] = m;
-      Hh[j] = h;
-      N[j] = n;
-    }
+      if constexpr (KC > 0) {
+        mr[c] = m; hr[c] = h; nr[c] = n;
+      } else {
+        Ms[j] = m; Hs[j] = h; Ns[j] = n;
+      }
+    });
     __syncthreads();
     // (2) per section, one pass of forward elimination (reciprocal pivot) and back
-    // substitution for the three right-hand sides
-    for (int s = tid; s < ns; s += bs) {
-      const int j0 = SST[s], j1 = SEN[s];
-      double cprev = 0.0, xprev = 0.0, sprev = 0.0, eprev = 0.0;
-      for (int j = j0; j < j1; ++j) {
-        const double lw = j > j0 ? __ldg(H.low + c0 + j) : 0.0;
-        const double piv = recip(DG[j] - lw * cprev);
-        cprev = __ldg(H.up + c0 + j) * piv;
-        DG[j] = cprev;   // the diagonal is not needed again
-        X[j] = (X[j] - lw * xprev) * piv;
-        US[j] = ((j == j0 ? RF[s] : 0.0) - lw * sprev) * piv;
-        UE[j] = ((j == j1 - 1 ? RL[s] : 0.0) - lw * eprev) * piv;
-        xprev = X[j];
-        sprev = US[j];
-        eprev = UE[j];
+    // substitution for the three right-hand sides.  The pivots are one chain per section:
+    // the next compartment's operands are loaded ahead of it (clamped, not branched) and what
+    // is passed along stays in registers.  u_end is 0 before the last compartment of the
+    // forward pass; the couplings into a section's first and out of its last compartment are 0.
+    for (int s = tid; s < ns; s += BS) {
+      const int j0 = SST[s], last = SEN[s] - 1;
+      auto couplings = [&](int j) {
+        return KC > 0 ? LU[j] : make_double2(__ldg(H.low + c0 + j), __ldg(H.up + c0 + j));
+      };
+      double2 lu = couplings(j0), dx = DX[j0];
+      double rs = RF[s];
+      const double rl = RL[s];
+      double cprev = 0.0, xprev = 0.0, sprev = 0.0, piv = 0.0;
+#pragma unroll 2
+      for (int j = j0; j <= last; ++j) {
+        const int jn = min(j + 1, last);
+        const double2 lun = couplings(jn), dxn = DX[jn];
+        piv = recip(dx.x - lu.x * cprev);
+        cprev = lu.y * piv;
+        xprev = (dx.y - lu.x * xprev) * piv;
+        sprev = (rs - lu.x * sprev) * piv;
+        DX[j] = make_double2(cprev, xprev);   // the diagonal is not needed again
+        US[j] = sprev;
+        lu = lun;
+        dx = dxn;
+        rs = 0.0;
       }
-      for (int j = j1 - 2; j >= j0; --j) {
-        X[j] -= DG[j] * X[j + 1];
-        US[j] -= DG[j] * US[j + 1];
-        UE[j] -= DG[j] * UE[j + 1];
+      double eprev = rl * piv;
+      DX[last].x = eprev;
+      int j = max(last - 1, j0);
+      dx = DX[j];
+      double us = US[j];
+#pragma unroll 2
+      for (j = last - 1; j >= j0; --j) {
+        const int jn = max(j - 1, j0);
+        const double2 dxn = DX[jn];
+        const double un = US[jn];
+        xprev = dx.y - dx.x * xprev;
+        sprev = us - dx.x * sprev;
+        eprev = -(dx.x * eprev);
+        DX[j] = make_double2(eprev, xprev);
+        US[j] = sprev;
+        dx = dxn;
+        us = un;
       }
     }
     __syncthreads();
-    // (3) node equations: node i's current balance in its own voltage (DN), its parent
-    // node's (TOWARD) and its children's end nodes' (INTO, stored with the child node)
-    for (int i = tid; i < nB; i += bs) {
+    // (3) node equations: node i's current balance in its own voltage, its parent node's
+    // and its children's end nodes' (stored with the child node)
+    for (int k = tid; k < nB; k += BS) {
+      const int4 r = REC[k];
+      const int i = r.x >> 4;
       double dn, rh;
       if (i == 0) {
         // the root's start takes the voltage of the root's first compartment
         const int f = SST[0];
         dn = US[f] - 1.0;
-        rh = -X[f];
-        INTO[1] = UE[f];
+        rh = -DX[f].y;
+        IT[1].x = DX[f].x;
       } else {
-        const int s = i - 1;
-        const int l = SEN[s] - 1;
-        dn = GN[s] * (1.0 - UE[l]);
-        TOWARD[i] = -GN[s] * US[l];
-        rh = GN[s] * X[l];
-        for (int e = COFF[i]; e < COFF[i + 1]; ++e) {
-          const int cs = CSEC[e];
-          const int f = SST[cs];
-          dn += G0[cs] * (1.0 - US[f]);
-          INTO[cs + 1] = -G0[cs] * UE[f];
-          rh += G0[cs] * X[f];
-        }
+        const int s = i - 1, l = SEN[s] - 1;
+        const double2 ex = DX[l];
+        dn = GN[s] * (1.0 - ex.x);
+        IT[i].y = -GN[s] * US[l];
+        rh = GN[s] * ex.y;
+        auto child = [&](int cn) {   // cn: the child section's end node
+          const int f = SST[cn - 1];
+          const double g = G0[cn - 1];
+          const double2 exf = DX[f];
+          dn += g * (1.0 - US[f]);
+          IT[cn].x = -g * exf.x;
+          rh += g * exf.y;
+        };
+        if ((r.y >> 4) < nB) child(r.y >> 4);
+        if ((r.z >> 4) < nB) child(r.z >> 4);
+        if (any_more)
+          for (int e = MORE[k] & 0xffff; e < (int)((unsigned)MORE[k] >> 16); ++e)
+            child(CSEC[e] + 1);
       }
-      DN[i] = dn;
-      RHSN[i] = rh;
+      EQ[i] = make_double2(dn, rh);
     }
     __syncthreads();
-    // (4)-(5) the node system on the first warp alone, level by level with warp barriers (a
-    // level holds few nodes; CTA-wide barriers per level would idle every other warp)
+    // (4)-(5) the node system on the first warp alone, group by group of at most 32 nodes of
+    // one depth, with warp barriers.  Records hold byte offsets into EQ and IT and are loaded
+    // two groups ahead, what else does not depend on the group before it one ahead; the dummy
+    // child of a node with fewer than two subtracts 0.
     if (tid < 32) {
-      // (4) elimination, deepest level first: each node takes in its children's equations;
-      // a record gives the node and its child edges at once, and children are taken in
-      // pairs so that their loads and divisions overlap (the order of the updates is the
-      // children's order)
-      for (int L = nlev - 1; L >= 0; --L) {
-        for (int k = LOFF[L] + tid; k < LOFF[L + 1]; k += 32) {
-          const int4 r = REC[k];
-          double dn = DN[r.x], rh = RHSN[r.x];
-          int e = r.z;
-          for (; e + 1 < r.w; e += 2) {
-            const int ca = CSEC[e] + 1, cb = CSEC[e + 1] + 1;   // the children's end nodes
-            const double fa = INTO[ca] * INV[ca], fb = INTO[cb] * INV[cb];
-            dn -= fa * TOWARD[ca];
-            rh -= fa * RHSN[ca];
-            dn -= fb * TOWARD[cb];
-            rh -= fb * RHSN[cb];
-          }
-          if (e < r.w) {
-            const int c = CSEC[e] + 1;
-            const double f = INTO[c] * INV[c];
-            dn -= f * TOWARD[c];
-            rh -= f * RHSN[c];
-          }
-          DN[r.x] = dn;
-          RHSN[r.x] = rh;
-          INV[r.x] = recip(dn);   // the node's equation is final here
+      char* const eqb = reinterpret_cast<char*>(EQ);
+      char* const itb = reinterpret_cast<char*>(IT);
+      auto eq_at = [&](int off) -> double2& { return *reinterpret_cast<double2*>(eqb + off); };
+      auto it_at = [&](int off) -> double2& { return *reinterpret_cast<double2*>(itb + off); };
+      // (4) elimination, deepest group first: each node takes in its children's equations in
+      // the children's order
+      int hi = nB, lo = LOFF[nlev - 1], lo1 = LOFF[max(nlev - 2, 0)];
+      if (!any_more) {
+        int4 r = REC[min(lo + tid, nB - 1)], rn = REC[min(lo1 + tid, nB - 1)];
+        double2 eq = eq_at(r.x), ia = it_at(r.y), ib = it_at(r.z);
+        for (int L = nlev - 1; L >= 0; --L) {
+          const double2 a = eq_at(r.y), c = eq_at(r.z);
+          const int lo2 = LOFF[max(L - 2, 0)];
+          const double2 eqn = eq_at(rn.x), ian = it_at(rn.y), ibn = it_at(rn.z);
+          const int4 rnn = REC[min(lo2 + tid, nB - 1)];
+          const double fa = ia.x * a.x, fb = ib.x * c.x;
+          double dn = eq.x, rh = eq.y;
+          dn -= fa * ia.y;
+          rh -= fa * a.y;
+          dn -= fb * ib.y;
+          rh -= fb * c.y;
+          const double inv = recip(dn);   // the node's equation is final here
+          if (lo + tid < hi) eq_at(r.x) = make_double2(inv, rh);
+          __syncwarp();
+          r = rn; eq = eqn; ia = ian; ib = ibn; rn = rnn;
+          hi = lo; lo = lo1; lo1 = lo2;
         }
-        __syncwarp();
+      } else {
+        for (int L = nlev - 1; L >= 0; --L) {
+          const int k = LOFF[L] + tid;
+          if (k < LOFF[L + 1]) {
+            const int4 r = REC[k];
+            double2 eq = eq_at(r.x);
+            auto take = [&](int off) {
+              const double2 it = it_at(off), c = eq_at(off);
+              const double f = it.x * c.x;
+              eq.x -= f * it.y;
+              eq.y -= f * c.y;
+            };
+            take(r.y);
+            take(r.z);
+            for (int e = MORE[k] & 0xffff; e < (int)((unsigned)MORE[k] >> 16); ++e)
+              take(16 * (CSEC[e] + 1));
+            eq_at(r.x) = make_double2(recip(eq.x), eq.y);
+          }
+          __syncwarp();
+        }
       }
-      // (5) substitution, root first: RHSN becomes the node voltage
-      if (tid == 0) RHSN[0] = RHSN[0] * INV[0];
+      // (5) substitution, root first: the right-hand side becomes the node voltage
+      if (tid == 0) EQ[0].y = EQ[0].y * EQ[0].x;
+      lo = LOFF[min(1, nlev)];
+      hi = LOFF[min(2, nlev)];
+      int hi1 = LOFF[min(3, nlev)];
+      int4 r = REC[min(lo + tid, nB - 1)], rn = REC[min(hi + tid, nB - 1)];
+      double2 eq = eq_at(r.x);
+      double toward = it_at(r.x).y;
       __syncwarp();
       for (int L = 1; L < nlev; ++L) {
-        for (int k = LOFF[L] + tid; k < LOFF[L + 1]; k += 32) {
-          const int4 r = REC[k];
-          RHSN[r.x] = (RHSN[r.x] - TOWARD[r.x] * RHSN[r.y]) * INV[r.x];
-        }
+        const double vp = eq_at(r.w).y;
+        const double2 eqn = eq_at(rn.x);
+        const double towardn = it_at(rn.x).y;
+        const int hi2 = LOFF[min(L + 3, nlev)];
+        const int4 rnn = REC[min(hi1 + tid, nB - 1)];
+        if (lo + tid < hi) eq_at(r.x).y = (eq.y - toward * vp) * eq.x;
         __syncwarp();
+        r = rn; eq = eqn; toward = towardn; rn = rnn;
+        lo = hi; hi = hi1; hi1 = hi2;
       }
     }
     __syncthreads();
     // (6) v = x* + V_start u_start + V_end u_end; capacitive current
     const bool last_step = step == n_steps - 1;
-    for (int j = tid; j < nc; j += bs) {
-      const int s = __ldg(H.sec_of_comp + c0 + j);
-      const double vn = X[j] + RHSN[SPN[s]] * US[j] + RHSN[s + 1] * UE[j];
-      if (last_step && write_currents) H.Ic[c0 + j] = H.Cm * (vn - V[j]) / H.dt;
-      V[j] = vn;
-    }
+    for_comps([&](int j, int c) {
+      int pn, s;
+      if constexpr (KC > 0) {
+        pn = nodes[c] & 0xffff;
+        s = nodes[c] >> 16;
+      } else {
+        s = __ldg(H.sec_of_comp + c0 + j);
+        pn = SPN[s];
+      }
+      const double2 ex = DX[j];
+      const double vn = ex.y + EQ[pn].y * US[j] + EQ[s + 1].y * ex.x;
+      const double v = KC > 0 ? vr[c] : Vs[j];
+      if (last_step && write_currents) H.Ic[c0 + j] = H.Cm * (vn - v) / H.dt;
+      if constexpr (KC > 0) vr[c] = vn; else Vs[j] = vn;
+    });
     // no barrier: a thread owns the same compartments here and in the next step's channel
     // phase (and thread 0 owns compartment 0); the next step's first barrier orders the rest
     if (tid == 0) {
-      const int ab = V[0] > H.Vthr ? 1 : 0;
+      const int ab = (KC > 0 ? vr[0] : Vs[0]) > H.Vthr ? 1 : 0;
       if (ab && !above) ++spikes;
       above = ab;
     }
@@ -323,22 +455,59 @@ hines_kernel(HinesDev H, int n_steps, int write_currents) {
   RC* wm = static_cast<RC*>(H.m);
   RC* wh = static_cast<RC*>(H.h);
   RC* wn = static_cast<RC*>(H.n);
-  for (int j = tid; j < nc; j += bs) {
-    H.v[c0 + j] = V[j];
-    wm[c0 + j] = M[j];
-    wh[c0 + j] = Hh[j];
-    wn[c0 + j] = N[j];
-  }
+  for_comps([&](int j, int c) {
+    H.v[c0 + j] = KC > 0 ? vr[c] : Vs[j];
+    wm[c0 + j] = KC > 0 ? mr[c] : Ms[j];
+    wh[c0 + j] = KC > 0 ? hr[c] : Hs[j];
+    wn[c0 + j] = KC > 0 ? nr[c] : Ns[j];
+  });
   if (tid == 0) {
     H.spikes[b] += spikes;
     H.above[b] = above;
   }
 }
 
-size_t hines_smem(int nc, int ns, int nlev, int rc_size) {
-  const size_t NB = (size_t)ns + 1;
-  return 16 * NB + sizeof(double) * (5 * (size_t)nc + 5 * NB + 4 * (size_t)ns) +
-         rc_size * 3 * (size_t)nc + sizeof(int32_t) * (4 * (size_t)ns + NB + 1 + (size_t)nlev + 1);
+// Shared memory of a neuron's image of nlev node groups (in_regs: its compartments' state is in
+// registers).
+size_t hines_smem(int nc, int ns, int nlev, int rc_size, bool in_regs) {
+  const size_t ND = (size_t)ns + 2;
+  return 48 * ND + sizeof(double) * ((in_regs ? 5 : 4) * (size_t)nc + 4 * (size_t)ns) +
+         (in_regs ? 0 : rc_size * 3 * (size_t)nc) +
+         sizeof(int32_t) * (4 * (size_t)ns + ND + (size_t)nlev + 1);
+}
+
+using HinesKernel = void (*)(HinesDev, int, int);
+
+// The kernel and its threads per CTA for a class of neurons of up to nc compartments.
+struct HinesVariant {
+  HinesKernel kern;
+  int block;
+};
+template <typename RC, int KC, int BS, int MINB>
+HinesVariant variant() {
+  return {hines_kernel<RC, KC, BS, MINB>, BS};
+}
+// Neurons that have an SM each are pure latency: 512 threads, so that fewer compartments share a
+// thread (61 neurons of up to 400 compartments, float64 channels: 10.2 -> 5.3 us per step with
+// the rest of the kernel's chains, 15.3 before both).  Otherwise as many neurons per SM as
+// registers and shared memory allow cover each other's chains: the float32 variant of 1024
+// compartments at 4 per SM with a few spills 20.2, at 3 without 21.6 us per step (1024 neurons of
+// 200-1000 compartments); those of up to 768 at 5 per SM 13.4, at 4 12.1 (200-400 compartments).
+template <typename RC>
+HinesVariant hines_variant(int nc, bool one_per_sm) {
+  constexpr bool f32 = sizeof(RC) == 4;
+  if (one_per_sm) {
+    if (nc <= kHinesWide) return variant<RC, 1, kHinesWide, 1>();
+    if (nc <= 2 * kHinesWide) return variant<RC, 2, kHinesWide, 1>();
+    return variant<RC, 0, kHinesBlock, 3>();
+  }
+  switch ((nc + kHinesBlock - 1) / kHinesBlock) {
+    case 1: return variant<RC, 1, kHinesBlock, 4>();
+    case 2: return variant<RC, 2, kHinesBlock, 4>();
+    case 3: return variant<RC, 3, kHinesBlock, f32 ? 4 : 3>();
+    case 4: return variant<RC, 4, kHinesBlock, f32 ? 4 : 3>();
+    default: return variant<RC, 0, kHinesBlock, 3>();
+  }
 }
 
 }  // namespace
@@ -355,7 +524,7 @@ struct b2b_hines {
   // own size beside the others (on stream2, forked from and joined to the net's stream), so
   // that small neurons do not reserve the largest neuron's shared memory.
   int32_t n_large = 0;                   // CTAs of the first launch (all neurons when 1 class)
-  bool large_fits5 = false;              // the first launch's image fits 5 CTAs per SM too
+  b2b::HinesVariant var{}, var_small{};   // kernels of the two classes
   b2b::HinesDev dev_small{};
   size_t smem_small = 0;
   cudaStream_t stream2 = nullptr;
@@ -404,7 +573,8 @@ b2b_status b2b_hines_create(b2b_net* net, int32_t n_neurons, const int64_t* comp
     std::vector<double> low(n_comp, 0.0), diag(n_comp, 0.0), upr(n_comp, 0.0);
     std::vector<int32_t> soc(n_comp), sst(n_sec), sen(n_sec), spn(n_sec);
     std::vector<double> g0(n_sec), gn(n_sec), rfirst(n_sec), rlast(n_sec);
-    std::vector<int32_t> child_off, child_sec, level_rec, level_off, lvl_base;
+    std::vector<int32_t> child_off, child_sec, more_rec, level_off, lvl_base;
+    std::vector<int4> level_rec;
     // r: cross section over half the length; g: axial conductance into c from c - 1
     std::vector<double> area(n_comp), rl(n_comp), g(n_comp + 1, 0.0);
     std::vector<double> soma_area(n_neurons);
@@ -416,6 +586,8 @@ b2b_status b2b_hines_create(b2b_net* net, int32_t n_neurons, const int64_t* comp
       const int s0 = sec_off[b], s1 = sec_off[b + 1];
       const int nc = (int)(c1 - c0), ns = s1 - s0;
       if (nc <= 0 || ns <= 0 || nc > (1 << 20)) return B2B_ERR_INVALID_ARG;
+      // 16-bit node and edge indices; so many sections exceed a CTA's shared memory anyway
+      if (ns >= 32766) return B2B_ERR_UNSUPPORTED;
       nc_max = std::max(nc_max, nc);
       ns_max = std::max(ns_max, ns);
       // morphology checks: sections contiguous, in topological order, root first
@@ -464,9 +636,6 @@ b2b_status b2b_hines_create(b2b_net* net, int32_t n_neurons, const int64_t* comp
       for (int s = 1; s < ns; ++s) kids[spn[s0 + s]].push_back(s);
       std::vector<int> depth(nB, 0);
       for (int s = 0; s < ns; ++s) depth[s + 1] = depth[spn[s0 + s]] + 1;
-      const int nlev = *std::max_element(depth.begin(), depth.end()) + 1;
-      nlev_max = std::max(nlev_max, nlev);
-      nlev_of[b] = nlev;
       const int edge_base = (int)child_sec.size();
       std::vector<int> first_edge(nB + 1);
       for (int i = 0; i < nB; ++i) {
@@ -480,22 +649,34 @@ b2b_status b2b_hines_create(b2b_net* net, int32_t n_neurons, const int64_t* comp
       std::stable_sort(order.begin(), order.end(), [&](int a, int c) { return depth[a] < depth[c]; });
       lvl_base.push_back((int)level_off.size());
       for (int i : order) {
-        level_rec.push_back(i);
-        level_rec.push_back(i == 0 ? -1 : spn[s0 + i - 1]);
-        level_rec.push_back(first_edge[i]);
-        level_rec.push_back(first_edge[i + 1]);
+        const std::vector<int>& ch = kids[i];
+        const int ca = ch.size() > 0 ? ch[0] + 1 : nB, cb = ch.size() > 1 ? ch[1] + 1 : nB;
+        const int more = std::min(first_edge[i] + 2, first_edge[i + 1]);
+        level_rec.push_back(
+            make_int4(16 * i, 16 * ca, 16 * cb, i == 0 ? 0 : 16 * spn[s0 + i - 1]));
+        more_rec.push_back(more | first_edge[i + 1] << 16);
       }
-      int k = 0;
-      for (int L = 0; L <= nlev; ++L) {
-        while (k < nB && depth[order[k]] < L) ++k;
+      // groups of at most 32 nodes (one per lane of the warp that walks them) of one depth
+      int groups = 0;
+      for (int k = 0; k < nB; ++groups) {
         level_off.push_back(k);
+        const int first = k;
+        while (k < nB && k - first < 32 && depth[order[k]] == depth[order[first]]) ++k;
       }
+      level_off.push_back(nB);
+      nlev_of[b] = groups;
+      nlev_max = std::max(nlev_max, groups);
     }
     child_off.push_back((int)child_sec.size());
     lvl_base.push_back((int)level_off.size());
 
     const int rc = p->channel_dtype == B2B_F32 ? 4 : 8;
-    const size_t smem = hines_smem(nc_max, ns_max, nlev_max, rc);
+    // neurons beyond the register variants' size put the whole batch on the general one
+    const bool in_regs = nc_max <= kHinesMaxInRegs;
+    int sms = kNumSMs;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, net->cfg.device);
+    const bool one_per_sm = n_neurons <= sms;   // latency alone counts: wide CTAs, one class
+    const size_t smem = hines_smem(nc_max, ns_max, nlev_max, rc, in_regs);
     int dev_smem = 0;
     cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, net->cfg.device);
     if ((int64_t)smem > dev_smem) return B2B_ERR_UNSUPPORTED;
@@ -525,9 +706,9 @@ b2b_status b2b_hines_create(b2b_net* net, int32_t n_neurons, const int64_t* comp
     up(&D.sec_start, sst); up(&D.sec_end, sen); up(&D.sec_pnode, spn);
     up(&D.g0, g0); up(&D.gn, gn); up(&D.rhs_first, rfirst); up(&D.rhs_last, rlast);
     up(&D.child_off, child_off); up(&D.child_sec, child_sec);
-    up(&D.level_rec, level_rec); up(&D.level_off, level_off);
-    // cost of a neuron's step: the node system walks its levels on one warp (~1000 cycles
-    // per level, the largest phase), the compartment-parallel phases grow with its size
+    up(&D.level_rec, level_rec); up(&D.more_rec, more_rec); up(&D.level_off, level_off);
+    // cost of a neuron's step: the node system walks its levels on one warp, the
+    // compartment-parallel phases grow with its size
     std::vector<int32_t> order(n_neurons);
     std::vector<double> cost(n_neurons);
     for (int b = 0; b < n_neurons; ++b) {
@@ -540,17 +721,16 @@ b2b_status b2b_hines_create(b2b_net* net, int32_t n_neurons, const int64_t* comp
     int sm_bytes = 0, reserved = 0;
     cudaDeviceGetAttribute(&sm_bytes, cudaDevAttrMaxSharedMemoryPerMultiprocessor, net->cfg.device);
     cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, net->cfg.device);
-    const size_t small_cap = sm_bytes > 0 ? (size_t)(sm_bytes / 5 - reserved) : 0;
+    const size_t small_cap = sm_bytes > 0 ? (size_t)(sm_bytes / kHinesSmallCtas - reserved) : 0;
     std::vector<char> small(n_neurons, 0);
     int n_small = 0;
     for (int b = 0; b < n_neurons; ++b) {
       const int nc = (int)(comp_off[b + 1] - comp_off[b]), ns = sec_off[b + 1] - sec_off[b];
-      small[b] = hines_smem(nc, ns, nlev_of[b], rc) <= small_cap ? 1 : 0;
+      small[b] = hines_smem(nc, ns, nlev_of[b], rc, in_regs) <= small_cap ? 1 : 0;
       n_small += small[b];
     }
-    if (n_small == 0 || n_small == n_neurons || smem <= small_cap)
+    if (n_small == 0 || n_small == n_neurons || smem <= small_cap || one_per_sm)
       std::fill(small.begin(), small.end(), 0);   // one class, one launch
-    h->large_fits5 = smem <= small_cap;
     std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t c) {
       if (small[a] != small[c]) return small[a] < small[c];
       return cost[a] > cost[c];
@@ -570,8 +750,8 @@ b2b_status b2b_hines_create(b2b_net* net, int32_t n_neurons, const int64_t* comp
     if (n_large < n_neurons) {
       // the large class's image bounds its own arrays; the small class has its own bounds
       D.nc_max = ncl; D.ns_max = nsl; D.nlev_max = nll;
-      h->smem = hines_smem(ncl, nsl, nll, rc);
-      h->smem_small = hines_smem(ncs, nss, nls, rc);
+      h->smem = hines_smem(ncl, nsl, nll, rc, in_regs);
+      h->smem_small = hines_smem(ncs, nss, nls, rc, in_regs);
       if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&h->stream2, cudaStreamNonBlocking);
       if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming);
       if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming);
@@ -596,19 +776,18 @@ b2b_status b2b_hines_create(b2b_net* net, int32_t n_neurons, const int64_t* comp
       h->dev_small.nc_max = ncs; h->dev_small.ns_max = nss; h->dev_small.nlev_max = nls;
       h->dev_small.order = D.order + n_large;
     }
-    // shared memory of each kernel variant: the first launch's image for the variant it runs
-    // (5 CTAs per SM when its image fits them), the small class's for the other
-    const int s5 = (int)std::max(h->large_fits5 ? smem : 0, n_large < n_neurons ? h->smem_small : 0);
-    if (e == cudaSuccess && !h->large_fits5)
-      e = rc == 4 ? cudaFuncSetAttribute(hines_kernel<float, kHinesLargeCtas>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
-                  : cudaFuncSetAttribute(hines_kernel<double, kHinesLargeCtas>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess && s5 > 0)
-      e = rc == 4 ? cudaFuncSetAttribute(hines_kernel<float, kHinesSmallCtas>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, s5)
-                  : cudaFuncSetAttribute(hines_kernel<double, kHinesSmallCtas>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, s5);
+    // in a batch of the general variant both classes run it
+    auto pick = [&](int nc) {
+      if (!in_regs) nc = nc_max;
+      return rc == 4 ? hines_variant<float>(nc, one_per_sm) : hines_variant<double>(nc, one_per_sm);
+    };
+    h->var = pick(D.nc_max);
+    h->var_small = pick(n_large < n_neurons ? ncs : D.nc_max);
+    // the limit is a property of the kernel, shared by every batch that runs it: the device's
+    for (HinesKernel k : {h->var.kern, h->var_small.kern})
+      if (e == cudaSuccess)
+        e = cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 dev_smem);
     if (e != cudaSuccess) {
       b2b_hines_destroy(h);
       return e == cudaErrorMemoryAllocation ? B2B_ERR_OOM : B2B_ERR_CUDA;
@@ -676,23 +855,11 @@ b2b_status b2b_hines_run(b2b_hines* h, int64_t n_steps) {
       if (cudaEventRecord(h->ev_fork, s) != cudaSuccess) return B2B_ERR_CUDA;
       if (cudaStreamWaitEvent(h->stream2, h->ev_fork, 0) != cudaSuccess) return B2B_ERR_CUDA;
     }
-    if (h->channel_dtype == B2B_F32) {
-      if (h->n_large > 0 && h->large_fits5)
-        hines_kernel<float, kHinesSmallCtas><<<h->n_large, kHinesBlock, h->smem, s>>>(h->dev, k, wc);
-      else if (h->n_large > 0)
-        hines_kernel<float, kHinesLargeCtas><<<h->n_large, kHinesBlock, h->smem, s>>>(h->dev, k, wc);
-      if (two)
-        hines_kernel<float, kHinesSmallCtas><<<h->n_neurons - h->n_large, kHinesBlock, h->smem_small,
-                              h->stream2>>>(h->dev_small, k, wc);
-    } else {
-      if (h->n_large > 0 && h->large_fits5)
-        hines_kernel<double, kHinesSmallCtas><<<h->n_large, kHinesBlock, h->smem, s>>>(h->dev, k, wc);
-      else if (h->n_large > 0)
-        hines_kernel<double, kHinesLargeCtas><<<h->n_large, kHinesBlock, h->smem, s>>>(h->dev, k, wc);
-      if (two)
-        hines_kernel<double, kHinesSmallCtas><<<h->n_neurons - h->n_large, kHinesBlock, h->smem_small,
-                               h->stream2>>>(h->dev_small, k, wc);
-    }
+    if (h->n_large > 0)
+      h->var.kern<<<h->n_large, h->var.block, h->smem, s>>>(h->dev, k, wc);
+    if (two)
+      h->var_small.kern<<<h->n_neurons - h->n_large, h->var_small.block, h->smem_small,
+                          h->stream2>>>(h->dev_small, k, wc);
     if (cudaGetLastError() != cudaSuccess) return B2B_ERR_CUDA;
     if (two) {
       if (cudaEventRecord(h->ev_join, h->stream2) != cudaSuccess) return B2B_ERR_CUDA;
