@@ -946,6 +946,70 @@ b2b_status setup_two_launch(b2b_net* net) {
   return B2B_OK;
 }
 
+// The per-step form as one launch per step (neuron.cu, fused_step_kernel) applies to one LIF/HH
+// population without TimedArray or PoissonInput inputs, gating surrogate or state monitors,
+// whose synapses onto itself are all additive onto ge/gi, without delays or weights of their own
+// and with one weight per target variable.  Up to the size where the two counts read per
+// neuron stay a small part of the update.
+void setup_fused(b2b_net* net) {
+  net->fused_ok = false;
+  if (net->cfg.flags & B2B_NET_CHECKED) return;
+  if (!net->smons.empty() || net->pops.size() != 1 || net->projs.empty() ||
+      net->projs.size() > (size_t)kMaxProjBatch)
+    return;
+  const Pop& pop = net->pops[0];
+  if ((pop.kind != KIND_LIF && pop.kind != KIND_HH) || pop.surr_img || pop.inputs ||
+      pop.late_reset || pop.n > kAutoTwoLaunchMaxNeurons)
+    return;
+  FusedDev& F = net->fused;
+  PopDev& U = net->fused_pop;
+  U = pop.dev;
+  F.n_proj = (int32_t)net->projs.size();
+  bool seen[3] = {false, false, false};
+  int64_t longest = 1;
+  for (size_t p = 0; p < net->projs.size(); ++p) {
+    const Proj& pr = net->projs[p];
+    if (pr.effect != B2B_EFFECT_ADD || pr.dmin != 0 || pr.dmax != 0 || pr.dev.w != nullptr ||
+        pr.dev.aggregate || pr.src_pop != 0 || pr.dst_pop != 0 || pr.retire_after >= 0 ||
+        pr.dev.src_lo > net->ts)
+      return;
+    for (int m : pr.members) {
+      const Syn& sy = net->syns[m];
+      if (sy.target_var != B2B_VAR_GE && sy.target_var != B2B_VAR_GI) return;
+      if (seen[sy.target_var] && U.fold_w[sy.target_var] != sy.w_scalar) return;
+      seen[sy.target_var] = true;
+      U.fold_w[sy.target_var] = sy.w_scalar;
+    }
+    F.proj[p] = pr.dev;
+    F.var[p] = pr.target_var;
+    longest = std::max(longest, pr.max_bundle);
+  }
+  F.spread = (int32_t)std::min<int64_t>((longest + 31) / 32, 4);
+  for (int v = 0; v < 3; ++v) {
+    if (seen[v] && !F.cnt[v]) {
+      void* c = nullptr;
+      if (cudaMalloc(&c, 2 * sizeof(int32_t) * pop.n) != cudaSuccess ||
+          cudaMemset(c, 0, 2 * sizeof(int32_t) * pop.n) != cudaSuccess) {
+        cudaGetLastError();   // without the counts the two launches run
+        if (c) cudaFree(c);
+        return;
+      }
+      net->fused_allocs.push_back(c);
+      F.cnt[v] = static_cast<int32_t*>(c);
+    }
+    U.fold[v] = seen[v] ? F.cnt[v] : nullptr;
+  }
+  net->fused_ok = true;
+}
+
+// Whether the per-step form runs fused: a tuned delivery shape asks for the delivery's launch.
+bool fused_in_use(const b2b_net* net) {
+  if (!net->fused_ok || net->prof_ev) return false;
+  for (const AddTune& t : net->add_tune)
+    if (t.group > 0 || t.grid > 0 || t.cluster) return false;
+  return true;
+}
+
 // ---------------------------------------------------------------------------------------
 // Records profiling event `which` (0 before, 1 after) of launch site `site` of step k on s,
 // when b2b_profile_graph has set the net's event table; under stream capture the record is
@@ -1018,7 +1082,19 @@ b2b_status enqueue_steps(b2b_net* net, int kk) {
     return B2B_OK;
   }
   cudaStream_t s = net->stream;
+  const bool fused = fused_in_use(net);
   for (int k = 0; k < kk; ++k) {
+    if (fused) {
+      CU(launch_fused_step(net->pops[0], net->fused_pop, net->fused, net->d_clock, k,
+                           net->cfg.dt, net->d_status, s));
+      ++net->launches;
+      if (!net->rmons.empty()) {
+        CU(launch_ratemon(net->d_rmons, (int)net->rmons.size(), net->d_clock, k, net->d_status,
+                          s));
+        ++net->launches;
+      }
+      continue;
+    }
     int si = 0;   // profiling site, in the order of b2b_profile's site list
     if (!net->smons.empty()) {
       CU(prof_mark(net, k, si, 0, s));
@@ -1083,6 +1159,10 @@ b2b_status enqueue_steps(b2b_net* net, int kk) {
       CU(prof_mark(net, k, si++, 1, s));
       ++net->launches;
     }
+  }
+  if (fused) {
+    CU(launch_fold_counts(net->pops[0], net->fused_pop, kk - 1, s));
+    ++net->launches;
   }
   CU(launch_tick(net->d_clock, kk, s));
   ++net->launches;
@@ -1411,6 +1491,7 @@ b2b_status b2b_destroy(b2b_net* net) {
   for (Snapshot& sn : net->snapshots)
     for (void* a : sn.buffers) cudaFree(a);
   for (void* a : net->pending_allocs) cudaFree(a);
+  for (void* a : net->fused_allocs) cudaFree(a);
   if (net->pull_buf) cudaFree(net->pull_buf);
   if (net->fetch_pinned) cudaFreeHost(net->fetch_pinned);
   if (net->stream2) cudaStreamDestroy(net->stream2);
@@ -1844,6 +1925,7 @@ b2b_status b2b_finalize(b2b_net* net) {
   if (st == B2B_OK) st = setup_two_launch(net);
   if (st == B2B_OK) st = setup_small(net);
   if (st != B2B_OK) return st;
+  setup_fused(net);
   if (net->pops.size() > 1) {
     CU(cudaEventCreateWithFlags(&net->ev_pop_fork, cudaEventDisableTiming));
     for (size_t p = 1; p < net->pops.size(); ++p) {
@@ -3151,6 +3233,7 @@ b2b_status b2b_syn_set_delays(b2b_net* net, int32_t sid, const int32_t* delay_st
   }
   build_add_batches(net);
   refresh_two_launch(net);
+  setup_fused(net);
   return B2B_OK;
   GUARD_END
 }

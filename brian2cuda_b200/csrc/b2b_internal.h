@@ -114,6 +114,9 @@ struct PopDev {
   // The step as two concurrent launches (pending.cu): per variable (v, ge, gi), [2][n] input
   // delivered during the previous step, which the update adds in and clears (NULL: none).
   void* fold[3];
+  // The fused step (neuron.cu): fold holds int32 event counts instead, each count one addition
+  // of the variable's weight.
+  double fold_w[3];
 };
 
 // Device view of a projection (merged Synapses objects with one source population, one
@@ -203,6 +206,16 @@ struct PendingDev {
   void* acc[3];                   // per target variable (v, ge, gi): [2][pop.n] or NULL
   int32_t group;                  // delivery: lanes per work item (2, 4, 8 or 16)
   int32_t pad_group;
+};
+
+// Device view of the fused step's delivery (neuron.cu): additive projections of a population
+// onto its own ge/gi without delays or weights of their own, one weight per target variable.
+struct FusedDev {
+  ProjDev proj[kMaxProjBatch];
+  int32_t var[kMaxProjBatch];     // target variable of a projection with one member
+  int32_t n_proj;
+  int32_t spread;                 // warps that share one spike's bundle
+  int32_t* cnt[3];                // per target variable (v, ge, gi): [2][pop.n] or NULL
 };
 
 // Device view of the one-CTA path for small networks (small.cu): one LIF/HH population of at
@@ -401,6 +414,12 @@ struct b2b_net {
   bool one_launch_ok = false;
   int one_launch_grid = 0;
   bool one_launch_chained = false;         // programmatic dependent launch between steps
+  // the per-step form's update and delivery of a step as one launch (setup_fused); its
+  // population view holds the event counts
+  bool fused_ok = false;
+  b2b::FusedDev fused{};
+  b2b::PopDev fused_pop{};
+  std::vector<void*> fused_allocs;
   cudaStream_t stream2 = nullptr;
   // per-step form with several populations: populations 1.. update on streams of their own,
   // forked from and joined to the net's stream every step (the updates are independent)
@@ -480,4 +499,10 @@ cudaError_t launch_one_launch_step(const Pop& pop, const PopDev& U, const Pendin
                                    int deliver_ctas, bool chained, const int64_t* clock, int k,
                                    double dt, int32_t* status, cudaStream_t s);
 cudaError_t launch_fold_pending(const PendingDev& F, int dtype, int k_last, cudaStream_t s);
+// The fused step of a population (view U: its counts as fold buffers), and the addition of the
+// last step's counts at the end of a chunk.
+cudaError_t launch_fused_step(const Pop& pop, const PopDev& U, const FusedDev& F,
+                              const int64_t* clock, int k, double dt, int32_t* status,
+                              cudaStream_t s);
+cudaError_t launch_fold_counts(const Pop& pop, const PopDev& U, int k_last, cudaStream_t s);
 }  // namespace b2b

@@ -40,6 +40,37 @@ __device__ __forceinline__ R* fold_in(const PopDev& P, int v, int k, int64_t q,
   return a;
 }
 
+// The same from event counts (the fused step): count additions of the variable's weight one by
+// one, which rounds as the delivery's own additions would; nothing to clear where no event came.
+template <typename R, int E>
+__device__ __forceinline__ int32_t* fold_counts(const PopDev& P, int v, int k, int64_t q,
+                                                Pack<R, E>& X) {
+  if (!P.fold[v]) return nullptr;
+  int32_t* a = static_cast<int32_t*>(P.fold[v]) + (int64_t)((k & 1) ^ 1) * P.n + E * q;
+  const R w = (R)P.fold_w[v];
+  int32_t n[E];
+  if constexpr (E == 2) {
+    const int2 c = *reinterpret_cast<const int2*>(a);
+    n[0] = c.x;
+    n[1] = c.y;
+  } else {
+    n[0] = a[0];
+  }
+  int32_t any = 0;
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    any |= n[e];
+    for (int32_t c = n[e]; c > 0; --c) X.x[e] += w;
+  }
+  return any ? a : nullptr;
+}
+template <int E>
+__device__ __forceinline__ void clear_counts(int32_t* a) {
+  if (!a) return;
+#pragma unroll
+  for (int e = 0; e < E; ++e) a[e] = 0;
+}
+
 template <typename R, int E>
 __device__ __forceinline__ void fold_clear(R* a, int64_t q) {
   if (!a) return;
@@ -52,9 +83,12 @@ __device__ __forceinline__ void fold_clear(R* a, int64_t q) {
 // ---- LIF, exact integration ------------------------------------------------------------
 // INPUTS: the population has TimedArray or PoissonInput inputs (compiled out otherwise).
 // The work of CTA `blk` of the update (blockDim.x threads, E neurons each).
-template <typename R, int E, bool INPUTS>
+// FUSED: the step's delivery is part of it (fused_step_kernel): the input pending from the step
+// before comes as event counts, and the CTA's spikes go through emit(q, fl, ts, slot).
+template <typename R, int E, bool INPUTS, bool FUSED = false, class Emit = int>
 __device__ __forceinline__ void lif_step_body(const PopDev& P, const int64_t* __restrict__ clock,
-                                              int k, double dt, int32_t* status, int64_t blk) {
+                                              int k, double dt, int32_t* status, int64_t blk,
+                                              Emit emit = 0) {
   const int64_t ts = clock[0] + k;
   const double t = (double)ts * dt;
   const double inv_dt = 1.0 / dt;
@@ -75,8 +109,15 @@ __device__ __forceinline__ void lif_step_body(const PopDev& P, const int64_t* __
     Pack<R, E> GI = load_pack<R, E>(P.var[B2B_VAR_GI], q);
     Pack<R, E> LS;
     if (refr) LS = load_pack<R, E>(P.var[B2B_VAR_LASTSPIKE], q);
-    R* fge = fold_in<R, E>(P, B2B_VAR_GE, k, q, GE);
-    R* fgi = fold_in<R, E>(P, B2B_VAR_GI, k, q, GI);
+    R *fge = nullptr, *fgi = nullptr;
+    int32_t *cge = nullptr, *cgi = nullptr;
+    if constexpr (FUSED) {
+      cge = fold_counts<R, E>(P, B2B_VAR_GE, k, q, GE);
+      cgi = fold_counts<R, E>(P, B2B_VAR_GI, k, q, GI);
+    } else {
+      fge = fold_in<R, E>(P, B2B_VAR_GE, k, q, GE);
+      fgi = fold_in<R, E>(P, B2B_VAR_GI, k, q, GI);
+    }
     uint32_t NRout = 0;
 #pragma unroll
     for (int e = 0; e < E; ++e) {
@@ -112,10 +153,16 @@ __device__ __forceinline__ void lif_step_body(const PopDev& P, const int64_t* __
       if (fl) store_pack<R, E>(P.var[B2B_VAR_LASTSPIKE], q, LS);   // changes only on a spike
       store_flags<E>(P.var[B2B_VAR_NOT_REFRACTORY], q, NRout);
     }
-    fold_clear<R, E>(fge, q);
-    fold_clear<R, E>(fgi, q);
+    if constexpr (FUSED) {
+      clear_counts<E>(cge);
+      clear_counts<E>(cgi);
+    } else {
+      fold_clear<R, E>(fge, q);
+      fold_clear<R, E>(fgi, q);
+    }
   }
-  emit_spikes<E>(P, q, fl, ts, slot, status);
+  if constexpr (FUSED) emit(q, fl, ts, slot);
+  else emit_spikes<E>(P, q, fl, ts, slot, status);
   clear_next_slot(P, ts, blk);
 }
 
@@ -127,9 +174,10 @@ lif_step_kernel(PopDev P, const int64_t* __restrict__ clock, int k, double dt,
 }
 
 // ---- Hodgkin-Huxley (COBAHH), exponential Euler (hh_advance) ------------------------
-template <typename R, int E, bool INPUTS>
+template <typename R, int E, bool INPUTS, bool FUSED = false, class Emit = int>
 __device__ __forceinline__ void hh_step_body(const PopDev& P, const int64_t* __restrict__ clock,
-                                             int k, double dt, int32_t* status, int64_t blk) {
+                                             int k, double dt, int32_t* status, int64_t blk,
+                                             Emit emit = 0) {
   const int64_t ts = clock[0] + k;
   const double t = (double)ts * dt;
   const double inv_dt = 1.0 / dt;
@@ -152,8 +200,15 @@ __device__ __forceinline__ void hh_step_body(const PopDev& P, const int64_t* __r
     Pack<R, E> GI = load_pack<R, E>(P.var[B2B_VAR_GI], q);
     Pack<R, E> LS;
     if (refr) LS = load_pack<R, E>(P.var[B2B_VAR_LASTSPIKE], q);
-    R* fge = fold_in<R, E>(P, B2B_VAR_GE, k, q, GE);
-    R* fgi = fold_in<R, E>(P, B2B_VAR_GI, k, q, GI);
+    R *fge = nullptr, *fgi = nullptr;
+    int32_t *cge = nullptr, *cgi = nullptr;
+    if constexpr (FUSED) {
+      cge = fold_counts<R, E>(P, B2B_VAR_GE, k, q, GE);
+      cgi = fold_counts<R, E>(P, B2B_VAR_GI, k, q, GI);
+    } else {
+      fge = fold_in<R, E>(P, B2B_VAR_GE, k, q, GE);
+      fgi = fold_in<R, E>(P, B2B_VAR_GI, k, q, GI);
+    }
     uint32_t NRout = 0;
 #pragma unroll
     for (int e = 0; e < E; ++e) {
@@ -183,10 +238,16 @@ __device__ __forceinline__ void hh_step_body(const PopDev& P, const int64_t* __r
       if (fl) store_pack<R, E>(P.var[B2B_VAR_LASTSPIKE], q, LS);   // changes only on a spike
       store_flags<E>(P.var[B2B_VAR_NOT_REFRACTORY], q, NRout);
     }
-    fold_clear<R, E>(fge, q);
-    fold_clear<R, E>(fgi, q);
+    if constexpr (FUSED) {
+      clear_counts<E>(cge);
+      clear_counts<E>(cgi);
+    } else {
+      fold_clear<R, E>(fge, q);
+      fold_clear<R, E>(fgi, q);
+    }
   }
-  emit_spikes<E>(P, q, fl, ts, slot, status);
+  if constexpr (FUSED) emit(q, fl, ts, slot);
+  else emit_spikes<E>(P, q, fl, ts, slot, status);
   clear_next_slot(P, ts, blk);
 }
 
@@ -263,6 +324,69 @@ cudaError_t launch_one_k(const PopDev& U, const PendingDev& F, bool f32, unsigne
                                             n_upd, s)
              : launch_one_r<double, KIND, E>(U, F, grid, block, chained, clock, k, dt, status,
                                              n_upd, s);
+}
+
+// ---- update and delivery of a step without delays as one launch ------------------------
+// Synapses without delays deliver the step's own spikes, so the per-step form runs the update
+// and then a delivery launch that waits for it.  Where a variable's events all carry one
+// weight, counting them separates the two: a CTA that finds spikes among its neurons adds 1 to
+// the targets' counts for this step (row k & 1) as soon as it has updated them, whether the
+// targets' own CTAs have updated theirs or not, and the update of the next step adds the weight
+// count times before it integrates.  The additions and their order per target are those of the
+// two launches, so the state is the same bit for bit.  Between chunks the last step's counts are
+// added in (fold_counts_kernel).  CUBA 4000, float64: 5.5 -> @FUSED@ us per step.
+template <typename R, int KIND, int E>
+__global__ void __launch_bounds__(kBlock)
+fused_step_kernel(const __grid_constant__ PopDev U, const __grid_constant__ FusedDev F,
+                  const int64_t* __restrict__ clock, int k, double dt, int32_t* status) {
+  __shared__ int32_t s_list[kBlock * E];
+  auto deliver = [&](int total) {
+    const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+    const int64_t row = (int64_t)(k & 1) * U.n;
+    for (int p = 0; p < F.n_proj; ++p) {
+      const ProjDev& J = F.proj[p];
+      for (int it = threadIdx.x >> 5; it < total * F.spread; it += warps) {
+        const int x = it / F.spread, part = it - x * F.spread;
+        const int32_t pre = s_list[x];
+        const int64_t b0 = __ldg(J.off + pre), b1 = __ldg(J.off + pre + 1);
+        if (b0 == b1) continue;
+        int32_t* c = F.cnt[J.n_mem > 1 ? J.mem_var[member_of(J, pre)] : F.var[p]] + row;
+        for (int64_t s = b0 + 32 * part + lane; s < b1; s += 32 * F.spread)
+          atomicAdd(c + __ldg(J.post + s), 1);
+      }
+    }
+  };
+  auto emit = [&](int64_t q, unsigned fl, int64_t ts, int slot) {
+    emit_spikes_use<E>(U, q, fl, ts, slot, status, s_list, deliver);
+  };
+  if constexpr (KIND == KIND_HH)
+    hh_step_body<R, E, false, true>(U, clock, k, dt, status, blockIdx.x, emit);
+  else
+    lif_step_body<R, E, false, true>(U, clock, k, dt, status, blockIdx.x, emit);
+}
+
+// Adds the counts of the chunk's last step (row `row`) into the target variables.
+template <typename R>
+__global__ void fold_counts_kernel(const __grid_constant__ PopDev U, int row) {
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int v = B2B_VAR_GE; v <= B2B_VAR_GI; ++v) {
+    if (!U.fold[v]) continue;
+    R* X = static_cast<R*>(U.var[v]);
+    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < U.n; q += stride) {
+      Pack<R, 1> x{{X[q]}};
+      if (int32_t* a = fold_counts<R, 1>(U, v, row ^ 1, q, x)) {
+        X[q] = x.x[0];
+        a[0] = 0;
+      }
+    }
+  }
+}
+
+template <typename R, int KIND>
+void launch_fused_rk(const PopDev& U, const FusedDev& F, int e, unsigned grid, int block,
+                     const int64_t* clock, int k, double dt, int32_t* status, cudaStream_t s) {
+  if (e == 2) fused_step_kernel<R, KIND, 2><<<grid, block, 0, s>>>(U, F, clock, k, dt, status);
+  else fused_step_kernel<R, KIND, 1><<<grid, block, 0, s>>>(U, F, clock, k, dt, status);
 }
 
 // Large HH populations: a persistent grid (resident CTAs only) walks the population in
@@ -568,6 +692,31 @@ cudaError_t launch_one_launch_step(const Pop& pop, const PopDev& U, const Pendin
                                             status, n_upd, s)
                 : launch_one_k<KIND_LIF, 1>(U, F, f32, grid, block, chained, clock, k, dt,
                                             status, n_upd, s);
+}
+
+cudaError_t launch_fused_step(const Pop& pop, const PopDev& U, const FusedDev& F,
+                              const int64_t* clock, int k, double dt, int32_t* status,
+                              cudaStream_t s) {
+  const UpdateShape shape = update_shape(pop, U.n);
+  const int e = shape.e >= 2 ? 2 : 1, block = shape.block;
+  const unsigned grid = (unsigned)((U.n / e + block - 1) / block);
+  const bool f32 = pop.dtype == B2B_F32;
+  if (pop.kind == KIND_HH) {
+    if (f32) launch_fused_rk<float, KIND_HH>(U, F, e, grid, block, clock, k, dt, status, s);
+    else launch_fused_rk<double, KIND_HH>(U, F, e, grid, block, clock, k, dt, status, s);
+  } else {
+    if (f32) launch_fused_rk<float, KIND_LIF>(U, F, e, grid, block, clock, k, dt, status, s);
+    else launch_fused_rk<double, KIND_LIF>(U, F, e, grid, block, clock, k, dt, status, s);
+  }
+  return cudaGetLastError();
+}
+
+cudaError_t launch_fold_counts(const Pop& pop, const PopDev& U, int k_last, cudaStream_t s) {
+  const unsigned grid =
+      (unsigned)std::min<int64_t>((U.n + kBlock - 1) / kBlock, 4 * kNumSMs);
+  if (pop.dtype == B2B_F32) fold_counts_kernel<float><<<grid, kBlock, 0, s>>>(U, k_last & 1);
+  else fold_counts_kernel<double><<<grid, kBlock, 0, s>>>(U, k_last & 1);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_pop_late_reset(const Pop& pop, const int64_t* clock, int k, cudaStream_t s) {

@@ -107,6 +107,54 @@ __device__ __forceinline__ void emit_spikes(const PopDev& P, int64_t q, unsigned
   }
 }
 
+// emit_spikes of a CTA that also uses its spikes itself: they are listed in s_list (blockDim.x * E
+// entries), use(total) is called by the whole CTA while the reservation in the ring slot and the
+// monitor is under way, and the record is written after it.  Every thread of the CTA must call
+// this.
+template <int E, class Use>
+__device__ __forceinline__ void emit_spikes_use(const PopDev& P, int64_t q, unsigned fl,
+                                                int64_t ts, int slot, int32_t* status,
+                                                int32_t* s_list, Use use) {
+  __shared__ int s_warp[33];
+  __shared__ int s_base;
+  __shared__ unsigned long long s_mbase;
+  if (!__syncthreads_or(fl != 0)) return;
+  int total;
+  const int c = __popc(fl);
+  const int excl = block_exclusive_scan(c, s_warp, &total);
+  int base = 0;
+  unsigned long long mbase = 0;
+  if (threadIdx.x == 0) {
+    base = atomicAdd(&P.ring_cnt[slot], total);
+    if (P.mon_cnt) mbase = atomicAdd(P.mon_cnt, (unsigned long long)total);
+  }
+  int pos = excl;
+#pragma unroll
+  for (int e = 0; e < E; ++e)
+    if (fl & (1u << e)) s_list[pos++] = (int32_t)(E * q + e);
+  __syncthreads();
+  use(total);
+  if (threadIdx.x == 0) {
+    s_base = base;
+    s_mbase = mbase;
+  }
+  __syncthreads();
+  int32_t* out = P.ring_idx + (int64_t)slot * P.n + s_base;
+  for (int x = threadIdx.x; x < total; x += blockDim.x) {
+    const int32_t idx = s_list[x];
+    out[x] = idx;
+    if (P.mon_cnt) {
+      const unsigned long long mpos = s_mbase + (unsigned long long)x;
+      if (mpos < (unsigned long long)P.mon_cap) {
+        P.mon_idx[mpos] = idx;
+        P.mon_step[mpos] = ts;
+      } else {
+        set_status(status, B2B_ERR_QUEUE_OVERFLOW);
+      }
+    }
+  }
+}
+
 // emit_spikes for kernels that call it in a loop (hh_stream_kernel): every lane of a warp
 // must call this, which synchronises the warp, not the block, so the warps of a CTA are not
 // held in step once per iteration.  A warp with spikes reserves its range in the slot (and
