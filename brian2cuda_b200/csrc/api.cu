@@ -981,7 +981,13 @@ void setup_fused(b2b_net* net) {
       U.fold_w[sy.target_var] = sy.w_scalar;
     }
     F.proj[p] = pr.dev;
-    F.var[p] = pr.target_var;
+    F.var[p][0] = pr.target_var;
+    if (pr.dev.n_mem > 1)
+      for (size_t m = 0; m < pr.members.size() && m < (size_t)kFusedMembers; ++m) {
+        const Syn& sy = net->syns[pr.members[m]];
+        F.hi[p][m] = net->groups[sy.pre_gid].offset + sy.pre_hi;
+        F.var[p][m] = sy.target_var;
+      }
     longest = std::max(longest, pr.max_bundle);
   }
   F.spread = (int32_t)std::min<int64_t>((longest + 31) / 32, 4);

@@ -210,9 +210,13 @@ struct PendingDev {
 
 // Device view of the fused step's delivery (neuron.cu): additive projections of a population
 // onto its own ge/gi without delays or weights of their own, one weight per target variable.
+constexpr int kFusedMembers = 4;   // members whose table travels in the launch's parameters
 struct FusedDev {
   ProjDev proj[kMaxProjBatch];
-  int32_t var[kMaxProjBatch];     // target variable of a projection with one member
+  // per projection, member m: presynaptic indices below hi[m], target variable var[m]; with more
+  // than kFusedMembers members (n_mem of the projection) they are looked up in its own tables
+  int64_t hi[kMaxProjBatch][kFusedMembers];
+  int32_t var[kMaxProjBatch][kFusedMembers];
   int32_t n_proj;
   int32_t spread;                 // warps that share one spike's bundle
   int32_t* cnt[3];                // per target variable (v, ge, gi): [2][pop.n] or NULL

@@ -334,12 +334,20 @@ cudaError_t launch_one_k(const PopDev& U, const PendingDev& F, bool f32, unsigne
 // targets' own CTAs have updated theirs or not, and the update of the next step adds the weight
 // count times before it integrates.  The additions and their order per target are those of the
 // two launches, so the state is the same bit for bit.  Between chunks the last step's counts are
-// added in (fold_counts_kernel).  CUBA 4000, float64: 5.5 -> @FUSED@ us per step.
+// added in (fold_counts_kernel).  CUBA 4000, float64: 5.5 -> 3.8 us per step (4.0 with the
+// bundle bounds and member tables loaded after the spike).
 template <typename R, int KIND, int E>
 __global__ void __launch_bounds__(kBlock)
 fused_step_kernel(const __grid_constant__ PopDev U, const __grid_constant__ FusedDev F,
                   const int64_t* __restrict__ clock, int k, double dt, int32_t* status) {
   __shared__ int32_t s_list[kBlock * E];
+  // the bundle bounds of the CTA's own neurons are loaded with their state and kept for those
+  // that spike, so that a delivery starts at its targets
+  __shared__ int64_t s_b0[kBlock * E], s_b1[kBlock * E];
+  const int64_t q0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  int64_t off[E + 1];
+#pragma unroll
+  for (int e = 0; e <= E; ++e) off[e] = q0 < U.n / E ? __ldg(F.proj[0].off + E * q0 + e) : 0;
   auto deliver = [&](int total) {
     const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
     const int64_t row = (int64_t)(k & 1) * U.n;
@@ -348,16 +356,28 @@ fused_step_kernel(const __grid_constant__ PopDev U, const __grid_constant__ Fuse
       for (int it = threadIdx.x >> 5; it < total * F.spread; it += warps) {
         const int x = it / F.spread, part = it - x * F.spread;
         const int32_t pre = s_list[x];
-        const int64_t b0 = __ldg(J.off + pre), b1 = __ldg(J.off + pre + 1);
+        const int64_t b0 = p == 0 ? s_b0[x] : __ldg(J.off + pre);
+        const int64_t b1 = p == 0 ? s_b1[x] : __ldg(J.off + pre + 1);
         if (b0 == b1) continue;
-        int32_t* c = F.cnt[J.n_mem > 1 ? J.mem_var[member_of(J, pre)] : F.var[p]] + row;
+        int var = F.var[p][0];
+        if (J.n_mem > kFusedMembers) {
+          var = J.mem_var[member_of(J, pre)];
+        } else {
+#pragma unroll
+          for (int m = 1; m < kFusedMembers; ++m)
+            if (m < J.n_mem && pre >= F.hi[p][m - 1]) var = F.var[p][m];
+        }
+        int32_t* c = F.cnt[var] + row;
         for (int64_t s = b0 + 32 * part + lane; s < b1; s += 32 * F.spread)
           atomicAdd(c + __ldg(J.post + s), 1);
       }
     }
   };
   auto emit = [&](int64_t q, unsigned fl, int64_t ts, int slot) {
-    emit_spikes_use<E>(U, q, fl, ts, slot, status, s_list, deliver);
+    emit_spikes_use<E>(U, q, fl, ts, slot, status, s_list, [&](int e, int pos) {
+      s_b0[pos] = off[e];
+      s_b1[pos] = off[e + 1];
+    }, deliver);
   };
   if constexpr (KIND == KIND_HH)
     hh_step_body<R, E, false, true>(U, clock, k, dt, status, blockIdx.x, emit);

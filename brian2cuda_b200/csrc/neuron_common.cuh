@@ -108,13 +108,13 @@ __device__ __forceinline__ void emit_spikes(const PopDev& P, int64_t q, unsigned
 }
 
 // emit_spikes of a CTA that also uses its spikes itself: they are listed in s_list (blockDim.x * E
-// entries), use(total) is called by the whole CTA while the reservation in the ring slot and the
+// entries; keep(e, place) is called for the thread's neuron e), use(total) is called by the whole CTA while the reservation in the ring slot and the
 // monitor is under way, and the record is written after it.  Every thread of the CTA must call
 // this.
-template <int E, class Use>
+template <int E, class Keep, class Use>
 __device__ __forceinline__ void emit_spikes_use(const PopDev& P, int64_t q, unsigned fl,
                                                 int64_t ts, int slot, int32_t* status,
-                                                int32_t* s_list, Use use) {
+                                                int32_t* s_list, Keep keep, Use use) {
   __shared__ int s_warp[33];
   __shared__ int s_base;
   __shared__ unsigned long long s_mbase;
@@ -131,7 +131,10 @@ __device__ __forceinline__ void emit_spikes_use(const PopDev& P, int64_t q, unsi
   int pos = excl;
 #pragma unroll
   for (int e = 0; e < E; ++e)
-    if (fl & (1u << e)) s_list[pos++] = (int32_t)(E * q + e);
+    if (fl & (1u << e)) {
+      s_list[pos] = (int32_t)(E * q + e);
+      keep(e, pos++);
+    }
   __syncthreads();
   use(total);
   if (threadIdx.x == 0) {

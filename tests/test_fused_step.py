@@ -95,3 +95,29 @@ def test_fused_step_around_profiles_snapshots_and_delays(gpu_factory):
     for v in out[True][0]:
         np.testing.assert_array_equal(out[True][0][v], out[True][1][v], err_msg=v)
     np.testing.assert_array_equal(out[False][3][0], out[True][3][0])
+
+
+def test_fused_step_with_many_synapses_objects(gpu_factory):
+    """More members than the launch's parameters hold, and two projections (overlapping source
+    ranges do not merge)."""
+    out = {}
+    for checked in (False, True):
+        net = gpu_factory(DT, checked=checked)
+        rng = np.random.default_rng(8)
+        n = 900
+        P = net.lif_group(n, models.cuba_lif(), "float64")
+        net.set_state(P, "v", rng.uniform(-60e-3, -50e-3, n))
+        for lo in range(0, n, 150):            # six objects of one projection
+            i, j = rng.integers(lo, lo + 150, 4000), rng.integers(0, n, 4000)
+            exc = lo < 600
+            net.synapses(P, P, "ge" if exc else "gi", i, j, w_scalar=1.62e-3 if exc else -9e-3)
+        net.synapses(P, P, "ge", rng.integers(0, n, 9000), rng.integers(0, n, 9000),
+                     w_scalar=1.62e-3)         # from every neuron: a projection of its own
+        net.spike_monitor(P, 10**5)
+        net.finalize()
+        net.run(120)
+        out[checked] = (net.spikes(P), _state(net, P, "lif"))
+    assert len(out[True][0][0]) > 0
+    np.testing.assert_array_equal(out[False][0][0], out[True][0][0])
+    for v in out[True][1]:
+        np.testing.assert_array_equal(out[False][1][v], out[True][1][v], err_msg=v)
