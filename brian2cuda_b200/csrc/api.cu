@@ -807,6 +807,152 @@ b2b_status setup_monitors(b2b_net* net) {
 // cluster: one LIF/HH population of at most 4096 neurons (no gating surrogate) whose
 // Synapses objects are all additive and target it, with the state fitting the CTA's shared
 // memory.  B2B_NET_SMALL selects the path; otherwise b2b_autotune may (site kind 14).
+// The pull form's connectivity split by the slices of sdev (cluster and slice set): for each
+// rank, offsets by presynaptic neuron and slice-local targets, uploaded to the device; false
+// when a slice's targets do not fit a CTA's shared memory.
+bool build_pull_slices(b2b_net* net) {
+  SmallDev& D = net->sdev;
+  const int64_t n = net->pops[0].n, S = D.slice;
+  const int C = D.cluster;
+  const int P = (int)net->projs.size();
+  std::vector<int32_t> hoff((size_t)P * C * (n + 1));
+  std::vector<int64_t> base((size_t)P * (C + 1), 0);
+  std::vector<int64_t> per_rank(C, 0);
+  for (int p = 0; p < P; ++p) {
+    const std::vector<int64_t>& off = net->pull_host_off[p];
+    const std::vector<int32_t>& post = net->pull_host_post[p];
+    std::vector<int64_t> cnt((size_t)C * (n + 1), 0);
+    for (int64_t pre = 0; pre < n; ++pre)
+      for (int64_t s = off[pre]; s < off[pre + 1]; ++s)
+        ++cnt[(size_t)(post[s] / S) * (n + 1) + pre];
+    for (int r = 0; r < C; ++r) {
+      int64_t acc = 0;
+      int32_t* o = hoff.data() + ((size_t)p * C + r) * (n + 1);
+      for (int64_t pre = 0; pre < n; ++pre) {
+        o[pre] = (int32_t)acc;
+        acc += cnt[(size_t)r * (n + 1) + pre];
+      }
+      o[n] = (int32_t)acc;
+      base[(size_t)p * (C + 1) + r + 1] = base[(size_t)p * (C + 1) + r] + acc;
+      per_rank[r] += acc;
+    }
+  }
+  // targets: projection-major, then rank, then presynaptic neuron
+  std::vector<int64_t> pstart(P + 1, 0);
+  for (int p = 0; p < P; ++p) pstart[p + 1] = pstart[p] + base[(size_t)p * (C + 1) + C];
+  std::vector<uint16_t> htgt((size_t)std::max<int64_t>(pstart[P], 1));
+  for (int p = 0; p < P; ++p) {
+    const std::vector<int64_t>& off = net->pull_host_off[p];
+    const std::vector<int32_t>& post = net->pull_host_post[p];
+    std::vector<int32_t> fill((size_t)C * (n + 1), 0);
+    for (int64_t pre = 0; pre < n; ++pre)
+      for (int64_t s = off[pre]; s < off[pre + 1]; ++s) {
+        const int r = (int)(post[s] / S);
+        const size_t at = (size_t)(pstart[p] + base[(size_t)p * (C + 1) + r] +
+                                   hoff[((size_t)p * C + r) * (n + 1) + pre] +
+                                   fill[(size_t)r * (n + 1) + pre]++);
+        htgt[at] = (uint16_t)(post[s] - (int64_t)r * S);
+      }
+    for (int r = 0; r <= C; ++r) base[(size_t)p * (C + 1) + r] += pstart[p];   // absolute
+  }
+  D.pull_max_tgt = (int32_t)*std::max_element(per_rank.begin(), per_rank.end());
+  int optin = 0;
+  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, net->cfg.device);
+  const size_t need = small_cluster_smem(D, net->pops[0].kind, net->pops[0].dtype);
+  if (optin > 0 && need > (size_t)optin - 4096) return false;
+  const size_t bb = sizeof(int64_t) * base.size(), ob = sizeof(int32_t) * hoff.size();
+  const size_t tb = sizeof(uint16_t) * htgt.size();
+  void* buf = nullptr;
+  if (cudaMalloc(&buf, bb + ob + tb) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  uint8_t* b8 = static_cast<uint8_t*>(buf);
+  if (cudaMemcpy(b8, base.data(), bb, cudaMemcpyHostToDevice) != cudaSuccess ||
+      cudaMemcpy(b8 + bb, hoff.data(), ob, cudaMemcpyHostToDevice) != cudaSuccess ||
+      cudaMemcpy(b8 + bb + ob, htgt.data(), tb, cudaMemcpyHostToDevice) != cudaSuccess) {
+    cudaFree(buf);
+    return false;
+  }
+  if (net->pull_buf) cudaFree(net->pull_buf);
+  net->pull_buf = buf;
+  D.pull_base = reinterpret_cast<const int64_t*>(b8);
+  D.pull_off = reinterpret_cast<const int32_t*>(b8 + bb);
+  D.pull_tgt = reinterpret_cast<const uint16_t*>(b8 + bb + ob);
+  return true;
+}
+
+// Turns the one-CTA form into small_lif_kernel where it applies: a LIF population whose synapses
+// have no delays or weights of their own and add into ge/gi only; the connectivity in shared
+// memory where it fits.
+void set_small_lif(b2b_net* net) {
+  SmallDev& D = net->sdev;
+  const Pop& pop = net->pops[0];
+  D.lif_regs = 0;
+  if (!net->pull_ok || pop.kind != KIND_LIF || pop.late_reset || D.n_proj == 0) return;
+  int64_t longest = 1;
+  for (const Proj& pr : net->projs) {
+    if (pr.dev.n_mem > 16) return;                // the kernel's member tables
+    for (int m : pr.members)
+      if (net->syns[m].target_var == B2B_VAR_V) return;
+    longest = std::max(longest, pr.max_bundle);
+  }
+  int optin = 0;
+  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, net->cfg.device);
+  if (optin > 0 && !small_lif_fits(D, pop.dtype, false, (size_t)optin)) return;
+  D.total_syn = 0;
+  for (const Proj& pr : net->projs) D.total_syn += pr.n_syn;
+  D.local = optin > 0 && small_lif_fits(D, pop.dtype, true, (size_t)optin) ? 1 : 0;
+  D.spread = (int32_t)std::min<int64_t>((longest + 31) / 32, 8);
+  D.lif_regs = 1;
+}
+
+// The small-network path as one CTA (c == 1) or one cluster of c CTAs, each holding a slice
+// of the population, pushing the effects or (pull) gathering them at the targets; false
+// (nothing changed) when that form cannot run the net.
+bool set_small_cluster(b2b_net* net, int c, bool pull) {
+  SmallDev& D = net->sdev;
+  const Pop& pop = net->pops[0];
+  const int32_t c0 = D.cluster, p0 = D.pull;
+  const int64_t s0 = D.slice;
+  // the connectivity of the form that stays, which the refused one's may have replaced
+  auto restore_form = [&]() {
+    if (c0 == 1) set_small_lif(net);
+    else if (p0) build_pull_slices(net);
+  };
+  D.lif_regs = 0;
+  if (c == 1 && !pull) {
+    D.cluster = 1;
+    D.pull = 0;
+    D.slice = pop.n;
+    set_small_lif(net);
+  } else {
+    if ((c != 8 && c != 16) || (pull && !net->pull_ok)) return false;
+    D.cluster = c;
+    D.pull = pull ? 1 : 0;
+    D.slice = ((pop.n + c - 1) / c + 3) / 4 * 4;
+    if (pull && !build_pull_slices(net)) {
+      D.cluster = c0;
+      D.pull = p0;
+      D.slice = s0;
+      restore_form();
+      return false;
+    }
+    if (!small_cluster_possible(D, pop.kind, pop.dtype)) {
+      D.cluster = c0;
+      D.pull = p0;
+      D.slice = s0;
+      restore_form();
+      return false;
+    }
+  }
+  if (net->graph) {
+    cudaGraphExecDestroy(net->graph);
+    net->graph = nullptr;
+  }
+  return true;
+}
+
 b2b_status setup_small(b2b_net* net) {
   const int32_t flags = net->cfg.flags;
   if (flags & (B2B_NET_CHECKED | B2B_NET_TWO_LAUNCH | B2B_NET_ONE_LAUNCH)) return B2B_OK;
@@ -863,6 +1009,7 @@ b2b_status setup_small(b2b_net* net) {
   }
   net->small_ok = true;
   net->small = (flags & B2B_NET_SMALL) != 0;
+  if (net->small) set_small_cluster(net, 1, false);
   return B2B_OK;
 }
 
@@ -1957,10 +2104,13 @@ b2b_status b2b_run(b2b_net* net, int64_t n_steps) {
   const int K = net->cfg.steps_per_graph;
   const bool use_graph = !(net->cfg.flags & B2B_NET_NO_GRAPH);
   if (b2b_status st = drop_retired(net)) return st;
+  // one launch of the small-network path may hold many chunks' steps (its nets draw no random
+  // numbers)
+  const int longest = net->small ? small_max_steps(net->sdev) : 0;
   while (n_steps > 0) {
-    const int kk = (int)std::min<int64_t>(n_steps, K);
+    const int kk = (int)std::min<int64_t>(n_steps, std::max(K, longest));
     if (b2b_status st = refill_rng(net, kk)) return st;
-    if (use_graph && kk == K) {
+    if (use_graph && kk == K && longest <= K) {
       if (!net->graph) {
         if (b2b_status st = capture_graph(net)) return st;
       }
@@ -2156,118 +2306,6 @@ b2b_status b2b_profile_graph(b2b_net* net, int64_t n_steps, double* mean_ms,
 namespace {
 
 constexpr double kTuneMargin = 0.98;
-
-// The pull form's connectivity split by the slices of sdev (cluster and slice set): for each
-// rank, offsets by presynaptic neuron and slice-local targets, uploaded to the device; false
-// when a slice's targets do not fit a CTA's shared memory.
-bool build_pull_slices(b2b_net* net) {
-  SmallDev& D = net->sdev;
-  const int64_t n = net->pops[0].n, S = D.slice;
-  const int C = D.cluster;
-  const int P = (int)net->projs.size();
-  std::vector<int32_t> hoff((size_t)P * C * (n + 1));
-  std::vector<int64_t> base((size_t)P * (C + 1), 0);
-  std::vector<int64_t> per_rank(C, 0);
-  for (int p = 0; p < P; ++p) {
-    const std::vector<int64_t>& off = net->pull_host_off[p];
-    const std::vector<int32_t>& post = net->pull_host_post[p];
-    std::vector<int64_t> cnt((size_t)C * (n + 1), 0);
-    for (int64_t pre = 0; pre < n; ++pre)
-      for (int64_t s = off[pre]; s < off[pre + 1]; ++s)
-        ++cnt[(size_t)(post[s] / S) * (n + 1) + pre];
-    for (int r = 0; r < C; ++r) {
-      int64_t acc = 0;
-      int32_t* o = hoff.data() + ((size_t)p * C + r) * (n + 1);
-      for (int64_t pre = 0; pre < n; ++pre) {
-        o[pre] = (int32_t)acc;
-        acc += cnt[(size_t)r * (n + 1) + pre];
-      }
-      o[n] = (int32_t)acc;
-      base[(size_t)p * (C + 1) + r + 1] = base[(size_t)p * (C + 1) + r] + acc;
-      per_rank[r] += acc;
-    }
-  }
-  // targets: projection-major, then rank, then presynaptic neuron
-  std::vector<int64_t> pstart(P + 1, 0);
-  for (int p = 0; p < P; ++p) pstart[p + 1] = pstart[p] + base[(size_t)p * (C + 1) + C];
-  std::vector<uint16_t> htgt((size_t)std::max<int64_t>(pstart[P], 1));
-  for (int p = 0; p < P; ++p) {
-    const std::vector<int64_t>& off = net->pull_host_off[p];
-    const std::vector<int32_t>& post = net->pull_host_post[p];
-    std::vector<int32_t> fill((size_t)C * (n + 1), 0);
-    for (int64_t pre = 0; pre < n; ++pre)
-      for (int64_t s = off[pre]; s < off[pre + 1]; ++s) {
-        const int r = (int)(post[s] / S);
-        const size_t at = (size_t)(pstart[p] + base[(size_t)p * (C + 1) + r] +
-                                   hoff[((size_t)p * C + r) * (n + 1) + pre] +
-                                   fill[(size_t)r * (n + 1) + pre]++);
-        htgt[at] = (uint16_t)(post[s] - (int64_t)r * S);
-      }
-    for (int r = 0; r <= C; ++r) base[(size_t)p * (C + 1) + r] += pstart[p];   // absolute
-  }
-  D.pull_max_tgt = (int32_t)*std::max_element(per_rank.begin(), per_rank.end());
-  const size_t need = small_cluster_smem(D, net->pops[0].kind, net->pops[0].dtype);
-  int optin = 0;
-  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, net->cfg.device);
-  if (optin > 0 && need > (size_t)optin - 4096) return false;
-  const size_t bb = sizeof(int64_t) * base.size(), ob = sizeof(int32_t) * hoff.size();
-  const size_t tb = sizeof(uint16_t) * htgt.size();
-  void* buf = nullptr;
-  if (cudaMalloc(&buf, bb + ob + tb) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
-  uint8_t* b8 = static_cast<uint8_t*>(buf);
-  if (cudaMemcpy(b8, base.data(), bb, cudaMemcpyHostToDevice) != cudaSuccess ||
-      cudaMemcpy(b8 + bb, hoff.data(), ob, cudaMemcpyHostToDevice) != cudaSuccess ||
-      cudaMemcpy(b8 + bb + ob, htgt.data(), tb, cudaMemcpyHostToDevice) != cudaSuccess) {
-    cudaFree(buf);
-    return false;
-  }
-  if (net->pull_buf) cudaFree(net->pull_buf);
-  net->pull_buf = buf;
-  D.pull_base = reinterpret_cast<const int64_t*>(b8);
-  D.pull_off = reinterpret_cast<const int32_t*>(b8 + bb);
-  D.pull_tgt = reinterpret_cast<const uint16_t*>(b8 + bb + ob);
-  return true;
-}
-
-// The small-network path as one CTA (c == 1) or one cluster of c CTAs, each holding a slice
-// of the population, pushing the effects or (pull) gathering them at the targets; false
-// (nothing changed) when that form cannot run the net.
-bool set_small_cluster(b2b_net* net, int c, bool pull) {
-  SmallDev& D = net->sdev;
-  const Pop& pop = net->pops[0];
-  const int32_t c0 = D.cluster, p0 = D.pull;
-  const int64_t s0 = D.slice;
-  if (c == 1 && !pull) {
-    D.cluster = 1;
-    D.pull = 0;
-    D.slice = pop.n;
-  } else {
-    if ((c != 8 && c != 16) || (pull && !net->pull_ok)) return false;
-    D.cluster = c;
-    D.pull = pull ? 1 : 0;
-    D.slice = ((pop.n + c - 1) / c + 3) / 4 * 4;
-    if (pull && !build_pull_slices(net)) {
-      D.cluster = c0;
-      D.pull = p0;
-      D.slice = s0;
-      return false;
-    }
-    if (!small_cluster_possible(D, pop.kind, pop.dtype)) {
-      D.cluster = c0;
-      D.pull = p0;
-      D.slice = s0;
-      return false;
-    }
-  }
-  if (net->graph) {
-    cudaGraphExecDestroy(net->graph);
-    net->graph = nullptr;
-  }
-  return true;
-}
 
 void set_one_launch_grid(b2b_net* net, int grid) {
   int sms = kNumSMs;

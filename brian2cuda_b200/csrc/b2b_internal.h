@@ -242,7 +242,10 @@ struct SmallDev {
   const uint16_t* pull_tgt;
   const int64_t* pull_base;
   int32_t pull_max_tgt;                 // most synapses (of all projections) into one slice
-  int32_t pull_pad;
+  // the one-CTA form of LIF nets without delays (small_lif_kernel): in use, with the connectivity
+  // (total_syn synapses) in shared memory, warps that share one spike's bundle
+  int32_t lif_regs, local, spread;
+  int64_t total_syn;
 };
 
 struct Group {
@@ -486,6 +489,10 @@ int mlp_device(const b2b_mlp* m);
 size_t small_smem(const SmallDev& D, int kind, int dtype);
 // Shared memory of one CTA of the small path's cluster forms.
 size_t small_cluster_smem(const SmallDev& D, int kind, int dtype);
+// Whether small_lif_kernel's shared memory (local: with the connectivity) fits `limit` bytes, and
+// the steps one launch of the small-network path may take beyond a chunk (0: chunks only).
+bool small_lif_fits(const SmallDev& D, int dtype, bool local, size_t limit);
+int small_max_steps(const SmallDev& D);
 // Whether the cluster form of the small-network path (D.cluster CTAs of D.slice neurons) can
 // be launched on the current device.
 bool small_cluster_possible(const SmallDev& D, int kind, int dtype);

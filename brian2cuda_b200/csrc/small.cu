@@ -14,10 +14,11 @@
 // shared-memory targets,
 // applies a deferred reset if the schedule needs one, and writes the state back at the end.
 // Block barriers separate the phases, so Brian2's order within a step (groups, thresholds,
-// synapses, resets) is kept, delays of zero steps included.  Measured on B200 against the
-// per-step kernels: CUBA-type LIF nets of 500 / 1000 / 2000 neurons 3.8 / 4.4 / 5.8 us per
-// step against 4.9 / 5.5 / 6.6 us; at 4000 neurons, or with many delays (COBAHH with delays
-// of 1-50 steps), one SM's issue rate loses to the whole GPU, so the path is opt-in.
+// synapses, resets) is kept, delays of zero steps included.  LIF nets without delays have a form
+// of their own (small_lif_kernel): CUBA of 500 / 1000 / 2000 / 4000 neurons 0.8 / 1.1 / 1.7 / 3.6
+// us per step against 2.8 / 3.0 / 3.7 / 4.1 us of the per-step form's one launch per step; with
+// many delays (COBAHH with delays of 1-50 steps) one SM's issue rate loses to the whole GPU, so
+// the path is opt-in.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -285,6 +286,177 @@ small_net_kernel(const __grid_constant__ SmallDev D, const int64_t* __restrict__
     for (int64_t q = tid; q < n; q += blockDim.x) g[q] = snr[q];
   }
   if (tid == 0 && P.mon_cnt) *P.mon_cnt = s_mon;
+}
+
+// ---- one CTA, LIF without delays: the state in registers -------------------------------
+// A LIF network whose synapses have no delays and no weights of their own and add into ge/gi
+// only (the CUBA example) needs little of the general one-CTA kernel: a thread keeps v, lastspike
+// and its group's constants of its E neurons in registers for the whole chunk, ge and gi are in
+// shared memory, and spikes of the step go through one shared list.  A step without spikes is
+// one update and one block barrier; with spikes, the warps of the CTA share their bundles (from
+// shared memory where the connectivity fits, else from L2), a second barrier, and the next
+// update sees every event.  What bounds it is the latency of those two phases.
+// Measured (CUBA, float64), us per step: 700 neurons 4.2 in the general kernel, 0.92 here; 2000
+// neurons 5.8 / 1.7 (2.5 on a cluster of 8 gathering the effects), 4000 neurons 9.6 / 3.6 (3.1).
+constexpr int kSmallMaxSteps = 1000;   // steps of one launch
+
+template <typename R, int E>
+__global__ void __launch_bounds__(kSmallThreads, 1)
+small_lif_kernel(const __grid_constant__ SmallDev D, const int64_t* __restrict__ clock,
+                 int steps, double dt, int32_t* status) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  const PopDev& P = D.pop;
+  const int64_t n = P.n;                         // a multiple of 128
+  R* const sG = reinterpret_cast<R*>(smem);      // ge, gi
+  int32_t* const s_list = reinterpret_cast<int32_t*>(sG + 2 * n);   // the step's spikes
+  int32_t* const s_off = s_list + n;             // [n_proj][n + 1], with the targets
+  uint16_t* const s_tgt = reinterpret_cast<uint16_t*>(s_off + (int64_t)D.n_proj * (n + 1));
+  const bool local = D.local != 0;
+  // each spike's members: target variable and weight (ge / gi only)
+  __shared__ int64_t s_mhi[kMaxProjBatch][kPullMaxMembers];
+  __shared__ R* s_mtgt[kMaxProjBatch][kPullMaxMembers];
+  __shared__ R s_mw[kMaxProjBatch][kPullMaxMembers];
+  // spikes of the step by step number mod 3: the next step's is cleared while the one before
+  // may still be read
+  __shared__ int s_cnt[3];
+  const int tid = threadIdx.x, lane = tid & 31, warps = blockDim.x >> 5;
+  const int64_t ts0 = clock[0];
+  for (int64_t x = tid; x < n; x += blockDim.x) {
+    sG[x] = static_cast<const R*>(P.var[B2B_VAR_GE])[x];
+    sG[n + x] = static_cast<const R*>(P.var[B2B_VAR_GI])[x];
+  }
+  for (int x = tid; x < D.n_proj * kPullMaxMembers; x += blockDim.x) {
+    const int p = x / kPullMaxMembers, m = x - p * kPullMaxMembers;
+    const ProjDev& J = D.proj[p];
+    if (m < J.n_mem) {
+      const int var = J.n_mem == 1 ? D.proj_target[p] : (int)J.mem_var[m];
+      s_mhi[p][m] = J.n_mem == 1 ? INT64_MAX : J.mem_hi[m];
+      s_mtgt[p][m] = sG + (var == B2B_VAR_GE ? 0 : n);
+      s_mw[p][m] = (R)(J.mem_w ? J.mem_w[m] : J.w_scalar);
+    }
+  }
+  if (local) {
+    int64_t at = 0;
+    for (int p = 0; p < D.n_proj; ++p) {
+      const ProjDev& J = D.proj[p];              // without delays: one bundle per neuron
+      for (int64_t x = tid; x <= n; x += blockDim.x)
+        s_off[p * (n + 1) + x] = (int32_t)(at + J.off[x]);
+      const int64_t syn = J.off[n];
+      for (int64_t x = tid; x < syn; x += blockDim.x) s_tgt[at + x] = (uint16_t)J.post[x];
+      at += syn;
+    }
+  }
+  if (tid < 3) s_cnt[tid] = 0;
+  // this thread's neurons E tid .. E tid + E - 1, all of one group
+  const int64_t i0 = (int64_t)E * tid;
+  const bool mine = i0 < n;
+  const int gidx = mine && P.vec_group ? P.vec_group[i0 >> 2] : 0;
+  const LifDev g = static_cast<const LifDev*>(P.params)[gidx];
+  const bool refr = g.ref_steps >= 0;
+  const R Vt = (R)g.Vt, Vr = (R)g.Vr;
+  Pack<R, E> V{}, LS{};
+  uint32_t nrf = 0;
+  if (mine) {
+    V = load_pack<R, E>(P.var[B2B_VAR_V], tid);
+    LS = load_pack<R, E>(P.var[B2B_VAR_LASTSPIKE], tid);
+  }
+  unsigned long long mon = P.mon_cnt ? *P.mon_cnt : 0ull;   // the same in every thread
+  __syncthreads();
+
+  const double inv_dt = 1.0 / dt;
+  int slot = ring_slot(ts0, P.ring_len), next;
+  int par = 0;
+  for (int k = 0; k < steps; ++k, slot = next, par = par == 2 ? 0 : par + 1) {
+    next = slot + 1 == P.ring_len ? 0 : slot + 1;
+    const int64_t ts = ts0 + k;
+    const double t = (double)ts * dt;
+    // ---- groups, thresholds and resets
+    unsigned fl = 0;
+    if (mine) {
+      Pack<R, E> GE = load_pack<R, E>(sG, tid), GI = load_pack<R, E>(sG + n, tid);
+      nrf = 0;
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        bool nr = true;
+        if (refr) nr = past_refractory(t - (double)LS.x[e], dt, inv_dt, g.ref_steps);
+        R vn = lif_advance<R>(
+            g, V.x[e], GE.x[e], GI.x[e], nr,
+            P.inputs ? timed_input<R>(P.inputs[gidx].ta, ts, i0 + e - g.offset) : R(0));
+        if (g.has_threshold && (i0 + e - g.offset) < g.n && vn > Vt && nr) {
+          nr = false;
+          if (refr) LS.x[e] = (R)t;
+          if (g.has_reset) vn = Vr;
+          fl |= 1u << e;
+        }
+        V.x[e] = vn;
+        nrf |= (nr ? 1u : 0u) << (8 * e);
+      }
+      store_pack<R, E>(sG, tid, GE);
+      store_pack<R, E>(sG + n, tid, GI);
+      if (fl) {
+        int pos = atomicAdd(&s_cnt[par], __popc(fl));
+#pragma unroll
+        for (int e = 0; e < E; ++e)
+          if (fl & (1u << e)) s_list[pos++] = (int32_t)(i0 + e);
+      }
+    }
+    if (tid == 0) {
+      s_cnt[par == 2 ? 0 : par + 1] = 0;
+      P.ring_cnt[next] = 0;
+    }
+    const bool any = __syncthreads_or(fl != 0);
+    const int total = any ? s_cnt[par] : 0;
+    if (tid == 0) P.ring_cnt[slot] = total;
+    if (!any) continue;
+    // ---- synapses: each spike's bundle over D.spread warps
+    for (int it = tid >> 5; it < total * D.spread; it += warps) {
+      const int x = it / D.spread, part = it - x * D.spread;
+      const int32_t pre = s_list[x];
+      for (int p = 0; p < D.n_proj; ++p) {
+        const ProjDev& J = D.proj[p];
+        int m = 0, mh = J.n_mem - 1;
+        while (m < mh) {
+          const int mid = (m + mh) >> 1;
+          if (pre < s_mhi[p][mid]) mh = mid; else m = mid + 1;
+        }
+        R* T = s_mtgt[p][m];
+        const R w = s_mw[p][m];
+        if (local) {
+          const int32_t* o = s_off + p * (n + 1) + pre;
+          for (int32_t s = o[0] + 32 * part + lane; s < o[1]; s += 32 * D.spread)
+            atomicAdd(T + s_tgt[s], w);
+        } else {
+          const int64_t b1 = __ldg(J.off + pre + 1);
+          for (int64_t s = __ldg(J.off + pre) + 32 * part + lane; s < b1; s += 32 * D.spread)
+            atomicAdd(T + __ldg(J.post + s), w);
+        }
+      }
+    }
+    // ---- the step's record: ring slot and monitor
+    int32_t* out = P.ring_idx + (int64_t)slot * n;
+    for (int x = tid; x < total; x += blockDim.x) {
+      const int32_t idx = s_list[x];
+      out[x] = idx;
+      if (P.mon_cnt) {
+        if (mon + x < (unsigned long long)P.mon_cap) {
+          P.mon_idx[mon + x] = idx;
+          P.mon_step[mon + x] = ts;
+        } else {
+          set_status(status, B2B_ERR_QUEUE_OVERFLOW);
+        }
+      }
+    }
+    mon += (unsigned long long)total;
+    __syncthreads();
+  }
+  if (mine) {
+    store_pack<R, E>(P.var[B2B_VAR_V], tid, V);
+    store_pack<R, E>(P.var[B2B_VAR_LASTSPIKE], tid, LS);
+    store_pack<R, E>(P.var[B2B_VAR_GE], tid, load_pack<R, E>(sG, tid));
+    store_pack<R, E>(P.var[B2B_VAR_GI], tid, load_pack<R, E>(sG + n, tid));
+    if (refr && steps > 0) store_flags<E>(P.var[B2B_VAR_NOT_REFRACTORY], tid, nrf);
+  }
+  if (tid == 0 && P.mon_cnt) *P.mon_cnt = mon;
 }
 
 // Shared-memory copies of what the cluster kernels' step loops read repeatedly (the cluster
@@ -790,6 +962,15 @@ size_t small_smem(const SmallDev& D, int kind, int dtype) {
   return bytes;
 }
 
+// Shared memory of the LIF form; local: with the connectivity.
+size_t small_lif_smem(const SmallDev& D, int dtype, bool local) {
+  const size_t n = (size_t)D.pop.n, rs = dtype == B2B_F32 ? 4 : 8;
+  return 2 * rs * n + sizeof(int32_t) * n +
+         (local ? sizeof(int32_t) * (size_t)D.n_proj * (n + 1) +
+                      sizeof(uint16_t) * (size_t)D.total_syn
+                : 0);
+}
+
 // Shared memory of one CTA of the cluster form: its slice of the state and flags, then the
 // ring counts (push form) or the slice's bit rows, two local spike lists and the step's list
 // (pull form).
@@ -870,10 +1051,45 @@ bool small_cluster_possible(const SmallDev& D, int kind, int dtype) {
   return ok;
 }
 
+namespace {
+template <typename R, int E>
+cudaError_t launch_small_lif_e(const SmallDev& D, const int64_t* clock, int steps, double dt,
+                               int32_t* status, cudaStream_t s) {
+  const size_t smem = small_lif_smem(D, sizeof(R) == 4 ? B2B_F32 : B2B_F64, D.local != 0);
+  // static and dynamic shared memory together stay below the device's limit (small_lif_fits)
+  cudaError_t e = cudaFuncSetAttribute(small_lif_kernel<R, E>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  const int threads = (int)std::max<int64_t>(128, D.pop.n / E);   // n is a multiple of 128
+  small_lif_kernel<R, E><<<1, (threads + 31) / 32 * 32, smem, s>>>(D, clock, steps, dt, status);
+  return cudaGetLastError();
+}
+
+// A thread per neuron up to 1024 neurons, then two and four.
+template <typename R>
+cudaError_t launch_small_lif(const SmallDev& D, const int64_t* clock, int steps, double dt,
+                             int32_t* status, cudaStream_t s) {
+  if (D.pop.n <= kSmallThreads) return launch_small_lif_e<R, 1>(D, clock, steps, dt, status, s);
+  if (D.pop.n <= 2 * kSmallThreads)
+    return launch_small_lif_e<R, 2>(D, clock, steps, dt, status, s);
+  return launch_small_lif_e<R, 4>(D, clock, steps, dt, status, s);
+}
+}  // namespace
+
+bool small_lif_fits(const SmallDev& D, int dtype, bool local, size_t limit) {
+  const size_t fixed = sizeof(int64_t) * kMaxProjBatch * kPullMaxMembers * 3 + 256;
+  return small_lif_smem(D, dtype, local) + fixed <= limit;
+}
+
+int small_max_steps(const SmallDev& D) { return D.lif_regs ? kSmallMaxSteps : 0; }
+
 cudaError_t launch_small(const SmallDev& D, int kind, int dtype, const int64_t* clock,
                          int steps, double dt, int32_t* status, cudaStream_t s) {
   if (D.cluster > 1)
     return launch_cluster(D, kind, dtype, clock, steps, dt, status, s, false);
+  if (D.lif_regs)
+    return dtype == B2B_F32 ? launch_small_lif<float>(D, clock, steps, dt, status, s)
+                            : launch_small_lif<double>(D, clock, steps, dt, status, s);
   const size_t smem = small_smem(D, kind, dtype);
   cudaError_t e = cudaSuccess;
 #define B2B_SMALL(R, K)                                                                       \
