@@ -1606,6 +1606,7 @@ b2b_status b2b_create(const b2b_config* cfg, b2b_net** out) {
   *out = nullptr;
   b2b_net* net = new (std::nothrow) b2b_net();
   if (!net) return B2B_ERR_OOM;
+  readback_net_created();
   net->cfg = *cfg;
   if (net->cfg.steps_per_graph <= 0) net->cfg.steps_per_graph = 50;
   cudaError_t e = cudaSetDevice(cfg->device);
@@ -1661,6 +1662,7 @@ b2b_status b2b_destroy(b2b_net* net) {
   cudaFree(net->d_clock);
   cudaFree(net->d_status);
   if (net->own_stream) cudaStreamDestroy(net->stream);
+  readback_net_destroyed();
   delete net;
   return B2B_OK;
 }
@@ -1891,8 +1893,7 @@ b2b_status b2b_state_get(b2b_net* net, int32_t gid, int32_t var, void* host, int
   CHECK(net->finalized, B2B_ERR_STATE, "state is on the device only after b2b_finalize");
   const size_t es = var_size(g.dtype, var);
   const uint8_t* d = (const uint8_t*)net->pops[g.pop].dev.var[var] + es * g.offset;
-  CU(cudaMemcpyAsync(host, d, es * n, cudaMemcpyDeviceToHost, net->stream));
-  CU(cudaStreamSynchronize(net->stream));
+  CU(read_array(net, host, d, es * n));
   return B2B_OK;
 }
 
@@ -3311,15 +3312,33 @@ b2b_status b2b_syn_get(b2b_net* net, int32_t sid, int32_t var, void* host, int64
   const void* arr = var == B2B_SYN_W ? (stdp ? pr.dev.stdp_w : pr.w) : nullptr;
   const int64_t* inv = sy.inv;  // NULL for generated synapses: positions are the numbering
   const size_t es = (var <= B2B_SYN_DELAY) ? 4 : real_size(pr.dtype);
-  void* d_out = nullptr;
-  CU(cudaMalloc(&d_out, es * n));
   const int64_t key_lo = (gpre.offset + sy.pre_lo) * (int64_t)nd;
   const int64_t key_hi = (gpre.offset + sy.pre_hi) * (int64_t)nd;
-  cudaError_t e =
-      var > B2B_SYN_W
-          ? gather_syn_trace(pr, var, inv, sy.base, n, key_lo, key_hi, d_out, net->stream)
-          : gather_syn_var(pr, var, inv, sy.base, n, key_lo, key_hi, gpre.offset, gpost.offset,
-                           arr, sy.w_scalar, d_out, net->stream);
+  // values [q0, q0 + m) of the synapses' order into the device array out
+  auto gather = [&](int64_t q0, int64_t m, void* out, cudaStream_t s) {
+    const int64_t* at = inv ? inv + q0 : nullptr;
+    return var > B2B_SYN_W
+               ? gather_syn_trace(pr, var, at, sy.base + q0, m, key_lo, key_hi, out, s)
+               : gather_syn_var(pr, var, at, sy.base + q0, m, key_lo, key_hi, gpre.offset,
+                                gpost.offset, arr, sy.w_scalar, out, s);
+  };
+  if (read_back_worth(es * n)) {
+    GUARD_BEGIN
+    const cudaError_t e = read_back(
+        net, host, es * n,
+        [&](size_t off, size_t len, void* scratch, const void** src, cudaStream_t s) {
+          *src = scratch;
+          return gather((int64_t)(off / es), (int64_t)(len / es), scratch, s);
+        });
+    if (e != cudaErrorMemoryAllocation) {
+      CU(e);
+      return B2B_OK;
+    }
+    GUARD_END
+  }
+  void* d_out = nullptr;
+  CU(cudaMalloc(&d_out, es * n));
+  cudaError_t e = gather(0, n, d_out, net->stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(host, d_out, es * n, cudaMemcpyDeviceToHost, net->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(net->stream);
   cudaFree(d_out);

@@ -6,6 +6,7 @@
 
 #include <cmath>
 #include <cstdio>
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -364,6 +365,11 @@ struct Proj {
 }  // namespace b2b
 
 namespace b2b {
+// Bytes [off, off + len) of a value on the device (readback.cu): *src receives their address,
+// either in the value itself or, after work enqueued on s, in scratch (of len bytes).
+using ReadSource = std::function<cudaError_t(size_t off, size_t len, void* scratch,
+                                             const void** src, cudaStream_t s)>;
+
 struct Snapshot {
   bool valid = false;
   int64_t ts = 0;
@@ -450,6 +456,15 @@ struct b2b_net {
 
 // Kernel launch entry points (implemented in the .cu files, called by api.cu).
 namespace b2b {
+// Reads `bytes` from source into the host array, complete on return (readback.cu); for values
+// worth its threads.
+bool read_back_worth(size_t bytes);
+cudaError_t read_back(b2b_net* net, void* host, size_t bytes, const ReadSource& source);
+// A device array: by read_back, or a plain copy on the net's stream.
+cudaError_t read_array(b2b_net* net, void* host, const void* dev, size_t bytes);
+// Every net's creation and destruction: the slots of large reads go with the last net.
+void readback_net_created();
+void readback_net_destroyed();
 cudaError_t launch_pop_step(const Pop& pop, const int64_t* clock, int k, double dt,
                             int32_t* status, cudaStream_t s);
 // The same with another device view of the population (its fold buffers set).

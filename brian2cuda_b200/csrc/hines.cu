@@ -839,8 +839,7 @@ b2b_status b2b_hines_state_get(b2b_hines* h, int32_t var, void* host, int64_t n)
   void* d = hines_var(h, var, &es);
   if (!d) return B2B_ERR_INVALID_ARG;
   cudaSetDevice(h->net->cfg.device);
-  cudaStreamSynchronize(h->net->stream);
-  return cudaMemcpy(host, d, es * n, cudaMemcpyDeviceToHost) == cudaSuccess ? B2B_OK : B2B_ERR_CUDA;
+  return read_array(h->net, host, d, es * n) == cudaSuccess ? B2B_OK : B2B_ERR_CUDA;
 }
 
 b2b_status b2b_hines_run(b2b_hines* h, int64_t n_steps) {
