@@ -152,22 +152,38 @@ __device__ __forceinline__ void store_row16(uint8_t* base, int r, float v0, floa
 }
 
 // Loads 64 accumulator columns of this thread's row, adds bias (or nothing) and applies
-// tanh in bf16: hp receives the 64 activations as packed bf16 pairs.
+// tanh in bf16: hp receives the 64 activations as packed bf16 pairs.  WIDE: in one load (64
+// registers, for kernels that have them to spare).
+template <bool WIDE>
 __device__ __forceinline__ void epilogue_tanh64(uint32_t taddr, const float* bias,
                                                 uint32_t (&hp)[32]) {
+  constexpr int kCols = WIDE ? 64 : 16;
 #pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    float v[16];
-    tmem_ld16(taddr + 16 * c, v);
+  for (int c = 0; c < 64; c += kCols) {
+    float v[kCols];
+    if constexpr (WIDE) tmem_ld64(taddr, v);
+    else tmem_ld16(taddr + c, v);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int i = 0; i < kCols / 2; ++i) {
       float a = v[2 * i], b = v[2 * i + 1];
       if (bias) {
-        a += bias[16 * c + 2 * i];
-        b += bias[16 * c + 2 * i + 1];
+        a += bias[c + 2 * i];
+        b += bias[c + 2 * i + 1];
       }
-      hp[8 * c + i] = tanh_bf16x2(pack_bf16x2(a, b));
+      hp[c / 2 + i] = tanh_bf16x2(pack_bf16x2(a, b));
     }
+  }
+}
+
+// gz = d * (1 - h^2) of this thread's row: d the 64 accumulator columns, h the packed activations.
+__device__ __forceinline__ void scale_by_dtanh(uint32_t taddr, const uint32_t (&h)[32],
+                                               uint32_t (&gz)[32]) {
+  float v[64];
+  tmem_ld64(taddr, v);
+#pragma unroll
+  for (int i = 0; i < 32; ++i) {
+    const float a = bf16_lo(h[i]), b = bf16_hi(h[i]);
+    gz[i] = pack_bf16x2(v[2 * i] * (1.f - a * a), v[2 * i + 1] * (1.f - b * b));
   }
 }
 
@@ -242,7 +258,7 @@ __device__ bool mlp_tile_forward(FwdSmem& S, uint32_t& phase, const float (&xh)[
   }
   if (!wait_mma(&S.bar, phase, status)) return false;
   uint32_t hp[32];
-  epilogue_tanh64(taddr, nullptr, hp);
+  epilogue_tanh64<false>(taddr, nullptr, hp);
   store_row64(S.H, r, hp);
   operands_ready();
   if (r == 0) {
@@ -254,7 +270,7 @@ __device__ bool mlp_tile_forward(FwdSmem& S, uint32_t& phase, const float (&xh)[
     mma_commit(&S.bar);
   }
   if (!wait_mma(&S.bar, phase, status)) return false;
-  epilogue_tanh64(taddr, I->b2, hp);
+  epilogue_tanh64<false>(taddr, I->b2, hp);
   store_row64(S.H, r, hp);
   operands_ready();
   if (r == 0) {
@@ -423,13 +439,20 @@ struct TrainSmem {
   uint64_t bar;
   uint32_t tmem;
 };
-constexpr uint32_t kColS = 0, kColA = 64, kColB = 208, kTrainCols = 512;
-constexpr int kNA = 144, kNB = 80;   // columns of the two weight-gradient accumulators
+// Two CTAs per SM share its 512 TMEM columns: the products' scratch (64), the accumulator of
+// features 0-127 x all gradients (x, h1 and the first 48 of h2: 144 columns) and that of [h1 | h2]
+// x dy (16; the W3 gradient of all h2).  A tile is a chain of seven products with an epilogue
+// each, so a second CTA fills the waits of the first; more do not fit TMEM.  b2b_mlp_grad of 1e6
+// samples: 289 us with one CTA of 512 columns per SM, 195 us (2e5 samples: 122 / 108 us; the
+// call's copies and its wait are 80 us of either).
+constexpr uint32_t kColS = 0, kColA = 64, kColB = 208, kTrainCols = 256;
+constexpr int kNA = 144, kNB = 16;   // columns of the two weight-gradient accumulators
+constexpr int kTrainCtas = 2;        // per SM
 
 // Gradient of the mean loss over samples [mb_start, mb_start + mb_n) of the (permuted)
 // dataset; adds into grad (fp32, parameter order) and the summed squared error into *loss.
 // Sample s of the minibatch is dataset row (a * (mb_start + s) + c) mod n.
-__global__ void __launch_bounds__(kTile)
+__global__ void __launch_bounds__(kTile, kTrainCtas)
 mlp_grad_kernel(const MlpImage* __restrict__ img, const float4* __restrict__ x,
                 const float* __restrict__ tgt, int64_t n, int64_t mb_start, int64_t mb_n,
                 int64_t pa, int64_t pc, float inv_batch, float* __restrict__ grad,
@@ -485,7 +508,7 @@ mlp_grad_kernel(const MlpImage* __restrict__ img, const float4* __restrict__ x,
     }
     if (!(ok = wait_mma(&S.bar, phase, status))) break;
     uint32_t h1[32], h2[32];
-    epilogue_tanh64(taddr + kColS, nullptr, h1);
+    epilogue_tanh64<true>(taddr + kColS, nullptr, h1);
     store_row64(S.FS + 2 * kG, r, h1);
     operands_ready();
     if (r == 0) {
@@ -497,7 +520,7 @@ mlp_grad_kernel(const MlpImage* __restrict__ img, const float4* __restrict__ x,
       mma_commit(&S.bar);
     }
     if (!(ok = wait_mma(&S.bar, phase, status))) break;
-    epilogue_tanh64(taddr + kColS, I->b2, h2);
+    epilogue_tanh64<true>(taddr + kColS, I->b2, h2);
     store_row64(S.FS + 10 * kG, r, h2);
     operands_ready();
     if (r == 0) {
@@ -531,16 +554,7 @@ mlp_grad_kernel(const MlpImage* __restrict__ img, const float4* __restrict__ x,
     if (!(ok = wait_mma(&S.bar, phase, status))) break;
     // dz2 = dh2 * (1 - h2^2), then dz1 = (dz2 W2) * (1 - h1^2)
     uint32_t gz[32];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      tmem_ld16(taddr + kColS + 16 * c, v);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const uint32_t hh = h2[8 * c + i];
-        const float a = bf16_lo(hh), b = bf16_hi(hh);
-        gz[8 * c + i] = pack_bf16x2(v[2 * i] * (1.f - a * a), v[2 * i + 1] * (1.f - b * b));
-      }
-    }
+    scale_by_dtanh(taddr + kColS, h2, gz);
     store_row64(S.GS + 8 * kG, r, gz);
     operands_ready();
     if (r == 0) {
@@ -552,16 +566,7 @@ mlp_grad_kernel(const MlpImage* __restrict__ img, const float4* __restrict__ x,
       mma_commit(&S.bar);
     }
     if (!(ok = wait_mma(&S.bar, phase, status))) break;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      tmem_ld16(taddr + kColS + 16 * c, v);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const uint32_t hh = h1[8 * c + i];
-        const float a = bf16_lo(hh), b = bf16_hi(hh);
-        gz[8 * c + i] = pack_bf16x2(v[2 * i] * (1.f - a * a), v[2 * i + 1] * (1.f - b * b));
-      }
-    }
+    scale_by_dtanh(taddr + kColS, h1, gz);
     store_row64(S.GS, r, gz);
     operands_ready();
     // weight gradients: A = features^T (MN-major), B = gradients (MN-major), K = samples
@@ -573,7 +578,7 @@ mlp_grad_kernel(const MlpImage* __restrict__ img, const float4* __restrict__ x,
         mma_bf16(tmem + kColA, sdesc(sFS + kk * 256, 128, kG), sdesc(sGS + kk * 256, 128, kG),
                  idA, acc);
         mma_bf16(tmem + kColB, sdesc(sFS + 2 * kG + kk * 256, 128, kG),
-                 sdesc(sGS + 8 * kG + kk * 256, 128, kG), idB, acc);
+                 sdesc(sGS + 16 * kG + kk * 256, 128, kG), idB, acc);
       }
       mma_commit(&S.bar);
     }
@@ -602,19 +607,19 @@ mlp_grad_kernel(const MlpImage* __restrict__ img, const float4* __restrict__ x,
         }
       }
     }
-    // second accumulator: rows 0..63 = h1 features x dz2 columns 0..63; rows 64..127 = h2
-    // features x dy columns 64..66
-    for (int c = 0; c < kNB; c += 16) {
+    // rows 16..79: h1 features x dz2 (columns 64..127).  Warp 2 holds rows 64..95, so the first
+    // three warps load together
+    if (r < 96) {
+      float a[64];
+      tmem_ld64(taddr + kColA + kHid, a);
+      if (r >= 16 && r < 16 + kHid)
+        for (int col = 0; col < kHid; ++col) atomicAdd(&grad[kW2 + col * kHid + r - 16], a[col]);
+    }
+    // second accumulator: rows 64..127 = h2 features x dy columns 0..2
+    if (r >= kHid) {
       float b[16];
-      tmem_ld16(taddr + kColB + c, b);
-      for (int i = 0; i < 16; ++i) {
-        const int col = c + i;
-        if (r < kHid) {
-          if (col < kHid) atomicAdd(&grad[kW2 + col * kHid + r], b[i]);
-        } else if (col >= kHid && col < kHid + kOut) {
-          atomicAdd(&grad[kW3 + (col - kHid) * kHid + (r - kHid)], b[i]);
-        }
-      }
+      tmem_ld16(taddr + kColB, b);
+      for (int o = 0; o < kOut; ++o) atomicAdd(&grad[kW3 + o * kHid + (r - kHid)], b[o]);
     }
   }
   fence_before_sync();
@@ -1000,9 +1005,10 @@ b2b_status b2b_mlp_forward(b2b_mlp* m, const float* dev_x, float* dev_out, int64
 namespace {
 b2b_status launch_grad(b2b_mlp* m, const float* dev_x, const float* dev_t, int64_t n,
                        int64_t mb_start, int64_t mb_n, int64_t pa, int64_t pc) {
-  // more than half an SM's shared memory, so that one CTA (holding all 512 TMEM columns)
-  // runs per SM and no CTA waits in tcgen05.alloc for another
-  const size_t smem = std::max<size_t>(sizeof(TrainSmem), 120 * 1024);
+  // more than a third of an SM's shared memory, so that two CTAs (holding 256 TMEM columns
+  // each) run per SM and no CTA waits in tcgen05.alloc for another
+  const size_t smem = std::max<size_t>(sizeof(TrainSmem), 96 * 1024);
+  static_assert(sizeof(TrainSmem) <= 112 * 1024, "two CTAs per SM");
   static bool attr[64] = {};
   if (m->device < 64 && !attr[m->device]) {
     MCU(cudaFuncSetAttribute(mlp_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1010,7 +1016,7 @@ b2b_status launch_grad(b2b_mlp* m, const float* dev_x, const float* dev_t, int64
     attr[m->device] = true;
   }
   const int64_t ntiles = (mb_n + kTile - 1) / kTile;
-  const unsigned grid = (unsigned)std::min<int64_t>(ntiles, sm_count(m->device));
+  const unsigned grid = (unsigned)std::min<int64_t>(ntiles, kTrainCtas * sm_count(m->device));
   mlp_grad_kernel<<<grid, kTile, smem, m->stream>>>(
       m->img, reinterpret_cast<const float4*>(dev_x), dev_t, n, mb_start, mb_n, pa, pc,
       1.0f / (float)mb_n, m->g, m->loss, m->status);
