@@ -251,6 +251,99 @@ __device__ __forceinline__ void hh_step_body(const PopDev& P, const int64_t* __r
   clear_next_slot(P, ts, blk);
 }
 
+// The same with a neuron's v, m, h and n in four warps of the CTA (warp 4 g + r: variable r of the
+// CTA's neurons 32 g .. 32 g + 31): in a population that does not fill the GPU the update is one
+// thread's chain of exponentials and quotients, and the four equations are independent given the
+// state at the start of the step.  A barrier between the loads and the stores keeps that state.
+// Float64, us per step of the update alone, one thread per neuron / here: 4000 neurons 4.12 / 2.89,
+// 8000 4.24 / 3.09, 20,000 4.48 / 3.52, 40,000 4.92 / 5.33 (the added warps are work there);
+// float32, whose hardware exponentials are short, 4000 neurons 2.17 / 2.33, so it is not used.
+template <typename R>
+__device__ __forceinline__ int64_t split_neuron(int64_t blk) {
+  return blk * (blockDim.x >> 2) + 32 * (threadIdx.x >> 7) + (threadIdx.x & 31);
+}
+template <typename R, bool FUSED = false, class Emit = int>
+__device__ __forceinline__ void hh_split_body(const PopDev& P, const int64_t* __restrict__ clock,
+                                              int k, double dt, int32_t* status, int64_t blk,
+                                              Emit emit = 0) {
+  const int64_t ts = clock[0] + k;
+  const int slot = ring_slot(ts, P.ring_len);
+  const int role = (threadIdx.x >> 5) & 3;
+  const int64_t q = split_neuron<R>(blk);
+  const bool mine = q < P.n;
+  const R dtR = (R)dt;
+  HhRun<R> g{};
+  if (mine) g = hh_run(static_cast<const HhDev*>(P.params)[group_of<1>(P, q)], R());
+  R v = 0;
+  if (mine) v = static_cast<const R*>(P.var[B2B_VAR_V])[q];
+  unsigned fl = 0;
+  if (role == 0) {
+    Pack<R, 1> GE{}, GI{};
+    R m = 0, h = 0, n = 0, ls = 0;
+    R *fge = nullptr, *fgi = nullptr;
+    int32_t *cge = nullptr, *cgi = nullptr;
+    if (mine) {
+      m = static_cast<const R*>(P.var[B2B_VAR_M])[q];
+      h = static_cast<const R*>(P.var[B2B_VAR_H])[q];
+      n = static_cast<const R*>(P.var[B2B_VAR_N])[q];
+      GE = load_pack<R, 1>(P.var[B2B_VAR_GE], q);
+      GI = load_pack<R, 1>(P.var[B2B_VAR_GI], q);
+      ls = static_cast<const R*>(P.var[B2B_VAR_LASTSPIKE])[q];
+      if constexpr (FUSED) {
+        cge = fold_counts<R, 1>(P, B2B_VAR_GE, k, q, GE);
+        cgi = fold_counts<R, 1>(P, B2B_VAR_GI, k, q, GI);
+      } else {
+        fge = fold_in<R, 1>(P, B2B_VAR_GE, k, q, GE);
+        fgi = fold_in<R, 1>(P, B2B_VAR_GI, k, q, GI);
+      }
+    }
+    __syncthreads();
+    if (mine) {
+      const double t = (double)ts * dt;
+      const bool refr = g.ref_steps >= 0;
+      bool nr = true;
+      if (refr) nr = past_refractory(t - (double)ls, dt, 1.0 / dt, g.ref_steps);
+      const R vn = hh_membrane<R>(g, v, m, h, n, GE.x[0], GI.x[0], dtR);
+      if (q - g.offset < g.n && vn > (R)g.Vthr && nr) {
+        nr = false;
+        if (refr) static_cast<R*>(P.var[B2B_VAR_LASTSPIKE])[q] = (R)t;
+        fl = 1u;
+      }
+      static_cast<R*>(P.var[B2B_VAR_V])[q] = vn;
+      static_cast<R*>(P.var[B2B_VAR_GE])[q] = (R)g.De * GE.x[0];
+      static_cast<R*>(P.var[B2B_VAR_GI])[q] = (R)g.Di * GI.x[0];
+      if (refr) static_cast<uint8_t*>(P.var[B2B_VAR_NOT_REFRACTORY])[q] = nr ? 1 : 0;
+      if constexpr (FUSED) {
+        clear_counts<1>(cge);
+        clear_counts<1>(cgi);
+      } else {
+        fold_clear<R, 1>(fge, q);
+        fold_clear<R, 1>(fgi, q);
+      }
+    }
+  } else {
+    R* X = static_cast<R*>(P.var[role == 1 ? B2B_VAR_M : role == 2 ? B2B_VAR_H : B2B_VAR_N]);
+    R x = 0;
+    if (mine) x = X[q];
+    __syncthreads();
+    if (mine) {
+      if (role == 1) x = hh_gate_m<R>((R)g.VT, v, x, dtR);
+      else if (role == 2) x = hh_gate_h<R>((R)g.VT, v, x, dtR);
+      else x = hh_gate_n<R>((R)g.VT, v, x, dtR);
+      X[q] = x;
+    }
+  }
+  if constexpr (FUSED) emit(q, fl, ts, slot);
+  else emit_spikes<1>(P, q, fl, ts, slot, status);
+  clear_next_slot(P, ts, blk);
+}
+
+template <typename R>
+__global__ void __launch_bounds__(kBlock)
+hh_split_kernel(PopDev P, const int64_t* __restrict__ clock, int k, double dt, int32_t* status) {
+  hh_split_body<R>(P, clock, k, dt, status, blockIdx.x);
+}
+
 template <typename R, int E, bool INPUTS>
 __global__ void __launch_bounds__(kBlock)
 hh_step_kernel(PopDev P, const int64_t* __restrict__ clock, int k, double dt,
@@ -265,8 +358,9 @@ hh_step_kernel(PopDev P, const int64_t* __restrict__ clock, int k, double dt,
 // bundles due at step t into acc[t & 1] (t counted from the chunk's start).  Consecutive steps are consecutive launches on one
 // stream, so one launch boundary orders step t+1 after both halves of step t, where the two
 // concurrent launches need a boundary each and dependencies across two streams.
+// E = 0: a HH neuron's variables in four warps (hh_split_body).
 template <typename R, int KIND, int E, int GROUP>
-__global__ void __launch_bounds__(kBlock, E == 1 ? (sizeof(R) == 4 ? 5 : 4) : 3)
+__global__ void __launch_bounds__(kBlock, E <= 1 ? (sizeof(R) == 4 ? 5 : 4) : 3)
 one_launch_step_kernel(const __grid_constant__ PopDev U, const __grid_constant__ PendingDev F,
                        const int64_t* __restrict__ clock, int k, double dt, int32_t* status,
                        int n_upd) {
@@ -276,7 +370,9 @@ one_launch_step_kernel(const __grid_constant__ PopDev U, const __grid_constant__
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;");
   if ((int)blockIdx.x < n_upd) {
-    if constexpr (KIND == KIND_HH)
+    if constexpr (E == 0)
+      hh_split_body<R>(U, clock, k, dt, status, blockIdx.x);
+    else if constexpr (KIND == KIND_HH)
       hh_step_body<R, E, false>(U, clock, k, dt, status, blockIdx.x);
     else
       lif_step_body<R, E, false>(U, clock, k, dt, status, blockIdx.x);
@@ -340,14 +436,18 @@ template <typename R, int KIND, int E>
 __global__ void __launch_bounds__(kBlock)
 fused_step_kernel(const __grid_constant__ PopDev U, const __grid_constant__ FusedDev F,
                   const int64_t* __restrict__ clock, int k, double dt, int32_t* status) {
-  __shared__ int32_t s_list[kBlock * E];
+  constexpr int kMine = E > 0 ? E : 1;          // neurons per thread
+  constexpr int kList = E > 0 ? kBlock * E : kBlock / 4;
+  __shared__ int32_t s_list[kList];
   // the bundle bounds of the CTA's own neurons are loaded with their state and kept for those
   // that spike, so that a delivery starts at its targets
-  __shared__ int64_t s_b0[kBlock * E], s_b1[kBlock * E];
-  const int64_t q0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  int64_t off[E + 1];
+  __shared__ int64_t s_b0[kList], s_b1[kList];
+  const int64_t q0 = E > 0 ? (int64_t)blockIdx.x * blockDim.x + threadIdx.x
+                           : split_neuron<R>(blockIdx.x);
+  int64_t off[kMine + 1];
 #pragma unroll
-  for (int e = 0; e <= E; ++e) off[e] = q0 < U.n / E ? __ldg(F.proj[0].off + E * q0 + e) : 0;
+  for (int e = 0; e <= kMine; ++e)
+    off[e] = q0 < U.n / kMine ? __ldg(F.proj[0].off + kMine * q0 + e) : 0;
   auto deliver = [&](int total) {
     const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
     const int64_t row = (int64_t)(k & 1) * U.n;
@@ -374,12 +474,14 @@ fused_step_kernel(const __grid_constant__ PopDev U, const __grid_constant__ Fuse
     }
   };
   auto emit = [&](int64_t q, unsigned fl, int64_t ts, int slot) {
-    emit_spikes_use<E>(U, q, fl, ts, slot, status, s_list, [&](int e, int pos) {
+    emit_spikes_use<kMine>(U, q, fl, ts, slot, status, s_list, [&](int e, int pos) {
       s_b0[pos] = off[e];
       s_b1[pos] = off[e + 1];
     }, deliver);
   };
-  if constexpr (KIND == KIND_HH)
+  if constexpr (E == 0)
+    hh_split_body<R, true>(U, clock, k, dt, status, blockIdx.x, emit);
+  else if constexpr (KIND == KIND_HH)
     hh_step_body<R, E, false, true>(U, clock, k, dt, status, blockIdx.x, emit);
   else
     lif_step_body<R, E, false, true>(U, clock, k, dt, status, blockIdx.x, emit);
@@ -405,6 +507,11 @@ __global__ void fold_counts_kernel(const __grid_constant__ PopDev U, int row) {
 template <typename R, int KIND>
 void launch_fused_rk(const PopDev& U, const FusedDev& F, int e, unsigned grid, int block,
                      const int64_t* clock, int k, double dt, int32_t* status, cudaStream_t s) {
+  if constexpr (KIND == KIND_HH && sizeof(R) == 8)
+    if (e == 0) {
+      fused_step_kernel<R, KIND, 0><<<grid, block, 0, s>>>(U, F, clock, k, dt, status);
+      return;
+    }
   if (e == 2) fused_step_kernel<R, KIND, 2><<<grid, block, 0, s>>>(U, F, clock, k, dt, status);
   else fused_step_kernel<R, KIND, 1><<<grid, block, 0, s>>>(U, F, clock, k, dt, status);
 }
@@ -602,6 +709,8 @@ __global__ void lif_late_reset_kernel(PopDev P, const int64_t* __restrict__ cloc
   }
 }
 
+// Float64 HH populations below this size run hh_split_body.
+constexpr int64_t kSplitNeurons = 32000;
 // Neurons per thread and threads per CTA of a population's update: the autotuner's choice, else
 // by kind, type and size.  Small populations are bound by one neuron's chain of loads and
 // arithmetic, so every neuron gets a thread, in CTAs of 128 that spread over more SMs; once a
@@ -616,14 +725,23 @@ __global__ void lif_late_reset_kernel(PopDev P, const int64_t* __restrict__ cloc
 // 3.42 / 3.10 / 3.03.
 struct UpdateShape {
   int e, block;
+  bool split;                     // a HH neuron's variables in four warps (hh_split_body; e = 1)
 };
 UpdateShape update_shape(const Pop& pop, int64_t n) {
   const bool f32 = pop.dtype == B2B_F32;
   int e = 1;
+  if (pop.kind == KIND_HH && pop.tune_e == 0 && !pop.inputs && !f32 && n < kSplitNeurons)
+    return {1, pop.tune_block > 0 ? pop.tune_block : 128, true};
   if (pop.kind == KIND_POISSON) e = n >= 200000 ? 4 : 2;
   else if (f32) e = n >= 280000 ? 4 : (n >= 90000 ? 2 : 1);
   else if (pop.kind == KIND_LIF) e = n >= 130000 ? 2 : 1;
-  return {pop.tune_e > 0 ? pop.tune_e : e, pop.tune_block > 0 ? pop.tune_block : 128};
+  return {pop.tune_e > 0 ? pop.tune_e : e, pop.tune_block > 0 ? pop.tune_block : 128, false};
+}
+
+// CTAs of an update of n neurons at e neurons per thread (0: four threads per neuron).
+unsigned update_grid(const UpdateShape& shape, int e, int64_t n) {
+  const int64_t threads = e == 0 ? 4 * n : n / e;
+  return (unsigned)((threads + shape.block - 1) / shape.block);
 }
 
 template <int E, bool IN>
@@ -675,7 +793,13 @@ cudaError_t launch_pop_step_dev(const Pop& pop, const PopDev& dev, const int64_t
     spikegen_step_kernel<<<1, kBlock, 0, s>>>(pop.dev, clock, k, status);
     return cudaGetLastError();
   }
-  const int e = update_shape(pop, pop.dev.n).e;
+  const UpdateShape shape = update_shape(pop, pop.dev.n);
+  const int e = shape.e;
+  if (shape.split) {
+    hh_split_kernel<double>
+        <<<update_grid(shape, 0, dev.n), shape.block, 0, s>>>(dev, clock, k, dt, status);
+    return cudaGetLastError();
+  }
   if (pop.inputs) {
     if (e == 4) return launch_e<4, true>(pop, dev, clock, k, dt, status, s);
     if (e == 2) return launch_e<2, true>(pop, dev, clock, k, dt, status, s);
@@ -699,10 +823,13 @@ cudaError_t launch_one_launch_step(const Pop& pop, const PopDev& U, const Pendin
   // threads per CTA); the delivery half the same threads per CTA, deliver_ctas counted in
   // CTAs of kBlock threads
   const UpdateShape shape = update_shape(pop, U.n);
-  const int e = shape.e >= 2 ? 2 : 1, block = shape.block;
-  const int n_upd = (int)((U.n / e + block - 1) / block);
+  const int e = shape.split ? 0 : shape.e >= 2 ? 2 : 1, block = shape.block;
+  const int n_upd = (int)update_grid(shape, e, U.n);
   const unsigned grid = (unsigned)(n_upd + (int64_t)deliver_ctas * kBlock / block);
   const bool f32 = pop.dtype == B2B_F32;
+  if (e == 0)
+    return launch_one_r<double, KIND_HH, 0>(U, F, grid, block, chained, clock, k, dt, status,
+                                            n_upd, s);
   if (pop.kind == KIND_HH)
     return e == 2 ? launch_one_k<KIND_HH, 2>(U, F, f32, grid, block, chained, clock, k, dt,
                                              status, n_upd, s)
@@ -718,8 +845,8 @@ cudaError_t launch_fused_step(const Pop& pop, const PopDev& U, const FusedDev& F
                               const int64_t* clock, int k, double dt, int32_t* status,
                               cudaStream_t s) {
   const UpdateShape shape = update_shape(pop, U.n);
-  const int e = shape.e >= 2 ? 2 : 1, block = shape.block;
-  const unsigned grid = (unsigned)((U.n / e + block - 1) / block);
+  const int e = shape.split ? 0 : shape.e >= 2 ? 2 : 1, block = shape.block;
+  const unsigned grid = update_grid(shape, e, U.n);
   const bool f32 = pop.dtype == B2B_F32;
   if (pop.kind == KIND_HH) {
     if (f32) launch_fused_rk<float, KIND_HH>(U, F, e, grid, block, clock, k, dt, status, s);

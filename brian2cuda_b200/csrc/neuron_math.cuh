@@ -85,17 +85,29 @@ __device__ __forceinline__ R expeuler(R x, R A, R B, R dt) {
 // of m, h, n over one dt at membrane potential v.  Rates in SI units; the three of the form
 // x/(exp(x/a) - 1) go through z/(exp(z) - 1) (hz_over_expm1, Brian2's exprel).
 template <typename R>
-__device__ __forceinline__ void hh_gating(R VT, R v, R& m, R& h, R& n, R dt) {
+__device__ __forceinline__ R hh_gate_m(R VT, R v, R m, R dt) {
   // 0.32/mV*(13mV-v+VT)/(exp((13mV-v+VT)/4mV)-1)/ms = 1280 * z/expm1(z), z = (..)/4mV
   const R am = (R)1280 * hz_over_expm1(hdivc((R)13e-3 - v + VT, 4e-3));
   const R bm = (R)1400 * hz_over_expm1(hdivc(v - VT - (R)40e-3, 5e-3));
+  return expeuler(m, -(am + bm), am, dt);
+}
+template <typename R>
+__device__ __forceinline__ R hh_gate_h(R VT, R v, R h, R dt) {
   const R ah = (R)128 * hexp(hdivc((R)17e-3 - v + VT, 18e-3));
   const R bh = hdiv((R)4000, (R)1 + hexp(hdivc((R)40e-3 - v + VT, 5e-3)));
+  return expeuler(h, -(ah + bh), ah, dt);
+}
+template <typename R>
+__device__ __forceinline__ R hh_gate_n(R VT, R v, R n, R dt) {
   const R an = (R)160 * hz_over_expm1(hdivc((R)15e-3 - v + VT, 5e-3));
   const R bn = (R)500 * hexp(hdivc((R)10e-3 - v + VT, 40e-3));
-  m = expeuler(m, -(am + bm), am, dt);
-  h = expeuler(h, -(ah + bh), ah, dt);
-  n = expeuler(n, -(an + bn), an, dt);
+  return expeuler(n, -(an + bn), an, dt);
+}
+template <typename R>
+__device__ __forceinline__ void hh_gating(R VT, R v, R& m, R& h, R& n, R dt) {
+  m = hh_gate_m(VT, v, m, dt);
+  h = hh_gate_h(VT, v, h, dt);
+  n = hh_gate_n(VT, v, n, dt);
 }
 
 // A group's HH constants in the arithmetic type R of the update (float32: the host-rounded

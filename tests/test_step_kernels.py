@@ -47,3 +47,28 @@ def test_pending_input_across_odd_chunks(gpu_factory, form, n):
         out.append([net.get_state(ids["P"], v) for v in ("v", "m", "ge", "gi", "lastspike")])
     for a, b in zip(*out):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("form", [{"two_launch": False}, {"two_launch": True},
+                                  {"one_launch": True}])
+@pytest.mark.parametrize("n,dmin", [(5, 1), (33, 1), (127, 1), (1000, 1), (31_900, 1), (2000, 0)])
+def test_split_hh_update_equals_one_thread_per_neuron(gpu_factory, form, n, dmin):
+    """Float64 COBAHH networks below 32,000 neurons update a neuron's variables in four warps;
+    the tuned shape of one thread per neuron gives the same state, bit for bit.  dmin = 0: the
+    per-step form's single launch without delays."""
+    if dmin == 0 and form != {"two_launch": False}:
+        pytest.skip("the other forms need delays of at least one step")
+    out = []
+    for e in (0, 1):
+        net = gpu_factory(DT, **form)
+        ids = models.build_cobahh(net, n=n, p=min(1.0, 30 / n), dmin=dmin,
+                                  dmax=9 if dmin else 0, dtype="float64", monitor_capacity=10**6)
+        net.finalize()
+        if e:
+            net.tune_apply([{"site_kind": 1, "site_index": 0, "choice_a": e, "choice_b": 128}])
+        net.run(120)
+        out.append([net.get_state(ids["P"], v) for v in
+                    ("v", "m", "h", "n", "ge", "gi", "lastspike", "not_refractory")] +
+                   list(net.spikes(ids["P"])))
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
