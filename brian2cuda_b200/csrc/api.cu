@@ -611,6 +611,9 @@ b2b_status build_proj(b2b_net* net, int pj) {
       CU(cudaMemcpy(dw, mw.data(), 8 * mw.size(), cudaMemcpyHostToDevice));
       D.mem_w = dw;
     }
+    pr.mem_hi = hi;
+    pr.mem_var = var;
+    pr.mem_w = mw;
   }
   int64_t n_dst_valid = 0;
   for (int gi : dst.groups) n_dst_valid += net->groups[gi].n;
@@ -1058,7 +1061,7 @@ b2b_status setup_two_launch(b2b_net* net) {
   const size_t rs = real_size(pop.dtype);
   for (size_t p = 0; p < net->projs.size(); ++p) {
     const Proj& pr = net->projs[p];
-    F.proj[p] = pr.dev;
+    F.proj[p] = add_dev(pr);
     for (int m : pr.members) {
       const int v = net->syns[m].target_var;
       if (!F.acc[v]) {
@@ -1068,7 +1071,7 @@ b2b_status setup_two_launch(b2b_net* net) {
       }
       F.proj[p].targets[v] = F.acc[v];
     }
-    F.proj[p].target = F.acc[pr.target_var];
+    F.proj[p].targets[pr.target_var] = F.acc[pr.target_var];
   }
   int sms = kNumSMs;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, net->cfg.device);
@@ -1420,12 +1423,12 @@ void refresh_two_launch(b2b_net* net) {
   F.nd_max = nd_max;
   for (size_t p = 0; p < net->projs.size(); ++p) {
     const Proj& pr = net->projs[p];
-    F.proj[p] = pr.dev;
+    F.proj[p] = add_dev(pr);
     for (int m : pr.members) {
       const int v = net->syns[m].target_var;
       F.proj[p].targets[v] = F.acc[v];
     }
-    F.proj[p].target = F.acc[pr.target_var];
+    F.proj[p].targets[pr.target_var] = F.acc[pr.target_var];
   }
   net->fold_dev = pop.dev;
   for (int v = 0; v < 3; ++v) net->fold_dev.fold[v] = F.acc[v];

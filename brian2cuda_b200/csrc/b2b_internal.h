@@ -171,6 +171,30 @@ struct ProjDev {
   const int32_t* rec_of;
 };
 
+// An additive projection as its delivery kernels read it: what ProjDev holds for them in a third
+// of the size, with the tables of up to kInlineMembers members in place (a lookup of them in
+// memory would be two dependent loads in front of every bundle's effects).
+constexpr int kInlineMembers = 4;
+struct AddDev {
+  const int32_t* src_ring_cnt;
+  const int32_t* src_ring_idx;
+  int64_t src_n;
+  int32_t src_ring_len, dmin, nd, chunks;
+  int64_t src_lo, src_hi;
+  const int64_t* off;
+  const int32_t* post;
+  const void* w;
+  void* targets[3];
+  int32_t n_mem;
+  int32_t in_hi[kInlineMembers - 1];  // members 0 .. n_mem-2: presynaptic indices below
+  int32_t in_var[kInlineMembers];
+  double in_w[kInlineMembers];
+  const int64_t* mem_hi;              // more members: the projection's tables
+  const int8_t* mem_var;
+  const double* mem_w;
+  double w_scalar;
+};
+
 // Device view of a state monitor (monitor.cu): variable src (es-byte elements) of the
 // population rows idx[0..n_idx), one record [n_idx] per step divisible by `every`.
 struct StateMonDev {
@@ -202,12 +226,28 @@ struct RateMonDev {
 // additive projections, whose targets are redirected to double-buffered input accumulators.
 struct PendingDev {
   PopDev pop;
-  ProjDev proj[kMaxProjBatch];
+  AddDev proj[kMaxProjBatch];
   int32_t n_proj, nd_max;
   void* acc[3];                   // per target variable (v, ge, gi): [2][pop.n] or NULL
   int32_t group;                  // delivery: lanes per work item (2, 4, 8 or 16)
   int32_t pad_group;
 };
+// What its delivering CTAs read: the projections (one launch parameter block for the ordinary
+// case of one projection, one for several) and the rows of the accumulators.
+template <int NP>
+struct PendingArgs {
+  AddDev proj[NP];
+  int64_t n;                      // population size, the accumulators' row length
+  int32_t n_proj, pad;
+};
+template <int NP>
+inline PendingArgs<NP> pending_args(const PendingDev& F) {
+  PendingArgs<NP> a{};
+  for (int p = 0; p < F.n_proj && p < NP; ++p) a.proj[p] = F.proj[p];
+  a.n = F.pop.n;
+  a.n_proj = F.n_proj;
+  return a;
+}
 
 // Device view of the fused step's delivery (neuron.cu): additive projections of a population
 // onto its own ge/gi without delays or weights of their own, one weight per target variable.
@@ -340,6 +380,9 @@ struct Syn {  // one user-level Synapses object
   int32_t pre_lo = 0, pre_hi = 0;            // presynaptic subgroup (group-local)
 };
 
+struct Proj;
+AddDev add_dev(const Proj& pr);            // delivery.cuh's view of an additive projection
+
 struct Proj {
   int src_pop = -1, dst_pop = -1, target_var = 0, effect = 0, dtype = 0;
   bool multi_target = false;                 // members add into different variables
@@ -348,6 +391,10 @@ struct Proj {
   int64_t n_syn = 0;
   int64_t max_bundle = 0, max_post_bundle = 0;
   double mean_bundle = 0;                    // synapses per (pre, delay) bundle of the members
+  // host copies of the member tables (dev.n_mem > 1)
+  std::vector<int64_t> mem_hi;
+  std::vector<int8_t> mem_var;
+  std::vector<double> mem_w;
   ProjDev dev{};
   int64_t* off = nullptr;
   int32_t* post = nullptr;

@@ -45,22 +45,51 @@ __device__ __forceinline__ bool in_window(int64_t ts, int d, int64_t lo, int64_t
   return s >= 0 && s >= lo && s < hi;
 }
 
-__device__ __forceinline__ DuePrefix due_prefix_warp(const int32_t* __restrict__ ring_cnt,
+// The due counts themselves, delay indices lane and 32 + lane.  A ring of at most 64 slots is read
+// whole before the step is known (its loads run beside the clock's) and picked from by shuffles.
+struct DueCounts {
+  int c0, c1;
+};
+__device__ __forceinline__ DueCounts due_counts_warp(const int32_t* __restrict__ ring_cnt,
                                                      int ring_len, int64_t ts, int dmin, int nd,
                                                      int64_t lo, int64_t hi) {
   const int lane = threadIdx.x & 31;
+  DueCounts c{0, 0};
+  if (ring_len <= 64) {   // the same in every lane
+    const int r0 = lane < ring_len ? ring_cnt[lane] : 0;
+    const int r1 = 32 + lane < ring_len ? ring_cnt[32 + lane] : 0;
+    const int base = ring_slot(ts, ring_len);
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const int di = 32 * half + lane;
+      const int slot = ring_back(base, di < nd ? dmin + di : 0, ring_len);
+      const int a = __shfl_sync(kFull, r0, slot & 31), b = __shfl_sync(kFull, r1, slot & 31);
+      const int v = di < nd && in_window(ts, dmin + di, lo, hi) ? (slot < 32 ? a : b) : 0;
+      if (half == 0) c.c0 = v; else c.c1 = v;
+    }
+    return c;
+  }
   const int base = ring_slot(ts, ring_len);
-  int c0 = 0, c1 = 0;
   if (lane < nd && in_window(ts, dmin + lane, lo, hi))
-    c0 = ring_cnt[ring_back(base, dmin + lane, ring_len)];
+    c.c0 = ring_cnt[ring_back(base, dmin + lane, ring_len)];
   if (32 + lane < nd && in_window(ts, dmin + 32 + lane, lo, hi))
-    c1 = ring_cnt[ring_back(base, dmin + 32 + lane, ring_len)];
+    c.c1 = ring_cnt[ring_back(base, dmin + 32 + lane, ring_len)];
+  return c;
+}
+
+__device__ __forceinline__ DuePrefix due_prefix_of(const DueCounts& c) {
   DuePrefix p;
-  p.incl0 = warp_incl_scan(c0);
+  p.incl0 = warp_incl_scan(c.c0);
   const int t0 = __shfl_sync(kFull, p.incl0, 31);
-  p.incl1 = warp_incl_scan(c1) + t0;
+  p.incl1 = warp_incl_scan(c.c1) + t0;
   p.total = __shfl_sync(kFull, p.incl1, 31);
   return p;
+}
+
+__device__ __forceinline__ DuePrefix due_prefix_warp(const int32_t* __restrict__ ring_cnt,
+                                                     int ring_len, int64_t ts, int dmin, int nd,
+                                                     int64_t lo, int64_t hi) {
+  return due_prefix_of(due_counts_warp(ring_cnt, ring_len, ts, dmin, nd, lo, hi));
 }
 
 // Delay index of due spike number sp (0 <= sp < total) and its rank within its slot.
@@ -140,8 +169,12 @@ __device__ __forceinline__ int find_delay_block(const int* s_pref, int nd, int s
 // call item together; len, the longest b1 - b0 of the warp's groups, is the same in every
 // lane.  WARP_PREFIX requires J.nd <= 64; otherwise every thread of the CTA must call this
 // (block prefix in s_pref, J.nd + 1 ints).
-template <bool WARP_PREFIX, int GROUP = 32, class Item>
-__device__ __forceinline__ void for_each_due_item(const ProjDev& J, int64_t ts, int64_t warp0,
+//
+// In a quiet step (no slot holds more due items than two rounds of its share of the warps) warps
+// are dealt out to the delays and take the slot's items in turn, without the prefix over the
+// counts and the search in it; a burst's items, all in few slots, go by the prefix to all warps.
+template <bool WARP_PREFIX, int GROUP = 32, class Proj_, class Item>
+__device__ __forceinline__ void for_each_due_item(const Proj_& J, int64_t ts, int64_t warp0,
                                                   int64_t nwarps, int* s_pref, Item item) {
   static_assert(GROUP == 32 || GROUP == 16 || GROUP == 8 || GROUP == 4 || GROUP == 2,
                 "group size");
@@ -149,17 +182,53 @@ __device__ __forceinline__ void for_each_due_item(const ProjDev& J, int64_t ts, 
   const int lane = threadIdx.x & 31;
   const int grp = lane / GROUP;
   DuePrefix wp{};
-  int nspk;
+  int nspk = 0;
+  const int base = ring_slot(ts, J.src_ring_len);
+  // one round of the warp: the lane's group takes item `it` (if any) of delay index di
+  auto round = [&](bool have, int di, int kk, int ch) {
+    int64_t b0 = 0, b1 = 0, head_key = -1;
+    int32_t pre = 0;
+    if (have) {
+      const int slot = ring_back(base, J.dmin + di, J.src_ring_len);
+      pre = J.src_ring_idx[(int64_t)slot * J.src_n + kk];
+      const int64_t key = (int64_t)pre * J.nd + di;
+      b0 = J.off[key] + (int64_t)ch * kChunk;
+      b1 = J.off[key + 1];
+      if (b1 > b0 + kChunk) b1 = b0 + kChunk;
+      if (ch == 0) head_key = key;
+    }
+    // rounds until the longest bundle of this warp's groups is done (warp-uniform)
+    int64_t len = b1 - b0;
+#pragma unroll
+    for (int o = 16; o >= GROUP; o >>= 1) len = max(len, __shfl_xor_sync(kFull, len, o));
+    item(b0, b1, len, pre, head_key);
+  };
   if constexpr (WARP_PREFIX) {
-    wp = due_prefix_warp(J.src_ring_cnt, J.src_ring_len, ts, J.dmin, J.nd, J.src_lo,
-                         J.src_hi);
+    const DueCounts c = due_counts_warp(J.src_ring_cnt, J.src_ring_len, ts, J.dmin, J.nd,
+                                        J.src_lo, J.src_hi);
+    const int most = __reduce_max_sync(kFull, max(c.c0, c.c1));
+    if (most == 0) return;
+    const int share = nwarps <= INT32_MAX ? (int)((uint32_t)nwarps / (uint32_t)J.nd) : 0;
+    if (share > 0 && (int64_t)most * J.chunks <= 2ll * share * G) {
+      const int di = (int)((uint32_t)warp0 / (uint32_t)share);
+      if (di >= J.nd) return;
+      const int a = __shfl_sync(kFull, c.c0, di & 31), b = __shfl_sync(kFull, c.c1, di & 31);
+      const int items = (di < 32 ? a : b) * J.chunks;
+      for (int r0 = ((int)warp0 - di * share) * G; r0 < items; r0 += share * G) {
+        const int it = r0 + grp;
+        const bool have = it < items;
+        const int kk = J.chunks == 1 ? it : it / J.chunks;
+        round(have, di, kk, have ? it - kk * J.chunks : 0);
+      }
+      return;
+    }
+    wp = due_prefix_of(c);
     nspk = wp.total;
   } else {
     nspk = due_prefix_block(J.src_ring_cnt, J.src_ring_len, ts, J.dmin, J.nd, J.src_lo,
                             J.src_hi, s_pref);
   }
   const int64_t items = (int64_t)nspk * J.chunks;
-  const int base = ring_slot(ts, J.src_ring_len);
   for (int64_t r0 = warp0 * G; r0 < items; r0 += nwarps * G) {
     const int64_t it = r0 + grp;
     const bool have = it < items;
@@ -182,22 +251,7 @@ __device__ __forceinline__ void for_each_due_item(const ProjDev& J, int64_t ts, 
     } else {
       di = find_delay_block(s_pref, J.nd, sp, &kk);
     }
-    int64_t b0 = 0, b1 = 0, head_key = -1;
-    int32_t pre = 0;
-    if (have) {
-      const int slot = ring_back(base, J.dmin + di, J.src_ring_len);
-      pre = J.src_ring_idx[(int64_t)slot * J.src_n + kk];
-      const int64_t key = (int64_t)pre * J.nd + di;
-      b0 = J.off[key] + (int64_t)ch * kChunk;
-      b1 = J.off[key + 1];
-      if (b1 > b0 + kChunk) b1 = b0 + kChunk;
-      if (ch == 0) head_key = key;
-    }
-    // rounds until the longest bundle of this warp's groups is done (warp-uniform)
-    int64_t len = b1 - b0;
-#pragma unroll
-    for (int o = 16; o >= GROUP; o >>= 1) len = max(len, __shfl_xor_sync(kFull, len, o));
-    item(b0, b1, len, pre, head_key);
+    round(have, di, kk, ch);
   }
 }
 
@@ -250,6 +304,34 @@ __device__ __forceinline__ void member_lookup(const ProjDev& J, int32_t pre, Mem
   const int m = member_of(J, pre);
   c.target = static_cast<R*>(J.targets[J.mem_var[m]]);
   c.w = J.mem_w ? (R)J.mem_w[m] : (R)J.w_scalar;
+}
+
+template <typename R>
+__device__ __forceinline__ void member_lookup(const AddDev& J, int32_t pre, MemberCache<R>& c) {
+  if (pre == c.pre) return;
+  c.pre = pre;
+  if (J.n_mem <= kInlineMembers) {
+    int var = J.in_var[0];
+    double w = J.in_w[0];
+#pragma unroll
+    for (int m = 1; m < kInlineMembers; ++m)
+      if (m < J.n_mem && pre >= J.in_hi[m - 1]) {
+        var = J.in_var[m];
+        w = J.in_w[m];
+      }
+    c.target = static_cast<R*>(var == B2B_VAR_V    ? J.targets[0]
+                               : var == B2B_VAR_GE ? J.targets[1]
+                                                   : J.targets[2]);
+    c.w = (R)w;
+    return;
+  }
+  int lo = 0, hi = J.n_mem - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (pre < J.mem_hi[mid]) hi = mid; else lo = mid + 1;
+  }
+  c.target = static_cast<R*>(J.targets[J.mem_var[lo]]);
+  c.w = J.mem_w ? (R)J.mem_w[lo] : (R)J.w_scalar;
 }
 
 }  // namespace b2b

@@ -359,9 +359,10 @@ hh_step_kernel(PopDev P, const int64_t* __restrict__ clock, int k, double dt,
 // stream, so one launch boundary orders step t+1 after both halves of step t, where the two
 // concurrent launches need a boundary each and dependencies across two streams.
 // E = 0: a HH neuron's variables in four warps (hh_split_body).
-template <typename R, int KIND, int E, int GROUP>
+template <typename R, int KIND, int E, int GROUP, int NP>
 __global__ void __launch_bounds__(kBlock, E <= 1 ? (sizeof(R) == 4 ? 5 : 4) : 3)
-one_launch_step_kernel(const __grid_constant__ PopDev U, const __grid_constant__ PendingDev F,
+one_launch_step_kernel(const __grid_constant__ PopDev U,
+                       const __grid_constant__ PendingArgs<NP> F,
                        const int64_t* __restrict__ clock, int k, double dt, int32_t* status,
                        int n_upd) {
   // chained launches (programmatic dependent launch): wait for the previous step's grid to
@@ -377,8 +378,8 @@ one_launch_step_kernel(const __grid_constant__ PopDev U, const __grid_constant__
     else
       lif_step_body<R, E, false>(U, clock, k, dt, status, blockIdx.x);
   } else {
-    deliver_pending_body<R, true, GROUP>(F, clock, k, (int64_t)blockIdx.x - n_upd,
-                                         (int64_t)gridDim.x - n_upd, nullptr);
+    deliver_pending_body<R, true, GROUP, NP>(F, clock, k, (int64_t)blockIdx.x - n_upd,
+                                             (int64_t)gridDim.x - n_upd, nullptr);
   }
 }
 
@@ -395,8 +396,11 @@ cudaError_t launch_one_g(const PopDev& U, const PendingDev& F, unsigned grid, in
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = chained ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, one_launch_step_kernel<R, KIND, E, GROUP>, U, F, clock, k,
-                            dt, status, n_upd);
+  if (F.n_proj == 1)
+    return cudaLaunchKernelEx(&cfg, one_launch_step_kernel<R, KIND, E, GROUP, 1>, U,
+                              pending_args<1>(F), clock, k, dt, status, n_upd);
+  return cudaLaunchKernelEx(&cfg, one_launch_step_kernel<R, KIND, E, GROUP, kMaxProjBatch>, U,
+                            pending_args<kMaxProjBatch>(F), clock, k, dt, status, n_upd);
 }
 
 template <typename R, int KIND, int E>

@@ -25,12 +25,12 @@ namespace b2b {
 namespace {
 
 // Bundles due at step clock+k (spikes of steps ts - d, d >= 1) added into acc[k & 1].
-template <typename R, bool WARP_PREFIX, int GROUP>
+template <typename R, bool WARP_PREFIX, int GROUP, int NP>
 __global__ void __launch_bounds__(kPendingBlock)
-deliver_pending_kernel(const __grid_constant__ PendingDev F, const int64_t* __restrict__ clock,
-                       int k) {
-  extern __shared__ int s_pref[];  // F.nd_max + 1 ints when !WARP_PREFIX
-  deliver_pending_body<R, WARP_PREFIX, GROUP>(F, clock, k, blockIdx.x, gridDim.x, s_pref);
+deliver_pending_kernel(const __grid_constant__ PendingArgs<NP> F,
+                       const int64_t* __restrict__ clock, int k) {
+  extern __shared__ int s_pref[];  // nd_max + 1 ints when !WARP_PREFIX
+  deliver_pending_body<R, WARP_PREFIX, GROUP, NP>(F, clock, k, blockIdx.x, gridDim.x, s_pref);
 }
 
 // Adds the input delivered in step clock+k_last into the target variables and zeroes it.
@@ -50,18 +50,26 @@ __global__ void fold_pending_kernel(const __grid_constant__ PendingDev F, int k_
   }
 }
 
+template <typename R, bool WP, int NP>
+cudaError_t launch_pending_n(const PendingDev& D, dim3 g, size_t smem, const int64_t* clock,
+                             int k, cudaStream_t s) {
+  const PendingArgs<NP> F = pending_args<NP>(D);
+  if (D.group == 16)
+    deliver_pending_kernel<R, WP, 16, NP><<<g, kPendingBlock, smem, s>>>(F, clock, k);
+  else if (D.group == 4)
+    deliver_pending_kernel<R, WP, 4, NP><<<g, kPendingBlock, smem, s>>>(F, clock, k);
+  else if (D.group == 2)
+    deliver_pending_kernel<R, WP, 2, NP><<<g, kPendingBlock, smem, s>>>(F, clock, k);
+  else
+    deliver_pending_kernel<R, WP, 8, NP><<<g, kPendingBlock, smem, s>>>(F, clock, k);
+  return cudaGetLastError();
+}
+
 template <typename R, bool WP>
 cudaError_t launch_pending_r(const PendingDev& F, dim3 g, size_t smem, const int64_t* clock,
                              int k, cudaStream_t s) {
-  if (F.group == 16)
-    deliver_pending_kernel<R, WP, 16><<<g, kPendingBlock, smem, s>>>(F, clock, k);
-  else if (F.group == 4)
-    deliver_pending_kernel<R, WP, 4><<<g, kPendingBlock, smem, s>>>(F, clock, k);
-  else if (F.group == 2)
-    deliver_pending_kernel<R, WP, 2><<<g, kPendingBlock, smem, s>>>(F, clock, k);
-  else
-    deliver_pending_kernel<R, WP, 8><<<g, kPendingBlock, smem, s>>>(F, clock, k);
-  return cudaGetLastError();
+  return F.n_proj == 1 ? launch_pending_n<R, WP, 1>(F, g, smem, clock, k, s)
+                       : launch_pending_n<R, WP, kMaxProjBatch>(F, g, smem, clock, k, s);
 }
 
 }  // namespace

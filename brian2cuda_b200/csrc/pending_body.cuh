@@ -12,17 +12,17 @@ constexpr int kPendingBlock = 256;
 constexpr int kPendingUnroll = 4;   // rounds of a bundle whose loads a lane issues together
 
 // The work of CTA `blk` of `nblk` delivering CTAs (blockDim.x threads each).
-template <typename R, bool WARP_PREFIX, int GROUP>
-__device__ __forceinline__ void deliver_pending_body(const PendingDev& F,
+template <typename R, bool WARP_PREFIX, int GROUP, int NP>
+__device__ __forceinline__ void deliver_pending_body(const PendingArgs<NP>& F,
                                                      const int64_t* __restrict__ clock, int k,
                                                      int64_t blk, int64_t nblk, int* s_pref) {
   const int64_t ts = clock[0] + k;
   const int64_t warp0 = (blk * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = (nblk * blockDim.x) >> 5;
-  const int64_t row = (int64_t)(k & 1) * F.pop.n;
+  const int64_t row = (int64_t)(k & 1) * F.n;
   const int glane = (threadIdx.x & 31) % GROUP;
-  for (int p = 0; p < F.n_proj; ++p) {
-    const ProjDev& J = F.proj[p];
+  for (int p = 0; p < (NP == 1 ? 1 : F.n_proj); ++p) {
+    const AddDev& J = F.proj[p];
     const R* W = static_cast<const R*>(J.w);
     MemberCache<R> mc;
     for_each_due_item<WARP_PREFIX, GROUP>(J, ts, warp0, nwarps, s_pref,

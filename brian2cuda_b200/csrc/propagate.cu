@@ -59,19 +59,21 @@ __device__ __forceinline__ void add_to_target(R* T, int32_t post, R w, bool vali
   }
 }
 
-// Several additive projections in one launch: blockIdx.y picks the projection.
-struct ProjBatch {
-  ProjDev p[kMaxProjBatch];
-  int n;
+// Several additive projections in one launch: blockIdx.y picks the projection.  (One projection,
+// the ordinary case, travels in a parameter block of its own size.)
+template <int NP>
+struct AddBatch {
+  AddDev p[NP];
 };
+using ProjBatch = AddBatch<kMaxProjBatch>;
 
 // ---- on_pre: target[post] += w -------------------------------------------------------------
-template <typename R, bool HAS_W, bool AGG, bool WARP_PREFIX, int GROUP>
+template <typename R, bool HAS_W, bool AGG, bool WARP_PREFIX, int GROUP, int NP>
 __global__ void __launch_bounds__(kDeliverBlock)
-deliver_add_batch_kernel(const __grid_constant__ ProjBatch B, const int64_t* __restrict__ clock,
-                         int k) {
+deliver_add_batch_kernel(const __grid_constant__ AddBatch<NP> B,
+                         const int64_t* __restrict__ clock, int k) {
   extern __shared__ int s_pref[];
-  const ProjDev& P = B.p[blockIdx.y];
+  const AddDev& P = B.p[NP == 1 ? 0 : blockIdx.y];
   const int64_t ts = clock[0] + k;
   const R* __restrict__ W = static_cast<const R*>(P.w);
   const int64_t warp0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -259,11 +261,22 @@ unsigned deliver_grid(const Proj& pr) {
 template <typename R, bool HAS_W, bool AGG, int GROUP>
 void launch_add_g(const ProjBatch& B, dim3 g, bool warp_prefix, size_t smem,
                   const int64_t* clock, int k, cudaStream_t s) {
+  if (g.y == 1) {
+    const AddBatch<1> one{{B.p[0]}};
+    if (warp_prefix)
+      deliver_add_batch_kernel<R, HAS_W, AGG, true, GROUP, 1>
+          <<<g, kDeliverBlock, 0, s>>>(one, clock, k);
+    else
+      deliver_add_batch_kernel<R, HAS_W, AGG, false, GROUP, 1>
+          <<<g, kDeliverBlock, smem, s>>>(one, clock, k);
+    return;
+  }
   if (warp_prefix)
-    deliver_add_batch_kernel<R, HAS_W, AGG, true, GROUP><<<g, kDeliverBlock, 0, s>>>(B, clock, k);
+    deliver_add_batch_kernel<R, HAS_W, AGG, true, GROUP, kMaxProjBatch>
+        <<<g, kDeliverBlock, 0, s>>>(B, clock, k);
   else
-    deliver_add_batch_kernel<R, HAS_W, AGG, false, GROUP><<<g, kDeliverBlock, smem, s>>>(B, clock,
-                                                                                         k);
+    deliver_add_batch_kernel<R, HAS_W, AGG, false, GROUP, kMaxProjBatch>
+        <<<g, kDeliverBlock, smem, s>>>(B, clock, k);
 }
 
 // Lanes per work item: 8 (four items in flight per warp, the default), 2, 4, 16 or 32.
@@ -320,7 +333,7 @@ deliver_cluster_kernel(const __grid_constant__ ProjBatch B,
   for (int i = 4 * threadIdx.x; i < A.slice; i += 4 * blockDim.x)
     *reinterpret_cast<float4*>(s_acc + i) = make_float4(0.f, 0.f, 0.f, 0.f);
   cl.sync();
-  const ProjDev& P = B.p[blockIdx.y];
+  const AddDev& P = B.p[blockIdx.y];
   const int64_t ts = clock[0] + k;
   const float* __restrict__ W = static_cast<const float*>(P.w);
   const int64_t warp0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -466,6 +479,38 @@ void launch_stdp_pre(const ProjDev& P, unsigned grid, bool ag, bool wp, size_t s
 
 }  // namespace
 
+AddDev add_dev(const Proj& pr) {
+  const ProjDev& D = pr.dev;
+  AddDev A{};
+  A.src_ring_cnt = D.src_ring_cnt;
+  A.src_ring_idx = D.src_ring_idx;
+  A.src_n = D.src_n;
+  A.src_ring_len = D.src_ring_len;
+  A.dmin = D.dmin;
+  A.nd = D.nd;
+  A.chunks = D.chunks;
+  A.src_lo = D.src_lo;
+  A.src_hi = D.src_hi;
+  A.off = D.off;
+  A.post = D.post;
+  A.w = D.w;
+  for (int v = 0; v < 3; ++v) A.targets[v] = D.targets[v];
+  A.n_mem = D.n_mem;
+  A.mem_hi = D.mem_hi;
+  A.mem_var = D.mem_var;
+  A.mem_w = D.mem_w;
+  A.w_scalar = D.w_scalar;
+  A.in_var[0] = pr.target_var;
+  A.in_w[0] = D.w_scalar;
+  if (D.n_mem > 1 && D.n_mem <= kInlineMembers)
+    for (int m = 0; m < D.n_mem; ++m) {
+      if (m < kInlineMembers - 1) A.in_hi[m] = (int32_t)pr.mem_hi[m];
+      A.in_var[m] = pr.mem_var[m];
+      A.in_w[m] = D.mem_w ? pr.mem_w[m] : D.w_scalar;
+    }
+  return A;
+}
+
 // A work item is a bundle (up to kChunk synapses): as many lanes as keep most of them busy, so
 // that short bundles leave lanes to other items and long ones need few dependent rounds.
 // Measured, us per step at 2 / 4 / 8 / 16 / 32 lanes: 80 synapses per bundle (CUBA 4000) 8.81 /
@@ -491,11 +536,10 @@ cudaError_t launch_proj_add_batch(const Proj* const* prs, int n, const int64_t* 
                                   cudaStream_t s, const AddTune* tune) {
   if (n <= 0 || n > kMaxProjBatch) return cudaErrorInvalidValue;
   ProjBatch B{};
-  B.n = n;
   unsigned grid = 1;
   int nd = 1;
   for (int i = 0; i < n; ++i) {
-    B.p[i] = prs[i]->dev;
+    B.p[i] = add_dev(*prs[i]);
     grid = std::max(grid, deliver_grid(*prs[i]));
     nd = std::max(nd, (int)prs[i]->dev.nd);
   }
