@@ -259,7 +259,7 @@ struct FusedDev {
   int64_t hi[kMaxProjBatch][kFusedMembers];
   int32_t var[kMaxProjBatch][kFusedMembers];
   int32_t n_proj;
-  int32_t spread;                 // warps that share one spike's bundle
+  int32_t pad;
   int32_t* cnt[3];                // per target variable (v, ge, gi): [2][pop.n] or NULL
 };
 
@@ -572,9 +572,10 @@ cudaError_t launch_one_launch_step(const Pop& pop, const PopDev& U, const Pendin
                                    int deliver_ctas, bool chained, const int64_t* clock, int k,
                                    double dt, int32_t* status, cudaStream_t s);
 cudaError_t launch_fold_pending(const PendingDev& F, int dtype, int k_last, cudaStream_t s);
-// The fused step of a population (view U: its counts as fold buffers), and the addition of the
+// The fused step of a population (view U: its counts as fold buffers; chained: with programmatic
+// dependent launch on the previous launch of the stream), and the addition of the
 // last step's counts at the end of a chunk.
-cudaError_t launch_fused_step(const Pop& pop, const PopDev& U, const FusedDev& F,
+cudaError_t launch_fused_step(const Pop& pop, const PopDev& U, const FusedDev& F, bool chained,
                               const int64_t* clock, int k, double dt, int32_t* status,
                               cudaStream_t s);
 cudaError_t launch_fold_counts(const Pop& pop, const PopDev& U, int k_last, cudaStream_t s);

@@ -7,10 +7,10 @@
 // spikes with one global atomicAdd per spike (threshold.cu:19-45), and the resetter over
 // the spiking indices (templates/reset.cu:3-27).  Here a thread owns E consecutive neurons:
 // E = 4 for large populations (each state array read with one 128-bit access, two for
-// float64), E = 1 when the population is too small to fill the GPU that way.  The CTA
-// compacts its spikes with warp shuffles and a shared-memory scan and reserves its output
-// range with a single atomicAdd on the step's slot of the spike-history ring (the streaming
-// kernel, which compacts once per pack iteration, does this per warp instead).
+// float64), E = 1 when the population is too small to fill the GPU that way.  A warp
+// compacts its spikes with shuffles and reserves its output range with a single atomicAdd on
+// the step's slot of the spike-history ring (the Poisson kernel, whose every warp may have
+// spikes in every step, does this per CTA instead).
 //
 // The reset is applied in the same pass when no synaptic effect of the population writes a
 // variable the reset writes; otherwise `late_reset` defers it to a kernel that runs after
@@ -24,6 +24,16 @@
 namespace b2b {
 
 namespace {
+// Waits until the previous launch of the stream has completed and its memory is visible
+// (programmatic dependent launch; nothing to wait for without that launch attribute).
+__device__ __forceinline__ void previous_launch_done() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+// Lets the next launch of the stream start its CTAs as room comes free.
+__device__ __forceinline__ void let_next_launch_start() {
+  asm volatile("griddepcontrol.launch_dependents;");
+}
+
 // Adds the input delivered during the previous step (fold buffer of variable v, the row that
 // step k-1 of the chunk filled) into pack X and returns the pack's address in the buffer, to be
 // cleared after the update's stores; no-op when the population has no fold buffer for v.  The
@@ -85,7 +95,10 @@ __device__ __forceinline__ void fold_clear(R* a, int64_t q) {
 // The work of CTA `blk` of the update (blockDim.x threads, E neurons each).
 // FUSED: the step's delivery is part of it (fused_step_kernel): the input pending from the step
 // before comes as event counts, and the CTA's spikes go through emit(q, fl, ts, slot).
-template <typename R, int E, bool INPUTS, bool FUSED = false, class Emit = int>
+// CHAINED: the launch may start before the previous one of the stream has ended (programmatic
+// dependent launch); what does not depend on it comes before previous_launch_done().
+template <typename R, int E, bool INPUTS, bool FUSED = false, bool CHAINED = false,
+          class Emit = int>
 __device__ __forceinline__ void lif_step_body(const PopDev& P, const int64_t* __restrict__ clock,
                                               int k, double dt, int32_t* status, int64_t blk,
                                               Emit emit = 0) {
@@ -96,10 +109,11 @@ __device__ __forceinline__ void lif_step_body(const PopDev& P, const int64_t* __
   const int64_t nthr = P.n / E;
   const int64_t q = blk * blockDim.x + threadIdx.x;
   unsigned fl = 0;
+  const LifDev* prm = static_cast<const LifDev*>(P.params);
+  const int grp = q < nthr ? group_of<E>(P, q) : 0;
+  const LifDev g = prm[grp];
+  if constexpr (CHAINED) previous_launch_done();
   if (q < nthr) {
-    const LifDev* prm = static_cast<const LifDev*>(P.params);
-    const int grp = group_of<E>(P, q);
-    const LifDev g = prm[grp];
     const GroupInputs* gin = INPUTS ? P.inputs + grp : nullptr;
     const bool after_reset = INPUTS && gin->pin.after_reset;
     const R Vt = (R)g.Vt, Vr = (R)g.Vr;
@@ -162,7 +176,7 @@ __device__ __forceinline__ void lif_step_body(const PopDev& P, const int64_t* __
     }
   }
   if constexpr (FUSED) emit(q, fl, ts, slot);
-  else emit_spikes<E>(P, q, fl, ts, slot, status);
+  else emit_spikes_warp<E>(P, q, fl, ts, slot, status);
   clear_next_slot(P, ts, blk);
 }
 
@@ -174,7 +188,8 @@ lif_step_kernel(PopDev P, const int64_t* __restrict__ clock, int k, double dt,
 }
 
 // ---- Hodgkin-Huxley (COBAHH), exponential Euler (hh_advance) ------------------------
-template <typename R, int E, bool INPUTS, bool FUSED = false, class Emit = int>
+template <typename R, int E, bool INPUTS, bool FUSED = false, bool CHAINED = false,
+          class Emit = int>
 __device__ __forceinline__ void hh_step_body(const PopDev& P, const int64_t* __restrict__ clock,
                                              int k, double dt, int32_t* status, int64_t blk,
                                              Emit emit = 0) {
@@ -185,10 +200,11 @@ __device__ __forceinline__ void hh_step_body(const PopDev& P, const int64_t* __r
   const int64_t nthr = P.n / E;
   const int64_t q = blk * blockDim.x + threadIdx.x;
   unsigned fl = 0;
+  const HhDev* prm = static_cast<const HhDev*>(P.params);
+  const int grp = q < nthr ? group_of<E>(P, q) : 0;
+  const HhRun<R> g = hh_run(prm[grp], R());
+  if constexpr (CHAINED) previous_launch_done();
   if (q < nthr) {
-    const HhDev* prm = static_cast<const HhDev*>(P.params);
-    const int grp = group_of<E>(P, q);
-    const HhRun<R> g = hh_run(prm[grp], R());
     const GroupInputs* gin = INPUTS ? P.inputs + grp : nullptr;
     const R Vthr = (R)g.Vthr, dtR = (R)dt;
     const bool refr = g.ref_steps >= 0;
@@ -247,7 +263,7 @@ __device__ __forceinline__ void hh_step_body(const PopDev& P, const int64_t* __r
     }
   }
   if constexpr (FUSED) emit(q, fl, ts, slot);
-  else emit_spikes<E>(P, q, fl, ts, slot, status);
+  else emit_spikes_warp<E>(P, q, fl, ts, slot, status);
   clear_next_slot(P, ts, blk);
 }
 
@@ -262,7 +278,7 @@ template <typename R>
 __device__ __forceinline__ int64_t split_neuron(int64_t blk) {
   return blk * (blockDim.x >> 2) + 32 * (threadIdx.x >> 7) + (threadIdx.x & 31);
 }
-template <typename R, bool FUSED = false, class Emit = int>
+template <typename R, bool FUSED = false, bool CHAINED = false, class Emit = int>
 __device__ __forceinline__ void hh_split_body(const PopDev& P, const int64_t* __restrict__ clock,
                                               int k, double dt, int32_t* status, int64_t blk,
                                               Emit emit = 0) {
@@ -274,6 +290,7 @@ __device__ __forceinline__ void hh_split_body(const PopDev& P, const int64_t* __
   const R dtR = (R)dt;
   HhRun<R> g{};
   if (mine) g = hh_run(static_cast<const HhDev*>(P.params)[group_of<1>(P, q)], R());
+  if constexpr (CHAINED) previous_launch_done();
   R v = 0;
   if (mine) v = static_cast<const R*>(P.var[B2B_VAR_V])[q];
   unsigned fl = 0;
@@ -334,7 +351,7 @@ __device__ __forceinline__ void hh_split_body(const PopDev& P, const int64_t* __
     }
   }
   if constexpr (FUSED) emit(q, fl, ts, slot);
-  else emit_spikes<1>(P, q, fl, ts, slot, status);
+  else emit_spikes_warp<1>(P, q, fl, ts, slot, status);
   clear_next_slot(P, ts, blk);
 }
 
@@ -365,20 +382,19 @@ one_launch_step_kernel(const __grid_constant__ PopDev U,
                        const __grid_constant__ PendingArgs<NP> F,
                        const int64_t* __restrict__ clock, int k, double dt, int32_t* status,
                        int n_upd) {
-  // chained launches (programmatic dependent launch): wait for the previous step's grid to
-  // complete and its memory to be visible, then let the next step's grid be scheduled, so its
-  // CTAs are resident by the time this one ends; without that launch attribute both are no-ops
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;");
+  // chained launches (programmatic dependent launch): the next step's CTAs come in as this one's
+  // leave, and each reads its parameters, the clock and its group's constants before it waits for
+  // the previous step's grid to complete; without that launch attribute both are no-ops
+  let_next_launch_start();
   if ((int)blockIdx.x < n_upd) {
     if constexpr (E == 0)
-      hh_split_body<R>(U, clock, k, dt, status, blockIdx.x);
+      hh_split_body<R, false, true>(U, clock, k, dt, status, blockIdx.x);
     else if constexpr (KIND == KIND_HH)
-      hh_step_body<R, E, false>(U, clock, k, dt, status, blockIdx.x);
+      hh_step_body<R, E, false, false, true>(U, clock, k, dt, status, blockIdx.x);
     else
-      lif_step_body<R, E, false>(U, clock, k, dt, status, blockIdx.x);
+      lif_step_body<R, E, false, false, true>(U, clock, k, dt, status, blockIdx.x);
   } else {
-    deliver_pending_body<R, true, GROUP, NP>(F, clock, k, (int64_t)blockIdx.x - n_upd,
+    deliver_pending_body<R, true, GROUP, NP, true>(F, clock, k, (int64_t)blockIdx.x - n_upd,
                                              (int64_t)gridDim.x - n_upd, nullptr);
   }
 }
@@ -441,54 +457,69 @@ __global__ void __launch_bounds__(kBlock)
 fused_step_kernel(const __grid_constant__ PopDev U, const __grid_constant__ FusedDev F,
                   const int64_t* __restrict__ clock, int k, double dt, int32_t* status) {
   constexpr int kMine = E > 0 ? E : 1;          // neurons per thread
-  constexpr int kList = E > 0 ? kBlock * E : kBlock / 4;
-  __shared__ int32_t s_list[kList];
-  // the bundle bounds of the CTA's own neurons are loaded with their state and kept for those
-  // that spike, so that a delivery starts at its targets
-  __shared__ int64_t s_b0[kList], s_b1[kList];
+  constexpr int kAhead = 2;                     // projections whose bundle bounds are loaded ahead
+  let_next_launch_start();
+  // the bundle bounds of this thread's neurons are loaded with its group's constants, so that a
+  // spike's delivery starts at its targets
   const int64_t q0 = E > 0 ? (int64_t)blockIdx.x * blockDim.x + threadIdx.x
                            : split_neuron<R>(blockIdx.x);
-  int64_t off[kMine + 1];
+  int64_t off[kAhead][kMine + 1];
 #pragma unroll
-  for (int e = 0; e <= kMine; ++e)
-    off[e] = q0 < U.n / kMine ? __ldg(F.proj[0].off + kMine * q0 + e) : 0;
-  auto deliver = [&](int total) {
-    const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  for (int p = 0; p < kAhead; ++p)
+#pragma unroll
+    for (int e = 0; e <= kMine; ++e)
+      off[p][e] = p < F.n_proj && q0 < U.n / kMine ? __ldg(F.proj[p].off + kMine * q0 + e) : 0;
+  // every warp delivers its own spikes, one after the other, its lanes over a bundle's targets
+  auto deliver = [&](int64_t q, unsigned fl) {
+    const int lane = threadIdx.x & 31;
     const int64_t row = (int64_t)(k & 1) * U.n;
-    for (int p = 0; p < F.n_proj; ++p) {
-      const ProjDev& J = F.proj[p];
-      for (int it = threadIdx.x >> 5; it < total * F.spread; it += warps) {
-        const int x = it / F.spread, part = it - x * F.spread;
-        const int32_t pre = s_list[x];
-        const int64_t b0 = p == 0 ? s_b0[x] : __ldg(J.off + pre);
-        const int64_t b1 = p == 0 ? s_b1[x] : __ldg(J.off + pre + 1);
-        if (b0 == b1) continue;
-        int var = F.var[p][0];
-        if (J.n_mem > kFusedMembers) {
-          var = J.mem_var[member_of(J, pre)];
-        } else {
 #pragma unroll
-          for (int m = 1; m < kFusedMembers; ++m)
-            if (m < J.n_mem && pre >= F.hi[p][m - 1]) var = F.var[p][m];
+    for (int e = 0; e < kMine; ++e) {
+      for (unsigned m = __ballot_sync(kFull, (fl >> e) & 1u); m; m &= m - 1) {
+        const int src = __ffs(m) - 1;
+        const int32_t pre = (int32_t)(kMine * __shfl_sync(kFull, q, src) + e);
+        for (int p = 0; p < F.n_proj; ++p) {
+          const ProjDev& J = F.proj[p];
+          int64_t b0, b1;
+          if (p < kAhead) {
+            b0 = __shfl_sync(kFull, p == 0 ? off[0][e] : off[1][e], src);
+            b1 = __shfl_sync(kFull, p == 0 ? off[0][e + 1] : off[1][e + 1], src);
+          } else {
+            b0 = __ldg(J.off + pre);
+            b1 = __ldg(J.off + pre + 1);
+          }
+          if (b0 == b1) continue;
+          int var = F.var[p][0];
+          if (J.n_mem > kFusedMembers) {
+            var = J.mem_var[member_of(J, pre)];
+          } else {
+#pragma unroll
+            for (int mm = 1; mm < kFusedMembers; ++mm)
+              if (mm < J.n_mem && pre >= F.hi[p][mm - 1]) var = F.var[p][mm];
+          }
+          int32_t* c = F.cnt[var] + row;
+          // four rounds' targets are loaded before their additions
+          for (int64_t s = b0 + lane; s < b1; s += 128) {
+            int32_t post[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) post[u] = s + 32 * u < b1 ? __ldg(J.post + s + 32 * u) : -1;
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+              if (post[u] >= 0) atomicAdd(c + post[u], 1);
+          }
         }
-        int32_t* c = F.cnt[var] + row;
-        for (int64_t s = b0 + 32 * part + lane; s < b1; s += 32 * F.spread)
-          atomicAdd(c + __ldg(J.post + s), 1);
       }
     }
   };
   auto emit = [&](int64_t q, unsigned fl, int64_t ts, int slot) {
-    emit_spikes_use<kMine>(U, q, fl, ts, slot, status, s_list, [&](int e, int pos) {
-      s_b0[pos] = off[e];
-      s_b1[pos] = off[e + 1];
-    }, deliver);
+    emit_spikes_warp<kMine>(U, q, fl, ts, slot, status, [&]() { deliver(q, fl); });
   };
   if constexpr (E == 0)
-    hh_split_body<R, true>(U, clock, k, dt, status, blockIdx.x, emit);
+    hh_split_body<R, true, true>(U, clock, k, dt, status, blockIdx.x, emit);
   else if constexpr (KIND == KIND_HH)
-    hh_step_body<R, E, false, true>(U, clock, k, dt, status, blockIdx.x, emit);
+    hh_step_body<R, E, false, true, true>(U, clock, k, dt, status, blockIdx.x, emit);
   else
-    lif_step_body<R, E, false, true>(U, clock, k, dt, status, blockIdx.x, emit);
+    lif_step_body<R, E, false, true, true>(U, clock, k, dt, status, blockIdx.x, emit);
 }
 
 // Adds the counts of the chunk's last step (row `row`) into the target variables.
@@ -508,16 +539,31 @@ __global__ void fold_counts_kernel(const __grid_constant__ PopDev U, int row) {
   }
 }
 
+template <typename R, int KIND, int E>
+cudaError_t launch_fused_e(const PopDev& U, const FusedDev& F, unsigned grid, int block,
+                           bool chained, const int64_t* clock, int k, double dt, int32_t* status,
+                           cudaStream_t s) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = chained ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, fused_step_kernel<R, KIND, E>, U, F, clock, k, dt, status);
+}
 template <typename R, int KIND>
-void launch_fused_rk(const PopDev& U, const FusedDev& F, int e, unsigned grid, int block,
-                     const int64_t* clock, int k, double dt, int32_t* status, cudaStream_t s) {
+cudaError_t launch_fused_rk(const PopDev& U, const FusedDev& F, int e, unsigned grid, int block,
+                            bool chained, const int64_t* clock, int k, double dt,
+                            int32_t* status, cudaStream_t s) {
   if constexpr (KIND == KIND_HH && sizeof(R) == 8)
-    if (e == 0) {
-      fused_step_kernel<R, KIND, 0><<<grid, block, 0, s>>>(U, F, clock, k, dt, status);
-      return;
-    }
-  if (e == 2) fused_step_kernel<R, KIND, 2><<<grid, block, 0, s>>>(U, F, clock, k, dt, status);
-  else fused_step_kernel<R, KIND, 1><<<grid, block, 0, s>>>(U, F, clock, k, dt, status);
+    if (e == 0)
+      return launch_fused_e<R, KIND, 0>(U, F, grid, block, chained, clock, k, dt, status, s);
+  if (e == 2)
+    return launch_fused_e<R, KIND, 2>(U, F, grid, block, chained, clock, k, dt, status, s);
+  return launch_fused_e<R, KIND, 1>(U, F, grid, block, chained, clock, k, dt, status, s);
 }
 
 // Large HH populations: a persistent grid (resident CTAs only) walks the population in
@@ -845,21 +891,20 @@ cudaError_t launch_one_launch_step(const Pop& pop, const PopDev& U, const Pendin
                                             status, n_upd, s);
 }
 
-cudaError_t launch_fused_step(const Pop& pop, const PopDev& U, const FusedDev& F,
+cudaError_t launch_fused_step(const Pop& pop, const PopDev& U, const FusedDev& F, bool chained,
                               const int64_t* clock, int k, double dt, int32_t* status,
                               cudaStream_t s) {
   const UpdateShape shape = update_shape(pop, U.n);
-  const int e = shape.split ? 0 : shape.e >= 2 ? 2 : 1, block = shape.block;
+  const int e = shape.split ? 0 : shape.e >= 2 ? 2 : 1, b = shape.block;
   const unsigned grid = update_grid(shape, e, U.n);
   const bool f32 = pop.dtype == B2B_F32;
-  if (pop.kind == KIND_HH) {
-    if (f32) launch_fused_rk<float, KIND_HH>(U, F, e, grid, block, clock, k, dt, status, s);
-    else launch_fused_rk<double, KIND_HH>(U, F, e, grid, block, clock, k, dt, status, s);
-  } else {
-    if (f32) launch_fused_rk<float, KIND_LIF>(U, F, e, grid, block, clock, k, dt, status, s);
-    else launch_fused_rk<double, KIND_LIF>(U, F, e, grid, block, clock, k, dt, status, s);
-  }
-  return cudaGetLastError();
+  if (pop.kind == KIND_HH)
+    return f32 ? launch_fused_rk<float, KIND_HH>(U, F, e, grid, b, chained, clock, k, dt, status, s)
+               : launch_fused_rk<double, KIND_HH>(U, F, e, grid, b, chained, clock, k, dt, status,
+                                                  s);
+  return f32 ? launch_fused_rk<float, KIND_LIF>(U, F, e, grid, b, chained, clock, k, dt, status, s)
+             : launch_fused_rk<double, KIND_LIF>(U, F, e, grid, b, chained, clock, k, dt, status,
+                                                 s);
 }
 
 cudaError_t launch_fold_counts(const Pop& pop, const PopDev& U, int k_last, cudaStream_t s) {

@@ -12,7 +12,8 @@ constexpr int kPendingBlock = 256;
 constexpr int kPendingUnroll = 4;   // rounds of a bundle whose loads a lane issues together
 
 // The work of CTA `blk` of `nblk` delivering CTAs (blockDim.x threads each).
-template <typename R, bool WARP_PREFIX, int GROUP, int NP>
+// CHAINED: in a launch that may start before the previous step's has ended.
+template <typename R, bool WARP_PREFIX, int GROUP, int NP, bool CHAINED = false>
 __device__ __forceinline__ void deliver_pending_body(const PendingArgs<NP>& F,
                                                      const int64_t* __restrict__ clock, int k,
                                                      int64_t blk, int64_t nblk, int* s_pref) {
@@ -21,6 +22,14 @@ __device__ __forceinline__ void deliver_pending_body(const PendingArgs<NP>& F,
   const int64_t nwarps = (nblk * blockDim.x) >> 5;
   const int64_t row = (int64_t)(k & 1) * F.n;
   const int glane = (threadIdx.x & 31) % GROUP;
+  if constexpr (CHAINED) {
+    // the projection's fields and the clock are in registers before the wait
+    const AddDev& J = F.proj[0];
+    asm volatile("" ::"l"(J.src_ring_cnt), "l"(J.src_ring_idx), "l"(J.src_n), "r"(J.src_ring_len),
+                 "r"(J.dmin), "r"(J.nd), "r"(J.chunks), "l"(J.src_lo), "l"(J.src_hi), "l"(J.off),
+                 "l"(J.post), "l"(ts));
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+  }
   for (int p = 0; p < (NP == 1 ? 1 : F.n_proj); ++p) {
     const AddDev& J = F.proj[p];
     const R* W = static_cast<const R*>(J.w);
