@@ -1240,6 +1240,10 @@ b2b_status enqueue_steps(b2b_net* net, int kk) {
   }
   cudaStream_t s = net->stream;
   const bool fused = fused_in_use(net);
+  // launches within the chunk are chained to the one before them on the stream (the first of a
+  // chunk follows other work); not when every launch is timed or checked by itself
+  const bool may_chain = !net->prof_ev && !(net->cfg.flags & B2B_NET_CHECKED);
+  bool chained = false;
   for (int k = 0; k < kk; ++k) {
     if (fused) {
       // the first step of a chunk follows other kernels, and a rate monitor's launch the step's
@@ -1262,55 +1266,75 @@ b2b_status enqueue_steps(b2b_net* net, int kk) {
                          k, net->d_status, s));
       CU(prof_mark(net, k, si++, 1, s));
       ++net->launches;
+      chained = may_chain;
     }
-    // the populations' updates of a step are independent: the first on the net's stream,
-    // the others side by side on their own streams, joined before the deliveries
+    // the populations' updates of a step are independent: a driving and a driven one in one
+    // launch, else the first on the net's stream and the others side by side on their own
+    // streams, joined before the deliveries
     const size_t np = net->pops.size();
-    const bool fork = np > 1 && net->pop_streams.size() + 1 == np;
-    if (fork) {
-      CU(cudaEventRecord(net->ev_pop_fork, s));
-      for (cudaStream_t ps : net->pop_streams) CU(cudaStreamWaitEvent(ps, net->ev_pop_fork, 0));
-    }
-    for (size_t p = 0; p < np; ++p) {
-      cudaStream_t ps = fork && p > 0 ? net->pop_streams[p - 1] : s;
-      CU(prof_mark(net, k, si, 0, ps));
-      CU(launch_pop_step(net->pops[p], net->d_clock, k, net->cfg.dt, net->d_status, ps));
-      CU(prof_mark(net, k, si++, 1, ps));
+    const int pair_a = np == 2 && may_chain
+                           ? (pair_supported(net->pops[0], net->pops[1])   ? 0
+                              : pair_supported(net->pops[1], net->pops[0]) ? 1
+                                                                           : -1)
+                           : -1;
+    if (pair_a >= 0) {
+      CU(launch_pair_step(net->pops[pair_a], net->pops[1 - pair_a], net->d_clock, k, net->cfg.dt,
+                          net->d_status, s, chained));
       ++net->launches;
-    }
-    if (fork)
-      for (size_t p = 1; p < np; ++p) {
-        CU(cudaEventRecord(net->ev_pop_join[p - 1], net->pop_streams[p - 1]));
-        CU(cudaStreamWaitEvent(s, net->ev_pop_join[p - 1], 0));
+      si += 2;
+      chained = may_chain;
+    } else {
+      const bool fork = np > 1 && net->pop_streams.size() + 1 == np;
+      if (fork) {
+        CU(cudaEventRecord(net->ev_pop_fork, s));
+        for (cudaStream_t ps : net->pop_streams) CU(cudaStreamWaitEvent(ps, net->ev_pop_fork, 0));
       }
+      for (size_t p = 0; p < np; ++p) {
+        cudaStream_t ps = fork && p > 0 ? net->pop_streams[p - 1] : s;
+        CU(prof_mark(net, k, si, 0, ps));
+        CU(launch_pop_step(net->pops[p], net->d_clock, k, net->cfg.dt, net->d_status, ps));
+        CU(prof_mark(net, k, si++, 1, ps));
+        ++net->launches;
+        chained = may_chain && !fork;   // the launch after a join waits for several
+      }
+      if (fork)
+        for (size_t p = 1; p < np; ++p) {
+          CU(cudaEventRecord(net->ev_pop_join[p - 1], net->pop_streams[p - 1]));
+          CU(cudaStreamWaitEvent(s, net->ev_pop_join[p - 1], 0));
+        }
+    }
     for (size_t b = 0; b < net->add_batches.size(); ++b) {
       const auto& B = net->add_batches[b];
       CU(prof_mark(net, k, si, 0, s));
       CU(launch_proj_add_batch(B.data(), (int)B.size(), net->d_clock, k, s,
-                               b < net->add_tune.size() ? &net->add_tune[b] : nullptr));
+                               b < net->add_tune.size() ? &net->add_tune[b] : nullptr, chained));
       CU(prof_mark(net, k, si++, 1, s));
       ++net->launches;
+      chained = may_chain;
     }
     for (const Proj& pr : net->projs) {
       if (pr.effect != B2B_EFFECT_STDP) continue;
       CU(prof_mark(net, k, si, 0, s));
-      CU(launch_proj_pre(pr, net->d_clock, k, net->cfg.dt, net->d_status, s));
+      CU(launch_proj_pre(pr, net->d_clock, k, net->cfg.dt, net->d_status, s, chained));
       CU(prof_mark(net, k, si++, 1, s));
       ++net->launches;
+      chained = may_chain;
     }
     for (const Proj& pr : net->projs) {
       if (pr.effect != B2B_EFFECT_STDP) continue;
       CU(prof_mark(net, k, si, 0, s));
-      CU(launch_proj_post(pr, net->d_clock, k, net->cfg.dt, net->d_status, s));
+      CU(launch_proj_post(pr, net->d_clock, k, net->cfg.dt, net->d_status, s, chained));
       CU(prof_mark(net, k, si++, 1, s));
       ++net->launches;
+      chained = may_chain;
     }
     for (const Pop& pop : net->pops) {
       if (!pop.late_reset) continue;
       CU(prof_mark(net, k, si, 0, s));
-      CU(launch_pop_late_reset(pop, net->d_clock, k, s));
+      CU(launch_pop_late_reset(pop, net->d_clock, k, s, chained));
       CU(prof_mark(net, k, si++, 1, s));
       ++net->launches;
+      chained = may_chain;
     }
     if (!net->rmons.empty()) {
       CU(prof_mark(net, k, si, 0, s));
@@ -1318,6 +1342,7 @@ b2b_status enqueue_steps(b2b_net* net, int kk) {
                         s));
       CU(prof_mark(net, k, si++, 1, s));
       ++net->launches;
+      chained = may_chain;
     }
   }
   if (fused) {

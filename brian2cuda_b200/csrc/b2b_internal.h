@@ -517,15 +517,22 @@ cudaError_t launch_pop_step(const Pop& pop, const int64_t* clock, int k, double 
 // The same with another device view of the population (its fold buffers set).
 cudaError_t launch_pop_step_dev(const Pop& pop, const PopDev& dev, const int64_t* clock, int k,
                                 double dt, int32_t* status, cudaStream_t s);
+// Two populations of a step in one launch: a source without state (Poisson, spike generator) and a
+// LIF or HH population, both of built-in shapes and without inputs.  (chained, here and below: a
+// programmatic dependent launch on the previous kernel of the stream.)
+bool pair_supported(const Pop& a, const Pop& b);
+cudaError_t launch_pair_step(const Pop& a, const Pop& b, const int64_t* clock, int k, double dt,
+                             int32_t* status, cudaStream_t s, bool chained);
 cudaError_t launch_pop_late_reset(const Pop& pop, const int64_t* clock, int k,
-                                  cudaStream_t s);
+                                  cudaStream_t s, bool chained = false);
 cudaError_t launch_proj_pre(const Proj& pr, const int64_t* clock, int k, double dt,
-                            int32_t* status, cudaStream_t s);
+                            int32_t* status, cudaStream_t s, bool chained = false);
 cudaError_t launch_proj_post(const Proj& pr, const int64_t* clock, int k, double dt,
-                             int32_t* status, cudaStream_t s);
+                             int32_t* status, cudaStream_t s, bool chained = false);
 // One launch for n (<= kMaxProjBatch) additive projections of equal dtype / weight mode.
 cudaError_t launch_proj_add_batch(const Proj* const* prs, int n, const int64_t* clock, int k,
-                                  cudaStream_t s, const AddTune* tune = nullptr);
+                                  cudaStream_t s, const AddTune* tune = nullptr,
+                                  bool chained = false);
 // Lanes per work item of an additive delivery without tuning: for the per-step launch of
 // bundles of mean_bundle synapses, and for the delivery into the pending input (n neurons).
 int delivery_lanes(double mean_bundle);

@@ -65,6 +65,35 @@ __device__ __forceinline__ int block_exclusive_scan(int c, int* s_warp, int* tot
   return s_warp[warp] + x - c;
 }
 
+// Programmatic dependent launch: a kernel launched chained (launch_kernel) may start while the
+// previous one of its stream still runs.  It waits for that one's completion, and the visibility
+// of its memory, in previous_launch_done(), which every thread of every CTA calls before it touches
+// anything a kernel of the step writes; launched ordinarily there is nothing to wait for.  Ahead
+// of it a kernel may read what stays as it is for a chunk of steps: its parameters, the clock,
+// constants, random numbers.  A kernel that calls let_next_launch_start() lets the next one's CTAs
+// in as room comes free.
+__device__ __forceinline__ void previous_launch_done() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void let_next_launch_start() {
+  asm volatile("griddepcontrol.launch_dependents;");
+}
+template <class... KernelArgs, class... Args>
+inline cudaError_t launch_kernel(void (*kernel)(KernelArgs...), dim3 grid, int block, size_t smem,
+                                 cudaStream_t s, bool chained, const Args&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = chained ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, KernelArgs(args)...);
+}
+
 // Floor modulo of a (possibly negative) step by the ring length.  Every kernel of a step
 // starts with it, so steps below 2^31 (all but days of simulated time) take the 32-bit
 // remainder: a 64-bit one is a long serial sequence in software.

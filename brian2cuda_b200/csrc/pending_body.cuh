@@ -28,7 +28,7 @@ __device__ __forceinline__ void deliver_pending_body(const PendingArgs<NP>& F,
     asm volatile("" ::"l"(J.src_ring_cnt), "l"(J.src_ring_idx), "l"(J.src_n), "r"(J.src_ring_len),
                  "r"(J.dmin), "r"(J.nd), "r"(J.chunks), "l"(J.src_lo), "l"(J.src_hi), "l"(J.off),
                  "l"(J.post), "l"(ts));
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    previous_launch_done();
   }
   for (int p = 0; p < (NP == 1 ? 1 : F.n_proj); ++p) {
     const AddDev& J = F.proj[p];
