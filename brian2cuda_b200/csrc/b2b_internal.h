@@ -195,6 +195,22 @@ struct AddDev {
   double w_scalar;
 };
 
+// An additive projection delivered by counting (counted.cu): per class, the synapses onto one
+// target variable, the CTAs that count its events, the sums of their counts (16 bits per target,
+// zero between deliveries) and the weight.
+struct CountedDev {
+  AddDev add;
+  int64_t n;                          // targets (padded)
+  int32_t words;                      // 64-bit words of counts, four targets each
+  int32_t n_class;
+  int32_t cta_lo[4];                  // class c: CTAs [cta_lo[c], cta_lo[c + 1])
+  int32_t var[3];
+  int32_t per_round[3];               // due items a CTA of the class looks through at a time
+  void* target[3];
+  double w[3];
+  unsigned long long* sums[3];
+};
+
 // Device view of a state monitor (monitor.cu): variable src (es-byte elements) of the
 // population rows idx[0..n_idx), one record [n_idx] per step divisible by `every`.
 struct StateMonDev {
@@ -407,6 +423,8 @@ struct Proj {
   int64_t retire_after = -1;
   uint8_t var_mask = 0;                      // bit v: some member adds into variable v
   int64_t dst_n = 0;                         // padded size of the target population
+  bool counted_ok = false;                   // delivered by counting (setup_counted)
+  CountedDev counted{};
 };
 
 }  // namespace b2b
@@ -533,6 +551,15 @@ cudaError_t launch_proj_post(const Proj& pr, const int64_t* clock, int k, double
 cudaError_t launch_proj_add_batch(const Proj* const* prs, int n, const int64_t* clock, int k,
                                   cudaStream_t s, const AddTune* tune = nullptr,
                                   bool chained = false);
+// Delivery by counting (counted.cu): whether such a launch takes it, its two launches, whether
+// n_targets and n_delays fit, and the largest in-degree of n_syn synapses.
+bool counted_in_use(const Proj* const* prs, int n, const AddTune* tune);
+cudaError_t launch_counted(const Proj& pr, const int64_t* clock, int k, cudaStream_t s,
+                           bool chained);
+bool counted_fits(int64_t n_targets, int32_t n_delays);
+cudaError_t largest_in_degree(const int32_t* d_post, int64_t n_syn, int64_t n_targets,
+                              int64_t* largest, cudaStream_t s);
+AddDev add_dev(const Proj& pr);
 // Lanes per work item of an additive delivery without tuning: for the per-step launch of
 // bundles of mean_bundle synapses, and for the delivery into the pending input (n neurons).
 int delivery_lanes(double mean_bundle);

@@ -552,6 +552,12 @@ bool chained_delivery(int64_t n_syn) { return n_syn <= (int64_t)1 << 25; }
 cudaError_t launch_proj_add_batch(const Proj* const* prs, int n, const int64_t* clock, int k,
                                   cudaStream_t s, const AddTune* tune, bool chained) {
   if (n <= 0 || n > kMaxProjBatch) return cudaErrorInvalidValue;
+  if (counted_in_use(prs, n, tune)) {
+    cudaError_t e = cudaSuccess;
+    for (int i = 0; i < n && e == cudaSuccess; ++i)
+      e = launch_counted(*prs[i], clock, k, s, chained || i > 0);
+    return e;
+  }
   ProjBatch B{};
   unsigned grid = 1;
   int nd = 1;
