@@ -126,11 +126,13 @@ __device__ __forceinline__ int find_delay_lane(const DuePrefix& p, int sp, int* 
 }
 
 // Per-CTA prefix in shared memory (any nd): s_pref[0] = 0, s_pref[i] = counts of delay
-// indices < i.  Every thread of the CTA must call this.
+// indices < i.  Every thread of the CTA must call this.  The barrier in front: warps may still be
+// at the items of another projection, whose prefix stood in s_pref.
 __device__ __forceinline__ int due_prefix_block(const int32_t* __restrict__ ring_cnt,
                                                 int ring_len, int64_t ts, int dmin, int nd,
                                                 int64_t lo, int64_t hi, int* s_pref) {
   const int base = ring_slot(ts, ring_len);
+  __syncthreads();
   for (int di = threadIdx.x; di < nd; di += blockDim.x)
     s_pref[di + 1] = in_window(ts, dmin + di, lo, hi)
                          ? ring_cnt[ring_back(base, dmin + di, ring_len)] : 0;
