@@ -1102,11 +1102,80 @@ int builtin_pending_lanes(const b2b_net* net) {
   return pending_lanes(big ? big->mean_bundle : 0, net->pops[0].n);
 }
 
-// Populations up to this size run the two concurrent launches unless tuned otherwise
-// (measured: 1e5 HH neurons 38.6 vs 50.9 ms per simulated second).  Above it the pending
-// input's read and clear (16 B per neuron and step for ge and gi in float32) costs more HBM
-// time than the overlap saves: 3.9e6 HH neurons 70.1 vs 62.2 us per step.
-constexpr int64_t kAutoTwoLaunchMaxNeurons = 1 << 18;
+// CTAs of that launch: two per SM leave the update room; where the population is large its
+// update's waves pass anyway, and a third per SM shortens the delivery (at 2 / 3 / 4 per SM:
+// COBAHH 100,000 4.22 / 4.28 / 4.38 us per step, CUBA 150,000 4.05 / 4.12 / 4.41; merged
+// networks of 245,000 6.88 / 6.49 / 6.89, 460,000 10.3 / 9.8 / 10.1, 613,000 13.2 / 12.5 / 12.7).
+int pending_ctas(const b2b_net* net, int sms) {
+  return (net->pops[0].n >= kPendingLarge ? 3 : 2) * sms;
+}
+
+// Populations up to this size run the two concurrent launches unless tuned otherwise.  Above it
+// the pending input's read and clear (16 B per neuron and step for ge and gi in float32) cost more
+// than the overlap saves.  us per step, per-step form / two launches: HH f32 245,000 10.4 / 8.5,
+// 613,000 18.5 / 15.3, 920,000 28.4 / 25.8, 1.4e6 43.5 / 43.4, 2.1e6 63.9 / 67.1 (merged networks'
+// first 100 steps); LIF f32 600,000 8.6 / 7.0, 1.2e6 11.2 / 9.7, f64 600,000 10.9 / 8.8, 1.2e6
+// 14.9 / 15.5.
+// Up to kSumTwoLaunchMax the pending input is a sum of weights; beyond, event counts where those do
+// (count_pending), else the per-step form.
+constexpr int64_t kSumTwoLaunchMax = 1 << 18;
+int64_t auto_two_launch_max(int dtype) { return dtype == B2B_F32 ? 1 << 20 : 3 << 18; }
+constexpr int64_t kFusedMaxNeurons = 1 << 18;
+
+// The delivery and the update of the two launches, by event counts where net->count_gw says so
+// (the one-launch form has sums of weights).
+PendingDev pending_view(const b2b_net* net) {
+  PendingDev F = net->pdev;
+  if (net->count_gw && !net->one_launch) {
+    for (int p = 0; p < F.n_proj; ++p) {
+      F.proj[p].mem_w = nullptr;
+      F.proj[p].w_scalar = 1;
+      for (double& x : F.proj[p].in_w) x = 1;
+    }
+    F.pop.fold_gw = net->count_gw;
+  }
+  return F;
+}
+PopDev fold_view(const b2b_net* net) {
+  PopDev P = net->fold_dev;
+  if (net->count_gw && !net->one_launch) P.fold_gw = net->count_gw;
+  return P;
+}
+
+// Makes the pending input event counts (pending.cu) where all synapses of a group onto a variable
+// have one weight and no in-degree exceeds what a float32 counts exactly.
+b2b_status count_pending(b2b_net* net, bool* counted) {
+  *counted = false;
+  const Pop& pop = net->pops[0];
+  std::vector<double> w(3 * pop.groups.size(), 0);
+  std::vector<bool> seen(w.size(), false);
+  for (const Proj& pr : net->projs) {
+    if (pr.dev.w) return B2B_OK;
+    for (int m : pr.members) {
+      const Syn& sy = net->syns[m];
+      const size_t grp = (size_t)(std::find(pop.groups.begin(), pop.groups.end(), sy.post_gid) -
+                                  pop.groups.begin());
+      const size_t at = 3 * grp + (size_t)sy.target_var;
+      if (grp >= pop.groups.size() || (seen[at] && w[at] != sy.w_scalar)) return B2B_OK;
+      seen[at] = true;
+      w[at] = sy.w_scalar;
+    }
+  }
+  int64_t in_degree = 0;
+  for (const Proj& pr : net->projs) {
+    int64_t most = 0;
+    CU(largest_in_degree(pr.post, pr.n_syn, pr.dst_n, &most, net->stream));
+    in_degree += most;
+  }
+  if (in_degree > 1 << 20) return B2B_OK;   // (delay changes add projections for a while)
+  double* d = nullptr;
+  CU(cudaMalloc(&d, sizeof(double) * w.size()));
+  net->pending_allocs.push_back(d);
+  CU(cudaMemcpy(d, w.data(), sizeof(double) * w.size(), cudaMemcpyHostToDevice));
+  net->count_gw = d;
+  *counted = true;
+  return B2B_OK;
+}
 
 // The step as two concurrent launches (pending.cu) applies when the net is one LIF/HH
 // population (no gating surrogate, no state or rate monitor) whose synapses are all additive
@@ -1151,10 +1220,14 @@ b2b_status setup_two_launch(b2b_net* net) {
     }
     F.proj[p].targets[pr.target_var] = F.acc[pr.target_var];
   }
+  bool counted = false;
+  if (pop.n > kSumTwoLaunchMax && pop.n <= auto_two_launch_max(pop.dtype) &&
+      !(flags & (B2B_NET_TWO_LAUNCH | B2B_NET_ONE_LAUNCH)))
+    if (b2b_status st = count_pending(net, &counted)) return st;
   int sms = kNumSMs;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, net->cfg.device);
   F.group = builtin_pending_lanes(net);
-  net->pending_grid = 2 * sms;
+  net->pending_grid = pending_ctas(net, sms);
   // the update launch is the per-step neuron kernel, adding in the input that the previous
   // step's delivery left in acc
   net->fold_dev = pop.dev;
@@ -1165,7 +1238,7 @@ b2b_status setup_two_launch(b2b_net* net) {
   CU(cudaEventCreateWithFlags(&net->ev_d[1], cudaEventDisableTiming));
   net->two_launch_ok = true;
   net->two_launch = (flags & (B2B_NET_TWO_LAUNCH | B2B_NET_ONE_LAUNCH)) ||
-                    pop.n <= kAutoTwoLaunchMaxNeurons;
+                    pop.n <= kSumTwoLaunchMax || counted;
   net->one_launch_ok = one_launch_supported(pop, F);
   // delivering CTAs of the one-launch step: 1.5 per SM (in CTAs of kBlock threads) still fit
   // beside the update's in one wave for the populations this form is built for
@@ -1191,7 +1264,7 @@ void setup_fused(b2b_net* net) {
     return;
   const Pop& pop = net->pops[0];
   if ((pop.kind != KIND_LIF && pop.kind != KIND_HH) || pop.surr_img || pop.inputs ||
-      pop.late_reset || pop.n > kAutoTwoLaunchMaxNeurons)
+      pop.late_reset || pop.n > kFusedMaxNeurons)
     return;
   FusedDev& F = net->fused;
   PopDev& U = net->fused_pop;
@@ -1294,24 +1367,26 @@ b2b_status enqueue_steps(b2b_net* net, int kk) {
     // The deliveries run on the second stream; under stream capture this is a graph with
     // two branches per step.  Profiling sites: 0 the delivery, 1 the update.
     const Pop& pop = net->pops[0];
+    const PendingDev pending = pending_view(net);
+    const PopDev folding = fold_view(net);
     cudaStream_t s = net->stream, s2 = net->stream2;
     CU(cudaEventRecord(net->ev_n, s));
     for (int k = 0; k < kk; ++k) {
       CU(cudaStreamWaitEvent(s2, net->ev_n, 0));
       CU(prof_mark(net, k, 0, 0, s2));
-      CU(launch_pending_delivery(net->pdev, pop.dtype, net->pending_grid, net->d_clock, k, s2));
+      CU(launch_pending_delivery(pending, pop.dtype, net->pending_grid, net->d_clock, k, s2));
       CU(prof_mark(net, k, 0, 1, s2));
       CU(cudaEventRecord(net->ev_d[k & 1], s2));
       if (k > 0) CU(cudaStreamWaitEvent(s, net->ev_d[(k - 1) & 1], 0));
       CU(prof_mark(net, k, 1, 0, s));
-      CU(launch_pop_step_dev(pop, net->fold_dev, net->d_clock, k, net->cfg.dt, net->d_status,
+      CU(launch_pop_step_dev(pop, folding, net->d_clock, k, net->cfg.dt, net->d_status,
                              s));
       CU(prof_mark(net, k, 1, 1, s));
       CU(cudaEventRecord(net->ev_n, s));
       net->launches += 2;
     }
     CU(cudaStreamWaitEvent(s, net->ev_d[(kk - 1) & 1], 0));
-    CU(launch_fold_pending(net->pdev, pop.dtype, kk - 1, s));
+    CU(launch_fold_pending(pending, pop.dtype, kk - 1, s));
     CU(launch_tick(net->d_clock, kk, s));
     net->launches += 2;
     return B2B_OK;
@@ -2260,7 +2335,7 @@ b2b_status b2b_profile(b2b_net* net, int64_t n_steps, double* mean_ms, int32_t* 
       cudaError_t e = cudaSuccess;
       const int64_t* clk = net->d_clock;
       if (s.kind == 1)
-        e = launch_pop_step_dev(net->pops[s.idx], net->two_launch ? net->fold_dev : net->pops[s.idx].dev,
+        e = launch_pop_step_dev(net->pops[s.idx], net->two_launch ? fold_view(net) : net->pops[s.idx].dev,
                                 clk, 0, net->cfg.dt, net->d_status, net->stream);
       if (s.kind == 6)
         e = launch_proj_add_batch(net->add_batches[s.idx].data(), (int)net->add_batches[s.idx].size(),
@@ -2280,7 +2355,7 @@ b2b_status b2b_profile(b2b_net* net, int64_t n_steps, double* mean_ms, int32_t* 
         e = launch_small(net->sdev, net->pops[0].kind, net->pops[0].dtype, clk, 1, net->cfg.dt,
                          net->d_status, net->stream);
       if (s.kind == 5)
-        e = launch_pending_delivery(net->pdev, net->pops[0].dtype, net->pending_grid, clk, 0,
+        e = launch_pending_delivery(pending_view(net), net->pops[0].dtype, net->pending_grid, clk, 0,
                                     net->stream);
       if (s.kind == 13)
         e = launch_one_launch_step(net->pops[0], net->fold_dev, net->pdev, net->one_launch_grid,
@@ -2292,7 +2367,7 @@ b2b_status b2b_profile(b2b_net* net, int64_t n_steps, double* mean_ms, int32_t* 
     if (result != B2B_OK) break;
     // every profiled step is a chunk of its own (step 0 of it): its pending input is folded in
     cudaError_t e = net->two_launch
-                        ? launch_fold_pending(net->pdev, net->pops[0].dtype, 0, net->stream)
+                        ? launch_fold_pending(pending_view(net), net->pops[0].dtype, 0, net->stream)
                         : cudaSuccess;
     if (e == cudaSuccess) e = launch_tick(net->d_clock, 1, net->stream);
     ++net->launches;
@@ -2431,11 +2506,11 @@ void set_one_launch_grid(b2b_net* net, int grid) {
 }
 
 // Launch shape of the delivery launch of a net run with two launches per step (pending.cu):
-// lanes per work item (0: built in) and CTAs (0: two per SM).
+// lanes per work item (0: built in) and CTAs (0: pending_ctas).
 void set_pending_shape(b2b_net* net, int group, int grid) {
   int sms = kNumSMs;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, net->cfg.device);
-  net->pending_grid = grid > 0 ? grid : 2 * sms;
+  net->pending_grid = grid > 0 ? grid : pending_ctas(net, sms);
   net->pdev.group = group > 0 ? group : builtin_pending_lanes(net);
   if (net->graph) {
     cudaGraphExecDestroy(net->graph);

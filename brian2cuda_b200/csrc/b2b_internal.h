@@ -118,6 +118,9 @@ struct PopDev {
   // The fused step (neuron.cu): fold holds int32 event counts instead, each count one addition
   // of the variable's weight.
   double fold_w[3];
+  // Where set: the two launches' fold holds event counts (in the variable's type), each one
+  // addition of the weight of the neuron's group, [group][v, ge, gi].
+  const double* fold_gw;
 };
 
 // Device view of a projection (merged Synapses objects with one source population, one
@@ -486,6 +489,8 @@ struct b2b_net {
   b2b::PendingDev pdev{};
   b2b::PopDev fold_dev{};                  // the population's view whose update folds acc in
   int pending_grid = 0;
+  // pending input as event counts (count_pending): the weights, [group][v, ge, gi] on the device
+  const double* count_gw = nullptr;
   // the same two halves as one grid per step on the net's stream (neuron.cu), the delivery
   // with one_launch_grid CTAs after the update's; only where two_launch_ok
   bool one_launch = false;
@@ -564,6 +569,7 @@ AddDev add_dev(const Proj& pr);
 // bundles of mean_bundle synapses, and for the delivery into the pending input (n neurons).
 int delivery_lanes(double mean_bundle);
 int pending_lanes(double mean_bundle, int64_t n);
+constexpr int64_t kPendingLarge = 200000;   // neurons from which that delivery's shape differs
 // Whether such a launch can accumulate in thread-block clusters (AddTune::cluster).
 bool add_batch_cluster_capable(const Proj* const* prs, int n);
 cudaError_t launch_tick(int64_t* clock, int steps, cudaStream_t s);

@@ -17,6 +17,7 @@
 // the synaptic delivery, preserving Brian2's schedule (groups, thresholds, synapses,
 // resets).
 #include <algorithm>
+#include <type_traits>
 
 #include "neuron_common.cuh"
 #include "pending_body.cuh"
@@ -29,12 +30,20 @@ namespace {
 // cleared after the update's stores; no-op when the population has no fold buffer for v.  The
 // row goes by the step's place in its chunk (both rows are empty between chunks), a launch
 // argument, so its load does not wait for the clock's.
-template <typename R, int E>
+// COUNTED: the buffer holds event counts, each one addition of the group's weight.
+template <typename R, int E, bool COUNTED = false>
 __device__ __forceinline__ R* fold_in(const PopDev& P, int v, int k, int64_t q,
                                       Pack<R, E>& X) {
   if (!P.fold[v]) return nullptr;
   R* a = static_cast<R*>(P.fold[v]) + (int64_t)((k & 1) ^ 1) * P.n;
   const Pack<R, E> A = load_pack<R, E>(a, q);
+  if constexpr (COUNTED) {
+    const R w = (R)P.fold_gw[3 * group_of<E>(P, q) + v];
+#pragma unroll
+    for (int e = 0; e < E; ++e)
+      for (int c = (int)A.x[e]; c > 0; --c) X.x[e] += w;
+    return a;
+  }
 #pragma unroll
   for (int e = 0; e < E; ++e) X.x[e] += A.x[e];
   return a;
@@ -89,7 +98,7 @@ __device__ __forceinline__ void fold_clear(R* a, int64_t q) {
 // after the wait rather than at the top, so that its CTAs spread over SMs that the launch before
 // has left (pair_step_kernel before a delivery, STDP 3,001 -> 257: 9.06 -> 8.78 us per step).
 template <typename R, int E, bool INPUTS, bool FUSED = false, bool CHAINED = false,
-          bool NEXT = false, class Emit = int>
+          bool NEXT = false, bool COUNTED = false, class Emit = int>
 __device__ __forceinline__ void lif_step_body(const PopDev& P, const int64_t* __restrict__ clock,
                                               int k, double dt, int32_t* status, int64_t blk,
                                               Emit emit = 0) {
@@ -121,8 +130,8 @@ __device__ __forceinline__ void lif_step_body(const PopDev& P, const int64_t* __
       cge = fold_counts<R, E>(P, B2B_VAR_GE, k, q, GE);
       cgi = fold_counts<R, E>(P, B2B_VAR_GI, k, q, GI);
     } else {
-      fge = fold_in<R, E>(P, B2B_VAR_GE, k, q, GE);
-      fgi = fold_in<R, E>(P, B2B_VAR_GI, k, q, GI);
+      fge = fold_in<R, E, COUNTED>(P, B2B_VAR_GE, k, q, GE);
+      fgi = fold_in<R, E, COUNTED>(P, B2B_VAR_GI, k, q, GI);
     }
     uint32_t NRout = 0;
 #pragma unroll
@@ -172,16 +181,16 @@ __device__ __forceinline__ void lif_step_body(const PopDev& P, const int64_t* __
   clear_next_slot(P, ts, blk);
 }
 
-template <typename R, int E, bool INPUTS>
+template <typename R, int E, bool INPUTS, bool COUNTED>
 __global__ void __launch_bounds__(kBlock)
 lif_step_kernel(PopDev P, const int64_t* __restrict__ clock, int k, double dt,
                 int32_t* status) {
-  lif_step_body<R, E, INPUTS>(P, clock, k, dt, status, blockIdx.x);
+  lif_step_body<R, E, INPUTS, false, false, false, COUNTED>(P, clock, k, dt, status, blockIdx.x);
 }
 
 // ---- Hodgkin-Huxley (COBAHH), exponential Euler (hh_advance) ------------------------
 template <typename R, int E, bool INPUTS, bool FUSED = false, bool CHAINED = false,
-          bool NEXT = false, class Emit = int>
+          bool NEXT = false, bool COUNTED = false, class Emit = int>
 __device__ __forceinline__ void hh_step_body(const PopDev& P, const int64_t* __restrict__ clock,
                                              int k, double dt, int32_t* status, int64_t blk,
                                              Emit emit = 0) {
@@ -215,8 +224,8 @@ __device__ __forceinline__ void hh_step_body(const PopDev& P, const int64_t* __r
       cge = fold_counts<R, E>(P, B2B_VAR_GE, k, q, GE);
       cgi = fold_counts<R, E>(P, B2B_VAR_GI, k, q, GI);
     } else {
-      fge = fold_in<R, E>(P, B2B_VAR_GE, k, q, GE);
-      fgi = fold_in<R, E>(P, B2B_VAR_GI, k, q, GI);
+      fge = fold_in<R, E, COUNTED>(P, B2B_VAR_GE, k, q, GE);
+      fgi = fold_in<R, E, COUNTED>(P, B2B_VAR_GI, k, q, GI);
     }
     uint32_t NRout = 0;
 #pragma unroll
@@ -356,11 +365,11 @@ hh_split_kernel(PopDev P, const int64_t* __restrict__ clock, int k, double dt, i
   hh_split_body<R>(P, clock, k, dt, status, blockIdx.x);
 }
 
-template <typename R, int E, bool INPUTS>
+template <typename R, int E, bool INPUTS, bool COUNTED>
 __global__ void __launch_bounds__(kBlock)
 hh_step_kernel(PopDev P, const int64_t* __restrict__ clock, int k, double dt,
                int32_t* status) {
-  hh_step_body<R, E, INPUTS>(P, clock, k, dt, status, blockIdx.x);
+  hh_step_body<R, E, INPUTS, false, false, false, COUNTED>(P, clock, k, dt, status, blockIdx.x);
 }
 
 // ---- one launch per step (nets of the two-launch form, pending.cu) --------------------
@@ -570,7 +579,7 @@ __device__ __forceinline__ void hh_pack_load(const PopDev& P, int64_t q, HhPack<
   s.LS = load_pack<R, 4>(P.var[B2B_VAR_LASTSPIKE], q);
 }
 
-template <typename R, bool INPUTS>
+template <typename R, bool INPUTS, bool COUNTED>
 __global__ void __launch_bounds__(kBlock, 2)
 hh_stream_kernel(PopDev P, const int64_t* __restrict__ clock, int k, double dt,
                  int32_t* status) {
@@ -594,8 +603,8 @@ hh_stream_kernel(PopDev P, const int64_t* __restrict__ clock, int k, double dt,
       const HhRun<R> g = hh_run(prm[cur.grp], R());
       const GroupInputs* gin = INPUTS ? P.inputs + cur.grp : nullptr;
       const bool refr = g.ref_steps >= 0;
-      R* fge = fold_in<R, 4>(P, B2B_VAR_GE, k, q, cur.GE);
-      R* fgi = fold_in<R, 4>(P, B2B_VAR_GI, k, q, cur.GI);
+      R* fge = fold_in<R, 4, COUNTED>(P, B2B_VAR_GE, k, q, cur.GE);
+      R* fgi = fold_in<R, 4, COUNTED>(P, B2B_VAR_GI, k, q, cur.GI);
       uint32_t NRout = 0;
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
@@ -803,13 +812,15 @@ struct UpdateShape {
   int e, block;
   bool split;                     // a HH neuron's variables in four warps (hh_split_body; e = 1)
 };
-UpdateShape update_shape(const Pop& pop, int64_t n) {
+// Beside a delivery (beside: the update of the two launches) HH f32 keeps two: 460,000 9.83 ->
+// 9.11 us per step, 613,000 12.5 -> 11.7.
+UpdateShape update_shape(const Pop& pop, int64_t n, bool beside = false) {
   const bool f32 = pop.dtype == B2B_F32;
   int e = 1;
   if (pop.kind == KIND_HH && pop.tune_e == 0 && !pop.inputs && !f32 && n < kSplitNeurons)
     return {1, pop.tune_block > 0 ? pop.tune_block : 128, true};
   if (pop.kind == KIND_POISSON) e = n >= 200000 ? 4 : 2;
-  else if (f32) e = n >= 280000 ? 4 : (n >= 90000 ? 2 : 1);
+  else if (f32) e = n >= 280000 && !(beside && pop.kind == KIND_HH) ? 4 : (n >= 90000 ? 2 : 1);
   else if (pop.kind == KIND_LIF) e = n >= 130000 ? 2 : 1;
   return {pop.tune_e > 0 ? pop.tune_e : e, pop.tune_block > 0 ? pop.tune_block : 128, false};
 }
@@ -820,27 +831,27 @@ unsigned update_grid(const UpdateShape& shape, int e, int64_t n) {
   return (unsigned)((threads + shape.block - 1) / shape.block);
 }
 
-template <int E, bool IN>
+template <int E, bool IN, bool CNT>
 cudaError_t launch_e(const Pop& pop, const PopDev& P, const int64_t* clock, int k, double dt,
                      int32_t* status, cudaStream_t s) {
-  const int block = update_shape(pop, P.n).block;   // <= kBlock
+  const int block = update_shape(pop, P.n).block;   // <= kBlock (the same beside a delivery)
   const unsigned grid = (unsigned)((P.n / E + block - 1) / block);
   const bool f32 = pop.dtype == B2B_F32;
   switch (pop.kind) {
     case KIND_LIF:
-      if (f32) lif_step_kernel<float, E, IN><<<grid, block, 0, s>>>(P, clock, k, dt, status);
-      else lif_step_kernel<double, E, IN><<<grid, block, 0, s>>>(P, clock, k, dt, status);
+      if (f32) lif_step_kernel<float, E, IN, CNT><<<grid, block, 0, s>>>(P, clock, k, dt, status);
+      else lif_step_kernel<double, E, IN, CNT><<<grid, block, 0, s>>>(P, clock, k, dt, status);
       break;
     case KIND_HH:
       if (E == 4 && f32) {
         // resident CTAs only (2 per SM of 256 threads by the launch bounds); float64 keeps
         // one pack per thread (two packs of doubles do not fit the register budget)
         const unsigned g2 = std::min<unsigned>(grid, 2 * kNumSMs * (kBlock / block));
-        hh_stream_kernel<float, IN><<<g2, block, 0, s>>>(P, clock, k, dt, status);
+        hh_stream_kernel<float, IN, CNT><<<g2, block, 0, s>>>(P, clock, k, dt, status);
       } else if (f32) {
-        hh_step_kernel<float, E, IN><<<grid, block, 0, s>>>(P, clock, k, dt, status);
+        hh_step_kernel<float, E, IN, CNT><<<grid, block, 0, s>>>(P, clock, k, dt, status);
       } else {
-        hh_step_kernel<double, E, IN><<<grid, block, 0, s>>>(P, clock, k, dt, status);
+        hh_step_kernel<double, E, IN, CNT><<<grid, block, 0, s>>>(P, clock, k, dt, status);
       }
       break;
     case KIND_POISSON:
@@ -914,21 +925,24 @@ cudaError_t launch_pop_step_dev(const Pop& pop, const PopDev& dev, const int64_t
     spikegen_step_kernel<<<1, kBlock, 0, s>>>(pop.dev, clock, k, status);
     return cudaGetLastError();
   }
-  const UpdateShape shape = update_shape(pop, pop.dev.n);
+  const UpdateShape shape =
+      update_shape(pop, pop.dev.n, dev.fold[B2B_VAR_GE] || dev.fold[B2B_VAR_GI]);
   const int e = shape.e;
   if (shape.split) {
     hh_split_kernel<double>
         <<<update_grid(shape, 0, dev.n), shape.block, 0, s>>>(dev, clock, k, dt, status);
     return cudaGetLastError();
   }
-  if (pop.inputs) {
-    if (e == 4) return launch_e<4, true>(pop, dev, clock, k, dt, status, s);
-    if (e == 2) return launch_e<2, true>(pop, dev, clock, k, dt, status, s);
-    return launch_e<1, true>(pop, dev, clock, k, dt, status, s);
-  }
-  if (e == 4) return launch_e<4, false>(pop, dev, clock, k, dt, status, s);
-  if (e == 2) return launch_e<2, false>(pop, dev, clock, k, dt, status, s);
-  return launch_e<1, false>(pop, dev, clock, k, dt, status, s);
+  auto launch = [&](auto in, auto counted) {
+    constexpr bool IN = decltype(in)::value, CNT = decltype(counted)::value;
+    if (e == 4) return launch_e<4, IN, CNT>(pop, dev, clock, k, dt, status, s);
+    if (e == 2) return launch_e<2, IN, CNT>(pop, dev, clock, k, dt, status, s);
+    return launch_e<1, IN, CNT>(pop, dev, clock, k, dt, status, s);
+  };
+  using T = std::true_type;
+  using N = std::false_type;
+  if (dev.fold_gw) return pop.inputs ? launch(T{}, T{}) : launch(N{}, T{});
+  return pop.inputs ? launch(T{}, N{}) : launch(N{}, N{});
 }
 
 bool one_launch_supported(const Pop& pop, const PendingDev& F) {

@@ -12,6 +12,12 @@
 //                        that arrived during step t-1, acc[(t-1) & 1], and clears it
 // (t counted from the start of the chunk of steps, when both rows are empty).
 //
+// Sums of weights round differently from the per-step path, which adds every weight into the
+// target variable by itself.  Populations that take this form by their size beyond the one where
+// it always was the default keep the per-step path's results: their accumulators count events
+// (every weight is 1 there), and the update and the fold add the weight that often
+// (PopDev::fold_gw).
+//
 // The library launches the two side by side, the delivery on a second stream: the delivery
 // of step t waits for the update of step t-1, the update of step t for the update and the
 // delivery of step t-1 (api.cu, enqueue_steps).  The update of step t+1 sees exactly the
@@ -44,7 +50,13 @@ __global__ void fold_pending_kernel(const __grid_constant__ PendingDev F, int k_
     R* X = static_cast<R*>(F.pop.var[v]);
     R* A = static_cast<R*>(F.acc[v]) + (int64_t)last * n;
     for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += stride) {
-      X[q] += A[q];
+      if (F.pop.fold_gw) {
+        const int grp = F.pop.vec_group ? F.pop.vec_group[q >> 2] : 0;
+        const R w = (R)F.pop.fold_gw[3 * grp + v];
+        for (int c = (int)A[q]; c > 0; --c) X[q] += w;
+      } else {
+        X[q] += A[q];
+      }
       A[q] = (R)0;
     }
   }

@@ -537,10 +537,11 @@ int delivery_lanes(double mean_bundle) {
 // / 16 lanes: COBAHH 4000 3.82 / 3.79 / 3.78, CUBA with delays 20,000 3.80 / 3.78 / 3.74; COBAHH
 // 30,000 3.05 / 2.99 / 2.97).  Larger ones go by the bundle: 40 synapses (COBAHH 1e5) 3.83 / 3.74
 // / 3.69, 4-5 (8 merged networks) 5.38 / 5.47 / 6.18, (CUBA with delays 150,000) 4.66 / 4.62 /
-// 4.53.
+// 4.53.  From 200,000 neurons on, with three CTAs per SM, short bundles (4-5) are served best by
+// four: 245,000 6.49 / 6.87 / 8.07, 460,000 9.83 / 10.6 / 12.8, 613,000 12.5 / 13.7 / 17.2.
 int pending_lanes(double mean_bundle, int64_t n) {
   if (n <= 40000 || mean_bundle >= 24) return 16;
-  return 8;
+  return n >= kPendingLarge && mean_bundle < 8 ? 4 : 8;
 }
 
 // Chained, a delivery's CTAs take their places while the update's still run, where one has ended
