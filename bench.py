@@ -842,7 +842,8 @@ WORKLOADS = {
 }
 PROP_RATE = 300.0
 BYTES = {"cuba_neuron": 58, "cuba_event": 20, "stdp_neuron": 16, "poisson": 4,
-         "stdp_pre": 40, "stdp_post": 32, "hines_comp": 136}
+         # target or key 4, weight R/W 8, trace 8 (on_pre also the target's R/W 8)
+         "stdp_pre": 28, "stdp_post": 20, "hines_comp": 136}
 
 
 def build_propagation(net, monitor_capacity=0, rate=PROP_RATE):
@@ -1009,7 +1010,7 @@ def bench_small(args, world, rank, local):
                           ms / args.steps, WORKLOADS[wl],
                           {"sim_steps_per_step": steps_run, "neurons": 11_000,
                            "synapses": 10_000_000, "parallelism": f"replicas x{world}",
-                           "l2": "working set > L2 (1e7 synapses x 4 f32 variables = 160 MB)"},
+                           "l2": "working set > L2 (1e7 synapses x weight, key, target, place = 160 MB)"},
                           "f32")
         roof = _roofline(b, dom[1], kname, ms / (args.steps * steps_run))
         if kname == "deliver_stdp_post_kernel":
@@ -1064,10 +1065,15 @@ def bench_small(args, world, rank, local):
         per_step_bundles = nspk / (args.steps * steps_run) * (DMAX - DMIN + 1)
         db = BYTES_EVENT * per_step_events + BYTES_BUNDLE * per_step_bundles
         dmsk = [m for k, m in prof if k == 6]
-        roof = _roofline(db, dmsk[0], "deliver_add_batch_kernel", ms / (args.steps * steps_run))
-        roof["traffic"] = _traffic_lookup("deliver_add_batch_kernel@propagation")
+        shaped = any(t["site_kind"] in (6, 12) and (t["choice_a"] or t["choice_b"]) for t in tune)
+        kname = ("deliver_add_batch_kernel" if shaped
+                 else "count_events_kernel + apply_counts_kernel")
+        roof = _roofline(db, dmsk[0], kname, ms / (args.steps * steps_run))
+        roof["traffic"] = _traffic_lookup(kname + "@propagation")
         roof["note"] = ("12 B per event (target index 4 B + target read/write 8 B) + 8 B per "
-                        "(spike, delay) bundle; bound: one L2 atomic per event")
+                        "(spike, delay) bundle; bound: " +
+                        ("one L2 atomic per event" if shaped else
+                         "scattered bundles from DRAM, and the sums of the SMs' counts"))
         from brian2cuda_b200.network import atomic_rate
         loaded, hashed, dsmem = atomic_rate(2 * N_NEURONS, 60_000_000, device=local,
                                             stream=stream.cuda_stream)
@@ -1174,7 +1180,7 @@ def kernel_case(name: str):
     training on 2e6 transitions (mlp_grad_kernel, mlp_adam_kernel), propagation /
     propagation3000 = the propagation workload at 300 / 3000 Hz of input, 100 filling steps
     then 20 profiled ones (deliver_add_batch_kernel, 6e6 / 6e7 events per step), stdp /
-    stdp_synorder = the STDP workload with its records grouped by postsynaptic neuron / in
+    stdp_synorder = the STDP workload with its weights grouped by postsynaptic neuron / in
     synapse order, 200 steps then 20 profiled ones (deliver_stdp_post_kernel), hines = the
     1024-neuron multicompartment batch for one 1000-step launch (hines_kernel), model = a
     generated model (noisy adaptive LIF, 8e6 neurons, 20 steps: model_step_kernel), batched =

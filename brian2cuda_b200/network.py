@@ -170,12 +170,14 @@ class Network:
         step as two concurrent launches (the neuron update, and the delivery of earlier
         steps' spikes into a double-buffered input) where the net allows it, False always
         the per-step kernels, None (default) the two launches for nets that allow them with at
-        most 2^18 neurons, until autotune() picks the faster form.  `small`: run
+        most 2^18 neurons (2^20, in float64 3 * 2^18, where each group's synapses onto a variable
+        have one weight), until autotune() picks the faster form.  `small`: run
         a small network (one LIF/HH population of <= 4096 neurons, additive synapses onto
-        itself) in one CTA per chunk of steps with the state in shared memory; it pays off for
-        nets of a few hundred to ~2000 neurons with few delays.  `one_launch`: where the net
-        allows the two launches (and every projection has at most 64 delays, no TimedArray or
-        PoissonInput drives the population), run both halves of every step as one launch."""
+        itself) in one CTA per chunk of steps with the state on chip (in registers for LIF
+        without delays); it pays off for nets of a few hundred to ~2000 neurons with few delays.
+        `one_launch`: where the net allows the two launches (and every projection has at most 64
+        delays, no TimedArray or PoissonInput drives the population), run both halves of every
+        step as one launch, each step's launch chained to the previous one."""
         self._lib = N.lib()
         self.dt = float(dt)
         flags = (0 if graphs else N.NET_NO_GRAPH) | (N.NET_CHECKED if checked else 0)

@@ -68,7 +68,10 @@ enum {
                              synapses onto ge/gi only, all delays >= 1 step, no state or rate
                              monitor.  Without this flag or B2B_NET_PER_STEP such a net uses
                              the two launches when its population has at most 2^18 neurons,
-                             and b2b_autotune picks the faster of the two forms             */
+                             or, where the synapses of a group onto a variable all have one
+                             weight, 2^20 (float64: 3 * 2^18), the delivered input then
+                             counting events so that the results are the per-step form's;
+                             b2b_autotune picks the faster of the two forms                */
   B2B_NET_SMALL = 16,     /* run a small network (one LIF/HH population of <= 4096 neurons
                              with additive synapses onto itself) on the small-network path:
                              every step of a chunk in one launch, the state in shared
@@ -77,7 +80,8 @@ enum {
                              the effects or, for synapses without delays or weights of their
                              own, gathering them at the targets.  Without this flag such a
                              net runs the per-step kernels until b2b_autotune measures the
-                             path faster (CUBA 4000: 4.3 against 5.4 us per step)         */
+                             path faster.  LIF without delays or weights of its own runs
+                             with the state in registers, one CTA for up to 1000 steps    */
   B2B_NET_PER_STEP = 32,  /* always the per-step kernels (one launch per population, then
                              the delivery), never the two concurrent launches             */
   B2B_NET_ONE_LAUNCH = 64 /* where the net allows the two concurrent launches (see
@@ -405,7 +409,8 @@ b2b_status b2b_profile_graph(b2b_net* net, int64_t n_steps, double* mean_ms, int
  * steps run as b2b_run runs them (graph replays), so a shape is judged by the step time it
  * gives.  Populations: neurons per thread (1, 2 or 4) x threads per CTA (128 or 256), or, with a
  * gating surrogate, CTAs per SM (2..6); additive delivery launches: lanes per work item
- * (2, 4, 8, 16, 32) x CTAs (1/2, 1, 2, 4, 8 per SM); STDP projections: the order of the synapses'
+ * (2, 4, 8, 16, 32) x CTAs (1/2, 1, 2, 4, 8 per SM), 0 x 0 the built-in form, which counts the
+ * events of a heavily driven projection per target instead of one atomic each; STDP projections: the order of the synapses'
  * weights (0 synapse order, 1 grouped by postsynaptic neuron, where on_post reads contiguous
  * weights; the live weights and every snapshot are permuted together, and b2b_syn_get reads
  * through the order); a net that can run every step as two concurrent launches: the pending
