@@ -1179,7 +1179,7 @@ def kernel_case(name: str):
     gating surrogate attached (hh_surrogate_step_kernel), mlp_train = one epoch of surrogate
     training on 2e6 transitions (mlp_grad_kernel, mlp_adam_kernel), propagation /
     propagation3000 = the propagation workload at 300 / 3000 Hz of input, 100 filling steps
-    then 20 profiled ones (deliver_add_batch_kernel, 6e6 / 6e7 events per step), stdp /
+    then 20 profiled ones (count_events_kernel, 6e6 / 6e7 events per step), stdp /
     stdp_synorder = the STDP workload with its weights grouped by postsynaptic neuron / in
     synapse order, 200 steps then 20 profiled ones (deliver_stdp_post_kernel), hines = the
     1024-neuron multicompartment batch for one 1000-step launch (hines_kernel), model = a
