@@ -1253,6 +1253,18 @@ b2b_status setup_two_launch(b2b_net* net) {
   // beside the update's in one wave for the populations this form is built for
   net->one_launch_grid = 3 * sms / 2;
   net->one_launch = net->one_launch_ok && (flags & B2B_NET_ONE_LAUNCH);
+  // Taken by its size, the form runs as one chained grid up to kMergedMax neurons of one group: a
+  // step then waits for one launch, not for two streams.  us per step, two launches / one grid: LIF
+  // with delays f32 5000 3.11 / 2.72, 60,000 3.50 / 3.15, 150,000 4.09 / 3.56, 200,000 4.53 / 4.49;
+  // f64 60,000 3.79 / 2.98, 150,000 4.60 / 4.36, 200,000 5.22 / 5.27; HH f32 8000 3.58 / 3.23,
+  // 100,000 3.84 / 2.95; HH f64 8001 3.90 / 3.22, 31,000 4.77 / 3.84, but 33,000 (one thread per
+  // neuron, whose long CTAs hold up the delivering ones) 4.92 / 6.77.  Merged networks, whose many
+  // short bundles want more delivering CTAs than fit beside the update: 61,000 4.73 / 4.92,
+  // 245,000 7.5 / 8.5.
+  constexpr int64_t kMergedMax = 150000;
+  net->merged_ok = net->one_launch_ok && net->two_launch && pop.groups.size() == 1 &&
+                   !(flags & (B2B_NET_TWO_LAUNCH | B2B_NET_ONE_LAUNCH)) && pop.n <= kMergedMax + kPad &&
+                   (pop.kind == KIND_LIF || pop.dtype == B2B_F32 || update_is_split(pop));
   // chained: what a step's CTAs read before they wait (parameters, the clock, constants) and the
   // launch itself overlap the previous step.  COBAHH 1e5 3.85 -> 3.24, 4000 3.47 -> 2.89, 8001
   // float64 4.50 -> 3.84 us per step
@@ -1338,6 +1350,13 @@ cudaError_t prof_mark(b2b_net* net, int k, int site, int which, cudaStream_t s) 
                                   s, cudaEventRecordExternal);
 }
 
+// Whether the two launches that a net takes by its size run as one chained grid (merged_ok); timed
+// or with launch shapes of their own they stay two.
+bool merged_in_use(const b2b_net* net) {
+  return net->merged_ok && !net->prof_ev && net->pops[0].tune_e == 0 &&
+         net->pops[0].tune_block == 0;
+}
+
 b2b_status enqueue_steps(b2b_net* net, int kk) {
   if (net->small) {
     const Pop& pop = net->pops[0];
@@ -1349,7 +1368,7 @@ b2b_status enqueue_steps(b2b_net* net, int kk) {
     net->launches += 2;
     return B2B_OK;
   }
-  if (net->two_launch && net->one_launch) {
+  if (net->two_launch && (net->one_launch || merged_in_use(net))) {
     // The same two halves as one grid per step (neuron.cu): consecutive launches on the
     // net's stream order step k+1 after both halves of step k.  Profiling site 0.
     const Pop& pop = net->pops[0];
@@ -1626,7 +1645,7 @@ void refresh_two_launch(b2b_net* net) {
   net->fold_dev = pop.dev;
   for (int v = 0; v < 3; ++v) net->fold_dev.fold[v] = F.acc[v];
   net->one_launch_ok = one_launch_supported(pop, F);
-  if (!net->one_launch_ok) net->one_launch = false;
+  if (!net->one_launch_ok) net->one_launch = net->merged_ok = false;
 }
 
 // Grows population pi's spike-history ring to new_len slots, keeping the spikes of the last
@@ -2565,6 +2584,7 @@ b2b_status b2b_autotune(b2b_net* net, int32_t trial_steps, b2b_tune_result* out,
   CHECK(trial_steps > 0 && trial_steps <= 100000 && n_out, B2B_ERR_INVALID_ARG, "bad arguments");
   GUARD_BEGIN
   CU(cudaStreamSynchronize(net->stream));
+  net->merged_ok = false;   // the forms are measured as they are
   // the state to start every trial from, in a slot of its own; monitor counts to put back
   const int slot = (int)net->snapshots.size();
   if (b2b_status st = b2b_store(net, slot)) return st;
@@ -3009,6 +3029,7 @@ b2b_status b2b_tune_apply(b2b_net* net, const b2b_tune_result* r, int32_t n) {
             B2B_ERR_INVALID_ARG, "site kind 11 exists only for nets that allow both step forms");
       CHECK(t.choice_a < 2 || (net->one_launch_ok && t.choice_b >= 0 && t.choice_b <= 65535),
             B2B_ERR_INVALID_ARG, "the net does not allow the one-launch step");
+      net->merged_ok = false;
       net->two_launch = t.choice_a >= 1;
       net->one_launch = t.choice_a >= 2;
       net->one_launch_chained = t.choice_a == 3;
@@ -3020,6 +3041,7 @@ b2b_status b2b_tune_apply(b2b_net* net, const b2b_tune_result* r, int32_t n) {
              t.choice_a == 16) &&
                 t.choice_b >= 0 && t.choice_b <= 65535,
             B2B_ERR_INVALID_ARG, "bad delivery launch shape");
+      net->merged_ok = false;
       set_pending_shape(net, t.choice_a, t.choice_b);
     } else if (t.site_kind == 14) {
       CHECK(net->small_ok && t.site_index == 0, B2B_ERR_INVALID_ARG,

@@ -496,6 +496,7 @@ struct b2b_net {
   bool one_launch = false;
   bool one_launch_ok = false;
   int one_launch_grid = 0;
+  bool merged_ok = false;                  // two_launch by size: run as the one launch (enqueue_steps)
   bool one_launch_chained = false;         // programmatic dependent launch between steps
   // the per-step form's update and delivery of a step as one launch (setup_fused); its
   // population view holds the event counts
@@ -544,6 +545,8 @@ cudaError_t launch_pop_step_dev(const Pop& pop, const PopDev& dev, const int64_t
 // LIF or HH population, both of built-in shapes and without inputs.  (chained, here and below: a
 // programmatic dependent launch on the previous kernel of the stream.)
 bool pair_supported(const Pop& a, const Pop& b);
+// Whether the built-in update of a population spreads a neuron's equations over four warps.
+bool update_is_split(const Pop& pop);
 cudaError_t launch_pair_step(const Pop& a, const Pop& b, const int64_t* clock, int k, double dt,
                              int32_t* status, cudaStream_t s, bool chained);
 cudaError_t launch_pop_late_reset(const Pop& pop, const int64_t* clock, int k,

@@ -895,6 +895,8 @@ cudaError_t launch_pop_step(const Pop& pop, const int64_t* clock, int k, double 
   return launch_pop_step_dev(pop, pop.dev, clock, k, dt, status, s);
 }
 
+bool update_is_split(const Pop& pop) { return update_shape(pop, pop.dev.n).split; }
+
 bool pair_supported(const Pop& a, const Pop& b) {
   for (const Pop* p : {&a, &b})
     if (p->inputs || p->surr_img || p->tune_e != 0 || p->tune_block != 0) return false;

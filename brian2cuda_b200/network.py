@@ -171,7 +171,8 @@ class Network:
         steps' spikes into a double-buffered input) where the net allows it, False always
         the per-step kernels, None (default) the two launches for nets that allow them with at
         most 2^18 neurons (2^20, in float64 3 * 2^18, where each group's synapses onto a variable
-        have one weight), until autotune() picks the faster form.  `small`: run
+        have one weight; as one chained grid per step for one group of at most 150,000), until
+        autotune() picks the faster form.  `small`: run
         a small network (one LIF/HH population of <= 4096 neurons, additive synapses onto
         itself) in one CTA per chunk of steps with the state on chip (in registers for LIF
         without delays); it pays off for nets of a few hundred to ~2000 neurons with few delays.

@@ -368,7 +368,9 @@ b2b_status b2b_time(b2b_net* net, int64_t* timestep, double* t);
 /* Number of kernels launched so far by b2b_run (eager launches plus graph kernel nodes). */
 b2b_status b2b_kernel_launches(b2b_net* net, int64_t* n);
 /* How b2b_run advances the net (after b2b_finalize): *mode = 1 for every step as two
- * concurrent launches (B2B_NET_TWO_LAUNCH, or chosen automatically), 3 for both halves of
+ * concurrent launches (B2B_NET_TWO_LAUNCH, or chosen automatically; in the latter case a
+ * population of one group of up to 150,000 neurons runs the two as the CTAs of one chained grid
+ * while nothing is tuned or profiled), 3 for both halves of
  * every step as one launch (B2B_NET_ONE_LAUNCH or the autotuner), 2 for a small network run by
  * one CTA or one thread-block cluster per chunk of steps, 0 for per-step kernels replayed from
  * CUDA graphs. */
