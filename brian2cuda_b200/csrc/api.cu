@@ -3099,10 +3099,15 @@ b2b_status b2b_store(b2b_net* net, int32_t slot) {
   if ((int)net->snapshots.size() <= slot) net->snapshots.resize(slot + 1);
   Snapshot& sn = net->snapshots[slot];
   const auto arrays = state_arrays(net);
-  if (sn.buffers.size() != arrays.size()) {
+  sn.valid = false;                // until the copies are complete
+  std::vector<size_t> sizes;
+  for (const auto& a : arrays) sizes.push_back(a.second);
+  if (sn.sizes != sizes) {         // the slot's first use, or a ring has grown since (grow_ring)
     for (void* p : sn.buffers) cudaFree(p);
+    sn.sizes.clear();
     sn.buffers.assign(arrays.size(), nullptr);
-    for (size_t k = 0; k < arrays.size(); ++k) CU(cudaMalloc(&sn.buffers[k], arrays[k].second));
+    for (size_t k = 0; k < arrays.size(); ++k) CU(cudaMalloc(&sn.buffers[k], sizes[k]));
+    sn.sizes = sizes;
   }
   for (size_t k = 0; k < arrays.size(); ++k)
     CU(cudaMemcpyAsync(sn.buffers[k], arrays[k].first, arrays[k].second,

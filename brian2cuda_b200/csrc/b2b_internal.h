@@ -443,6 +443,7 @@ struct Snapshot {
   int64_t ts = 0;
   unsigned long long rng_offset = 0;
   std::vector<void*> buffers;      // device copies, one per entry of the state list
+  std::vector<size_t> sizes;       // their bytes
 };
 }  // namespace b2b
 
