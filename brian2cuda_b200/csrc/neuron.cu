@@ -295,15 +295,17 @@ __device__ __forceinline__ void hh_split_body(const PopDev& P, const int64_t* __
   if (mine) g = hh_run(static_cast<const HhDev*>(P.params)[group_of<1>(P, q)], R());
   if constexpr (CHAINED) previous_launch_done();
   if constexpr (NEXT) let_next_launch_start();
-  R v = 0;
-  if (mine) v = static_cast<const R*>(P.var[B2B_VAR_V])[q];
-  unsigned fl = 0;
-  if (role == 0) {
-    Pack<R, 1> GE{}, GI{};
-    R m = 0, h = 0, n = 0, ls = 0;
-    R *fge = nullptr, *fgi = nullptr;
-    int32_t *cge = nullptr, *cgi = nullptr;
-    if (mine) {
+  // the state at the start of the step: all of it for the membrane's warp (role 0), v and its own
+  // gate for the others
+  R v = 0, m = 0, h = 0, n = 0, ls = 0, x = 0;
+  R* const X =
+      static_cast<R*>(P.var[role == 1 ? B2B_VAR_M : role == 2 ? B2B_VAR_H : B2B_VAR_N]);
+  Pack<R, 1> GE{}, GI{};
+  R *fge = nullptr, *fgi = nullptr;
+  int32_t *cge = nullptr, *cgi = nullptr;
+  if (mine) {
+    v = static_cast<const R*>(P.var[B2B_VAR_V])[q];
+    if (role == 0) {
       m = static_cast<const R*>(P.var[B2B_VAR_M])[q];
       h = static_cast<const R*>(P.var[B2B_VAR_H])[q];
       n = static_cast<const R*>(P.var[B2B_VAR_N])[q];
@@ -317,42 +319,39 @@ __device__ __forceinline__ void hh_split_body(const PopDev& P, const int64_t* __
         fge = fold_in<R, 1>(P, B2B_VAR_GE, k, q, GE);
         fgi = fold_in<R, 1>(P, B2B_VAR_GI, k, q, GI);
       }
+    } else {
+      x = X[q];
     }
-    __syncthreads();
-    if (mine) {
-      const double t = (double)ts * dt;
-      const bool refr = g.ref_steps >= 0;
-      bool nr = true;
-      if (refr) nr = past_refractory(t - (double)ls, dt, 1.0 / dt, g.ref_steps);
-      const R vn = hh_membrane<R>(g, v, m, h, n, GE.x[0], GI.x[0], dtR);
-      if (q - g.offset < g.n && vn > (R)g.Vthr && nr) {
-        nr = false;
-        if (refr) static_cast<R*>(P.var[B2B_VAR_LASTSPIKE])[q] = (R)t;
-        fl = 1u;
-      }
-      static_cast<R*>(P.var[B2B_VAR_V])[q] = vn;
-      static_cast<R*>(P.var[B2B_VAR_GE])[q] = (R)g.De * GE.x[0];
-      static_cast<R*>(P.var[B2B_VAR_GI])[q] = (R)g.Di * GI.x[0];
-      if (refr) static_cast<uint8_t*>(P.var[B2B_VAR_NOT_REFRACTORY])[q] = nr ? 1 : 0;
-      if constexpr (FUSED) {
-        clear_counts<1>(cge);
-        clear_counts<1>(cgi);
-      } else {
-        fold_clear<R, 1>(fge, q);
-        fold_clear<R, 1>(fgi, q);
-      }
+  }
+  __syncthreads();   // every thread of the CTA, whatever its role
+  unsigned fl = 0;
+  if (mine && role == 0) {
+    const double t = (double)ts * dt;
+    const bool refr = g.ref_steps >= 0;
+    bool nr = true;
+    if (refr) nr = past_refractory(t - (double)ls, dt, 1.0 / dt, g.ref_steps);
+    const R vn = hh_membrane<R>(g, v, m, h, n, GE.x[0], GI.x[0], dtR);
+    if (q - g.offset < g.n && vn > (R)g.Vthr && nr) {
+      nr = false;
+      if (refr) static_cast<R*>(P.var[B2B_VAR_LASTSPIKE])[q] = (R)t;
+      fl = 1u;
     }
-  } else {
-    R* X = static_cast<R*>(P.var[role == 1 ? B2B_VAR_M : role == 2 ? B2B_VAR_H : B2B_VAR_N]);
-    R x = 0;
-    if (mine) x = X[q];
-    __syncthreads();
-    if (mine) {
-      if (role == 1) x = hh_gate_m<R>((R)g.VT, v, x, dtR);
-      else if (role == 2) x = hh_gate_h<R>((R)g.VT, v, x, dtR);
-      else x = hh_gate_n<R>((R)g.VT, v, x, dtR);
-      X[q] = x;
+    static_cast<R*>(P.var[B2B_VAR_V])[q] = vn;
+    static_cast<R*>(P.var[B2B_VAR_GE])[q] = (R)g.De * GE.x[0];
+    static_cast<R*>(P.var[B2B_VAR_GI])[q] = (R)g.Di * GI.x[0];
+    if (refr) static_cast<uint8_t*>(P.var[B2B_VAR_NOT_REFRACTORY])[q] = nr ? 1 : 0;
+    if constexpr (FUSED) {
+      clear_counts<1>(cge);
+      clear_counts<1>(cgi);
+    } else {
+      fold_clear<R, 1>(fge, q);
+      fold_clear<R, 1>(fgi, q);
     }
+  } else if (mine) {
+    if (role == 1) x = hh_gate_m<R>((R)g.VT, v, x, dtR);
+    else if (role == 2) x = hh_gate_h<R>((R)g.VT, v, x, dtR);
+    else x = hh_gate_n<R>((R)g.VT, v, x, dtR);
+    X[q] = x;
   }
   if constexpr (FUSED) emit(q, fl, ts, slot);
   else emit_spikes_warp<1>(P, q, fl, ts, slot, status);
