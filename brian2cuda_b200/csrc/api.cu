@@ -626,7 +626,6 @@ b2b_status build_proj(b2b_net* net, int pj) {
   if (pr.effect == B2B_EFFECT_STDP) {
     const b2b_stdp_params& sp = net->syns[pr.members[0]].stdp;
     CHECK(pr.n_syn < (1ll << 31), B2B_ERR_UNSUPPORTED, "STDP projection above 2^31 synapses");
-    CHECK(nkeys < (1ll << 31), B2B_ERR_UNSUPPORTED, "STDP source size x delay range above 2^31");
     // the scattered initial weights are the synapses' weights; the traces start at 0
     D.stdp_w = pr.w;
     pr.w = nullptr;
@@ -651,8 +650,8 @@ b2b_status build_proj(b2b_net* net, int pj) {
     D.post_chunks = (int32_t)std::max<int64_t>(1, (maxp + kChunk - 1) / kChunk);
     D.post_off = poff;
     D.post_syn = psyn;
-    int32_t* key_of = nullptr;
-    CU(dalloc(pr, &key_of, (size_t)pr.n_syn));
+    uint8_t* key_of = nullptr;
+    CU(dalloc(pr, &key_of, (wide_keys(nkeys) ? 8 : 4) * (size_t)pr.n_syn));
     CU(build_key_of(psyn, pr.off, nkeys, pr.n_syn, key_of, s));
     D.key_of = key_of;
     if (b2b_status st = set_record_order(net, pr, stdp_post_grouped(pr))) return st;

@@ -45,7 +45,7 @@ cudaError_t permute_stdp_weights(const void* d_in, void* d_out, const int32_t* d
 // rec_of[post_syn[r]] = r: the post-grouped place of each synapse position.
 cudaError_t build_rec_of(const int32_t* d_post_syn, int64_t n, int32_t* d_rec_of,
                          cudaStream_t s);
-// key_of[r]: bundle key of synapse position post_syn[r].
+// key_of[r]: bundle key of synapse position post_syn[r], as ProjDev::key_of holds it.
 cudaError_t build_key_of(const int32_t* d_post_syn, const int64_t* d_off, int64_t nkeys,
-                         int64_t n, int32_t* d_key_of, cudaStream_t s);
+                         int64_t n, void* d_key_of, cudaStream_t s);
 }  // namespace b2b

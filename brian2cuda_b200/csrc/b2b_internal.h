@@ -156,7 +156,8 @@ struct ProjDev {
   void* stdp_w;                   // [n_syn], in the order rec_of gives
   void* tr_pre;                   // [n_src*nd] by bundle key
   void* tr_post;                  // [n_post]
-  const int32_t* key_of;          // [n_syn] bundle key of each synapse, post-grouped order
+  const void* key_of;             // [n_syn] bundle key of each synapse, post-grouped order: int32,
+                                  // int64 where wide_keys(n_src*nd)
   double taupre, taupost, dApre, dApost, wmin, wmax;
   int32_t pre_adds_weight;
   int32_t aggregate;              // warp-aggregate atomics (few targets)
@@ -173,6 +174,8 @@ struct ProjDev {
   // contiguous weights) and rec_of[s] is the place of synapse position s's weight.
   const int32_t* rec_of;
 };
+
+constexpr bool wide_keys(int64_t nkeys) { return nkeys > INT32_MAX; }
 
 // An additive projection as its delivery kernels read it: what ProjDev holds for them in a third
 // of the size, with the tables of up to kInlineMembers members in place (a lookup of them in

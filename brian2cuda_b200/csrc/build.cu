@@ -192,16 +192,24 @@ cudaError_t counts_to_offsets(int64_t* d_counts, int64_t nkeys, int64_t* max_cou
   cudaError_t e;
   int64_t* d_max = nullptr;
   if ((e = dmalloc(&d_max, 1)) != cudaSuccess) return e;
-  size_t bytes = 0, bytes2 = 0;
-  cub::DeviceReduce::Max(nullptr, bytes, d_counts, d_max, (int)nkeys, s);
-  cub::DeviceScan::ExclusiveSum(nullptr, bytes2, d_counts, d_counts, (int)(nkeys + 1), s);
-  if (bytes2 > bytes) bytes = bytes2;
   void* tmp = nullptr;
-  if ((e = cudaMalloc(&tmp, bytes)) != cudaSuccess) { cudaFree(d_max); return e; }
-  cub::DeviceReduce::Max(tmp, bytes, d_counts, d_max, (int)nkeys, s);
-  cub::DeviceScan::ExclusiveSum(tmp, bytes, d_counts, d_counts, (int)(nkeys + 1), s);
-  e = cudaMemcpyAsync(max_count, d_max, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  auto scan = [&](auto n) {   // n: nkeys in the type that CUB counts with
+    size_t bytes = 0, bytes2 = 0;
+    e = cub::DeviceReduce::Max(nullptr, bytes, d_counts, d_max, n, s);
+    if (e == cudaSuccess)
+      e = cub::DeviceScan::ExclusiveSum(nullptr, bytes2, d_counts, d_counts, n + 1, s);
+    if (bytes2 > bytes) bytes = bytes2;
+    if (e == cudaSuccess) e = cudaMalloc(&tmp, bytes);
+    if (e == cudaSuccess) e = cub::DeviceReduce::Max(tmp, bytes, d_counts, d_max, n, s);
+    if (e == cudaSuccess)
+      e = cub::DeviceScan::ExclusiveSum(tmp, bytes, d_counts, d_counts, n + 1, s);
+  };
+  if (nkeys < INT32_MAX) scan((int)nkeys);
+  else scan(nkeys);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(max_count, d_max, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
+  const cudaError_t done = cudaStreamSynchronize(s);
+  if (e == cudaSuccess) e = done;
   cudaFree(tmp);
   cudaFree(d_max);
   if (e == cudaSuccess) e = cudaGetLastError();
@@ -267,12 +275,13 @@ __device__ __forceinline__ int64_t key_at(const int64_t* __restrict__ off, int64
   return lo;
 }
 
+template <typename Key>
 __global__ void key_of_kernel(const int32_t* __restrict__ post_syn,
                               const int64_t* __restrict__ off, int64_t nkeys, int64_t n,
-                              int32_t* __restrict__ key_of) {
+                              Key* __restrict__ key_of) {
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n;
        r += (int64_t)gridDim.x * blockDim.x)
-    key_of[r] = (int32_t)key_at(off, 0, nkeys, post_syn[r]);
+    key_of[r] = (Key)key_at(off, 0, nkeys, post_syn[r]);
 }
 
 // Apre, Apost or lastupdate of STDP synapses in input order, from the bundles' and targets'
@@ -329,9 +338,14 @@ cudaError_t build_rec_of(const int32_t* d_post_syn, int64_t n, int32_t* d_rec_of
 }
 
 cudaError_t build_key_of(const int32_t* d_post_syn, const int64_t* d_off, int64_t nkeys,
-                         int64_t n, int32_t* d_key_of, cudaStream_t s) {
+                         int64_t n, void* d_key_of, cudaStream_t s) {
   if (n == 0) return cudaSuccess;
-  key_of_kernel<<<grid_for(n), 256, 0, s>>>(d_post_syn, d_off, nkeys, n, d_key_of);
+  if (wide_keys(nkeys))
+    key_of_kernel<<<grid_for(n), 256, 0, s>>>(d_post_syn, d_off, nkeys, n,
+                                              static_cast<int64_t*>(d_key_of));
+  else
+    key_of_kernel<<<grid_for(n), 256, 0, s>>>(d_post_syn, d_off, nkeys, n,
+                                              static_cast<int32_t*>(d_key_of));
   return cudaGetLastError();
 }
 

@@ -204,8 +204,8 @@ deliver_stdp_pre_kernel(ProjDev P, const int64_t* __restrict__ clock, int k, dou
 }
 
 // on_post: every synapse of each neuron of the target population that spiked this step,
-// reached through the transposed (post-sorted) index.
-template <typename R>
+// reached through the transposed (post-sorted) index.  Key: the type of the bundle keys.
+template <typename R, typename Key>
 __global__ void __launch_bounds__(kDeliverBlock)
 deliver_stdp_post_kernel(ProjDev P, const int64_t* __restrict__ clock, int k, double dt) {
   const int64_t ts = clock[0] + k;
@@ -248,7 +248,7 @@ deliver_stdp_post_kernel(ProjDev P, const int64_t* __restrict__ clock, int k, do
       at[u] = r < b1 ? (P.rec_of ? r : (int64_t)__ldg(P.post_syn + r)) : -1;
       if (at[u] >= 0) {
         wt[u] = W[at[u]];
-        p[u] = tr_pre[__ldg(P.key_of + r)];
+        p[u] = tr_pre[__ldg(static_cast<const Key*>(P.key_of) + r)];
       }
     }
     if (ch == 0 && lane == 0) {
@@ -644,11 +644,14 @@ cudaError_t launch_proj_post(const Proj& pr, const int64_t* clock, int k, double
   const ProjDev& P = pr.dev;
   int64_t want = (P.post_src_n * (int64_t)P.post_chunks) / 8 + 1;
   const unsigned grid = (unsigned)(want < 4 * kNumSMs ? want : 4 * kNumSMs);
-  return pr.dtype == B2B_F32
-             ? launch_kernel(deliver_stdp_post_kernel<float>, dim3(grid), kDeliverBlock, 0, s,
-                             chained, P, clock, k, dt)
-             : launch_kernel(deliver_stdp_post_kernel<double>, dim3(grid), kDeliverBlock, 0, s,
-                             chained, P, clock, k, dt);
+  auto launch = [&](auto kernel) {
+    return launch_kernel(kernel, dim3(grid), kDeliverBlock, 0, s, chained, P, clock, k, dt);
+  };
+  if (wide_keys(P.src_n * (int64_t)P.nd))
+    return pr.dtype == B2B_F32 ? launch(deliver_stdp_post_kernel<float, int64_t>)
+                               : launch(deliver_stdp_post_kernel<double, int64_t>);
+  return pr.dtype == B2B_F32 ? launch(deliver_stdp_post_kernel<float, int32_t>)
+                             : launch(deliver_stdp_post_kernel<double, int32_t>);
 }
 
 }  // namespace b2b
