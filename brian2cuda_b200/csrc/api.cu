@@ -8,6 +8,7 @@
 #include <dlfcn.h>
 
 #include <algorithm>
+#include <array>
 #include <cstdarg>
 #include <cstdlib>
 #include <cstring>
@@ -1252,18 +1253,6 @@ b2b_status setup_two_launch(b2b_net* net) {
   // beside the update's in one wave for the populations this form is built for
   net->one_launch_grid = 3 * sms / 2;
   net->one_launch = net->one_launch_ok && (flags & B2B_NET_ONE_LAUNCH);
-  // Taken by its size, the form runs as one chained grid up to kMergedMax neurons of one group: a
-  // step then waits for one launch, not for two streams.  us per step, two launches / one grid: LIF
-  // with delays f32 5000 3.11 / 2.72, 60,000 3.50 / 3.15, 150,000 4.09 / 3.56, 200,000 4.53 / 4.49;
-  // f64 60,000 3.79 / 2.98, 150,000 4.60 / 4.36, 200,000 5.22 / 5.27; HH f32 8000 3.58 / 3.23,
-  // 100,000 3.84 / 2.95; HH f64 8001 3.90 / 3.22, 31,000 4.77 / 3.84, but 33,000 (one thread per
-  // neuron, whose long CTAs hold up the delivering ones) 4.92 / 6.77.  Merged networks, whose many
-  // short bundles want more delivering CTAs than fit beside the update: 61,000 4.73 / 4.92,
-  // 245,000 7.5 / 8.5.
-  constexpr int64_t kMergedMax = 150000;
-  net->merged_ok = net->one_launch_ok && net->two_launch && pop.groups.size() == 1 &&
-                   !(flags & (B2B_NET_TWO_LAUNCH | B2B_NET_ONE_LAUNCH)) && pop.n <= kMergedMax + kPad &&
-                   (pop.kind == KIND_LIF || pop.dtype == B2B_F32 || update_is_split(pop));
   // chained: what a step's CTAs read before they wait (parameters, the clock, constants) and the
   // launch itself overlap the previous step.  COBAHH 1e5 3.85 -> 3.24, 4000 3.47 -> 2.89, 8001
   // float64 4.50 -> 3.84 us per step
@@ -1349,11 +1338,25 @@ cudaError_t prof_mark(b2b_net* net, int k, int site, int which, cudaStream_t s) 
                                   s, cudaEventRecordExternal);
 }
 
-// Whether the two launches that a net takes by its size run as one chained grid (merged_ok); timed
-// or with launch shapes of their own they stay two.
+// Whether the two launches that a net takes by its size run as one chained grid, up to kMergedMax
+// neurons of one group: a step then waits for one launch, not for two streams.  Timed, or with a
+// form or launch shapes of their own, they stay two.  us per step, two launches / one grid: LIF
+// with delays f32 5000 3.11 / 2.72, 60,000 3.50 / 3.15, 150,000 4.09 / 3.56, 200,000 4.53 / 4.49;
+// f64 60,000 3.79 / 2.98, 150,000 4.60 / 4.36, 200,000 5.22 / 5.27; HH f32 8000 3.58 / 3.23,
+// 100,000 3.84 / 2.95; HH f64 8001 3.90 / 3.22, 31,000 4.77 / 3.84, but 33,000 (one thread per
+// neuron, whose long CTAs hold up the delivering ones) 4.92 / 6.77.  Merged networks, whose many
+// short bundles want more delivering CTAs than fit beside the update: 61,000 4.73 / 4.92,
+// 245,000 7.5 / 8.5.
+constexpr int64_t kMergedMax = 150000;
 bool merged_in_use(const b2b_net* net) {
-  return net->merged_ok && !net->prof_ev && net->pops[0].tune_e == 0 &&
-         net->pops[0].tune_block == 0;
+  if (!net->two_launch || net->one_launch || !net->one_launch_ok || net->prof_ev ||
+      net->form_tuned || net->pending_tuned ||
+      (net->cfg.flags & (B2B_NET_TWO_LAUNCH | B2B_NET_ONE_LAUNCH)))
+    return false;
+  const Pop& pop = net->pops[0];
+  return pop.groups.size() == 1 && pop.n <= kMergedMax + kPad && pop.tune_e == 0 &&
+         pop.tune_block == 0 &&
+         (pop.kind == KIND_LIF || pop.dtype == B2B_F32 || update_is_split(pop));
 }
 
 b2b_status enqueue_steps(b2b_net* net, int kk) {
@@ -1644,7 +1647,7 @@ void refresh_two_launch(b2b_net* net) {
   net->fold_dev = pop.dev;
   for (int v = 0; v < 3; ++v) net->fold_dev.fold[v] = F.acc[v];
   net->one_launch_ok = one_launch_supported(pop, F);
-  if (!net->one_launch_ok) net->one_launch = net->merged_ok = false;
+  if (!net->one_launch_ok) net->one_launch = false;
 }
 
 // Grows population pi's spike-history ring to new_len slots, keeping the spikes of the last
@@ -2545,6 +2548,37 @@ void set_pending_shape(b2b_net* net, int group, int grid) {
   }
 }
 
+// The form of the step and the launch shapes that a trial changes.
+struct StepShapes {
+  bool two_launch, one_launch, one_launch_chained, form_tuned, pending_tuned;
+  int one_launch_grid, pending_grid, group;
+  std::vector<std::array<int, 3>> pops;
+  std::vector<AddTune> add;
+  explicit StepShapes(const b2b_net* net)
+      : two_launch(net->two_launch), one_launch(net->one_launch),
+        one_launch_chained(net->one_launch_chained), form_tuned(net->form_tuned),
+        pending_tuned(net->pending_tuned), one_launch_grid(net->one_launch_grid),
+        pending_grid(net->pending_grid), group(net->pdev.group), add(net->add_tune) {
+    for (const Pop& p : net->pops) pops.push_back({p.tune_e, p.tune_block, p.tune_ctas});
+  }
+  void put_back(b2b_net* net) const {
+    net->two_launch = two_launch;
+    net->one_launch = one_launch;
+    net->one_launch_chained = one_launch_chained;
+    net->form_tuned = form_tuned;
+    net->pending_tuned = pending_tuned;
+    net->one_launch_grid = one_launch_grid;
+    net->pending_grid = pending_grid;
+    net->pdev.group = group;
+    net->add_tune = add;
+    for (size_t k = 0; k < pops.size(); ++k) {
+      net->pops[k].tune_e = pops[k][0];
+      net->pops[k].tune_block = pops[k][1];
+      net->pops[k].tune_ctas = pops[k][2];
+    }
+  }
+};
+
 // Advances the net by n_steps the way b2b_run does (CUDA-graph replays of the current launch
 // shapes, captured afresh before the timing starts), timed with a CUDA event pair on the
 // net's stream; *mean_ms receives the mean device time of one whole step.  A shape is judged
@@ -2583,7 +2617,6 @@ b2b_status b2b_autotune(b2b_net* net, int32_t trial_steps, b2b_tune_result* out,
   CHECK(trial_steps > 0 && trial_steps <= 100000 && n_out, B2B_ERR_INVALID_ARG, "bad arguments");
   GUARD_BEGIN
   CU(cudaStreamSynchronize(net->stream));
-  net->merged_ok = false;   // the forms are measured as they are
   // the state to start every trial from, in a slot of its own; monitor counts to put back
   const int slot = (int)net->snapshots.size();
   if (b2b_status st = b2b_store(net, slot)) return st;
@@ -2627,6 +2660,11 @@ b2b_status b2b_autotune(b2b_net* net, int32_t trial_steps, b2b_tune_result* out,
     double ms = 0;
     st = trial(&ms);
   }
+  // the forms are measured as they are, and kept by name; the untuned net's one chained grid is
+  // among them (a tuner that fails leaves all as it was)
+  const StepShapes untuned(net);
+  const bool builtin_merged = merged_in_use(net);
+  if (st == B2B_OK) net->form_tuned = true;
   if (net->small) {
     // the small-network path: one CTA, or one thread-block cluster of 8 or 16 CTAs pushing
     // the effects or pulling them at the targets
@@ -2746,6 +2784,20 @@ b2b_status b2b_autotune(b2b_net* net, int32_t trial_steps, b2b_tune_result* out,
     if (net->two_launch_ok && st == B2B_OK) {
       const double per_step_ms = res.empty() ? 1e30 : res.back().best_ms;
       net->two_launch = true;
+      Pop& pop0 = net->pops[0];
+      const int ps_e = pop0.tune_e, ps_block = pop0.tune_block;
+      // the built-in form where it is the one chained grid: with the built-in shapes
+      double merged_ms = 1e30;
+      if (builtin_merged) {
+        pop0.tune_e = pop0.tune_block = 0;
+        net->one_launch = net->one_launch_chained = true;
+        set_pending_shape(net, 0, 0);
+        set_one_launch_grid(net, 0);
+        st = trial(&merged_ms);
+        net->one_launch = false;
+        pop0.tune_e = ps_e;
+        pop0.tune_block = ps_block;
+      }
       // the step's delivery launch: lanes per work item x CTAs (the neuron launch has one
       // thread per neuron)
       std::vector<std::pair<int, int>> cands = {{0, 0}};
@@ -2771,8 +2823,6 @@ b2b_status b2b_autotune(b2b_net* net, int32_t trial_steps, b2b_tune_result* out,
       // followed by its own delivery, and the forms rank the shapes differently (COBAHH 1e5:
       // 1 x 256 against 2 x 128 neurons per thread x threads, 45.8 against 37.7 ms per
       // simulated second with two launches)
-      Pop& pop0 = net->pops[0];
-      const int ps_e = pop0.tune_e, ps_block = pop0.tune_block;
       b2b_tune_result r1{1, 0, ps_e, ps_block, best, best};
       {
         const std::pair<int, int> shapes[] = {{0, 0}, {1, 128}, {1, 256}, {2, 128}, {2, 256},
@@ -2879,15 +2929,23 @@ b2b_status b2b_autotune(b2b_net* net, int32_t trial_steps, b2b_tune_result* out,
       // the form of the step: 0 per-step kernels, 1 two concurrent launches, 2 one launch, 3 one
       // launch chained; the built-in form stays unless another is 2 % faster
       const double form_ms[4] = {per_step_ms, two_launch_ms, plain_ms, one_launch_ms};
-      const int builtin = builtin_two_launch ? (builtin_one_launch ? 3 : 1) : 0;
-      int other = -1;
+      const int builtin =
+          builtin_two_launch ? (builtin_one_launch || builtin_merged ? 3 : 1) : 0;
+      const double builtin_ms = builtin_merged ? merged_ms : form_ms[builtin];
+      int other = -1;   // (the chained grid of tuned shapes is another form than the built-in's)
       for (int f = 0; f < 4; ++f)
-        if (f != builtin && (other < 0 || form_ms[f] < form_ms[other])) other = f;
-      const int form = form_ms[other] < kTuneMargin * form_ms[builtin] ? other : builtin;
+        if ((f != builtin || builtin_merged) && (other < 0 || form_ms[f] < form_ms[other])) other = f;
+      const bool kept = !(form_ms[other] < kTuneMargin * builtin_ms);
+      const int form = kept ? builtin : other;
       net->two_launch = form >= 1;
       net->one_launch = form >= 2;
       net->one_launch_chained = form != 2;
-      if (form == 0) {
+      if (kept && builtin_merged) {
+        res.push_back(b2b_tune_result{1, 0, 0, 0, merged_ms, merged_ms});
+        res.push_back(b2b_tune_result{5, 0, 0, 0, merged_ms, merged_ms});
+        pop0.tune_e = pop0.tune_block = 0;
+        one_grid = 3 * sms / 2;
+      } else if (form == 0) {
         // the per-step form keeps the shape tuned for it
         pop0.tune_e = ps_e;
         pop0.tune_block = ps_block;
@@ -2902,14 +2960,16 @@ b2b_status b2b_autotune(b2b_net* net, int32_t trial_steps, b2b_tune_result* out,
           res.push_back(b2b_tune_result{1, 0, one_e, one_block, form_ms[form], r1.best_ms});
         }
       }
-      set_pending_shape(net, r.choice_a, r.choice_b);
-      if (form >= 2 && one_group != two_group) {
+      if (kept && builtin_merged) set_pending_shape(net, 0, 0);
+      else set_pending_shape(net, r.choice_a, r.choice_b);
+      if (form >= 2 && one_group != two_group && !(kept && builtin_merged)) {
         // the one-launch form's lanes per item (the pending delivery's CTAs stay as tuned)
         set_pending_shape(net, one_group, r.choice_b);
         res.push_back(b2b_tune_result{5, 0, one_group, r.choice_b, form_ms[form], r.best_ms});
       }
-      res.push_back(b2b_tune_result{11, 0, form, form >= 2 ? one_grid : 0, form_ms[form],
-                                    form_ms[builtin]});
+      if (form >= 2) set_one_launch_grid(net, one_grid);
+      res.push_back(b2b_tune_result{11, 0, form, form >= 2 ? one_grid : 0,
+                                    kept ? builtin_ms : form_ms[form], builtin_ms});
     }
     // STDP projections: order of the weights (0 synapse order, 1 post-grouped), the built-in
     // one first
@@ -2933,11 +2993,6 @@ b2b_status b2b_autotune(b2b_net* net, int32_t trial_steps, b2b_tune_result* out,
       if (st == B2B_OK) st = set_record_order(net, pr, r.choice_a == 1);
       r.best_ms = best;
       res.push_back(r);
-    }
-    if (st != B2B_OK && net->two_launch_ok) {
-      net->two_launch = builtin_two_launch;
-      net->one_launch = builtin_one_launch;
-      net->one_launch_chained = true;
     }
     // a net that allows the small-network path: its forms against the step as tuned above
     if (net->small_ok && st == B2B_OK) {
@@ -2975,8 +3030,11 @@ b2b_status b2b_autotune(b2b_net* net, int32_t trial_steps, b2b_tune_result* out,
     cudaGraphExecDestroy(net->graph);
     net->graph = nullptr;
   }
-  if (st != B2B_OK) return st;
-  if (st2 != B2B_OK) return st2;
+  if (st == B2B_OK) st = st2;
+  if (st != B2B_OK) {
+    untuned.put_back(net);
+    return st;
+  }
   *n_out = (int32_t)res.size();
   for (size_t k = 0; k < res.size() && (int32_t)k < cap; ++k)
     if (out) out[k] = res[k];
@@ -3028,7 +3086,7 @@ b2b_status b2b_tune_apply(b2b_net* net, const b2b_tune_result* r, int32_t n) {
             B2B_ERR_INVALID_ARG, "site kind 11 exists only for nets that allow both step forms");
       CHECK(t.choice_a < 2 || (net->one_launch_ok && t.choice_b >= 0 && t.choice_b <= 65535),
             B2B_ERR_INVALID_ARG, "the net does not allow the one-launch step");
-      net->merged_ok = false;
+      net->form_tuned = true;
       net->two_launch = t.choice_a >= 1;
       net->one_launch = t.choice_a >= 2;
       net->one_launch_chained = t.choice_a == 3;
@@ -3040,7 +3098,7 @@ b2b_status b2b_tune_apply(b2b_net* net, const b2b_tune_result* r, int32_t n) {
              t.choice_a == 16) &&
                 t.choice_b >= 0 && t.choice_b <= 65535,
             B2B_ERR_INVALID_ARG, "bad delivery launch shape");
-      net->merged_ok = false;
+      net->pending_tuned = t.choice_a > 0 || t.choice_b > 0;
       set_pending_shape(net, t.choice_a, t.choice_b);
     } else if (t.site_kind == 14) {
       CHECK(net->small_ok && t.site_index == 0, B2B_ERR_INVALID_ARG,

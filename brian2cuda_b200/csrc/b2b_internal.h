@@ -500,7 +500,10 @@ struct b2b_net {
   bool one_launch = false;
   bool one_launch_ok = false;
   int one_launch_grid = 0;
-  bool merged_ok = false;                  // two_launch by size: run as the one launch (enqueue_steps)
+  // the step's form, and the pending delivery's shape, are the tuner's or the caller's choice and
+  // not the built-in ones (merged_in_use)
+  bool form_tuned = false;
+  bool pending_tuned = false;
   bool one_launch_chained = false;         // programmatic dependent launch between steps
   // the per-step form's update and delivery of a step as one launch (setup_fused); its
   // population view holds the event counts
