@@ -1723,6 +1723,7 @@ b2b_status drop_retired(b2b_net* net) {
   if (any) {
     build_add_batches(net);
     refresh_two_launch(net);
+    setup_fused(net);   // a net without delays that waited for the last delayed spikes
     if (net->graph) {
       cudaGraphExecDestroy(net->graph);
       net->graph = nullptr;
