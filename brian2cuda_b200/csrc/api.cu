@@ -1264,7 +1264,14 @@ b2b_status setup_two_launch(b2b_net* net) {
 // population without TimedArray or PoissonInput inputs, gating surrogate or state monitors,
 // whose synapses onto itself are all additive onto ge/gi, without delays or weights of their own
 // and with one weight per target variable.  Up to the size where the two counts read per
-// neuron stay a small part of the update.
+// neuron stay a small part of the update, and up to fused_mean_limit synapses per neuron: only the
+// CTAs that find spikes deliver them, where a delivery launch has the whole GPU for them.  Update and
+// delivery / fused, us per step, LIF f32, at 19 Hz and at 200 Hz: 4000 neurons, 500 synapses each
+// 5.32 / 3.96 and 5.39 / 7.01, 1000 each 5.32 / 4.19 and 5.59 / 7.56, 2500 each 5.16 / 4.92 and 5.67 /
+// 11.8; 20,000, 500 5.55 / 4.48 and 7.03 / 8.35, 1000 5.67 / 5.06 and 8.95 / 11.0; 100,000, 300 6.03 /
+// 4.77 and 10.3 / 11.3, 500 6.31 / 5.13 and 13.3 / 15.5; 200,000, 80 6.00 / 4.90 and 8.90 / 9.92, 130
+// 6.15 / 5.25 and 11.0 / 12.4, 300 6.68 / 6.41 and 15.3 / 18.0.
+double fused_mean_limit(int64_t n) { return n <= 20000 ? 500 : n <= 150000 ? 300 : 100; }
 void setup_fused(b2b_net* net) {
   net->fused_ok = false;
   if (net->cfg.flags & B2B_NET_CHECKED) return;
@@ -1275,10 +1282,14 @@ void setup_fused(b2b_net* net) {
   if ((pop.kind != KIND_LIF && pop.kind != KIND_HH) || pop.surr_img || pop.inputs ||
       pop.late_reset || pop.n > kFusedMaxNeurons)
     return;
+  double synapses = 0;
+  for (const Proj& pr : net->projs) synapses += (double)pr.n_syn;
+  if (synapses > fused_mean_limit(pop.n) * (double)pop.n) return;
   FusedDev& F = net->fused;
   PopDev& U = net->fused_pop;
   U = pop.dev;
   F.n_proj = (int32_t)net->projs.size();
+  F.share = 0;
   bool seen[3] = {false, false, false};
   for (size_t p = 0; p < net->projs.size(); ++p) {
     const Proj& pr = net->projs[p];
@@ -1294,6 +1305,7 @@ void setup_fused(b2b_net* net) {
       U.fold_w[sy.target_var] = sy.w_scalar;
     }
     F.proj[p] = pr.dev;
+    if (pr.max_bundle > kFusedAlone) F.share = 1;
     F.var[p][0] = pr.target_var;
     if (pr.dev.n_mem > 1)
       for (size_t m = 0; m < pr.members.size() && m < (size_t)kFusedMembers; ++m) {

@@ -273,6 +273,7 @@ inline PendingArgs<NP> pending_args(const PendingDev& F) {
 
 // Device view of the fused step's delivery (neuron.cu): additive projections of a population
 // onto its own ge/gi without delays or weights of their own, one weight per target variable.
+constexpr int kFusedAlone = 128;   // targets that the warp of a spike adds to by itself
 constexpr int kFusedMembers = 4;   // members whose table travels in the launch's parameters
 struct FusedDev {
   ProjDev proj[kMaxProjBatch];
@@ -281,7 +282,7 @@ struct FusedDev {
   int64_t hi[kMaxProjBatch][kFusedMembers];
   int32_t var[kMaxProjBatch][kFusedMembers];
   int32_t n_proj;
-  int32_t pad;
+  int32_t share;                  // bundles longer than kFusedAlone are shared by a CTA's warps
   int32_t* cnt[3];                // per target variable (v, ge, gi): [2][pop.n] or NULL
 };
 

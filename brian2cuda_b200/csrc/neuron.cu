@@ -447,13 +447,29 @@ cudaError_t launch_one_k(const PopDev& U, const PendingDev& F, bool f32, unsigne
 // two launches, so the state is the same bit for bit.  Between chunks the last step's counts are
 // added in (fold_counts_kernel).  CUBA 4000, float64: 5.5 -> 3.8 us per step (4.0 with the
 // bundle bounds and member tables loaded after the spike).
-template <typename R, int KIND, int E>
+//
+// SHARE: a bundle longer than one round of its warp's loads (kFusedAlone) goes on a list in shared
+// memory, which all warps of the CTA work off after the update.  Walked by its own warp alone / shared,
+// us per step: LIF f32 4000 with 1000 synapses per neuron at 19 Hz 6.35 / 4.19, at 200 Hz 12.9 / 7.6;
+// 100,000 with 40 and 10 neurons of 100,000 9.1 / 5.2.
+constexpr int kFusedListed = 128;
+template <typename R, int KIND, int E, bool SHARE>
 __global__ void __launch_bounds__(kBlock)
 fused_step_kernel(const __grid_constant__ PopDev U, const __grid_constant__ FusedDev F,
                   const int64_t* __restrict__ clock, int k, double dt, int32_t* status) {
   constexpr int kMine = E > 0 ? E : 1;          // neurons per thread
   constexpr int kAhead = 2;                     // projections whose bundle bounds are loaded ahead
   let_next_launch_start();
+  struct Listed {
+    const int32_t* post;
+    int32_t len, var;
+  };
+  __shared__ Listed s_list[SHARE ? kFusedListed : 1];
+  __shared__ int s_listed;
+  if constexpr (SHARE) {
+    if (threadIdx.x == 0) s_listed = 0;
+    __syncthreads();
+  }
   // the bundle bounds of this thread's neurons are loaded with its group's constants, so that a
   // spike's delivery starts at its targets
   const int64_t q0 = E > 0 ? (int64_t)blockIdx.x * blockDim.x + threadIdx.x
@@ -493,6 +509,15 @@ fused_step_kernel(const __grid_constant__ PopDev U, const __grid_constant__ Fuse
               if (mm < J.n_mem && pre >= F.hi[p][mm - 1]) var = F.var[p][mm];
           }
           int32_t* c = F.cnt[var] + row;
+          if (SHARE && b1 - b0 > kFusedAlone) {
+            int at = 0;
+            if (lane == 0) at = atomicAdd(&s_listed, 1);
+            at = __shfl_sync(kFull, at, 0);
+            if (at < kFusedListed) {   // (a full list: the warp adds by itself)
+              if (lane == 0) s_list[at] = {J.post + b0, (int32_t)(b1 - b0), var};
+              continue;
+            }
+          }
           // four rounds' targets are loaded before their additions
           for (int64_t s = b0 + lane; s < b1; s += 128) {
             int32_t post[4];
@@ -515,6 +540,30 @@ fused_step_kernel(const __grid_constant__ PopDev U, const __grid_constant__ Fuse
     hh_step_body<R, E, false, true, true>(U, clock, k, dt, status, blockIdx.x, emit);
   else
     lif_step_body<R, E, false, true, true>(U, clock, k, dt, status, blockIdx.x, emit);
+  if constexpr (SHARE) {
+    __syncthreads();
+    const int listed = min(s_listed, kFusedListed);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const int64_t row = (int64_t)(k & 1) * U.n;
+    for (int i = 0; i < listed; ++i) {
+      const Listed b = s_list[i];
+      int32_t* c = F.cnt[b.var] + row;
+      // the bundles' pieces of 128 targets start at another warp each; two pieces' targets are
+      // loaded before their additions
+      const int first = (warp + i) % warps * 128 + lane, ahead = warps * 128;
+      for (int s = first; s < b.len; s += 2 * ahead) {
+        int32_t post[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const int at = s + 32 * (u & 3) + (u >> 2) * ahead;
+          post[u] = at < b.len ? __ldg(b.post + at) : -1;
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+          if (post[u] >= 0) atomicAdd(c + post[u], 1);
+      }
+    }
+  }
 }
 
 // Adds the counts of the chunk's last step (row `row`) into the target variables.
@@ -538,8 +587,10 @@ template <typename R, int KIND, int E>
 cudaError_t launch_fused_e(const PopDev& U, const FusedDev& F, unsigned grid, int block,
                            bool chained, const int64_t* clock, int k, double dt, int32_t* status,
                            cudaStream_t s) {
-  return launch_kernel(fused_step_kernel<R, KIND, E>, dim3(grid), block, 0, s, chained, U, F,
-                       clock, k, dt, status);
+  return F.share ? launch_kernel(fused_step_kernel<R, KIND, E, true>, dim3(grid), block, 0, s,
+                                 chained, U, F, clock, k, dt, status)
+                 : launch_kernel(fused_step_kernel<R, KIND, E, false>, dim3(grid), block, 0, s,
+                                 chained, U, F, clock, k, dt, status);
 }
 template <typename R, int KIND>
 cudaError_t launch_fused_rk(const PopDev& U, const FusedDev& F, int e, unsigned grid, int block,
@@ -977,10 +1028,16 @@ cudaError_t launch_one_launch_step(const Pop& pop, const PopDev& U, const Pendin
                                             status, n_upd, s);
 }
 
+// Its warps deliver as well, so a thread per neuron pays up to one wave of CTAs of 128 (us per step at
+// 1 / 2 neurons per thread, LIF f32, 80 synapses per neuron at 19 and 200 Hz: 100,000 3.89 / 4.13 and
+// 6.14 / 6.82, 150,000 4.18 / 4.35 and 7.18 / 8.40, 200,000 5.72 / 4.89 and 9.33 / 10.1; f64 140,000
+// with 130 synapses 4.56 / 5.46; HH f32 140,000 4.87 / 5.44, 180,000 6.08 / 5.53).
+constexpr int64_t kFusedOneEach = 150000;
 cudaError_t launch_fused_step(const Pop& pop, const PopDev& U, const FusedDev& F, bool chained,
                               const int64_t* clock, int k, double dt, int32_t* status,
                               cudaStream_t s) {
-  const UpdateShape shape = update_shape(pop, U.n);
+  UpdateShape shape = update_shape(pop, U.n);
+  if (pop.tune_e == 0 && U.n <= kFusedOneEach) shape.e = 1;
   const int e = shape.split ? 0 : shape.e >= 2 ? 2 : 1, b = shape.block;
   const unsigned grid = update_grid(shape, e, U.n);
   const bool f32 = pop.dtype == B2B_F32;
