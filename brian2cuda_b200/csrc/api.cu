@@ -1097,20 +1097,28 @@ b2b_status setup_small(b2b_net* net) {
   return B2B_OK;
 }
 
-// Lanes per work item of the pending delivery, by the largest projection's bundles.
-int builtin_pending_lanes(const b2b_net* net) {
+// Mean bundle of the largest projection, by which the pending delivery is shaped, and its lanes per
+// work item.
+double pending_bundle(const b2b_net* net) {
   const Proj* big = nullptr;
   for (const Proj& pr : net->projs)
     if (!big || pr.n_syn > big->n_syn) big = &pr;
-  return pending_lanes(big ? big->mean_bundle : 0, net->pops[0].n);
+  return big ? big->mean_bundle : 0;
+}
+int builtin_pending_lanes(const b2b_net* net) {
+  return pending_lanes(pending_bundle(net), net->pops[0].n);
 }
 
 // CTAs of that launch: two per SM leave the update room; where the population is large its
 // update's waves pass anyway, and a third per SM shortens the delivery (at 2 / 3 / 4 per SM:
 // COBAHH 100,000 4.22 / 4.28 / 4.38 us per step, CUBA 150,000 4.05 / 4.12 / 4.41; merged
-// networks of 245,000 6.88 / 6.49 / 6.89, 460,000 10.3 / 9.8 / 10.1, 613,000 13.2 / 12.5 / 12.7).
+// networks of 245,000 6.88 / 6.49 / 6.89, 460,000 10.3 / 9.8 / 10.1, 613,000 13.2 / 12.5 / 12.7), and where
+// the bundles are long a heavily driven one is too long for two (LIF f32 at 2 / 3 per SM, at 12 and 220
+// Hz: 60,000 with 500 synapses per neuron over 20 delays 4.08 / 4.21 and 12.5 / 10.6, 100,000 with 1000 4.93 /
+// 4.91 and 21.8 / 19.9).
 int pending_ctas(const b2b_net* net, int sms) {
-  return (net->pops[0].n >= kPendingLarge ? 3 : 2) * sms;
+  const int64_t n = net->pops[0].n;
+  return (n >= kPendingLarge || (n > 40000 && pending_bundle(net) >= kLongBundle) ? 3 : 2) * sms;
 }
 
 // Populations up to this size run the two concurrent launches unless tuned otherwise.  Above it
@@ -1249,9 +1257,7 @@ b2b_status setup_two_launch(b2b_net* net) {
   net->two_launch = (flags & (B2B_NET_TWO_LAUNCH | B2B_NET_ONE_LAUNCH)) ||
                     pop.n <= kSumTwoLaunchMax || counted;
   net->one_launch_ok = one_launch_supported(pop, F);
-  // delivering CTAs of the one-launch step: 1.5 per SM (in CTAs of kBlock threads) still fit
-  // beside the update's in one wave for the populations this form is built for
-  net->one_launch_grid = 3 * sms / 2;
+  net->one_launch_grid = builtin_one_launch_grid(pop, F, pending_bundle(net), sms);
   net->one_launch = net->one_launch_ok && (flags & B2B_NET_ONE_LAUNCH);
   // chained: what a step's CTAs read before they wait (parameters, the clock, constants) and the
   // launch itself overlap the previous step.  COBAHH 1e5 3.85 -> 3.24, 4000 3.47 -> 2.89, 8001
@@ -2541,7 +2547,8 @@ constexpr double kTuneMargin = 0.98;
 void set_one_launch_grid(b2b_net* net, int grid) {
   int sms = kNumSMs;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, net->cfg.device);
-  net->one_launch_grid = grid > 0 ? grid : 3 * sms / 2;   // 0: the built-in 1.5 per SM
+  net->one_launch_grid =
+      grid > 0 ? grid : builtin_one_launch_grid(net->pops[0], net->pdev, pending_bundle(net), sms);
   if (net->graph) {
     cudaGraphExecDestroy(net->graph);
     net->graph = nullptr;
@@ -2801,11 +2808,13 @@ b2b_status b2b_autotune(b2b_net* net, int32_t trial_steps, b2b_tune_result* out,
       const int ps_e = pop0.tune_e, ps_block = pop0.tune_block;
       // the built-in form where it is the one chained grid: with the built-in shapes
       double merged_ms = 1e30;
+      int merged_grid = 0;
       if (builtin_merged) {
         pop0.tune_e = pop0.tune_block = 0;
         net->one_launch = net->one_launch_chained = true;
         set_pending_shape(net, 0, 0);
         set_one_launch_grid(net, 0);
+        merged_grid = net->one_launch_grid;
         st = trial(&merged_ms);
         net->one_launch = false;
         pop0.tune_e = ps_e;
@@ -2861,18 +2870,20 @@ b2b_status b2b_autotune(b2b_net* net, int32_t trial_steps, b2b_tune_result* out,
       const double two_launch_ms = r1.best_ms;
       // the same halves as one grid per step: CTAs of the delivery after the update's
       double one_launch_ms = 1e30;
-      int one_grid = 3 * sms / 2;
+      const int builtin_grid =
+          builtin_one_launch_grid(pop0, net->pdev, pending_bundle(net), sms);
+      int one_grid = builtin_grid;
       const int two_group = net->pdev.group;
       int one_group = two_group;
       if (net->one_launch_ok && st == B2B_OK) {
         net->one_launch = true;
         net->one_launch_chained = true;
-        // the built-in 1.5 per SM first: between 1 and 2 per SM the delivering CTAs still fit
+        // the built-in number first: between 1 and 2 per SM the delivering CTAs still fit
         // beside the update's in one wave (COBAHH 1e5, update 2 x 128: 148, 185, 222, 259 gave
         // 38.1, 37.4, 36.9, 37.8 ms per simulated second, 148 against 222 38.1
         // against 37.2 on another; 296 needs a second wave), and the 2000-step window does not
         // tell 1 and 1.5 per SM apart by the 2 % margin
-        const int grids[] = {3 * sms / 2, net->pending_grid, sms / 2, sms, 5 * sms / 4,
+        const int grids[] = {builtin_grid, 3 * sms / 2, net->pending_grid, sms / 2, sms, 5 * sms / 4,
                              7 * sms / 4, 2 * sms, 4 * sms};
         auto tune_grid = [&](bool first) {
           for (size_t c = 0; c < sizeof(grids) / sizeof(grids[0]) && st == B2B_OK; ++c) {
@@ -2957,7 +2968,7 @@ b2b_status b2b_autotune(b2b_net* net, int32_t trial_steps, b2b_tune_result* out,
         res.push_back(b2b_tune_result{1, 0, 0, 0, merged_ms, merged_ms});
         res.push_back(b2b_tune_result{5, 0, 0, 0, merged_ms, merged_ms});
         pop0.tune_e = pop0.tune_block = 0;
-        one_grid = 3 * sms / 2;
+        one_grid = merged_grid;
       } else if (form == 0) {
         // the per-step form keeps the shape tuned for it
         pop0.tune_e = ps_e;

@@ -580,6 +580,7 @@ AddDev add_dev(const Proj& pr);
 // bundles of mean_bundle synapses, and for the delivery into the pending input (n neurons).
 int delivery_lanes(double mean_bundle);
 int pending_lanes(double mean_bundle, int64_t n);
+constexpr double kLongBundle = 24;          // synapses of bundles that 16 lanes share there
 constexpr int64_t kPendingLarge = 200000;   // neurons from which that delivery's shape differs
 // Whether such a launch can accumulate in thread-block clusters (AddTune::cluster).
 bool add_batch_cluster_capable(const Proj* const* prs, int n);
@@ -619,6 +620,8 @@ cudaError_t launch_pending_delivery(const PendingDev& F, int dtype, int grid,
 // (counted in CTAs of kBlock threads); chained: with programmatic dependent launch on the
 // previous launch of the stream.
 bool one_launch_supported(const Pop& pop, const PendingDev& F);
+// Its delivering CTAs (of 256 threads) without tuning.
+int builtin_one_launch_grid(const Pop& pop, const PendingDev& F, double mean_bundle, int sms);
 cudaError_t launch_one_launch_step(const Pop& pop, const PopDev& U, const PendingDev& F,
                                    int deliver_ctas, bool chained, const int64_t* clock, int k,
                                    double dt, int32_t* status, cudaStream_t s);

@@ -402,39 +402,38 @@ one_launch_step_kernel(const __grid_constant__ PopDev U,
   }
 }
 
-template <typename R, int KIND, int E, int GROUP>
-cudaError_t launch_one_g(const PopDev& U, const PendingDev& F, unsigned grid, int block,
-                         bool chained, const int64_t* clock, int k, double dt, int32_t* status,
-                         int n_upd, cudaStream_t s) {
-  if (F.n_proj == 1)
-    return launch_kernel(one_launch_step_kernel<R, KIND, E, GROUP, 1>, dim3(grid), block, 0, s,
-                         chained, U, pending_args<1>(F), clock, k, dt, status, n_upd);
-  return launch_kernel(one_launch_step_kernel<R, KIND, E, GROUP, kMaxProjBatch>, dim3(grid), block,
-                       0, s, chained, U, pending_args<kMaxProjBatch>(F), clock, k, dt, status,
-                       n_upd);
+// use(kernel, projections its parameters hold) with the one-launch kernel of a population at e
+// neurons per thread (0: four threads per neuron), `group` lanes per work item and n_proj projections.
+template <typename R, int KIND, int E, class Use>
+cudaError_t with_one_launch_e(int group, int n_proj, Use use) {
+  auto pick = [&](auto lanes) {
+    constexpr int G = decltype(lanes)::value;
+    return n_proj == 1 ? use(one_launch_step_kernel<R, KIND, E, G, 1>,
+                             std::integral_constant<int, 1>{})
+                       : use(one_launch_step_kernel<R, KIND, E, G, kMaxProjBatch>,
+                             std::integral_constant<int, kMaxProjBatch>{});
+  };
+  if (group == 16) return pick(std::integral_constant<int, 16>{});
+  if (group == 4) return pick(std::integral_constant<int, 4>{});
+  if (group == 2) return pick(std::integral_constant<int, 2>{});
+  return pick(std::integral_constant<int, 8>{});
 }
-
-template <typename R, int KIND, int E>
-cudaError_t launch_one_r(const PopDev& U, const PendingDev& F, unsigned grid, int block,
-                         bool chained, const int64_t* clock, int k, double dt, int32_t* status,
-                         int n_upd, cudaStream_t s) {
-  if (F.group == 16)
-    return launch_one_g<R, KIND, E, 16>(U, F, grid, block, chained, clock, k, dt, status, n_upd, s);
-  if (F.group == 4)
-    return launch_one_g<R, KIND, E, 4>(U, F, grid, block, chained, clock, k, dt, status, n_upd, s);
-  if (F.group == 2)
-    return launch_one_g<R, KIND, E, 2>(U, F, grid, block, chained, clock, k, dt, status, n_upd, s);
-  return launch_one_g<R, KIND, E, 8>(U, F, grid, block, chained, clock, k, dt, status, n_upd, s);
-}
-
-template <int KIND, int E>
-cudaError_t launch_one_k(const PopDev& U, const PendingDev& F, bool f32, unsigned grid,
-                         int block, bool chained, const int64_t* clock, int k, double dt,
-                         int32_t* status, int n_upd, cudaStream_t s) {
-  return f32 ? launch_one_r<float, KIND, E>(U, F, grid, block, chained, clock, k, dt, status,
-                                            n_upd, s)
-             : launch_one_r<double, KIND, E>(U, F, grid, block, chained, clock, k, dt, status,
-                                             n_upd, s);
+template <class Use>
+cudaError_t with_one_launch(const Pop& pop, int e, int group, int n_proj, Use use) {
+  const bool f32 = pop.dtype == B2B_F32;
+  if (pop.kind == KIND_HH) {
+    if (e == 0) return with_one_launch_e<double, KIND_HH, 0>(group, n_proj, use);
+    if (e == 2)
+      return f32 ? with_one_launch_e<float, KIND_HH, 2>(group, n_proj, use)
+                 : with_one_launch_e<double, KIND_HH, 2>(group, n_proj, use);
+    return f32 ? with_one_launch_e<float, KIND_HH, 1>(group, n_proj, use)
+               : with_one_launch_e<double, KIND_HH, 1>(group, n_proj, use);
+  }
+  if (e == 2)
+    return f32 ? with_one_launch_e<float, KIND_LIF, 2>(group, n_proj, use)
+               : with_one_launch_e<double, KIND_LIF, 2>(group, n_proj, use);
+  return f32 ? with_one_launch_e<float, KIND_LIF, 1>(group, n_proj, use)
+             : with_one_launch_e<double, KIND_LIF, 1>(group, n_proj, use);
 }
 
 // ---- update and delivery of a step without delays as one launch ------------------------
@@ -875,6 +874,9 @@ UpdateShape update_shape(const Pop& pop, int64_t n, bool beside = false) {
   return {pop.tune_e > 0 ? pop.tune_e : e, pop.tune_block > 0 ? pop.tune_block : 128, false};
 }
 
+// Neurons per thread of the forms that deliver as well (0: four threads per neuron).
+int one_launch_e(const UpdateShape& shape) { return shape.split ? 0 : shape.e >= 2 ? 2 : 1; }
+
 // CTAs of an update of n neurons at e neurons per thread (0: four threads per neuron).
 unsigned update_grid(const UpdateShape& shape, int e, int64_t n) {
   const int64_t threads = e == 0 ? 4 * n : n / e;
@@ -1010,22 +1012,42 @@ cudaError_t launch_one_launch_step(const Pop& pop, const PopDev& U, const Pendin
   // threads per CTA); the delivery half the same threads per CTA, deliver_ctas counted in
   // CTAs of kBlock threads
   const UpdateShape shape = update_shape(pop, U.n);
-  const int e = shape.split ? 0 : shape.e >= 2 ? 2 : 1, block = shape.block;
+  const int e = one_launch_e(shape), block = shape.block;
   const int n_upd = (int)update_grid(shape, e, U.n);
   const unsigned grid = (unsigned)(n_upd + (int64_t)deliver_ctas * kBlock / block);
-  const bool f32 = pop.dtype == B2B_F32;
-  if (e == 0)
-    return launch_one_r<double, KIND_HH, 0>(U, F, grid, block, chained, clock, k, dt, status,
-                                            n_upd, s);
-  if (pop.kind == KIND_HH)
-    return e == 2 ? launch_one_k<KIND_HH, 2>(U, F, f32, grid, block, chained, clock, k, dt,
-                                             status, n_upd, s)
-                  : launch_one_k<KIND_HH, 1>(U, F, f32, grid, block, chained, clock, k, dt,
-                                             status, n_upd, s);
-  return e == 2 ? launch_one_k<KIND_LIF, 2>(U, F, f32, grid, block, chained, clock, k, dt,
-                                            status, n_upd, s)
-                : launch_one_k<KIND_LIF, 1>(U, F, f32, grid, block, chained, clock, k, dt,
-                                            status, n_upd, s);
+  return with_one_launch(pop, e, F.group, F.n_proj, [&](auto kernel, auto np) {
+    return launch_kernel(kernel, dim3(grid), block, 0, s, chained, U,
+                         pending_args<decltype(np)::value>(F), clock, k, dt, status, n_upd);
+  });
+}
+
+// A step with many events is as long as its delivery, which the SMs' delivering warps bound, so there
+// are as many of them, up to three CTAs of 256 threads per SM, as run beside the update in one wave;
+// at least 1.5.  Up to 10,000 neurons a step has too few events for more to help, up to 40,000 for
+// more than two.  Beyond the wave long bundles of LIF (16 lanes each) are still worth three.  us per step at
+// 1.5 / 2 / 3 CTAs per SM, at 12 and 220 Hz: LIF f32 4000 (80 synapses per neuron over 20 delays) 2.75 /
+// 2.95 / 3.24 and 2.93 / 3.05 / 3.36; 20,000 (1000) 3.33 / 3.35 / 3.50 and 10.2 / 8.0 / 8.2; 60,000 (300)
+// 3.29 / 3.23 / 3.37 and 12.8 / 9.8 / 8.2, (1000) 3.95 / 3.81 / 3.95 and 25.8 / 20.5 / 15.4; 100,000
+// (two neurons per thread, so two CTAs fit) (300) 3.43 / 3.46 / 3.95 and 15.2 / 12.0 / 10.0, (1000) 4.51 /
+// 4.30 / 4.71 and 31.3 / 24.1 / 19.5; 150,000 (80) 3.48 / 3.83 / 4.08 and 17.0 / 15.4 / 12.3, (1000) 5.38 / 5.13 /
+// 5.12 and 37.6 / 36.2 / 27.1; HH f32 20,000 (300) 3.40 / 3.12 / 3.32 and, at 146 Hz, 5.44 / 5.12 / 4.85;
+// 100,000 (300) 3.38 / 3.63 / 3.96 and 11.5 / 10.1 / 8.9.
+int builtin_one_launch_grid(const Pop& pop, const PendingDev& F, double mean_bundle, int sms) {
+  const int64_t n = pop.dev.n;
+  int halves = 3;
+  if (n > 10000) {
+    const UpdateShape shape = update_shape(pop, n);
+    const int e = one_launch_e(shape);
+    int resident = 0;
+    with_one_launch(pop, e, F.group, F.n_proj, [&](auto kernel, auto) {
+      return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kernel, shape.block, 0);
+    });
+    const int64_t room = (int64_t)resident * sms - update_grid(shape, e, n);
+    const int64_t fit = 2 * (room * shape.block / kBlock) / sms;
+    halves = (int)std::min<int64_t>(n <= 40000 ? 4 : 6, std::max<int64_t>(3, fit));
+    if (pop.kind == KIND_LIF && n >= 90000 && mean_bundle >= kLongBundle) halves = 6;
+  }
+  return halves * sms / 2;
 }
 
 // Its warps deliver as well, so a thread per neuron pays up to one wave of CTAs of 128 (us per step at
@@ -1038,7 +1060,7 @@ cudaError_t launch_fused_step(const Pop& pop, const PopDev& U, const FusedDev& F
                               cudaStream_t s) {
   UpdateShape shape = update_shape(pop, U.n);
   if (pop.tune_e == 0 && U.n <= kFusedOneEach) shape.e = 1;
-  const int e = shape.split ? 0 : shape.e >= 2 ? 2 : 1, b = shape.block;
+  const int e = one_launch_e(shape), b = shape.block;
   const unsigned grid = update_grid(shape, e, U.n);
   const bool f32 = pop.dtype == B2B_F32;
   if (pop.kind == KIND_HH)

@@ -1,0 +1,68 @@
+"""Steps of many events in the step's single chained grid: the same state as from two launches, and
+delivering CTAs and lanes enough that it is no slower."""
+from dataclasses import replace
+
+import numpy as np
+import pytest
+
+from brian2cuda_b200 import models
+
+pytestmark = pytest.mark.gpu
+DT = 1e-4
+
+
+def _net(make, n, degree, delays, dtype="float32", **kw):
+    """LIF neurons that fire at about 220 Hz whatever they receive."""
+    net = make(DT, seed=3, **kw)
+    lif = models.cuba_lif()
+    P = net.lif_group(n, replace(lif, El=lif.Vt + 50e-3, refractory=1e-3), dtype)
+    net.set_state(P, "v", np.random.default_rng(n).uniform(-60e-3, -50e-3, n))
+    exc = int(0.8 * n)
+    net.synapses_random(P, P, "ge", degree / n, *delays, 1e-6, 1, (0, exc))
+    net.synapses_random(P, P, "gi", degree / n, *delays, -1e-6, 2, (exc, n))
+    net.finalize()
+    return net, P
+
+
+# bundles of about 2, 8, 25 and 100 synapses; populations on both sides of the rules' limits
+@pytest.mark.parametrize("dtype", ["float32", "float64"])
+@pytest.mark.parametrize("n,degree,delays", [(10_000, 160, (1, 20)), (10_300, 500, (1, 20)),
+                                             (39_900, 2000, (1, 20)), (40_100, 40, (5, 24)),
+                                             (60_000, 500, (1, 20)), (90_300, 500, (1, 5)),
+                                             (149_000, 40, (1, 20)), (149_000, 500, (60, 79))])
+def test_busy_steps_equal_two_launches(gpu_factory, n, degree, delays, dtype):
+    out = []
+    for kw in ({}, {"two_launch": True}):
+        net, P = _net(gpu_factory, n, degree, delays, dtype, **kw)
+        before = net.kernel_launches
+        net.run(delays[1] + 60)
+        out.append((net.kernel_launches - before,
+                    [net.get_state(P, v) for v in ("v", "ge", "gi", "lastspike")]))
+        net.close()
+    assert out[0][0] < out[1][0]                    # one launch per step against two
+    assert np.mean(out[0][1][3] > 0) > 0.5
+    for a, b in zip(out[0][1], out[1][1]):
+        np.testing.assert_array_equal(a, b)
+
+
+def test_busy_steps_take_no_longer_than_two_launches(gpu_factory):
+    """Measured 1.1 times (and 1.7 with 1.5 delivering CTAs per SM and eight lanes for all)."""
+    torch = pytest.importorskip("torch")
+    stream = torch.cuda.Stream()
+    took = []
+    for kw in ({}, {"two_launch": True}):
+        net, _ = _net(gpu_factory, 60_000, 1000, (1, 20), stream=stream.cuda_stream, **kw)
+        net.run(100)
+        net.store(0)
+        best = np.inf
+        for _ in range(5):
+            net.restore(0)
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            a.record(stream)
+            net.run(100)
+            b.record(stream)
+            b.synchronize()
+            best = min(best, a.elapsed_time(b))
+        took.append(best)
+        net.close()
+    assert took[0] < 1.35 * took[1]
