@@ -273,8 +273,9 @@ deliver_stdp_post_kernel(ProjDev P, const int64_t* __restrict__ clock, int k, do
   }
 }
 
-unsigned deliver_grid(const Proj& pr) {
-  const int64_t want = (pr.dev.src_n * (int64_t)pr.dev.chunks) / 64 + 1;
+// CTAs of a delivery with `group` lanes per work item: more lanes than eight leave a warp fewer items.
+unsigned deliver_grid(const Proj& pr, int group) {
+  const int64_t want = (pr.dev.src_n * (int64_t)pr.dev.chunks) * std::max(group / 8, 1) / 64 + 1;
   const int64_t cap = 4 * kNumSMs;
   return (unsigned)(want < cap ? want : cap);
 }
@@ -584,7 +585,6 @@ cudaError_t launch_proj_add_batch(const Proj* const* prs, int n, const int64_t* 
   for (int i = 0; i < n; ++i) {
     n_syn += prs[i]->n_syn;
     B.p[i] = add_dev(*prs[i]);
-    grid = std::max(grid, deliver_grid(*prs[i]));
     nd = std::max(nd, (int)prs[i]->dev.nd);
   }
   const bool wp = nd <= kWarpPrefixMaxDelays;
@@ -597,6 +597,7 @@ cudaError_t launch_proj_add_batch(const Proj* const* prs, int n, const int64_t* 
       mean = prs[i]->mean_bundle;
     }
   const int group = tune && tune->group > 0 ? tune->group : delivery_lanes(mean);
+  for (int i = 0; i < n; ++i) grid = std::max(grid, deliver_grid(*prs[i], group));
   ClusterAcc A;
   if (tune && tune->cluster && cluster_layout(prs, n, &A)) {
     const int pref_ints = ((nd + 1 + 3) / 4) * 4;
@@ -646,7 +647,7 @@ cudaError_t launch_proj_pre(const Proj& pr, const int64_t* clock, int k, double 
   if (pr.effect != B2B_EFFECT_STDP) return cudaErrorInvalidValue;
   const ProjDev& P = pr.dev;
   chained = chained && chained_delivery(pr.n_syn);
-  const unsigned grid = deliver_grid(pr);
+  const unsigned grid = deliver_grid(pr, 8);
   const bool wp = P.nd <= kWarpPrefixMaxDelays;
   const size_t smem = sizeof(int) * (size_t)(P.nd + 1);
   const bool ag = P.aggregate != 0;
