@@ -8,6 +8,8 @@
 // ballots, so no shared memory or block barrier is involved; larger delay ranges use a
 // per-CTA prefix in shared memory.
 #pragma once
+#include <type_traits>
+
 #include "kernels_common.cuh"
 
 namespace b2b {
@@ -175,7 +177,9 @@ __device__ __forceinline__ int find_delay_block(const int* s_pref, int nd, int s
 // In a quiet step (no slot holds more due items than two rounds of its share of the warps) warps
 // are dealt out to the delays and take the slot's items in turn, without the prefix over the
 // counts and the search in it; a burst's items, all in few slots, go by the prefix to all warps.
-template <bool WARP_PREFIX, int GROUP = 32, class Proj_, class Item>
+// QUIET: lanes of an item's group in a quiet step; item then gets its group's width, as a sixth
+// argument of std::integral_constant type.
+template <bool WARP_PREFIX, int GROUP = 32, int QUIET = 0, class Proj_, class Item>
 __device__ __forceinline__ void for_each_due_item(const Proj_& J, int64_t ts, int64_t warp0,
                                                   int64_t nwarps, int* s_pref, Item item) {
   static_assert(GROUP == 32 || GROUP == 16 || GROUP == 8 || GROUP == 4 || GROUP == 2,
@@ -183,11 +187,13 @@ __device__ __forceinline__ void for_each_due_item(const Proj_& J, int64_t ts, in
   constexpr int G = 32 / GROUP;  // items per warp per round
   const int lane = threadIdx.x & 31;
   const int grp = lane / GROUP;
+  constexpr int QG = QUIET > 0 ? 32 / QUIET : G;
+  const int qgrp = lane / (32 / QG);
   DuePrefix wp{};
   int nspk = 0;
   const int base = ring_slot(ts, J.src_ring_len);
   // one round of the warp: the lane's group takes item `it` (if any) of delay index di
-  auto round = [&](bool have, int di, int kk, int ch) {
+  auto round = [&](auto width, bool have, int di, int kk, int ch) {
     int64_t b0 = 0, b1 = 0, head_key = -1;
     int32_t pre = 0;
     if (have) {
@@ -202,25 +208,29 @@ __device__ __forceinline__ void for_each_due_item(const Proj_& J, int64_t ts, in
     // rounds until the longest bundle of this warp's groups is done (warp-uniform)
     int64_t len = b1 - b0;
 #pragma unroll
-    for (int o = 16; o >= GROUP; o >>= 1) len = max(len, __shfl_xor_sync(kFull, len, o));
-    item(b0, b1, len, pre, head_key);
+    for (int o = 16; o >= decltype(width)::value; o >>= 1)
+      len = max(len, __shfl_xor_sync(kFull, len, o));
+    if constexpr (QUIET > 0) item(b0, b1, len, pre, head_key, width);
+    else item(b0, b1, len, pre, head_key);
   };
+  using Width = std::integral_constant<int, GROUP>;
+  using QuietWidth = std::integral_constant<int, 32 / QG>;
   if constexpr (WARP_PREFIX) {
     const DueCounts c = due_counts_warp(J.src_ring_cnt, J.src_ring_len, ts, J.dmin, J.nd,
                                         J.src_lo, J.src_hi);
     const int most = __reduce_max_sync(kFull, max(c.c0, c.c1));
     if (most == 0) return;
     const int share = nwarps <= INT32_MAX ? (int)((uint32_t)nwarps / (uint32_t)J.nd) : 0;
-    if (share > 0 && (int64_t)most * J.chunks <= 2ll * share * G) {
+    if (share > 0 && (int64_t)most * J.chunks <= 2ll * share * QG) {
       const int di = (int)((uint32_t)warp0 / (uint32_t)share);
       if (di >= J.nd) return;
       const int a = __shfl_sync(kFull, c.c0, di & 31), b = __shfl_sync(kFull, c.c1, di & 31);
       const int items = (di < 32 ? a : b) * J.chunks;
-      for (int r0 = ((int)warp0 - di * share) * G; r0 < items; r0 += share * G) {
-        const int it = r0 + grp;
+      for (int r0 = ((int)warp0 - di * share) * QG; r0 < items; r0 += share * QG) {
+        const int it = r0 + qgrp;
         const bool have = it < items;
         const int kk = J.chunks == 1 ? it : it / J.chunks;
-        round(have, di, kk, have ? it - kk * J.chunks : 0);
+        round(QuietWidth{}, have, di, kk, have ? it - kk * J.chunks : 0);
       }
       return;
     }
@@ -253,7 +263,7 @@ __device__ __forceinline__ void for_each_due_item(const Proj_& J, int64_t ts, in
     } else {
       di = find_delay_block(s_pref, J.nd, sp, &kk);
     }
-    round(have, di, kk, ch);
+    round(Width{}, have, di, kk, ch);
   }
 }
 
