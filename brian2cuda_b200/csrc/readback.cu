@@ -97,7 +97,10 @@ void readback_net_created() {
 void readback_net_destroyed() {
   std::lock_guard<std::mutex> lock(g_mutex);
   if (--g_nets > 0) return;
+  int device = 0;                      // the caller's, which the sets' need not be
+  const bool known = cudaGetDevice(&device) == cudaSuccess;
   while (g_n_free > 0) release(g_free[--g_n_free]);
+  if (known) cudaSetDevice(device);
 }
 
 bool read_back_worth(size_t bytes) { return bytes >= 2 * kReadChunk; }
