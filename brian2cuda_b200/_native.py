@@ -112,6 +112,7 @@ PROTOTYPES = {
     "b2b_syn_set_delays": (I32, [P, I32, P, I64]),
     "b2b_wait_selftest": (I32, [I32, P, C.c_uint32, I32, PI32]),
     "b2b_recip_selftest": (I32, [I32, P, P, I64]),
+    "b2b_div_selftest": (I32, [I32, I32, I32, P, P, I64]),
     "b2b_group_model": (I32, [P, I64, I32, C.c_char_p, DBL, PI32]),
     "b2b_rng_normals_get": (I32, [P, I32, P, I64, I64]),
     "b2b_atomic_rate": (I32, [I32, P, I64, I64, I32, C.POINTER(DBL), C.POINTER(DBL),

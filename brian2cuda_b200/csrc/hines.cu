@@ -96,8 +96,10 @@ __device__ __forceinline__ RC hh_expeuler(RC x, RC a, RC b, RC dt) {
 // by its residual (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000
 // processor", 1990: with 1/c correctly rounded one fused residual step rounds the quotient
 // correctly).  Three operations without a branch, where the general quotient's range checks
-// keep the exponentials around it from overlapping.  An infinite quotient is kept as it is; x in
-// the subnormal range, whose residual is inexact, only feeds exponentials that round to 1.
+// keep the exponentials around it from overlapping.  The last place may differ where the residual is
+// inexact (|x| below 2^-101 in float32, 2^-968 in float64: its last place is below the smallest
+// subnormal number) and above 3e38 (kept uncorrected, as the residual may overflow), of values whose
+// exponentials are 1, 0 or infinite.
 template <typename RC>
 __device__ __forceinline__ RC div_lit(RC x, double c) {
   const RC b = (RC)c, y = (RC)(1.0 / (double)b);
@@ -899,7 +901,7 @@ b2b_status b2b_hines_destroy(b2b_hines* h) {
 
 }  // extern "C"
 
-// ---- the solver's reciprocal against the IEEE quotient ---------------------------------------
+// ---- the solver's reciprocal and quotients against the IEEE ones --------------------------------
 namespace b2b {
 namespace {
 __global__ void recip_selftest_kernel(const double* __restrict__ x, double* __restrict__ y,
@@ -908,26 +910,63 @@ __global__ void recip_selftest_kernel(const double* __restrict__ x, double* __re
        i += (int64_t)gridDim.x * blockDim.x)
     y[i] = recip(x[i]);
 }
+// x / c for the which-th of the rates' constants.
+template <typename RC>
+__global__ void div_selftest_kernel(int which, const RC* __restrict__ x, RC* __restrict__ y,
+                                    int64_t n) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+       i += (int64_t)gridDim.x * blockDim.x)
+    y[i] = which == 0   ? div_lit<RC>(x[i], 10e-3)
+           : which == 1 ? div_lit<RC>(x[i], 18e-3)
+           : which == 2 ? div_lit<RC>(x[i], 20e-3)
+                        : div_lit<RC>(x[i], 80e-3);
+}
 }  // namespace
 }  // namespace b2b
 
-extern "C" b2b_status b2b_recip_selftest(int32_t device, const double* x, double* y,
-                                         int64_t n) {
+namespace {
+// y[0..n) from x[0..n), host arrays of `es` bytes an element, by launch(device x, device y).
+template <class Launch>
+b2b_status run_selftest(int32_t device, const void* x, void* y, size_t es, int64_t n,
+                        Launch launch) {
   if (!x || !y || n <= 0) return B2B_ERR_INVALID_ARG;
   int prev = -1;
   if (cudaGetDevice(&prev) != cudaSuccess || cudaSetDevice(device) != cudaSuccess)
     return B2B_ERR_CUDA;
-  double *dx = nullptr, *dy = nullptr;
-  cudaError_t e = cudaMalloc(&dx, sizeof(double) * n);
-  if (e == cudaSuccess) e = cudaMalloc(&dy, sizeof(double) * n);
-  if (e == cudaSuccess) e = cudaMemcpy(dx, x, sizeof(double) * n, cudaMemcpyHostToDevice);
+  void *dx = nullptr, *dy = nullptr;
+  cudaError_t e = cudaMalloc(&dx, es * n);
+  if (e == cudaSuccess) e = cudaMalloc(&dy, es * n);
+  if (e == cudaSuccess) e = cudaMemcpy(dx, x, es * n, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) {
-    b2b::recip_selftest_kernel<<<256, 256>>>(dx, dy, n);
+    launch(dx, dy);
     e = cudaGetLastError();
   }
-  if (e == cudaSuccess) e = cudaMemcpy(y, dy, sizeof(double) * n, cudaMemcpyDeviceToHost);
+  if (e == cudaSuccess) e = cudaMemcpy(y, dy, es * n, cudaMemcpyDeviceToHost);
   if (dx) cudaFree(dx);
   if (dy) cudaFree(dy);
   cudaSetDevice(prev);
   return e == cudaSuccess ? B2B_OK : B2B_ERR_CUDA;
+}
+}  // namespace
+
+extern "C" b2b_status b2b_recip_selftest(int32_t device, const double* x, double* y,
+                                         int64_t n) {
+  return run_selftest(device, x, y, sizeof(double), n, [&](void* dx, void* dy) {
+    b2b::recip_selftest_kernel<<<256, 256>>>(static_cast<double*>(dx), static_cast<double*>(dy),
+                                             n);
+  });
+}
+
+extern "C" b2b_status b2b_div_selftest(int32_t device, int32_t dtype, int32_t which, const void* x,
+                                       void* y, int64_t n) {
+  if (which < 0 || which > 3 || (dtype != B2B_F32 && dtype != B2B_F64))
+    return B2B_ERR_INVALID_ARG;
+  return run_selftest(device, x, y, dtype == B2B_F32 ? 4 : 8, n, [&](void* dx, void* dy) {
+    if (dtype == B2B_F32)
+      b2b::div_selftest_kernel<<<256, 256>>>(which, static_cast<float*>(dx),
+                                             static_cast<float*>(dy), n);
+    else
+      b2b::div_selftest_kernel<<<256, 256>>>(which, static_cast<double*>(dx),
+                                             static_cast<double*>(dy), n);
+  });
 }

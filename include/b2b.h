@@ -309,16 +309,20 @@ b2b_status b2b_atomic_rate(int32_t device, void* stream, int64_t n_targets, int6
                            int32_t reps, double* loaded_per_s, double* hashed_per_s,
                            double* dsmem_per_s);
 
-/* Self-tests of two device-side building blocks (no counterpart in the reference):
+/* Self-tests of three device-side building blocks (no counterpart in the reference):
  * b2b_wait_selftest runs one CTA that waits with the kernels' bounded mbarrier wait (`polls`
  * polls, at most 2^20) on a barrier that nothing arrives on (arrive = 0: the wait gives up,
  * the CTA records B2B_ERR_TIMEOUT in the status word and returns) or that thread 0 arrives on
  * first (arrive = 1: B2B_OK); *device_status receives the status word.
  * b2b_recip_selftest evaluates the multicompartment solver's reciprocal (the reciprocal
- * unit's approximation refined by two Newton-Raphson steps) at x[0..n) into y. */
+ * unit's approximation refined by two Newton-Raphson steps) at x[0..n) into y.
+ * b2b_div_selftest evaluates its channel rates' quotient by a constant (which: 0 10e-3, 1 18e-3,
+ * 2 20e-3, 3 80e-3, as B2B_F32 or B2B_F64) at x[0..n) into y, arrays of that type. */
 b2b_status b2b_wait_selftest(int32_t device, void* stream, uint32_t polls, int32_t arrive,
                              int32_t* device_status);
 b2b_status b2b_recip_selftest(int32_t device, const double* x, double* y, int64_t n);
+b2b_status b2b_div_selftest(int32_t device, int32_t dtype, int32_t which, const void* x, void* y,
+                            int64_t n);
 
 /* Synapse variables. I, J, DELAY are int32; the others use the target group's dtype. */
 enum {
