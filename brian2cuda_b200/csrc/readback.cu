@@ -26,6 +26,10 @@ namespace {
 
 constexpr size_t kReadChunk = (size_t)1 << 20;
 constexpr int kReadSlots = 6;
+// A plain array below this is one copy: us for 0.6e6 / 0.8e6 / 1e6 / 2e6 floats, copied / by slots, into
+// pages in use 160 / 176, 200 / 260, 235 / 235, 430 / 440, into new ones (1e6, 2e6) 1830 / 680, 2100 / 970.
+// (A gathered value is spared its buffer as well: 0.6e6 855 / 333.)
+constexpr size_t kReadArrayMin = 4000000;
 
 // Sets of slots not in use.  Page-locking a set takes milliseconds, so a set outlives the read
 // (and the net) that needed it, at most kKeptSets of them, until the last net is destroyed.  A read
@@ -145,7 +149,7 @@ cudaError_t read_back(b2b_net* net, void* host, size_t bytes, const ReadSource& 
 }
 
 cudaError_t read_array(b2b_net* net, void* host, const void* dev, size_t bytes) {
-  if (read_back_worth(bytes)) {
+  if (bytes >= kReadArrayMin) {
     try {
       const cudaError_t e = read_back(
           net, host, bytes,
