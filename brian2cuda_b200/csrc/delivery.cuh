@@ -267,23 +267,6 @@ __device__ __forceinline__ void for_each_due_item(const Proj_& J, int64_t ts, in
   }
 }
 
-// Calls body(s, valid, pre) for every synapse position s of every bundle of projection J
-// due at step ts, GROUP lanes to a work item (for_each_due_item); all 32 lanes of a warp call
-// body together, valid marking real synapses.
-template <bool WARP_PREFIX, int GROUP = 32, class Body>
-__device__ __forceinline__ void for_each_due(const ProjDev& J, int64_t ts, int64_t warp0,
-                                             int64_t nwarps, int* s_pref, Body body) {
-  const int glane = (threadIdx.x & 31) % GROUP;
-  for_each_due_item<WARP_PREFIX, GROUP>(J, ts, warp0, nwarps, s_pref,
-                                        [&](int64_t b0, int64_t b1, int64_t len, int32_t pre,
-                                            int64_t) {
-    for (int64_t off = 0; off < len; off += GROUP) {
-      const int64_t s = b0 + off + glane;
-      body(s, s < b1, pre);
-    }
-  });
-}
-
 // Member of presynaptic neuron pre in a projection of several Synapses objects (binary
 // search over the members' upper bounds).
 __device__ __forceinline__ int member_of(const ProjDev& J, int32_t pre) {
