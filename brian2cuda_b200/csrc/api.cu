@@ -1272,7 +1272,7 @@ b2b_status setup_two_launch(b2b_net* net) {
 // and with one weight per target variable.  Up to the size where the two counts read per
 // neuron stay a small part of the update, and up to fused_mean_limit synapses per neuron: only the
 // CTAs that find spikes deliver them, where a delivery launch has the whole GPU for them.  Update and
-// delivery / fused, us per step, LIF f32, at 19 Hz and at 200 Hz: 4000 neurons, 500 synapses each
+// delivery / fused, us per step, LIF f32, at 12 Hz and at 220 Hz: 4000 neurons, 500 synapses each
 // 5.32 / 3.96 and 5.39 / 7.01, 1000 each 5.32 / 4.19 and 5.59 / 7.56, 2500 each 5.16 / 4.92 and 5.67 /
 // 11.8; 20,000, 500 5.55 / 4.48 and 7.03 / 8.35, 1000 5.67 / 5.06 and 8.95 / 11.0; 100,000, 300 6.03 /
 // 4.77 and 10.3 / 11.3, 500 6.31 / 5.13 and 13.3 / 15.5; 200,000, 80 6.00 / 4.90 and 8.90 / 9.92, 130

@@ -46,7 +46,7 @@ constexpr int kHinesBlock = 256;
 constexpr int kHinesMaxStepsPerLaunch = 1000;
 constexpr int kHinesWide = 512;      // threads per CTA when every neuron has an SM to itself
 constexpr int kHinesMaxInRegs = 1024;  // largest neuron whose state the registers hold
-constexpr int kHinesSmallCtas = 5;   // CTAs per SM that the small class's images fit
+constexpr int kHinesSmallCtas = 5;   // CTAs per SM whose images the small class's would fit
 
 struct HinesDev {
   int32_t n_neurons;
@@ -718,8 +718,8 @@ b2b_status b2b_hines_create(b2b_net* net, int32_t n_neurons, const int64_t* comp
       cost[b] = 1000.0 * (lvl_base[b + 1] - lvl_base[b] - 1) +
                 15.0 * (double)(comp_off[b + 1] - comp_off[b]);
     }
-    // two classes by shared-memory image: those that fit five CTAs per SM, and the rest; each
-    // class in decreasing order of cost, the large class first
+    // two classes by shared-memory image: those that fit five CTAs per SM (whose registers allow
+    // four), and the rest; each class in decreasing order of cost, the large class first
     int sm_bytes = 0, reserved = 0;
     cudaDeviceGetAttribute(&sm_bytes, cudaDevAttrMaxSharedMemoryPerMultiprocessor, net->cfg.device);
     cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, net->cfg.device);

@@ -444,12 +444,12 @@ cudaError_t with_one_launch(const Pop& pop, int e, int group, int n_proj, Use us
 // targets' own CTAs have updated theirs or not, and the update of the next step adds the weight
 // count times before it integrates.  The additions and their order per target are those of the
 // two launches, so the state is the same bit for bit.  Between chunks the last step's counts are
-// added in (fold_counts_kernel).  CUBA 4000, float64: 5.5 -> 3.8 us per step (4.0 with the
-// bundle bounds and member tables loaded after the spike).
+// added in (fold_counts_kernel).  CUBA 4000, float64: 6.1 -> 3.3 us per step, the launches chained
+// (unchained 3.8, and 4.0 with the bundle bounds and member tables loaded after the spike).
 //
 // SHARE: a bundle longer than one round of its warp's loads (kFusedAlone) goes on a list in shared
 // memory, which all warps of the CTA work off after the update.  Walked by its own warp alone / shared,
-// us per step: LIF f32 4000 with 1000 synapses per neuron at 19 Hz 6.35 / 4.19, at 200 Hz 12.9 / 7.6;
+// us per step: LIF f32 4000 with 1000 synapses per neuron at 12 Hz 6.35 / 4.19, at 220 Hz 12.9 / 7.6;
 // 100,000 with 40 and 10 neurons of 100,000 9.1 / 5.2.
 constexpr int kFusedListed = 128;
 template <typename R, int KIND, int E, bool SHARE>
@@ -1051,7 +1051,7 @@ int builtin_one_launch_grid(const Pop& pop, const PendingDev& F, double mean_bun
 }
 
 // Its warps deliver as well, so a thread per neuron pays up to one wave of CTAs of 128 (us per step at
-// 1 / 2 neurons per thread, LIF f32, 80 synapses per neuron at 19 and 200 Hz: 100,000 3.89 / 4.13 and
+// 1 / 2 neurons per thread, LIF f32, 80 synapses per neuron at 12 and 220 Hz: 100,000 3.89 / 4.13 and
 // 6.14 / 6.82, 150,000 4.18 / 4.35 and 7.18 / 8.40, 200,000 5.72 / 4.89 and 9.33 / 10.1; f64 140,000
 // with 130 synapses 4.56 / 5.46; HH f32 140,000 4.87 / 5.44, 180,000 6.08 / 5.53).
 constexpr int64_t kFusedOneEach = 150000;

@@ -169,7 +169,7 @@ class Network:
         default the network creates its own non-blocking stream.  `two_launch`: True runs every
         step as two concurrent launches (the neuron update, and the delivery of earlier
         steps' spikes into a double-buffered input) where the net allows it, False always
-        the per-step kernels, None (default) the two launches for nets that allow them with at
+        the per-step form, None (default) the two launches for nets that allow them with at
         most 2^18 neurons (2^20, in float64 3 * 2^18, where each group's synapses onto a variable
         have one weight; as one chained grid per step for one group of at most 150,000), until
         autotune() picks the faster form.  `small`: run
@@ -479,7 +479,8 @@ class Network:
         """Advances `steps` steps with every launch timed; returns (site kind, mean ms) per
         launch site (1 population, 6 additive on_pre delivery launch, 2 STDP on_pre delivery,
         3 on_post delivery, 4 late reset, 5 delivery into the pending input of the two-launch
-        step, 7 one-CTA step, 9 state monitors, 10 rate monitors)."""
+        step, 7 one-CTA step, 9 state monitors, 10 rate monitors).  Sites that run() has in one
+        launch are timed as launches of their own."""
         cap = 256
         ms = (C.c_double * cap)()
         kinds = (C.c_int32 * cap)()

@@ -82,8 +82,9 @@ enum {
                              net runs the per-step kernels until b2b_autotune measures the
                              path faster.  LIF without delays or weights of its own runs
                              with the state in registers, one CTA for up to 1000 steps    */
-  B2B_NET_PER_STEP = 32,  /* always the per-step kernels (one launch per population, then
-                             the delivery), never the two concurrent launches             */
+  B2B_NET_PER_STEP = 32,  /* always the per-step form (the populations' updates, then the
+                             deliveries; both in one launch where a net without delays allows
+                             it), never the two concurrent launches                       */
   B2B_NET_ONE_LAUNCH = 64 /* where the net allows the two concurrent launches (see
                              B2B_NET_TWO_LAUNCH) and every projection has at most 64
                              delays, no TimedArray or PoissonInput drives the population and
@@ -392,8 +393,10 @@ b2b_status b2b_run_mode(b2b_net* net, int32_t* mode);
  * concurrent launches (b2b_run_mode 1), the delivery into the pending input (kind 5) and the
  * neuron update folding it in (kind 1), launched one after the other; or, in the one-launch
  * form (b2b_run_mode 3), the one kernel of the step (kind 13); or, for a small network
- * run by one CTA or cluster (b2b_run_mode 2), that kernel advancing one step (kind 7).  *n_sites receives the number
- * of sites (<= cap filled). */
+ * run by one CTA or cluster (b2b_run_mode 2), that kernel advancing one step (kind 7).  Where
+ * b2b_run has two sites in one launch (the update and the delivery of a net without delays, the
+ * two launches taken by size, a driving and a driven population) they are timed as launches of
+ * their own.  *n_sites receives the number of sites (<= cap filled). */
 b2b_status b2b_profile(b2b_net* net, int64_t n_steps, double* mean_ms, int32_t* site_kind,
                        int32_t cap, int32_t* n_sites);
 /* The same sites timed where b2b_run runs them: the step graph of steps_per_graph steps is
@@ -422,11 +425,12 @@ b2b_status b2b_profile_graph(b2b_net* net, int64_t n_steps, double* mean_ms, int
  * through the order); a net that can run every step as two concurrent launches: the pending
  * delivery's lanes per item x CTAs (kind 5), then the form itself (kind 11: choice_a 2 one
  * launch per step holding both halves, with choice_b delivering CTAs (of 256 threads; 0: the
- * built-in 1.5 per SM) after the update's, 3 the
+ * built-in number, 1.5 to 3 per SM) after the update's, 3 the
  * same with each step's launch chained to the previous one by programmatic dependent launch;
  * 1 two launches; 0 the per-step kernels).  Afterwards the state, clock and monitor counts are as before the call,
  * and the next b2b_run captures its graph with the chosen shapes.  A candidate must be 2 % faster than the best so far (starting from the built-in
- * rule) to be chosen.  A choice of 0 means the built-in rule won.  The trials should cover a
+ * rule) to be chosen.  A choice of 0 means the built-in rule won (kind 11 names the form, 3 for the
+ * chained grid that an untuned net runs).  The trials should cover a
  * representative stretch of the run (bursts included). */
 typedef struct {
   int32_t site_kind;     /* 1 population, 6 additive delivery launch, 8 STDP weights,
