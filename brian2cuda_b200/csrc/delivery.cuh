@@ -177,8 +177,8 @@ __device__ __forceinline__ int find_delay_block(const int* s_pref, int nd, int s
 // In a quiet step (no slot holds more due items than two rounds of its share of the warps) warps
 // are dealt out to the delays and take the slot's items in turn, without the prefix over the
 // counts and the search in it; a burst's items, all in few slots, go by the prefix to all warps.
-// QUIET: lanes of an item's group in a quiet step; item then gets its group's width, as a sixth
-// argument of std::integral_constant type.
+// QUIET: lanes of an item's group in a quiet step (one round of the share, where they are more than
+// GROUP); item then gets its group's width, as a sixth argument of std::integral_constant type.
 template <bool WARP_PREFIX, int GROUP = 32, int QUIET = 0, class Proj_, class Item>
 __device__ __forceinline__ void for_each_due_item(const Proj_& J, int64_t ts, int64_t warp0,
                                                   int64_t nwarps, int* s_pref, Item item) {
@@ -189,6 +189,7 @@ __device__ __forceinline__ void for_each_due_item(const Proj_& J, int64_t ts, in
   const int grp = lane / GROUP;
   constexpr int QG = QUIET > 0 ? 32 / QUIET : G;
   const int qgrp = lane / (32 / QG);
+  constexpr int kQuietRounds = QG < G ? 1 : 2;
   DuePrefix wp{};
   int nspk = 0;
   const int base = ring_slot(ts, J.src_ring_len);
@@ -221,7 +222,7 @@ __device__ __forceinline__ void for_each_due_item(const Proj_& J, int64_t ts, in
     const int most = __reduce_max_sync(kFull, max(c.c0, c.c1));
     if (most == 0) return;
     const int share = nwarps <= INT32_MAX ? (int)((uint32_t)nwarps / (uint32_t)J.nd) : 0;
-    if (share > 0 && (int64_t)most * J.chunks <= 2ll * share * QG) {
+    if (share > 0 && (int64_t)most * J.chunks <= kQuietRounds * (int64_t)share * QG) {
       const int di = (int)((uint32_t)warp0 / (uint32_t)share);
       if (di >= J.nd) return;
       const int a = __shfl_sync(kFull, c.c0, di & 31), b = __shfl_sync(kFull, c.c1, di & 31);

@@ -17,6 +17,7 @@
 // the synaptic delivery, preserving Brian2's schedule (groups, thresholds, synapses,
 // resets).
 #include <algorithm>
+#include <cmath>
 #include <type_traits>
 
 #include "neuron_common.cuh"
@@ -1021,17 +1022,21 @@ cudaError_t launch_one_launch_step(const Pop& pop, const PopDev& U, const Pendin
   });
 }
 
-// A step with many events is as long as its delivery, which the SMs' delivering warps bound, so there
-// are as many of them, up to three CTAs of 256 threads per SM, as run beside the update in one wave;
-// at least 1.5.  Up to 10,000 neurons a step has too few events for more to help, up to 40,000 for
-// more than two.  Beyond the wave long bundles of LIF (16 lanes each) are still worth three.  us per step at
-// 1.5 / 2 / 3 CTAs per SM, at 12 and 220 Hz: LIF f32 4000 (80 synapses per neuron over 20 delays) 2.75 /
-// 2.95 / 3.24 and 2.93 / 3.05 / 3.36; 20,000 (1000) 3.33 / 3.35 / 3.50 and 10.2 / 8.0 / 8.2; 60,000 (300)
-// 3.29 / 3.23 / 3.37 and 12.8 / 9.8 / 8.2, (1000) 3.95 / 3.81 / 3.95 and 25.8 / 20.5 / 15.4; 100,000
-// (two neurons per thread, so two CTAs fit) (300) 3.43 / 3.46 / 3.95 and 15.2 / 12.0 / 10.0, (1000) 4.51 /
-// 4.30 / 4.71 and 31.3 / 24.1 / 19.5; 150,000 (80) 3.48 / 3.83 / 4.08 and 17.0 / 15.4 / 12.3, (1000) 5.38 / 5.13 /
-// 5.12 and 37.6 / 36.2 / 27.1; HH f32 20,000 (300) 3.40 / 3.12 / 3.32 and, at 146 Hz, 5.44 / 5.12 / 4.85;
-// 100,000 (300) 3.38 / 3.63 / 3.96 and 11.5 / 10.1 / 8.9.
+// A step with many events is as long as its delivery, which the SMs' delivering warps bound; in a quiet
+// one the launch is over sooner if the next step's CTAs find room beside it, so up to there the
+// delivering CTAs are as many as leave it (half of what an SM holds), at least 1.5 per SM.  Where the update alone leaves the next step no room, they are as many as
+// run in one wave, as the bundles need them: two per SM for short ones of LIF, 2.5, and three for long
+// (16 lanes each), which are worth them beyond the wave as well.  Up to 10,000 neurons a step has too few
+// events.  us per step at 1.5 / 2 / 2.5 / 3 CTAs per SM, at 12 and 220 Hz: LIF f32 (synapses per neuron over 20
+// delays) 4000 (80) 2.75 / 2.95 / - / 3.24 and 2.93 / 3.05 / - / 3.36; 12,000 (80) 2.96 / 2.88 / 3.12 / 3.21 and 3.6 /
+// 3.6 / 3.7 / 3.8; 20,000 (1000) 3.33 / 3.35 / - / 3.50 and 10.2 / 8.0 / - / 8.2; 35,000 (80) 2.90 / 3.18 / 3.14 / 3.13 and
+// 6.5 / 5.9 / 5.4 / 4.9; 45,000 (80) 3.14 / 3.14 / 3.13 / 3.17 and 5.6 / 5.2 / 4.6 / 4.4; 68,000 (80) 3.14 / 3.16 / 3.21 /
+// 3.31 and 6.8 / 6.6 / 6.0 / 5.7, (300) 3.18 / 3.26 / 3.33 / 3.37 and 11.2 / 11.2 / 9.6 / 8.5; 60,000 (1000) 3.95 / 3.81 / - /
+// 3.95 and 25.8 / 20.5 / - / 15.4; 100,000 (two neurons per thread) (300) 3.43 / 3.46 / - / 3.95 and 15.2 / 12.0 / - /
+// 10.0, (1000) 4.51 / 4.30 / - / 4.71 and 31.3 / 24.1 / - / 19.5; 150,000 (1000) 5.38 / 5.13 / - / 5.12 and 37.6 / 36.2 /
+// - / 27.1.  COBAHH f32 12,500 2.91 / 2.89 / 2.93 / 2.99, 18,786 2.75 / 2.46 / 2.75 / 2.81, 28,603 2.84 / 2.59 / 2.70 /
+// 2.77, 36,000 2.56 / 2.77 / 2.87 / 2.88, 50,186 3.00 / 3.02 / 3.10 / 3.11, 70,001 3.33 / 3.40 / 3.27 / 3.24, 85,000 3.59 /
+// 3.44 / 3.36 / 3.37; f64 20,000 3.25 / 3.46 / 3.58 / 3.61.
 int builtin_one_launch_grid(const Pop& pop, const PendingDev& F, double mean_bundle, int sms) {
   const int64_t n = pop.dev.n;
   int halves = 3;
@@ -1042,10 +1047,20 @@ int builtin_one_launch_grid(const Pop& pop, const PendingDev& F, double mean_bun
     with_one_launch(pop, e, F.group, F.n_proj, [&](auto kernel, auto) {
       return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kernel, shape.block, 0);
     });
-    const int64_t room = (int64_t)resident * sms - update_grid(shape, e, n);
-    const int64_t fit = 2 * (room * shape.block / kBlock) / sms;
-    halves = (int)std::min<int64_t>(n <= 40000 ? 4 : 6, std::max<int64_t>(3, fit));
-    if (pop.kind == KIND_LIF && n >= 90000 && mean_bundle >= kLongBundle) halves = 6;
+    const int64_t update = update_grid(shape, e, n);
+    // halves of a CTA of kBlock threads per SM that fit beside the update in `slots` CTAs
+    auto beside = [&](double slots) {
+      return (int)std::floor(2 * (slots - (double)update) * shape.block / kBlock / sms);
+    };
+    const bool lif = pop.kind == KIND_LIF;
+    const bool is_long = lif && mean_bundle >= kLongBundle;
+    const int with_next = beside(0.5 * resident * sms);
+    const int one_wave = beside((double)resident * sms);
+    const bool large = lif ? n > 40000 : update > 3 * sms;
+    if (large) halves = std::min(one_wave, is_long ? 6 : lif && mean_bundle < 10 ? 4 : 5);
+    else halves = is_long ? 4 : std::min(with_next, 4);
+    if (is_long && n >= 90000) halves = 6;
+    halves = std::max(halves, 3);
   }
   return halves * sms / 2;
 }

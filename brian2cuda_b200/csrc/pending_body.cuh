@@ -21,9 +21,10 @@ __device__ __forceinline__ void deliver_pending_body(const PendingArgs<NP>& F,
   const int64_t warp0 = (blk * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = (nblk * blockDim.x) >> 5;
   const int64_t row = (int64_t)(k & 1) * F.n;
-  // a quiet step has lanes to spare (us per step at 4 / 8 of them there, 4 in the others: LIF f32
-  // 150,000 neurons with bundles of 4 3.73 / 3.64, 100,000 3.20 / 3.16)
-  constexpr int kQuiet = GROUP < 8 ? 8 : GROUP;
+  // a quiet step has lanes to spare (us per step at as many as in a busy one / more: four there, LIF
+  // f32 150,000 neurons with bundles of 4 3.73 / 3.64, 100,000 3.20 / 3.16; eight, HH f64 8001 3.27 /
+  // 3.23, LIF f32 20,000 3.02 / 2.97)
+  constexpr int kQuiet = GROUP < 8 ? 8 : 16;
   if constexpr (CHAINED) {
     // the projection's fields and the clock are in registers before the wait
     const AddDev& J = F.proj[0];

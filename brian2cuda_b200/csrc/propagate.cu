@@ -547,18 +547,18 @@ int delivery_lanes(double mean_bundle) {
 
 // The pending delivery runs beside the update and, in a step of few events, is mostly latency: wide
 // items spread them over more warps.  In a step of many, lanes that a short bundle leaves idle are what it
-// takes longer by.  us per step of the chained grid at 4 / 8 / 16 lanes, at 12 and 220 Hz (LIF f32, synapses
-// per bundle): 4000 neurons (4) 2.82 / 2.76 / 2.75 and 2.93 / 2.88 / 2.93; 20,000 (4) 2.98 / 2.90 / 2.88 and 3.3 /
+// takes longer by (deliver_pending_body has more in the quiet steps).  us per step of the chained grid at
+// 4 / 8 / 16 lanes in both, at 12 and 220 Hz (LIF f32, synapses per bundle): 4000 neurons (4) 2.82 / 2.76 /
+// 2.75 and 2.93 / 2.88 / 2.93, 8000 (4) - / 2.90 / 2.86 and - / 3.36 / 4.19; 20,000 (4) 2.98 / 2.90 / 2.88 and 3.3 /
 // 4.4 / 5.8, (15) 3.46 / 3.03 / 2.98 and 4.8 / 4.9 / 5.9, (50) 4.66 / 3.83 / 3.33 and 11.2 / 9.7 / 10.2; 60,000
 // (8) 3.42 / 3.30 / 3.30 and 5.6 / 7.2 / 9.9, (25) 4.25 / 3.78 / 3.43 and 10.7 / 11.0 / 10.9; 100,000 (4) 3.14 /
 // 3.10 / 3.28 and 7.8 / 12.3 / 19.5, (15) 3.88 / 3.46 / 3.41 and 11.1 / 12.0 / 17.2, (50) 6.72 / 5.20 / 4.30 and
-// 25.7 / 23.9 / 24.1; two launches of 220,000 (15) 5.27 / 4.83 / 5.04 and 17.4 / 18.9 / 25.7, 300,000 (15) 6.48 / 6.22 /
-// 7.60 and 20.4 / 23.5 / 33.8, (25) 7.23 / 6.45 / 7.83 and 26.8 / 30.1 / 36.0, 700,000 (8) 8.89 / 9.24 / 9.97 and 38.0 /
-// 53.2 / 82.6; merged networks of 613,000 (4-5) 12.5 / 13.7 / 17.2 at their own rates.
+// 25.7 / 23.9 / 24.1; two launches of 220,000 (15) 5.27 / 4.83 / 5.04 and 17.4 / 18.9 / 25.7, 300,000 (15) 6.48 /
+// 6.22 / 7.60 and 20.4 / 23.5 / 33.8, (25) 7.23 / 6.45 / 7.83 and 26.8 / 30.1 / 36.0, 700,000 (8) 8.89 / 9.24 / 9.97
+// and 38.0 / 53.2 / 82.6; merged networks of 613,000 (4-5) 12.5 / 13.7 / 17.2 at their own rates.
 int pending_lanes(double mean_bundle, int64_t n) {
   const bool is_long = mean_bundle >= kLongBundle;
-  if (n <= 10000) return 16;
-  if (n <= 40000) return is_long ? 16 : 8;
+  if (n <= 10000) return mean_bundle < 8 ? 8 : 16;
   if (n < 250000) return mean_bundle < 10 ? 4 : is_long && n < kPendingLarge ? 16 : 8;
   return is_long ? 8 : 4;
 }
